@@ -211,3 +211,93 @@ def tolerance(case):
     # against the same attention in float64 the outputs differ by rel 1.2e-3 .. 3.5e-3 (bf16 operands, probabilities and
     # outputs; decode also rounds the dequantised cache to bf16) and by at most 0.025 of a value: four times that
     return {"rel": 0.012, "max": 0.1}
+
+
+# ---- the same results in plain torch, in 64 bits ------------------------------------------------------------------
+def _quant(x, block):
+    """bf16 / fp32 values -> (e4m3 values, fp32 scale per block), both widened to float64."""
+    xb = x.float().reshape(*x.shape[:-1], -1, block)
+    scale = xb.abs().amax(-1).clamp_min(1e-6) / 448
+    q8 = (xb / scale.unsqueeze(-1)).to(torch.float8_e4m3fn).reshape(x.shape)
+    return q8.double(), scale.double()
+
+
+def _rope(x, rope, interleave):
+    """x [T, ..., dim]: rotation of the first `rope` values at position = row."""
+    half = rope // 2
+    inv = 1.0 / (10000.0 ** (torch.arange(0, half, device=DEV, dtype=torch.float32) / half))
+    ang = torch.outer(torch.arange(x.shape[0], device=DEV, dtype=torch.float32), inv).view(x.shape[0], *([1] * (x.dim() - 2)), half)
+    cos, sin = ang.cos(), ang.sin()
+    a, b = (x[..., 0:rope:2], x[..., 1:rope:2]) if interleave else (x[..., :half], x[..., half:rope])
+    y = (a * cos - b * sin, a * sin + b * cos)
+    y = torch.stack(y, -1).flatten(-2).to(x.dtype) if interleave else torch.cat(y, -1)
+    return torch.cat((y, x[..., rope:].to(y.dtype)), -1)
+
+
+def _attend(q8, w, k8, ksc, first, q, kv, topk, out):
+    """Rows of one sequence, row i seeing the first `first + i` keys: scores, selection, attention; all in float64."""
+    rows, heads, keys = q8.shape[0], q8.shape[1], k8.shape[0]
+    k8t, pos = k8.double().t(), torch.arange(keys, device=DEV)
+    step = max(1, min(64, (1 << 27) // (heads * keys)))
+    for a in range(0, rows, step):
+        b = min(rows, a + step)
+        s = (q8[a:b].double().reshape(-1, q8.shape[2]) @ k8t).relu_().view(b - a, heads, keys)
+        s = torch.einsum("ths,th->ts", s, w[a:b].double()) * ksc.double()
+        window = torch.arange(first + a, first + b, device=DEV).unsqueeze(1)
+        top = s.masked_fill(pos >= window, -math.inf).topk(min(topk, keys), dim=-1)
+        for c in range(a, b, 32):
+            d = min(b, c + 32)
+            g = kv[top.indices[c - a:d - a]].double()
+            p = torch.bmm(q[c:d].double(), g.transpose(1, 2)) * SCALE
+            p = p.masked_fill((top.values[c - a:d - a] == -math.inf).unsqueeze(1), -math.inf).softmax(-1)
+            out[c:d] = torch.bmm(p, g[..., :512])
+    return out
+
+
+def exact(case, seed):
+    """What `run` returns for the inputs `prepare` makes, in float64 from the same quantised and bf16 operands.  A layer's
+    projections stay the bf16 Linears that its module consists of: their outputs are the operands."""
+    kind, st = case["kind"], prepare(case, seed)
+    if kind in ("prefill", "chunk"):
+        out = torch.empty(case["rows"], case["heads"], 512, dtype=torch.float64, device=DEV)
+        return _attend(st["q8"], st["w"], st["k8"], st["ksc"], case.get("keys", case["rows"]) - case["rows"] + 1, st["q"], st["kv"],
+                       TOPK, out)
+    if kind == "decode":
+        out = torch.empty(case["batch"], case["heads"], 512, dtype=torch.float64, device=DEV)
+        for b, n in enumerate(st["ctx"].tolist()):
+            row = torch.arange(n, device=DEV)
+            row = st["table"][b, row // 64].long() * 64 + row % 64
+            rec = st["latent"][row]
+            lat = rec[:, :512].contiguous().view(torch.float8_e4m3fn).double().view(n, 4, 128)
+            lat = lat * rec[:, 512:528].contiguous().view(torch.float32).double().unsqueeze(-1)
+            kv = torch.cat((lat.view(n, 512), rec[:, 528:].contiguous().view(torch.bfloat16).double()), -1)
+            k8 = st["kcache"].view(torch.uint8)[row].view(torch.float8_e4m3fn)
+            _attend(st["q8"][b:b + 1], st["w"][b:b + 1], k8, st["kscale"][row], n, st["q"][b:b + 1], kv, TOPK, out[b:b + 1])
+        return out
+    if kind == "layer":
+        _, _, ih, idim, rope, topk, heads, interleave = LAYERS[case["spec"]]
+        m, x, rows = st["layer"], st["x"], case["rows"]
+        linear = torch.nn.functional.linear
+        with torch.no_grad():
+            ql, ind = linear(x, m.q_a.weight), m.indexer
+            k = torch.nn.functional.layer_norm(linear(x, ind.wk.weight), (idim,), ind.k_norm.weight, ind.k_norm.bias, ind.k_norm.eps)
+            q8, qs = _quant(_rope(linear(ql, ind.wq_b.weight).view(rows, ih, idim), rope, interleave), idim)
+            k8, ksc = _quant(_rope(k, rope, interleave), idim)
+            w = (linear(x, ind.weights_proj.weight).float() * ih ** -0.5).double() * qs.squeeze(-1) * idim ** -0.5
+            q, kv = linear(ql, m.wq.weight).view(rows, heads, 576), linear(x, m.wkv.weight)
+            return _attend(q8, w, k8, ksc.squeeze(-1), 1, q, kv, topk,
+                           torch.empty(rows, heads, 512, dtype=torch.float64, device=DEV))
+    if kind == "block_sparse":
+        batch, seq, heads = case["batch"], case["seq"], case["heads"]
+        out = torch.empty(batch, seq, heads, 128, dtype=torch.float64, device=DEV)
+        for b in range(batch):
+            for h in range(heads):
+                k, v = (st[n][b, :, h].double().view(seq // 64, 64, 128) for n in ("k", "v"))
+                q = st["q"][b, :, h].double().view(seq // 64, 64, 128)
+                for i in range(0, seq // 64, 32):
+                    lut = st["idx"][b, h, i:i + 32].long()
+                    kk, vv = (t[lut].flatten(1, 2) for t in (k, v))
+                    p = (torch.bmm(q[i:i + 32], kk.transpose(1, 2)) * 128 ** -0.5).softmax(-1)
+                    out[b, i * 64:(i + 32) * 64, h] = torch.bmm(p, vv).flatten(0, 1)
+        return out
+    return None                                             # whole bytes, and scales that are compared bit for bit

@@ -26,6 +26,24 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ---- warp-uniform control ------------------------------------------------------
+// tcgen05.mma and the TMA copies take their descriptors and addresses from uniform registers.  Where the compiler cannot
+// see that a value is the same in the whole warp (a role picked by threadIdx.x >> 5, a counter advanced by the result of
+// a poll, a branch on lane == 0 around all of it) it serialises over the lanes that might differ, and every instruction
+// costs ~120 cycles to issue whatever its shape -- measured 115-168 cycles per kind::f16 MMA for all of N = 64, 128, 256
+// against 50, 64 and 128 with warp-uniform operands.  So an issuing warp walks its loop as a whole, on values made
+// uniform by a shuffle or a vote, and elects a lane only around the instruction.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -70,6 +88,25 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status) {
   return mbar_wait_limit(bar, parity, abort_flag, status, kSpinLimit);
+}
+
+// the same for a whole warp whose lanes all come here: one answer for all of them
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+}
+// One look, by a whole warp that polls several barriers in turn.  test_wait and not try_wait: a try_wait that finds its
+// phase open suspends the warp, which then misses the other barriers (a polling loop of try_waits by 32 lanes ran the
+// sparse MLA kernel at a third of its speed).
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
 }
 
 // ---- TMA (tiled bulk tensor copies, global -> this CTA's shared memory) ----
@@ -228,6 +265,12 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 

@@ -187,3 +187,35 @@ def test_decode_split_parts_match_the_single_part_path():
     ops.check_status("cuda")
     assert float((split.float() - single.float()).abs().max()) <= 1e-2
     check(split, O.sparse_mla_decode_paged(q.float().cpu(), cache.cpu(), table.cpu(), idx.cpu(), 0.06, round_bf16=True))
+
+
+@pytest.mark.parametrize("K", [1, 63, 64, 65, 128, 191, 193, 320, 321, 385, 640, 705])
+@pytest.mark.parametrize("H", [128, 16])
+def test_prefill_block_counts(H, K):
+    """Slot lists around whole numbers of 64-key blocks: one and two blocks (one warp set has nothing to do), the number
+    of KV buffers (five), and beyond."""
+    q, kv, idx = make(3, H, 1500, K, seed=K + H, causal=False)
+    out = ops.sparse_mla_prefill(q.cuda(), kv.cuda(), idx.cuda(), 0.06)
+    ops.check_status("cuda")
+    check(out, O.sparse_mla(q.float(), kv.float(), idx, 0.06))
+
+
+@pytest.mark.parametrize("T,H", [(4096, 16), (2048, 128)])
+def test_prefill_whole_output_and_repeats(T, H):
+    """Many waves of CTA pairs, every output value: against float64 on the GPU, and bit for bit the same in every run (a
+    hand-over between the two CTAs that comes too early shows here as a few wrong tokens in ten thousand)."""
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    S, K, scale = 8192, 1024, 192 ** -0.5
+    kv = torch.randn(S, 576, device="cuda", generator=g).to(torch.bfloat16)
+    q = torch.randn(T, H, 576, device="cuda", generator=g).to(torch.bfloat16)
+    idx = torch.rand(T, S, device="cuda", generator=g).topk(K, dim=-1).indices.int()
+    out = ops.sparse_mla_prefill(q, kv, idx, scale)
+    for _ in range(12):
+        assert torch.equal(ops.sparse_mla_prefill(q, kv, idx, scale), out)
+    ops.check_status("cuda")
+    worst = 0.0
+    for a in range(0, T, 64):
+        rows = kv[idx[a:a + 64].long()].double()
+        p = (torch.bmm(q[a:a + 64].double(), rows.transpose(1, 2)) * scale).softmax(-1)
+        worst = max(worst, float((out[a:a + 64].double() - torch.bmm(p, rows[..., :512])).abs().max()))
+    assert worst <= MAX_ABS, worst

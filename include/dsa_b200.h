@@ -55,6 +55,11 @@ const char* dsa_last_error_string(void);
 int dsa_fp8_quant_per_block(const void* x, int x_dtype, int64_t n_blocks, int block_size, void* q_fp8, float* scale,
                             void* stream);
 
+/* Write side of the paged FP8 latent cache, one kernel: rows kv [n_tokens, 576] (fp32 DSA_X_F32 or bf16 DSA_X_BF16,
+ * row_stride values apart, every row 16-byte aligned) -> records [n_tokens, 656] bytes (16-byte aligned, dense): the 512
+ * latent values as e4m3, their four fp32 scales (one per 128 values, quantised as above), the 64 rope values as bf16. */
+int dsa_pack_latent_cache(const void* kv, int kv_dtype, int64_t row_stride, int64_t n_tokens, void* records, void* stream);
+
 /* RoPE + per-row FP8 quantiser in one pass: stands in for DsaIndexer.rope followed by fp8_quant_per_block
  * (sparse_attn/DSA.py:513-524, 530-531).  x_bf16 [n_rows, head_dim] (head_dim 64 or 128 = one FP8 block per
  * row); row r is at position r / rows_per_pos (heads per token for q, 1 for k); cos_table / sin_table

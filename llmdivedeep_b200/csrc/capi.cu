@@ -63,6 +63,7 @@ int block_sparse_mha_launch(const void* q, const void* k, const void* v, const i
 
 int fp8_quant_launch(const void* x, int x_is_bf16, int64_t n_blocks, int block, void* q, float* scale,
                      cudaStream_t stream);
+int pack_latent_launch(const void* kv, int kv_is_bf16, int64_t row_stride, int64_t n, void* rec, cudaStream_t stream);
 int rope_fp8_quant_launch(const void* x, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
                           const float* cos_t, const float* sin_t, void* q, float* scale, cudaStream_t stream);
 
@@ -243,6 +244,19 @@ int dsa_fp8_quant_per_block(const void* x, int x_dtype, int64_t n_blocks, int bl
   if (!aligned16(x) || (reinterpret_cast<uintptr_t>(q_fp8) & 3))
     return set_error(DSA_ERR_ALIGN, "fp8_quant_per_block: x must be 16-byte and q_fp8 4-byte aligned");
   return fp8_quant_launch(x, x_dtype == DSA_X_BF16, n_blocks, block_size, q_fp8, scale, static_cast<cudaStream_t>(stream));
+}
+
+int dsa_pack_latent_cache(const void* kv, int kv_dtype, int64_t row_stride, int64_t n_tokens, void* records, void* stream) {
+  g_err[0] = 0;
+  if (n_tokens < 0) return set_error(DSA_ERR_SHAPE, "pack_latent_cache: negative size");
+  if (n_tokens == 0) return DSA_OK;
+  if (!kv || !records) return set_error(DSA_ERR_ARG, "pack_latent_cache: NULL pointer argument");
+  if (kv_dtype != DSA_X_F32 && kv_dtype != DSA_X_BF16) return set_error(DSA_ERR_ARG, "pack_latent_cache: bad kv_dtype");
+  const int64_t elt = kv_dtype == DSA_X_BF16 ? 2 : 4;
+  if (n_tokens > 1 && row_stride < 576) return set_error(DSA_ERR_SHAPE, "pack_latent_cache: row_stride below 576");
+  if (!aligned16(kv) || !aligned16(records) || (n_tokens > 1 && (row_stride * elt) % 16))
+    return set_error(DSA_ERR_ALIGN, "pack_latent_cache: every row and the records must be 16-byte aligned");
+  return pack_latent_launch(kv, kv_dtype == DSA_X_BF16, row_stride, n_tokens, records, static_cast<cudaStream_t>(stream));
 }
 
 int dsa_rope_fp8_quant(const void* x_bf16, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,

@@ -462,6 +462,22 @@ def fp8_quant_per_block(x: torch.Tensor, block_size: int = 128):
     return q, (scale.view(x.shape[:-1]) if nb == 1 else scale.view(*x.shape[:-1], nb))
 
 
+def pack_latent_records(kv: torch.Tensor, out: torch.Tensor) -> bool:
+    """Latent rows [N, 576] -> cache records uint8 [N, 656] in one kernel.  Takes bf16 or fp32 rows with unit column
+    stride and dense records, everything 16-byte aligned; returns False, having done nothing, for any other call."""
+    N = kv.shape[0]
+    if (not kv.is_cuda or kv.dtype not in (torch.bfloat16, torch.float32) or out.dtype != torch.uint8 or out.device != kv.device
+            or tuple(out.shape) != (N, 656) or not out.is_contiguous()):
+        return False
+    rs, cs = kv.stride()
+    if N and (cs != 1 or (N > 1 and (rs < 576 or rs * kv.element_size() % 16)) or (kv.data_ptr() | out.data_ptr()) % 16):
+        return False
+    lib = _lib.load()
+    with torch.cuda.device(kv.device):
+        check(lib.dsa_pack_latent_cache(_ptr(kv), 1 if kv.dtype == torch.bfloat16 else 0, rs, N, _ptr(out), _stream()))
+    return True
+
+
 def rope_fp8_quant(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rope_dim: int, interleave: bool,
                    rows_per_pos: int = 1):
     """RoPE on the first ``rope_dim`` values of every head row followed by the per-row FP8 quantiser, one kernel

@@ -108,3 +108,44 @@ def test_prefill_composition_small_config():
     want = O.sparse_mla(q[rows].float(), kv.float(), idx.cpu()[rows], 192 ** -0.5)
     d = (out.float().cpu()[rows] - want).abs()
     assert float(d.max()) <= 2e-2 and float(d.mean()) <= 2e-3
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2000])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_pack_latent_cache_records(n, dtype):
+    """Every form of input and record tensor gives the oracle's bytes: dense rows and rows cut out of wider ones (the
+    one-kernel path), strided columns, unaligned rows and strided records (the quantiser and copies)."""
+    from llmdivedeep_b200 import layer
+    g = torch.Generator().manual_seed(n)
+    kv = torch.randn(n, 576, generator=g).to(dtype)
+    kv[0, :128] = 0
+    kv[n - 1, 100:140] *= 1e4
+    want = O.pack_latent_cache(kv)
+    wide = torch.zeros(n, 640, dtype=dtype)
+    wide[:, 32:608] = kv
+    odd = torch.zeros(n, 577, dtype=dtype)
+    odd[:, 1:] = kv
+    forms = [kv.cuda(), wide.cuda()[:, 32:608], kv.t().contiguous().cuda().t()]
+    if n > 1:                                          # (one unaligned row counts as contiguous, and the quantiser refuses it)
+        forms.append(odd.cuda()[:, 1:])
+    for x in forms:
+        assert torch.equal(layer.pack_latent_cache(x).cpu(), want)
+        out = torch.zeros(n, 700, dtype=torch.uint8, device="cuda")
+        assert torch.equal(layer.pack_latent_cache(x, out=out[:, 3:659]).cpu(), want)
+        assert int(out[:, :3].sum()) == 0 and int(out[:, 659:].sum()) == 0
+
+
+@pytest.mark.parametrize("block", [64, 128])
+@pytest.mark.parametrize("n_blocks", [1, 3, 8, 33, 70001])
+def test_quantiser_ragged_block_counts_and_unaligned_output(n_blocks, block):
+    from llmdivedeep_b200 import _lib
+    x = torch.randn(n_blocks, block, generator=torch.Generator().manual_seed(n_blocks)).to(torch.bfloat16)
+    want_q, want_s = O.fp8_quant_per_block(x, block)
+    xd = x.cuda()
+    for off in (0, 4):
+        q = torch.zeros(n_blocks * block + 8, dtype=torch.uint8, device="cuda")
+        s = torch.zeros(n_blocks + 1, device="cuda")
+        _lib.check(_lib.load().dsa_fp8_quant_per_block(xd.data_ptr(), 1, n_blocks, block, q.data_ptr() + off, s.data_ptr(),
+                                                       torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(q[off:off + n_blocks * block].cpu(), want_q.view(torch.uint8).reshape(-1)) and not q[off + n_blocks * block:].any()
+        assert torch.equal(s[:n_blocks].cpu(), want_s.reshape(-1)) and float(s[n_blocks]) == 0

@@ -9,9 +9,8 @@
 // pair owns latent panels 4c..4c+3 -- its half of V -- and half of the rope panel's contraction:
 //   * it gathers only those 576 bytes of every selected row (36 KB per 64-key block, five blocks in
 //     flight), swizzled by the writing threads: cp.async straight out of the bf16 KV, or -- for the
-//     paged FP8 latent cache of decode -- cp.async of the raw rows into two shared-memory stages, two
-//     blocks ahead, and a shared -> shared conversion e4m3 x group scale -> bf16 (four KV buffers; the
-//     fifth one's space holds the raw stages);
+//     paged FP8 latent cache of decode -- cp.async of the raw rows two blocks ahead and a conversion
+//     e4m3 x group scale -> bf16 into one of four buffers;
 //   * its five Q panels live in tensor memory as the A operand, so Q.K^T reads no shared memory for
 //     Q, and it computes a PARTIAL score tile S_c = Q_c K_c^T (18 tcgen05.mma kind::f16 of N = 64);
 //   * the two partial tiles ([128 heads x 64 keys], rounded to fp16 for the way: 16 KB) are exchanged
@@ -31,17 +30,20 @@
 // (a warp keeps about eight 512-byte requests going, whether cp.async or TMA gather4), arrivals by the copies themselves.
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137
 // cycles each; see dsa_common.cuh) and TMA gather; 3125 with warp-uniform issue; 2860 with two sets of softmax warps;
-// 2418 with sixteen and setmaxnreg; 2274 as it stands (1027 TFLOP/s).  Tried on top: the exchange by st.async (3320:
+// 2418 with sixteen and setmaxnreg; 2228 as it stands (1049 TFLOP/s).  Tried on top: the exchange by st.async (3320:
 // the stores drain slowly and clog the gather), by loads from the peer's shared memory (3560: the release at cluster
 // scope costs ~2300 cycles), a quarter of the exponentials as polynomials on the FMA pipe (+3 %: the issue slots are
 // short too).
 //
-// Roles: warps 0-15 exchange + softmax + output, warp 16 MMA issuer (owns the TMEM allocation), warps 17-27 gather
-// (decode: 17-24).  Softmax warp w: set w / 8 takes the blocks of that parity, key half (w / 4) % 2, heads = TMEM lanes
+// Roles: warps 0-15 exchange + softmax + output, warp 16 MMA issuer (owns the TMEM allocation), warps 17-27 gather.
+//  Softmax warp w: set w / 8 takes the blocks of that parity, key half (w / 4) % 2, heads = TMEM lanes
 // 32 (w % 4)..; a thread owns one head and half of a block's keys.  The two threads of a head tell each other their
 // block maxima through shared memory (rounded up to bf16: any common reference point is exact for a softmax); from the
 // maxima of all blocks in order every thread follows the running reference by itself, so that one set can run ahead of
 // the other; row sums stay per thread until the end.
+// Decode, batch 64 (a call, launch included): 105 us with eight gather warps that met at two barriers per block, 72 us with
+// eleven that never wait for one another.  Loads into registers one block ahead in place of the raw stages: 94 us (the rows
+// take about 3000 cycles to come).  The gather then costs issue slots, about as many as the softmax.
 // Every wait is bounded (dsa_common.cuh); the two CTAs leave together through a cluster barrier.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -66,20 +68,15 @@ constexpr int kMlaRopeOff = 4 * kMlaKPanelBytes;   // in a buffer: four latent p
 constexpr int kMlaKBytes = kMlaRopeOff + kMlaBlk * 64;        // 36864 per buffer
 constexpr int kMlaXBytes = 128 * kMlaBlk * 2;      // one partial score tile, fp16: 16384
 constexpr int kMlaXWarp = kMlaXBytes / 8;          // ... a warp's part of it
-constexpr int kMlaRing = 2;                        // row-id slots: read only by the gather warps, inside the call that staged them
-constexpr int kMlaMaskRing = 8;                    // validity masks (64 bits per block) for the softmax: >= blocks in flight
+constexpr int kMlaValidRing = 8;                   // validity bytes (64 per block) for the softmax: >= blocks in flight
 // The registers of the launch (896 threads x 72) are dealt out again: setmaxnreg moves what the issuing and gathering
 // warps do not need to the softmax.
 template <bool FP8_PAGED>
-struct MlaCfg {
-  static constexpr int kThreads = 896;
-  static constexpr int kLaunchRegs = 72;
-  static constexpr int kSoftmaxRegs = FP8_PAGED ? 88 : 96, kOtherRegs = FP8_PAGED ? 48 : 40;
-  static constexpr int kGatherWarps = FP8_PAGED ? 8 : 11;      // at most 11: the warps of the last warpgroup
-  static constexpr int kGatherThreads = kGatherWarps * 32;
-  static_assert(512 * kSoftmaxRegs + 384 * kOtherRegs <= kThreads * kLaunchRegs, "more registers than the launch has");
+struct MlaRegs {                                   // decode's gather converts in registers
+  static constexpr int kSoftmax = FP8_PAGED ? 88 : 96, kOther = FP8_PAGED ? 48 : 40;
+  static_assert(512 * kSoftmax + 384 * kOther <= 896 * 72, "more registers than the launch has");
 };
-constexpr int kMlaSoftmaxWarps = 16, kMlaMmaWarp = 16, kMlaGatherWarp0 = 17;
+constexpr int kMlaThreads = 896, kMlaSoftmaxWarps = 16, kMlaMmaWarp = 16, kMlaGatherWarp0 = 17, kMlaGatherWarps = 11;
 template <int R>
 __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R>
@@ -87,7 +84,7 @@ __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.a
 constexpr int kMlaBarBytes = 512;                  // mbarriers and a few words
 constexpr int kMlaPairBytes = 4 * 2 * 128 * 2;     // block maxima: [block mod 4][key half][head], bf16
 constexpr int kMlaSmemBytes = kMlaBufs * kMlaKBytes + 2 * kMlaXBytes + kMlaBarBytes +
-                              kMlaMaskRing * 2 * 4 + kMlaPairBytes;
+                              kMlaValidRing * kMlaBlk + kMlaPairBytes;
 static_assert(kMlaSmemBytes <= 232448, "shared memory budget of one CTA");
 constexpr int kLatentTokenBytes = 656;             // 512 e4m3 + 4 fp32 scales + 64 bf16 rope
 constexpr int kLatentPage = 64;
@@ -107,9 +104,10 @@ struct MlaArgs {
   int num_phys_rows;              // decode: rows of the cache
   float scale_log2e;              // softmax scale * log2(e)
   int* status;
-  int n_split;                    // > 1: each query's slot list is cut into n_split parts (decode with few queries)
-  float* part_o;                  // [T * n_split, H, 512] fp32 normalised partial outputs
-  float* part_lse;                // [T * n_split, H] log2-sum-exp of each part (-inf = empty part)
+  int n_full;                     // the first n_full queries are one unit (CTA pair) each; ...
+  int n_split;                    // ... the slot list of every later one is cut into n_split parts, a unit each (decode)
+  float* part_o;                  // [(T - n_full) * n_split, H, 512] fp32 normalised partial outputs
+  float* part_lse;                // [(T - n_full) * n_split, H] log2-sum-exp of each part (-inf = empty part)
   int tma_out;                    // the output tensor map is valid: full 128-head groups leave through TMA stores
 };
 
@@ -177,11 +175,6 @@ __device__ __forceinline__ uint32_t bf16_bits_round_up(float x) {
 }
 
 // ---- paged FP8 latent cache (decode) ------------------------------------------------------------
-// A block's rows travel global -> shared memory as raw bytes with cp.async (asynchronous, two blocks ahead, no registers
-// held), and are converted shared -> shared.  A raw row is this CTA's 256 e4m3 values followed by the row's four scales.
-constexpr int kRawRow = kMlaDvHalf + 16;
-constexpr int kRawStage = kMlaBlk * kRawRow;         // 17408 bytes
-static_assert(2 * kRawStage + kMlaRing * kMlaBlk * 4 <= kMlaKBytes, "the two raw stages take the place of the fifth KV buffer");
 __device__ __forceinline__ void cp_async_16(void* dst, const void* src, int src_bytes) {      // src_bytes 0: zero fill
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -190,47 +183,38 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// A gather warp's raw rows of one block: per row this CTA's 256 e4m3 values, the four scales, this CTA's 64 rope bytes.
+constexpr int kRawRow = 256 + 16 + 64, kRawRows = (kMlaBlk + kMlaGatherWarps - 1) / kMlaGatherWarps, kRawBytes = kRawRows * kRawRow;
+constexpr int kRawInBuf = kMlaKBytes / kRawBytes;                     // of the 2 x 11 pieces, those in the fifth KV buffer
+constexpr int kMlaSmemDecode = kMlaSmemBytes + (2 * kMlaGatherWarps - kRawInBuf) * kRawBytes;
+static_assert(kRawRows % 2 == 0 && kMlaSmemBytes % 16 == 0 && kMlaSmemDecode <= 232448, "raw rows of decode");
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// e4m3 -> bf16 with the per-128 group scale, raw stage -> this CTA's four latent panels of a KV buffer.  Thread g of
-// GT gather threads; an empty slot was zero-filled (values and scales), so it converts to zeros.  (Tried and dropped:
-// decode's latent MMAs in fp16, so that e4m3 x scale is one conversion and one packed multiply per two values -- a third
-// of the instructions, and 9 % slower end to end: the conversion is not what paces the decode kernel.)
-template <int GT>
-__device__ __forceinline__ void convert_block(const uint8_t* stage, uint8_t* kv_s, int g, int cta) {
-  constexpr int kLat = kMlaBlk * 16 / GT;          // 16-value chunks per thread
+// Eight e4m3 values times their group scale, rounded to bf16; an empty slot's zeros (values and scale) stay zeros.
+__device__ __forceinline__ uint4 e4m3x8_to_bf16(uint2 raw, float sc) {
+  const uint32_t w[2] = {raw.x, raw.y};
+  const uint64_t sc2 = pack_f32x2(sc, sc);
+  uint32_t o[4];
 #pragma unroll
-  for (int u = 0; u < kLat; ++u) {
-    const int q = g + u * GT;
-    const int r = q >> 4, cc = q & 15;              // row, chunk inside this CTA's 256 latent dims
-    const uint4 raw = *reinterpret_cast<const uint4*>(stage + r * kRawRow + cc * 16);
-    const float sc = *reinterpret_cast<const float*>(stage + r * kRawRow + kMlaDvHalf + (cta * 2 + (cc >> 3)) * 4);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    uint32_t outw[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const __nv_fp8x2_storage_t pr = static_cast<__nv_fp8x2_storage_t>((w[i >> 1] >> (16 * (i & 1))) & 0xffffu);
-      const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(pr, __NV_E4M3);
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h2));
-      outw[i] = pack_bf16x2(f.x * sc, f.y * sc);
-    }
-    const int p = cc >> 2, c = (cc & 3) * 2;        // local panel, 16-byte chunk inside the 128-byte row (even)
-    uint8_t* base = kv_s + p * kMlaKPanelBytes + r * 128;
-    *reinterpret_cast<uint4*>(base + ((c ^ (r & 7)) << 4)) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
-    *reinterpret_cast<uint4*>(base + (((c + 1) ^ (r & 7)) << 4)) = make_uint4(outw[4], outw[5], outw[6], outw[7]);
+  for (int i = 0; i < 4; ++i) {
+    const __nv_fp8x2_storage_t pr = static_cast<__nv_fp8x2_storage_t>((w[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+    const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(pr, __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h2));
+    float x, y;
+    unpack_f32x2(mul_f32x2(pack_f32x2(f.x, f.y), sc2), x, y);
+    o[i] = pack_bf16x2(x, y);
   }
+  return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 template <bool FP8_PAGED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MlaCfg<FP8_PAGED>::kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMlaThreads, 1)
 sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
                   const __grid_constant__ CUtensorMap tmap_o, const MlaArgs a) {
+  constexpr int NB = FP8_PAGED ? kMlaBufs - 1 : kMlaBufs;      // KV buffers in use (decode: the fifth one's space holds raw rows)
   extern __shared__ __align__(1024) uint8_t smem[];            // the swizzled panels need 1024-byte alignment
-  constexpr int NB = FP8_PAGED ? kMlaBufs - 1 : kMlaBufs;      // KV buffers in use (decode: the fifth holds the raw stages)
-  constexpr int kMlaGatherWarps = MlaCfg<FP8_PAGED>::kGatherWarps, kMlaGatherThreads = MlaCfg<FP8_PAGED>::kGatherThreads;
-  constexpr int kMlaThreads = MlaCfg<FP8_PAGED>::kThreads;
   uint8_t* kv_s = smem;                                        // five buffers: four panels [64 keys x 128 B] and 64 x 64 B
   uint8_t* send_s = kv_s + kMlaBufs * kMlaKBytes;              // this CTA's partial score tile on its way out
   uint8_t* recv_s = send_s + kMlaXBytes;                       // the peer's
@@ -251,14 +235,16 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 59);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_s = const_cast<int*>(abort_flag) + 1;
-  uint32_t* masks = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(bars) + kMlaBarBytes);        // [kMlaMaskRing][2] bit s = slot s of the block is in use
-  uint16_t* pm_s = reinterpret_cast<uint16_t*>(masks + kMlaMaskRing * 2);          // block maxima, rounded up to bf16
+  uint8_t* valid_s = reinterpret_cast<uint8_t*>(bars) + kMlaBarBytes;       // [kMlaValidRing][64] 1 = the slot of the block is in use
+  uint16_t* pm_s = reinterpret_cast<uint16_t*>(valid_s + kMlaValidRing * kMlaBlk);          // block maxima, rounded up to bf16
 
   const int cta = blockIdx.x & 1, peer = cta ^ 1;              // rank in the cluster = V half = contraction part
   const int unit = blockIdx.x >> 1;
-  const int t = unit / a.n_split, split = unit % a.n_split, hg = blockIdx.z;
+  const int part = unit - a.n_full;                            // >= 0: a part of a split slot list
+  const int n_split = part < 0 ? 1 : a.n_split, t = part < 0 ? unit : a.n_full + part / n_split, split = part < 0 ? 0 : part % n_split;
+  const int hg = blockIdx.z;
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int k_per = ((a.K + a.n_split - 1) / a.n_split + kMlaBlk - 1) / kMlaBlk * kMlaBlk;   // slots per part
+  const int k_per = ((a.K + n_split - 1) / n_split + kMlaBlk - 1) / kMlaBlk * kMlaBlk;   // slots per part
   const int k_lo = min(a.K, split * k_per), k_cnt = min(a.K, k_lo + k_per) - k_lo;
   const int32_t* idx_row = a.idx + (int64_t)t * a.K + k_lo;
   const int heads_here = min(128, a.H - hg * 128);
@@ -283,7 +269,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       const uint32_t count = i == 1 ? 16u                                            // q_moved: lane 0 of the softmax warps
                              : (i == 3 || i == 4) ? 8u                               // s_free, p_full: lane 0 of a set's warps
                              : (i >= 9 && i <= 16) ? 2u                              // pm_full: the two warps of a quadrant
-                             : (i >= 49 && i <= 53) ? uint32_t(kMlaGatherThreads) + (FP8_PAGED ? 0u : 1u)
+                             : (i >= 49 && i <= 53) ? (FP8_PAGED ? uint32_t(kMlaGatherWarps) : kMlaGatherWarps * 33u)
                                                     : 1u;                            // the others
       mbar_init(bars + i, count);
     }
@@ -321,11 +307,11 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const int nblk = (*last_s + kMlaBlk) / kMlaBlk;
   if (nblk == 0) {   // nothing selected: the output row is zero (a part: weight zero in the combine); no cluster traffic yet
     if (threadIdx.x < 128 && threadIdx.x < heads_here) {
-      if (a.n_split == 1) {
+      if (part < 0) {
         uint4* o = reinterpret_cast<uint4*>(a.out + ((int64_t)t * a.H + hg * 128 + threadIdx.x) * kMlaDv + cta * kMlaDvHalf);
         for (int c = 0; c < kMlaDvHalf * 2 / 16; ++c) o[c] = make_uint4(0, 0, 0, 0);
       } else {
-        const int64_t prow = (int64_t)unit * a.H + hg * 128 + threadIdx.x;
+        const int64_t prow = (int64_t)part * a.H + hg * 128 + threadIdx.x;
         float4* o = reinterpret_cast<float4*>(a.part_o + prow * kMlaDv + cta * kMlaDvHalf);
         for (int c = 0; c < kMlaDvHalf / 4; ++c) o[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (cta == 0) a.part_lse[prow] = -CUDART_INF_F;
@@ -344,8 +330,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   // round trip through the cluster barrier is off the path to the first MMA.
   cluster_arrive();
 
-  if (warp >= kMlaSoftmaxWarps) regs_dec<MlaCfg<FP8_PAGED>::kOtherRegs>();
-  else regs_inc<MlaCfg<FP8_PAGED>::kSoftmaxRegs>();
+  if (warp >= kMlaSoftmaxWarps) regs_dec<MlaRegs<FP8_PAGED>::kOther>();
+  else regs_inc<MlaRegs<FP8_PAGED>::kSoftmax>();
   if (warp == kMlaMmaWarp) {
     // ------------------------------- MMA issuer -------------------------------
     // The partial scores of a block travel to the peer and through the softmax while the next blocks are scored: P.V of a
@@ -376,7 +362,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       int qk = 0, pv = 0;                              // next block to score, next block to accumulate
       auto pv_ready = [&]() { return pv < qk && mbar_test_warp(p_full, pv & 1); };
       auto issue_qk = [&](int i) {
-        if constexpr (!FP8_PAGED) fence_async_smem();  // the rows were written by cp.async, the tensor core reads through the async proxy
+        fence_async_smem();                            // the rows were written by cp.async or st, the tensor core reads through the async proxy
         tc_fence_after();
         if (elect_one()) {
           const uint64_t kd0 = kdesc0 + uint64_t(i % NB) * (kMlaKBytes >> 4);
@@ -418,74 +404,65 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
       }
     }
-  } else if (warp >= kMlaGatherWarp0 + kMlaGatherWarps) {
-    // (idle: fills up the warpgroup)
   } else if (warp >= kMlaGatherWarp0) {
     // ----------------------------- gather of the selected rows -----------------------------
-    const int g = threadIdx.x - kMlaGatherWarp0 * 32;                  // 0..kMlaGatherThreads-1
     const int w4 = warp - kMlaGatherWarp0;
+    constexpr int kG = kMlaGatherWarps;
     bool ok = true;
+    // A warp fetches every kG-th slot of a block, six at most: lane j < 6 keeps the id of slot w4 + 11 j.
+    const int slot = lane < kRawRows ? w4 + lane * kG : kMlaBlk;
+    auto load_pos = [&](int blk) -> int {
+      const int j = blk * kMlaBlk + slot;
+      return (slot < kMlaBlk && blk < nblk && j < k_cnt) ? __ldg(idx_row + j) : -1;
+    };
+    auto mark = [&](int blk, bool used) {
+      if (slot < kMlaBlk) valid_s[(blk % kMlaValidRing) * kMlaBlk + slot] = used;
+    };
     if constexpr (!FP8_PAGED) {
-      // Every warp keeps the block's 64 row ids in two registers per lane, requested one block ahead, and fetches every
-      // kG-th row: 512 latent bytes are one 16-byte cp.async per lane, this CTA's 64 rope bytes of eight rows another one.
-      // Nobody waits for the copies here: they arrive on the block's barrier by themselves, and the MMA warp orders them
-      // before the tensor core's reads (a proxy fence anywhere on the path between the two will do).
-      constexpr int kG = kMlaGatherWarps;
-      auto load_pos = [&](int blk, int hf) -> int {
-        const int j = blk * kMlaBlk + hf * 32 + lane;
-        return (blk < nblk && j < k_cnt) ? __ldg(idx_row + j) : -1;
-      };
-      auto translate = [&](int pos) -> int {           // -1 = empty slot; bad positions are flagged and skipped
-        if (pos >= a.S_kv) {
-          if (a.status) atomicCAS(a.status, kStatusOk, kStatusBadIndex);
-          return -1;
-        }
-        return pos < 0 ? -1 : pos;
-      };
-      int nxt0 = load_pos(0, 0), nxt1 = load_pos(0, 1);
+      // Row ids are requested one block ahead.  512 latent bytes are one 16-byte cp.async per lane, this CTA's 64 rope bytes
+      // of all six rows another one.  Nobody waits for the copies here: they arrive on the block's barrier by themselves,
+      // and the MMA warp orders them before the tensor core's reads (a proxy fence anywhere on the path between the two
+      // will do).
+      int nxt = load_pos(0);
       const uint8_t* src_lat = a.kv + cta * (kMlaDvHalf * 2) + lane * 16;
       const uint8_t* src_rope = a.kv + kMlaDv * 2 + cta * 64 + (lane & 3) * 16;
       for (int i = 0; i < nblk; ++i) {
         const int kvb = i % NB;
-        const int id0 = translate(nxt0), id1 = translate(nxt1);
-        nxt0 = load_pos(i + 1, 0);
-        nxt1 = load_pos(i + 1, 1);
-        const uint32_t used0 = __ballot_sync(0xffffffffu, id0 >= 0), used1 = __ballot_sync(0xffffffffu, id1 >= 0);
+        int id = nxt;                                  // -1 = empty slot; bad positions are flagged and skipped
+        if (id >= a.S_kv) {
+          if (a.status) atomicCAS(a.status, kStatusOk, kStatusBadIndex);
+          id = -1;
+        }
+        nxt = load_pos(i + 1);
         if (i == kQBuf0) ok = mbar_wait_warp(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
         if (i >= NB) ok = mbar_wait_warp(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
-        if (w4 == 0 && lane == 0) {
-          masks[(i % kMlaMaskRing) * 2] = used0;
-          masks[(i % kMlaMaskRing) * 2 + 1] = used1;
-          mbar_arrive(&kv_full[kvb]);
-        }
+        mark(i, id >= 0);
         uint8_t* dst = kv_s + kvb * kMlaKBytes;
         uint8_t* dst_lat = dst + (lane >> 3) * kMlaKPanelBytes;
-#pragma unroll 8
-        for (int r = w4; r < kMlaBlk; r += kG) {
-          const int id = __shfl_sync(0xffffffffu, r < 32 ? id0 : id1, r & 31);
-          cp_async_16(dst_lat + r * 128 + (((lane ^ r) & 7) << 4), src_lat + (int64_t)max(id, 0) * (kMlaDqk * 2), id >= 0 ? 16 : 0);
+#pragma unroll
+        for (int j = 0; j < kRawRows; ++j) {
+          const int r = w4 + j * kG, rid = __shfl_sync(0xffffffffu, id, j);
+          if (r < kMlaBlk)
+            cp_async_16(dst_lat + r * 128 + (((lane ^ r) & 7) << 4), src_lat + (int64_t)max(rid, 0) * (kMlaDqk * 2), rid >= 0 ? 16 : 0);
         }
-        if (const int r8 = kG - 1 - w4; r8 < kMlaBlk / 8) {      // the last warps have one row less
-          const int r = r8 * 8 + (lane >> 2);
-          const int id = __shfl_sync(0xffffffffu, r8 < 4 ? id0 : id1, r & 31);
-          cp_async_16(dst + kMlaRopeOff + r * 64 + (((lane ^ (r >> 1)) & 3) << 4),
-                      src_rope + (int64_t)max(id, 0) * (kMlaDqk * 2), id >= 0 ? 16 : 0);
+        {
+          const int r = w4 + (lane >> 2) * kG, rid = __shfl_sync(0xffffffffu, id, lane >> 2);
+          if (lane < 4 * kRawRows && r < kMlaBlk)
+            cp_async_16(dst + kMlaRopeOff + r * 64 + (((lane ^ (r >> 1)) & 3) << 4),
+                        src_rope + (int64_t)max(rid, 0) * (kMlaDqk * 2), rid >= 0 ? 16 : 0);
         }
-        cp_async_arrive(&kv_full[kvb]);                // this thread's arrival, once its copies have landed
+        cp_async_arrive(&kv_full[kvb]);                // this thread's arrival, once its copies have landed ...
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&kv_full[kvb]);     // ... and the warp's, for the validity bytes
       }
       cp_async_wait_all();                             // nothing of this thread's is in flight when it leaves
     } else {
-      // Decode.  Block b's raw rows are requested two blocks ahead with cp.async into one of two raw stages (the space of
-      // the fourth KV buffer), its rope halves with plain loads into registers; block b is converted into its KV buffer
-      // while blocks b+1 and b+2 are on their way.  The page-table entry of a slot is requested one call before it is
-      // examined, its position one call before that, so that no global-memory latency sits in the loop.
-      uint8_t* raw_s = kv_s + NB * kMlaKBytes;
-      int* ring = reinterpret_cast<int*>(raw_s + 2 * kRawStage);     // [kMlaRing][64] row id per slot, -1 = empty
-      auto load_pos = [&](int blk) -> int {
-        const int j = blk * kMlaBlk + g;
-        return (g < kMlaBlk && blk < nblk && j < k_cnt) ? __ldg(idx_row + j) : -1;
-      };
+      // Decode.  The same split of rows over the warps.  A warp keeps the raw rows of two blocks of its own in shared memory:
+      // cp.async two blocks ahead (a cache row is a DRAM and often a TLB miss away, ~3000 cycles), then 8 e4m3 values per
+      // lane and row through registers into the KV buffer.  The warps never wait for one another.  Positions travel four
+      // blocks ahead, page-table entries three.
+      constexpr int kRows = kRawRows;
       auto table_entry = [&](int pos) -> int {
         return (pos >= 0 && pos < a.S_kv) ? __ldg(a.block_table + (int64_t)t * a.table_stride + pos / kLatentPage) : -1;
       };
@@ -496,80 +473,76 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         if (a.status) atomicCAS(a.status, kStatusOk, kStatusBadIndex);
         return -1;
       };
-      constexpr int kRopePer = kMlaBlk * 4 / kMlaGatherThreads;      // 16-byte rope chunks per thread and block
-      uint4 rope_e[kRopePer], rope_o[kRopePer];        // rope chunks of the even / odd block in flight
-      // request block b: stage its row ids (and the validity mask for the softmax), then issue the copies
-      auto fetch = [&](int b, int row, uint4 (&rope)[kRopePer]) {
-        int* rows_s = ring + (b & 1) * kMlaBlk;
-        if (g < kMlaBlk) {
-          rows_s[g] = row;
-          const uint32_t used = __ballot_sync(0xffffffffu, row >= 0);            // the first two gather warps: 32 slots each
-          if (lane == 0) masks[(b % kMlaMaskRing) * 2 + w4] = used;
-        }
-        named_bar_sync(2, kMlaGatherThreads);            // ids staged; everyone is done with the raw stage that is overwritten next
-        if (b < nblk) {
-          uint8_t* stage = raw_s + (b & 1) * kRawStage;
-          constexpr int kCopies = kMlaBlk * 17;          // 16 value chunks + the scales, per row
-#pragma unroll
-          for (int u = 0; u < (kCopies + kMlaGatherThreads - 1) / kMlaGatherThreads; ++u) {
-            const int q = g + u * kMlaGatherThreads;
-            if (q < kCopies) {
-              const int r = q / 17, c = q - r * 17;
-              const int rr = rows_s[r];
-              const uint8_t* rec = a.cache + (int64_t)(rr >= 0 ? rr : 0) * kLatentTokenBytes;
-              cp_async_16(stage + r * kRawRow + c * 16, rec + (c < 16 ? cta * kMlaDvHalf + c * 16 : kMlaDv), rr >= 0 ? 16 : 0);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < kRopePer; ++u) {           // this CTA's two K-steps of the rope panel: 64 bytes per row
-            const int q = g + u * kMlaGatherThreads;
-            const int rr = rows_s[q >> 2];
-            rope[u] = make_uint4(0, 0, 0, 0);
-            if (rr >= 0)
-              rope[u] = __ldg(reinterpret_cast<const uint4*>(a.cache + (int64_t)rr * kLatentTokenBytes + kMlaDv + 16) + cta * 4 + (q & 3));
-          }
-        }
-        cp_async_commit();                               // one group per call, empty or not: the counting below relies on it
+      auto stage_of = [&](int blk) -> uint8_t* {       // the fifth KV buffer, and what does not fit there behind everything else
+        const int c = (blk & 1) * kG + w4;
+        return c < kRawInBuf ? kv_s + NB * kMlaKBytes + c * kRawBytes : smem + kMlaSmemBytes + (c - kRawInBuf) * kRawBytes;
       };
-      int P2, T2, P3;                                    // position / table entry of this thread's slot in block i+2, position in block i+3
+      const uint8_t* src_lat = a.cache + cta * kMlaDvHalf + (lane & 15) * 16;
+      const uint8_t* src_rope = a.cache + kMlaDv + 16 + cta * 64 + (lane & 3) * 16;
+      // request the warp's rows of a block; an empty slot is zero-filled, values and scales
+      auto fetch = [&](int blk, int id) {
+        uint8_t* st = stage_of(blk);
+#pragma unroll
+        for (int u = 0; u < kRows / 2; ++u) {          // two rows of 256 values per instruction
+          const int j = 2 * u + (lane >> 4), rid = __shfl_sync(0xffffffffu, id, j);
+          cp_async_16(st + j * kRawRow + (lane & 15) * 16, src_lat + (int64_t)max(rid, 0) * kLatentTokenBytes, rid >= 0 ? 16 : 0);
+        }
+        const int rid = __shfl_sync(0xffffffffu, id, lane >> 2);
+        if (lane < kRows)                              // a row's four scales
+          cp_async_16(st + lane * kRawRow + 256, a.cache + kMlaDv + (int64_t)max(id, 0) * kLatentTokenBytes, id >= 0 ? 16 : 0);
+        if (lane < 4 * kRows)                          // this CTA's two K-steps of the rope panel: 64 bytes per row
+          cp_async_16(st + (lane >> 2) * kRawRow + 272 + (lane & 3) * 16, src_rope + (int64_t)max(rid, 0) * kLatentTokenBytes, rid >= 0 ? 16 : 0);
+        cp_async_commit();
+      };
+      // row ids of blocks i and i+1 (which of them are used), page-table entry and position of i+2, position of i+3
+      int id_cur, id_nxt, pa, ta, pb;
       {
         const int p0 = load_pos(0), p1 = load_pos(1);
-        P2 = load_pos(2);
-        P3 = load_pos(3);
+        pa = load_pos(2);
+        pb = load_pos(3);
         const int t0 = table_entry(p0), t1 = table_entry(p1);
-        T2 = table_entry(P2);
-        fetch(0, cache_row(p0, t0), rope_e);
-        fetch(1, cache_row(p1, t1), rope_o);
+        ta = table_entry(pa);
+        id_cur = cache_row(p0, t0);
+        fetch(0, id_cur);
+        id_nxt = cache_row(p1, t1);
+        fetch(1, id_nxt);
       }
-      auto step = [&](int i, uint4 (&rope)[kRopePer]) -> bool {
+      for (int i = 0; i < nblk; ++i) {
         const int kvb = i % NB;
-        if (i == kQBuf0) mbar_wait(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
-        if (i >= NB) mbar_wait(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
-        cp_async_wait<1>();                              // this thread's copies of block i have landed (block i+1 may be in flight)
-        // ... and everyone else's; every thread of the group takes the same way out of a failed wait
-        if (named_bar_or(2, kMlaGatherThreads, *abort_flag != 0)) return false;
+        const int id2 = cache_row(pa, ta);             // block i+2
+        pa = pb;
+        ta = table_entry(pa);
+        pb = load_pos(i + 4);
+        if (i == kQBuf0) ok = mbar_wait_warp(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
+        if (i >= NB) ok = mbar_wait_warp(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
+        if (!ok) break;
+        mark(i, id_cur >= 0);
+        id_cur = id_nxt;
+        id_nxt = id2;
+        cp_async_wait<1>();                            // this lane's copies of block i have landed (block i+1 may be in flight) ...
+        __syncwarp();                                  // ... and the other lanes'
+        const uint8_t* st = stage_of(i);
         uint8_t* dst = kv_s + kvb * kMlaKBytes;
-        convert_block<kMlaGatherThreads>(raw_s + (i & 1) * kRawStage, dst, g, cta);
+        uint8_t* dst_lat = dst + (lane >> 3) * kMlaKPanelBytes;
 #pragma unroll
-        for (int u = 0; u < kRopePer; ++u) {
-          const int q = g + u * kMlaGatherThreads;
-          const int r = q >> 2;
-          *reinterpret_cast<uint4*>(dst + kMlaRopeOff + r * 64 + (((q ^ (r >> 1)) & 3) << 4)) = rope[u];
+        for (int j = 0; j < kRows; ++j) {
+          const int r = w4 + j * kG;
+          const uint2 raw = *reinterpret_cast<const uint2*>(st + j * kRawRow + lane * 8);
+          const float sc = *reinterpret_cast<const float*>(st + j * kRawRow + 256 + cta * 8 + (lane >> 4) * 4);
+          const uint4 v = e4m3x8_to_bf16(raw, sc);
+          if (r < kMlaBlk) *reinterpret_cast<uint4*>(dst_lat + r * 128 + (((lane ^ r) & 7) << 4)) = v;
         }
-        fence_async_smem();                              // make the panel writes visible to the tensor core's reads
-        mbar_arrive(&kv_full[kvb]);
-        const int row = cache_row(P2, T2);               // block i+2
-        P2 = P3;
-        T2 = table_entry(P2);
-        P3 = load_pos(i + 4);
-        fetch(i + 2, row, rope);
-        return true;
-      };
-      for (int i = 0; i < nblk && ok; i += 2) {
-        ok = step(i, rope_e);
-        if (ok && i + 1 < nblk) ok = step(i + 1, rope_o);
+        {
+          const int r = w4 + (lane >> 2) * kG;
+          if (lane < 4 * kRows && r < kMlaBlk)
+            *reinterpret_cast<uint4*>(dst + kMlaRopeOff + r * 64 + (((lane ^ (r >> 1)) & 3) << 4)) =
+                *reinterpret_cast<const uint4*>(st + (lane >> 2) * kRawRow + 272 + (lane & 3) * 16);
+        }
+        __syncwarp();                                  // (the MMA warp makes the writes visible to the tensor core's reads)
+        if (lane == 0) mbar_arrive(&kv_full[kvb]);
+        fetch(i + 2, id2);                             // into the stage just read: what was loaded from it has been stored
       }
-      cp_async_wait<0>();                                // nothing of this thread's is in flight into shared memory when it leaves
+      cp_async_wait_all();                             // nothing of this thread's is in flight when it leaves
     }
   } else {
     // ------------- partial-score exchange, softmax and output: thread = (head, half of a block's keys) -------------
@@ -658,7 +631,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
           add_f16x2(tw[k], __uint_as_float(sv[8 * c + 2 * k]), __uint_as_float(sv[8 * c + 2 * k + 1]), s[8 * c + 2 * k], s[8 * c + 2 * k + 1]);
         }
       }
-      const uint32_t used = masks[(n % kMlaMaskRing) * 2 + hf];
+      const uint32_t used = __ballot_sync(0xffffffffu, valid_s[(n % kMlaValidRing) * kMlaBlk + 32 * hf + lane]);
       if (used != 0xffffffffu) {                       // empty slots (the tail of a short row, holes): warp-uniform
 #pragma unroll
         for (int i = 0; i < 32; ++i) s[i] = (used >> i) & 1u ? s[i] : -CUDART_INF_F;
@@ -730,12 +703,12 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     // A full group of 128 heads leaves through shared memory and TMA stores: four [128 heads x 128 B] panels in the
     // (now idle) first two KV buffers, written asynchronously in whole lines.  16-byte stores from the threads -- every
     // lane its own 1 KB-strided row -- cost about 4 % of the kernel.
-    const bool by_tma = a.tma_out && a.n_split == 1 && heads_here == 128;
+    const bool by_tma = a.tma_out && part < 0 && heads_here == 128;
     // the row sum over all keys: the four threads of a head add theirs, relative to the later reference, through the idle
     // third KV buffer (every warp comes to the barrier, whatever became of its waits)
     float2* sum_s = reinterpret_cast<float2*>(kv_s + 2 * kMlaKBytes);
-    const int part = warp >> 2;                        // which quarter of the head's columns this thread writes
-    if (ok) sum_s[part * 128 + row] = make_float2(m, l);
+    const int quarter = warp >> 2;                     // which quarter of the head's columns this thread writes
+    if (ok) sum_s[quarter * 128 + row] = make_float2(m, l);
     named_bar_sync(3 + qd, 128);
     if (ok) {
       tc_fence_after();
@@ -750,11 +723,11 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       }
       const float inv = l > 0.f ? 1.f / l : 0.f;
       __nv_bfloat16* orow = a.out + ((int64_t)t * a.H + hg * 128 + row) * kMlaDv + cta * kMlaDvHalf;
-      const int64_t prow = (int64_t)unit * a.H + hg * 128 + row;
-      if (a.n_split > 1 && cta == 0 && part == 0 && row < heads_here)
+      const int64_t prow = (int64_t)part * a.H + hg * 128 + row;
+      if (part >= 0 && cta == 0 && quarter == 0 && row < heads_here)
         a.part_lse[prow] = l > 0.f ? mt + log2f(l) : -CUDART_INF_F;
 #pragma unroll 1
-      for (int c = part * (kMlaDvHalf / 4); c < (part + 1) * (kMlaDvHalf / 4); c += 32) {
+      for (int c = quarter * (kMlaDvHalf / 4); c < (quarter + 1) * (kMlaDvHalf / 4); c += 32) {
         uint32_t ov[32];
         tmem_ld32(t_row + kColO + c, ov);
         tmem_wait_ld();
@@ -770,7 +743,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
             w.w = pack_bf16x2(__uint_as_float(ov[i + 6]) * inv, __uint_as_float(ov[i + 7]) * inv);
             *reinterpret_cast<uint4*>(prow_s + (((ch0 + (i >> 3)) ^ (row & 7)) << 4)) = w;
           }
-        } else if (row < heads_here && a.n_split > 1) {
+        } else if (row < heads_here && part >= 0) {
           float4* po = reinterpret_cast<float4*>(a.part_o + prow * kMlaDv + cta * kMlaDvHalf + c);
 #pragma unroll
           for (int i = 0; i < 32; i += 4)
@@ -820,11 +793,11 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
 
 // out[t,h,:] = sum_s 2^(lse_s - M) o_s / sum_s 2^(lse_s - M): merges the parts of a split slot list.
 __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a) {
-  const int t = blockIdx.x, h = blockIdx.y;
+  const int u = blockIdx.x, t = a.n_full + u, h = blockIdx.y;
   float wgt[16];
   float mx = -CUDART_INF_F, den = 0.f;
   for (int sp = 0; sp < a.n_split; ++sp) {
-    wgt[sp] = a.part_lse[((int64_t)t * a.n_split + sp) * a.H + h];
+    wgt[sp] = a.part_lse[((int64_t)u * a.n_split + sp) * a.H + h];
     mx = fmaxf(mx, wgt[sp]);
   }
   for (int sp = 0; sp < a.n_split; ++sp) {
@@ -835,7 +808,7 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a
   const int d = threadIdx.x * 4;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int sp = 0; sp < a.n_split; ++sp) {
-    const float4 v = *reinterpret_cast<const float4*>(a.part_o + (((int64_t)t * a.n_split + sp) * a.H + h) * kMlaDv + d);
+    const float4 v = *reinterpret_cast<const float4*>(a.part_o + (((int64_t)u * a.n_split + sp) * a.H + h) * kMlaDv + d);
     acc.x += wgt[sp] * v.x; acc.y += wgt[sp] * v.y; acc.z += wgt[sp] * v.z; acc.w += wgt[sp] * v.w;
   }
   uint2 o;
@@ -858,16 +831,18 @@ static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaSt
   // 128 heads, no split, and the tensor can be mapped (16-byte aligned)
   a.tma_out = 0;
   to = tq;
-  if (a.n_split == 1 && a.H >= 128 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {
+  if (a.n_full > 0 && a.H >= 128 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) {
     if ((rc = make_tmap_2d_bytes(&to, a.out, (uint64_t)a.T * a.H, kMlaDv * 2, kMlaDv * 2, 128, 128))) return rc;
     a.tma_out = 1;
   }
   auto kern = sparse_mla_kernel<FP8_PAGED>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlaSmemBytes) != cudaSuccess)
-    return set_error(DSA_ERR_CUDA, "sparse_mla: cannot raise dynamic shared memory to %d", kMlaSmemBytes);
-  const dim3 grid(2 * a.T * a.n_split, 1, (a.H + 127) / 128);
-  kern<<<grid, MlaCfg<FP8_PAGED>::kThreads, kMlaSmemBytes, stream>>>(tq, to, a);
-  if (a.n_split > 1) sparse_mla_combine_kernel<<<dim3(a.T, a.H), 128, 0, stream>>>(a);
+  constexpr int smem_bytes = FP8_PAGED ? kMlaSmemDecode : kMlaSmemBytes;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
+    return set_error(DSA_ERR_CUDA, "sparse_mla: cannot raise dynamic shared memory to %d", smem_bytes);
+  const int n_parts = a.T - a.n_full;
+  const dim3 grid(2 * (a.n_full + n_parts * a.n_split), 1, (a.H + 127) / 128);
+  kern<<<grid, kMlaThreads, smem_bytes, stream>>>(tq, to, a);
+  if (n_parts > 0) sparse_mla_combine_kernel<<<dim3(n_parts, a.H), 128, 0, stream>>>(a);
   return check_launch("sparse_mla");
 }
 
@@ -880,24 +855,26 @@ int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx,
   a.T = T; a.H = H; a.K = K; a.S_kv = S_kv;
   a.scale_log2e = scale * 1.4426950408889634f;
   a.status = status;
+  a.n_full = T;
   a.n_split = 1;
   return launch_mla<false>(q, kv, a, stream);
 }
 
-// With few queries (decode) one CTA pair per query leaves most SMs idle and walks 2048 slots serially:
-// cut the slot list into parts of >= 256 slots while the grid still fits the GPU in one wave.  More
-// parts than that lose: every part pays the set-up again and writes an fp32 partial output that the
-// combine kernel reads back.
-int mla_decode_splits(int B, int H, int K) {
-  const int ctas = B * 2 * ((H + 127) / 128);
-  int ns = 1;
-  while (ns < 8 && ctas * ns * 2 <= sm_count() && K / (ns * 2) >= 256) ns *= 2;
-  return ns;
+// A CTA pair per query fills the GPU in rounds of (SMs / 2 / head groups) queries; the last, partly filled round would
+// take as long as a full one.  The queries of that round are cut into parts that share its pairs: as many as fit, at most
+// eight, of at least 256 slots.  More parts than that lose: every part pays the set-up again and writes an fp32 partial
+// output that the combine kernel reads back.  Batch 160 (two rounds and twelve queries in six parts each): 174 -> 156 us.
+struct MlaSplit { int n_full, n_split; };
+static MlaSplit mla_decode_split(int B, int H, int K) {
+  int pairs = sm_count() / (2 * ((H + 127) / 128));
+  if (pairs < 1) pairs = 1;
+  const int rest = B % pairs;
+  const int ns = rest == 0 ? 1 : min(min(8, K / 256), pairs / rest);
+  return ns > 1 ? MlaSplit{B - rest, ns} : MlaSplit{B, 1};
 }
 size_t mla_decode_workspace_bytes(int B, int H, int K) {
-  const int ns = mla_decode_splits(B, H, K);
-  if (ns <= 1) return 0;
-  return (size_t)B * ns * H * (kMlaDv + 1) * sizeof(float);
+  const MlaSplit sp = mla_decode_split(B, H, K);
+  return (size_t)(B - sp.n_full) * sp.n_split * H * (kMlaDv + 1) * sizeof(float);
 }
 
 int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* block_table, int64_t table_stride,
@@ -905,12 +882,14 @@ int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* bl
                              float scale, void* workspace, size_t workspace_bytes, int32_t* status,
                              cudaStream_t stream) {
   MlaArgs a{};
-  a.n_split = mla_decode_splits(B, H, K);
-  if (a.n_split > 1 && workspace && workspace_bytes >= mla_decode_workspace_bytes(B, H, K)) {
+  const MlaSplit sp = mla_decode_split(B, H, K);
+  a.n_full = B;
+  a.n_split = 1;
+  if (sp.n_split > 1 && workspace && workspace_bytes >= mla_decode_workspace_bytes(B, H, K)) {
+    a.n_full = sp.n_full;
+    a.n_split = sp.n_split;
     a.part_o = static_cast<float*>(workspace);
-    a.part_lse = a.part_o + (size_t)B * a.n_split * H * kMlaDv;
-  } else {
-    a.n_split = 1;
+    a.part_lse = a.part_o + (size_t)(B - sp.n_full) * sp.n_split * H * kMlaDv;
   }
   a.cache = static_cast<const uint8_t*>(cache);
   a.block_table = block_table;

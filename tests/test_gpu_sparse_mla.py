@@ -219,3 +219,24 @@ def test_prefill_whole_output_and_repeats(T, H):
         p = (torch.bmm(q[a:a + 64].double(), rows.transpose(1, 2)) * scale).softmax(-1)
         worst = max(worst, float((out[a:a + 64].double() - torch.bmm(p, rows[..., :512])).abs().max()))
     assert worst <= MAX_ABS, worst
+
+
+@pytest.mark.parametrize("B,H,K", [(74, 16, 512), (75, 128, 600), (80, 16, 2048), (111, 16, 700), (150, 40, 513), (37, 200, 640)])
+def test_decode_rounds_of_queries_with_a_split_remainder(B, H, K):
+    """Batches around whole rounds of CTA pairs: the queries of the last round are cut into parts and merged, the others
+    are not; both against the oracle, and against the call whose workspace is too small to split anything."""
+    g = torch.Generator().manual_seed(B + K)
+    P = 40
+    cache = O.pack_latent_cache(torch.randn(B * P * 64, 576, generator=g).to(torch.bfloat16))
+    table = torch.randperm(B * P, generator=g).int().view(B, P)
+    idx = torch.rand(B, P * 64, generator=g).topk(K, dim=-1).indices.int()
+    idx[B - 1, K // 3:] = -1                               # some parts of the last query are empty
+    idx[0, ::5] = -1
+    q = torch.randn(B, H, 576, generator=g).to(torch.bfloat16)
+    args = (q.cuda(), cache.cuda(), table.cuda(), idx.cuda(), 0.06)
+    out = ops.sparse_mla_decode_paged(*args)
+    one = ops.sparse_mla_decode_paged(*args, workspace=torch.empty(16, dtype=torch.uint8, device="cuda"))
+    ops.check_status("cuda")
+    assert float((out.float() - one.float()).abs().max()) <= MAX_ABS
+    rows = [0, 1, B // 2, B - 2, B - 1]
+    check(out[rows], O.sparse_mla_decode_paged(q[rows].float(), cache, table[rows], idx[rows], 0.06, round_bf16=True))

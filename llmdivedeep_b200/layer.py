@@ -410,8 +410,8 @@ def dsa_decode_step(q_idx_fp8, w, kcache, kscale, block_table, ctx_len, q, laten
     """One decode step for a batch of sequences: paged indexer scan, top-k over each sequence's
     context, sparse MLA over the paged FP8 latent cache.  Returns (idx, out) views of ``ws``."""
     B = q.shape[0]
+    idx, out = ws.idx[:B], ws.out[:B]
     logits = ops.fp8_paged_mqa_logits(q_idx_fp8, w, kcache, kscale, block_table, ctx_len, ws.max_ctx, out=ws.logits)
-    ops.topk_select(logits, ws.k, None, ctx_len, out=ws.idx[:B])
-    ops.sparse_mla_decode_paged(q, latent_cache, block_table, ws.idx[:B], softmax_scale, ws.max_ctx, out=ws.out[:B],
-                                workspace=ws.mla_ws)
-    return ws.idx[:B], ws.out[:B]
+    ops.topk_select(logits, ws.k, None, ctx_len, out=idx)
+    ops.sparse_mla_decode_paged(q, latent_cache, block_table, idx, softmax_scale, ws.max_ctx, out=out, workspace=ws.mla_ws)
+    return idx, out

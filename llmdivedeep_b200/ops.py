@@ -6,6 +6,7 @@ Nothing here computes on the CPU.
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Optional
 
 import torch
@@ -17,8 +18,18 @@ FP8 = torch.float8_e4m3fn
 _status = {}
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+# A call's host time is a few microseconds of launches; the generic torch helpers (device contexts, stream and device
+# objects) cost several times that, and small calls -- a decode step of one sequence, a cache write -- wait for the host.
+_NULL = contextlib.nullcontext()
+
+
+def _on(dev: torch.device):
+    """Context in which ``dev`` is the current device: nothing to do when it already is."""
+    return _NULL if torch._C._cuda_getDevice() == dev.index else torch.cuda.device(dev)
+
+
+def _stream(dev: torch.device) -> int:
+    return torch._C._cuda_getCurrentRawStream(dev.index)
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -55,10 +66,13 @@ def _dev_index(device) -> int:
 def status_word(device) -> torch.Tensor:
     """The per-device int32 the kernels report soft errors into (a device without an index means
     the current one)."""
-    key = _dev_index(device)
-    if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
-    return _status[key]
+    key = device.index if isinstance(device, torch.device) and device.type == "cuda" else None
+    if key is None:
+        key = _dev_index(device)
+    w = _status.get(key)
+    if w is None:
+        _status[key] = w = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
+    return w
 
 
 def check_status(device) -> None:
@@ -77,6 +91,12 @@ def _w_dtype(w: torch.Tensor) -> int:
     if w.dtype == torch.bfloat16:
         return 1
     raise DsaError(f"head weights must be fp32 or bf16, got {w.dtype}")
+
+
+def _flat_f32(t: torch.Tensor) -> torch.Tensor:
+    if t.dtype == torch.float32 and t.dim() == 1 and t.is_contiguous():
+        return t
+    return t.reshape(-1).to(torch.float32).contiguous()
 
 
 def _as_i32(t: Optional[torch.Tensor], n: int, name: str) -> Optional[torch.Tensor]:
@@ -120,7 +140,7 @@ def fp8_mqa_logits(q_fp8, kv, weights, ks, ke, clean_logits: bool = True,
     T, H, D = q_fp8.shape
     S = k_fp8.shape[0]
     q_fp8, k_fp8 = q_fp8.contiguous(), k_fp8.contiguous()
-    k_scale = k_scale.reshape(-1).to(torch.float32).contiguous()
+    k_scale = _flat_f32(k_scale)
     weights = weights.contiguous()
     if k_scale.numel() != S or tuple(weights.shape) != (T, H):
         raise DsaError("k_scale must have S entries and weights must be [T, H]")
@@ -134,10 +154,10 @@ def fp8_mqa_logits(q_fp8, kv, weights, ks, ke, clean_logits: bool = True,
     else:
         ld = out.stride(0)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_indexer_logits(_ptr(q_fp8), _ptr(k_fp8), _ptr(k_scale), _ptr(weights), _w_dtype(weights),
                                      _ptr(ks), _ptr(ke), _ptr(out), ld, T, S, H, D, int(bool(clean_logits)),
-                                     _ptr(status_word(q_fp8.device)), _stream()))
+                                     _ptr(status_word(dev)), _stream(dev)))
     return out[:T, :S]
 
 
@@ -158,18 +178,18 @@ def fp8_paged_mqa_logits(q_fp8, weights, kcache, kscale, block_table, ctx_len, m
         raise DsaError("block_table must be int32 [B, pages]")
     ctx_len = _as_i32(ctx_len, B, "ctx_len")
     q_fp8, kcache, weights = q_fp8.contiguous(), kcache.contiguous(), weights.contiguous()
-    kscale = kscale.reshape(-1).to(torch.float32).contiguous()
+    kscale = _flat_f32(kscale)
     ld = (max_ctx + 3) // 4 * 4
     if out is None:
         out = torch.empty(B, ld, dtype=torch.float32, device=q_fp8.device)
     else:
         ld = out.stride(0)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_indexer_logits_paged(_ptr(q_fp8), _ptr(weights), _w_dtype(weights), _ptr(kcache), _ptr(kscale),
                                            _ptr(block_table), block_table.stride(0), _ptr(ctx_len), _ptr(out), ld,
                                            B, H, D, kcache.shape[0] // 64, max_ctx,
-                                           _ptr(status_word(q_fp8.device)), _stream()))
+                                           _ptr(status_word(dev)), _stream(dev)))
     return out[:B, :max_ctx]
 
 
@@ -184,9 +204,9 @@ def topk_select(logits: torch.Tensor, k: int, ks=None, ke=None, out: Optional[to
     ke = _as_i32(ke, T, "ke")
     out = _check_idx_out(out, T, k, logits.device)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_topk_select(_ptr(logits), logits.stride(0) if T > 1 else max(S, logits.stride(0)), _ptr(ks),
-                                  _ptr(ke), T, S, k, _ptr(out), _stream()))
+                                  _ptr(ke), T, S, k, _ptr(out), _stream(dev)))
     return out
 
 
@@ -210,7 +230,7 @@ def indexer_topk(q_fp8, k_fp8, k_scale, weights, ks, ke, k: int, workspace: Opti
     S = k_fp8.shape[0]
     k = min(k, S)
     q_fp8, k_fp8, weights = q_fp8.contiguous(), k_fp8.contiguous(), weights.contiguous()
-    k_scale = k_scale.reshape(-1).to(torch.float32).contiguous()
+    k_scale = _flat_f32(k_scale)
     ks = _as_i32(ks, T, "ks")
     ke = _as_i32(ke, T, "ke")
     lib = _lib.load()
@@ -219,10 +239,10 @@ def indexer_topk(q_fp8, k_fp8, k_scale, weights, ks, ke, k: int, workspace: Opti
         row = full // max(T, 1)
         workspace = _workspace(q_fp8.device, min(full, max(max_workspace_bytes, 256 * row)))
     out = _check_idx_out(out, T, k, q_fp8.device)
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_indexer_topk(_ptr(q_fp8), _ptr(k_fp8), _ptr(k_scale), _ptr(weights), _w_dtype(weights),
                                    _ptr(ks), _ptr(ke), T, S, H, D, k, _ptr(out), _ptr(workspace), workspace.numel(),
-                                   _ptr(status_word(q_fp8.device)), _stream()))
+                                   _ptr(status_word(dev)), _stream(dev)))
     return out
 
 
@@ -244,10 +264,10 @@ def indexer_topk_static(q_fp8, k_fp8, k_scale, weights, ks, ke, k: int, out: Opt
     ke = _as_i32(ke, T, "ke")
     out = _check_idx_out(out, T, k, q_fp8.device)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_indexer_topk_static(_ptr(q_fp8), _ptr(k_fp8), _ptr(k_scale), _ptr(weights), _w_dtype(weights),
                                           _ptr(ks), _ptr(ke), T, S, H, D, k, _ptr(out),
-                                          _ptr(status_word(q_fp8.device)), _stream()))
+                                          _ptr(status_word(dev)), _stream(dev)))
     return out
 
 
@@ -263,9 +283,9 @@ def sparse_mla_prefill(q, kv, idx, scale: float, out: Optional[torch.Tensor] = N
     T, H, _ = q.shape
     out = _check_attn_out(out, (T, H, 512), q.device)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_sparse_mla_prefill(_ptr(q), _ptr(kv), _ptr(idx), _ptr(out), T, H, kv.shape[0], idx.shape[1],
-                                         float(scale), _ptr(status_word(q.device)), _stream()))
+                                         float(scale), _ptr(status_word(dev)), _stream(dev)))
     return out
 
 
@@ -285,9 +305,9 @@ def block_sparse_attn(q, k, v, lut, num, sm_scale: float, out: Optional[torch.Te
     if out is None:
         out = torch.empty_like(q)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_block_sparse_mha(_ptr(q), _ptr(k), _ptr(v), _ptr(lut), _ptr(num), _ptr(out), B, S, H, D,
-                                       lut.shape[3], float(sm_scale), _ptr(status_word(q.device)), _stream()))
+                                       lut.shape[3], float(sm_scale), _ptr(status_word(dev)), _stream(dev)))
     return out
 
 
@@ -309,11 +329,11 @@ def sparse_mla_decode_paged(q, cache, block_table, idx, scale: float, max_ctx: O
     if workspace is None:
         need = lib.dsa_sparse_mla_decode_workspace_bytes(B, H, idx.shape[1])
         workspace = _workspace(q.device, need) if need else None
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_sparse_mla_decode_paged(_ptr(q), _ptr(cache), _ptr(block_table), block_table.stride(0), _ptr(idx),
                                               _ptr(out), B, H, idx.shape[1], cache.shape[0] // 64, max_ctx, float(scale),
                                               _ptr(workspace), workspace.numel() if workspace is not None else 0,
-                                              _ptr(status_word(q.device)), _stream()))
+                                              _ptr(status_word(dev)), _stream(dev)))
     return out
 
 
@@ -456,9 +476,9 @@ def fp8_quant_per_block(x: torch.Tensor, block_size: int = 128):
     q = torch.empty(x.shape, dtype=FP8, device=x.device)
     scale = torch.empty(n_blocks, dtype=torch.float32, device=x.device)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_fp8_quant_per_block(_ptr(x), 1 if x.dtype == torch.bfloat16 else 0, n_blocks, block_size,
-                                          _ptr(q), _ptr(scale), _stream()))
+                                          _ptr(q), _ptr(scale), _stream(dev)))
     return q, (scale.view(x.shape[:-1]) if nb == 1 else scale.view(*x.shape[:-1], nb))
 
 
@@ -473,8 +493,8 @@ def pack_latent_records(kv: torch.Tensor, out: torch.Tensor) -> bool:
     if N and (cs != 1 or (N > 1 and (rs < 576 or rs * kv.element_size() % 16)) or (kv.data_ptr() | out.data_ptr()) % 16):
         return False
     lib = _lib.load()
-    with torch.cuda.device(kv.device):
-        check(lib.dsa_pack_latent_cache(_ptr(kv), 1 if kv.dtype == torch.bfloat16 else 0, rs, N, _ptr(out), _stream()))
+    with _on(kv.device):
+        check(lib.dsa_pack_latent_cache(_ptr(kv), 1 if kv.dtype == torch.bfloat16 else 0, rs, N, _ptr(out), _stream(kv.device)))
     return True
 
 
@@ -495,7 +515,7 @@ def rope_fp8_quant(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rope_d
     q = torch.empty(x.shape, dtype=FP8, device=x.device)
     scale = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on(dev):
         check(lib.dsa_rope_fp8_quant(_ptr(x), n_rows, D, rope_dim, int(bool(interleave)), rows_per_pos, _ptr(cos), _ptr(sin),
-                                     cos.shape[0], _ptr(q), _ptr(scale), _stream()))
+                                     cos.shape[0], _ptr(q), _ptr(scale), _stream(dev)))
     return q, scale

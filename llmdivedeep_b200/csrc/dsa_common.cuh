@@ -94,21 +94,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
 }
-// One look, by a whole warp that polls several barriers in turn.  test_wait and not try_wait: a try_wait that finds its
-// phase open suspends the warp, which then misses the other barriers (a polling loop of try_waits by 32 lanes ran the
-// sparse MLA kernel at a third of its speed).
-__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return __all_sync(0xffffffffu, ok != 0);
-}
-
 // ---- TMA (tiled bulk tensor copies, global -> this CTA's shared memory) ----
 __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, int y, uint64_t* bar) {
   asm volatile(

@@ -14,7 +14,8 @@
 //   * its five Q panels live in tensor memory as the A operand, so Q.K^T reads no shared memory for
 //     Q, and it computes a PARTIAL score tile S_c = Q_c K_c^T (18 tcgen05.mma kind::f16 of N = 64);
 //   * the two partial tiles ([128 heads x 64 keys], rounded to fp16 for the way: 16 KB) are exchanged
-//     through distributed shared memory, every warp sending its own 2 KB with one bulk copy.  Each
+//     through distributed shared memory, every warp sending its own 2 KB with one bulk copy (quadrants
+//     of tensor memory without heads stand by).  Each
 //     side adds what arrives to its own unrounded fp32 partial scores and runs the whole softmax; the
 //     two sides' P may differ in the last bit of an fp16 score, which is exact for each of them: a CTA
 //     normalises its half of O by the row sums of its own P.  fp16 carries 11 significant bits: an
@@ -123,10 +124,12 @@ __device__ __forceinline__ void cluster_arrive_wait() {
   cluster_arrive();
   cluster_wait();
 }
-// Arrive on the peer's barrier to say "I have READ the tile".  Relaxed on purpose: a release at cluster scope
-// costs a memory fence of thousands of cycles per block, and nothing written by this thread has to become
-// visible.  It orders nothing either: the caller must have consumed what it loaded (a value computed from all of it
-// stored or branched on) before it comes here.
+// Arrive on the peer's barrier to say "I have READ the tile".  Relaxed: a release at cluster scope costs a memory fence of
+// thousands of cycles per block, and nothing written by this thread has to become visible.  But a relaxed arrival orders
+// nothing, and straight after the loads it overtakes them -- they queue behind the gather's copies in the load/store unit,
+// and the next tile then lands on top of this one before it is read (seen: a few tokens in ten thousand).  The caller must
+// have stored or branched on a value computed from all that was loaded.  (A register-OR and warp reduction of the loaded
+// words as that value, to send the arrival earlier, cost more than it gained: 2228 -> 2280 us.)
 __device__ __forceinline__ void mbar_arrive_remote_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -248,6 +251,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const int k_lo = min(a.K, split * k_per), k_cnt = min(a.K, k_lo + k_per) - k_lo;
   const int32_t* idx_row = a.idx + (int64_t)t * a.K + k_lo;
   const int heads_here = min(128, a.H - hg * 128);
+  const int n_quad = (heads_here + 31) / 32;                   // quadrants of tensor memory with heads in them: the others' warps stand by
   // the five Q panels wait at the end of the KV buffers (from buffer kQBuf0 on) for their move into tensor memory
   constexpr int kQStage = NB * kMlaKBytes - kMlaPanels * kMlaQPanelBytes, kQBuf0 = kQStage / kMlaKBytes;
   static_assert(kQStage >= 0 && kQStage % 1024 == 0, "Q staging");
@@ -267,7 +271,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   if (warp == 0) {
     for (int i = lane; i < 59; i += 32) {
       const uint32_t count = i == 1 ? 16u                                            // q_moved: lane 0 of the softmax warps
-                             : (i == 3 || i == 4) ? 8u                               // s_free, p_full: lane 0 of a set's warps
+                             : (i == 3 || i == 4) ? 2u * n_quad                      // s_free, p_full: lane 0 of a set's warps
                              : (i >= 9 && i <= 16) ? 2u                              // pm_full: the two warps of a quadrant
                              : (i >= 49 && i <= 53) ? (FP8_PAGED ? uint32_t(kMlaGatherWarps) : kMlaGatherWarps * 33u)
                                                     : 1u;                            // the others
@@ -359,8 +363,6 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
         __syncwarp();
       };
-      int qk = 0, pv = 0;                              // next block to score, next block to accumulate
-      auto pv_ready = [&]() { return pv < qk && mbar_test_warp(p_full, pv & 1); };
       auto issue_qk = [&](int i) {
         fence_async_smem();                            // the rows were written by cp.async or st, the tensor core reads through the async proxy
         tc_fence_after();
@@ -380,27 +382,19 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
         __syncwarp();
       };
-      // Whatever is ready goes, P.V first: it is what frees a KV buffer (scores first: +1.5 %).  The arrival of the gathered
-      // rows, once seen, is not polled again.
-      uint32_t idle = 0;
-      bool rows_there = false;
-      while (ok && pv < nblk) {
-        if (qk < nblk && !rows_there) rows_there = mbar_test_warp(&kv_full[qk % NB], (qk / NB) & 1);
-        if (pv_ready()) {
-          pv_mmas(pv++);
-          idle = 0;
-        } else if (rows_there && (qk == 0 || mbar_test_warp(s_free, (qk - 1) & 1))) {
-          issue_qk(qk);
-          ++qk;
-          rows_there = false;
-          idle = 0;
-        } else if (++idle > kFastSpins) {              // bounded like every other wait (dsa_common.cuh)
-          if (__any_sync(0xffffffffu, *abort_flag)) ok = false;
-          else if (idle > kSpinLimit) {
-            *abort_flag = 1;
-            if (a.status && lane == 0) atomicCAS(a.status, kStatusOk, kStatusWaitTimeout);
-            ok = false;
-          } else __nanosleep(40);
+      // A fixed order: P.V two blocks behind the scores is about when its P is there, and what a KV buffer's round trip has
+      // time for.  (Whatever is ready first, by polling three barriers: the same speed, and every look costs ~100 cycles.)
+      for (int n = 0; n < nblk + 2 && ok; ++n) {
+        if (n < nblk) {
+          ok = mbar_wait_warp(&kv_full[n % NB], (n / NB) & 1, abort_flag, a.status);
+          if (ok && n > 0) ok = mbar_wait_warp(s_free, (n - 1) & 1, abort_flag, a.status);
+          if (!ok) break;
+          issue_qk(n);
+        }
+        if (n >= 2) {
+          ok = mbar_wait_warp(p_full, n & 1, abort_flag, a.status);
+          if (!ok) break;
+          pv_mmas(n - 2);
         }
       }
     }
@@ -574,8 +568,9 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
     cluster_wait();
     // this warp's part of the set's partial tile: 32 heads x 32 keys, 2 KB
-    uint8_t* send = send_s + (hf * 4 + qd) * kMlaXWarp;
-    const uint8_t* recv = recv_s + (hf * 4 + qd) * kMlaXWarp;
+    const int xw = hf * 4 + qd;
+    uint8_t* send = send_s + xw * kMlaXWarp;
+    const uint8_t* recv = recv_s + xw * kMlaXWarp;
     const uint32_t peer_recv = mapa_u32(smem_u32(recv), peer);
     // block maxima, four blocks deep: a warp may be two blocks behind its partner, never four (P.V orders them)
     auto pm_of = [&](int blk) -> uint16_t* { return pm_s + (blk & 3) * 256 + row; };      // [key half][head]
@@ -583,7 +578,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     auto pair_max = [&](const uint16_t* pm) {
       return fmaxf(__uint_as_float(uint32_t(pm[0]) << 16), __uint_as_float(uint32_t(pm[128]) << 16));
     };
-    for (int n = set; n < nblk && ok; n += 2) {
+    if (qd < n_quad && set < nblk && lane == 0) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
+    for (int n = qd < n_quad ? set : nblk; n < nblk && ok; n += 2) {
       const uint32_t ph = (n >> 1) & 1;
       uint32_t sv[32];                                 // this CTA's partial scores
       ok = mbar_wait_warp(&s_full[set], ph, abort_flag, a.status);
@@ -599,17 +595,13 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         if (!ok) break;
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-      {
+      for (int c = 0; c < 4; ++c) {
         auto h2 = [&](int k) { return pack_f16x2(__uint_as_float(sv[8 * c + 2 * k]), __uint_as_float(sv[8 * c + 2 * k + 1])); };
         *reinterpret_cast<uint4*>(send + xchg_off(lane, c)) = make_uint4(h2(0), h2(1), h2(2), h2(3));
       }
       fence_async_smem();                              // the bulk copy reads the tile through the async proxy
       __syncwarp();
-      if (elect_one()) {
-        mbar_expect_tx(&recv_full[warp], kMlaXWarp);   // the peer's block n-2 has been read: arm the stage again
-        bulk_copy_to_peer(peer_recv, send, kMlaXWarp, peer_recv_full);
-      }
+      if (elect_one()) bulk_copy_to_peer(peer_recv, send, kMlaXWarp, peer_recv_full);
       __syncwarp();
       // the reference of the block before, from that block's maxima: every thread follows the whole sequence by itself
       if (n > 0) {
@@ -644,10 +636,9 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (lane == 0) {
         mbar_arrive(&pm_full[set * 4 + qd]);
         // The peer may send into this stage again.  Only here: the block maximum just stored needed every value of the tile,
-        // so the loads have returned.  Straight after the loads the arrival can overtake them -- they queue behind the
-        // gather's copies in the load/store unit, and the next tile then landed on top of this one before it was read
-        // (a few tokens in ten thousand).
+        // so the loads have returned.
         mbar_arrive_remote_relaxed(peer_xchg_free);
+        if (n + 2 < nblk) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
       }
       ok = mbar_wait_warp(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
       if (!ok) break;

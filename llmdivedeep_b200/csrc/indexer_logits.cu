@@ -827,6 +827,19 @@ int make_tmap_2d_u8(CUtensorMap* m, const void* base, uint64_t rows, uint32_t ro
   return make_tmap_2d_bytes(m, base, rows, row_bytes, row_pitch, row_bytes, box_rows);
 }
 
+// Key tiles per work unit.  Units are dealt to the CTAs round-robin: keep at least six rounds of them so that the last,
+// partly filled round costs little, by cutting the key range finer when there are few query blocks -- down to eight tiles,
+// below which a unit's own start shows.  A call that would leave SMs without a unit goes on cutting, to single tiles if need
+// be: a start on an idle SM costs nothing (2048 rows x 2048 keys of 4 heads x 64: 32 units of eight tiles took 63.0 us, 30.7 with 256 units of one;
+// one sequence of 2000 tokens, paged: one unit 9.8 us, four 6.0; seven of 33000: 63 units 15.0 us, 119 units 12.0).
+static int pick_chunk_tiles(int n_qblocks, int n_tiles) {
+  auto units = [&](int chunk) { return (int64_t)n_qblocks * ((n_tiles + chunk - 1) / chunk); };
+  int chunk = kChunkTiles;
+  while (chunk > 8 && units(chunk) < 6LL * sm_count()) chunk /= 2;
+  while (chunk > 1 && units(chunk) < sm_count()) chunk /= 2;
+  return chunk;
+}
+
 template <int H, int D, int NQ, bool PAGED, int QB, int EPI>
 static int launch_indexer(const void* q, const void* k, const IndexerArgs& args, int clean, cudaStream_t stream) {
   using C = IdxCfg<H, D, NQ, PAGED, QB, EPI>;
@@ -841,12 +854,7 @@ static int launch_indexer(const void* q, const void* k, const IndexerArgs& args,
   const int n_groups = (a.T + NQ - 1) / NQ;
   const int n_qblocks = (n_groups + QB - 1) / QB;
   const int n_tiles = (a.S + C::TILE_KEYS - 1) / C::TILE_KEYS;
-  // Units are dealt to the CTAs round-robin: keep at least six rounds of them so that the last, partly
-  // filled round costs little, by cutting the key range finer when there are few query blocks.
-  a.chunk_tiles = kChunkTiles;
-  while (a.chunk_tiles > 8 &&
-         (int64_t)n_qblocks * ((n_tiles + a.chunk_tiles - 1) / a.chunk_tiles) < 6LL * sm_count())
-    a.chunk_tiles /= 2;
+  a.chunk_tiles = pick_chunk_tiles(n_qblocks, n_tiles);
   const int n_chunks = (n_tiles + a.chunk_tiles - 1) / a.chunk_tiles;
   const int64_t n_units64 = (int64_t)n_qblocks * n_chunks;
   if (n_units64 > 0x7fffffff) return set_error(DSA_ERR_SHAPE, "indexer: too many work units");
@@ -874,9 +882,7 @@ static int launch_indexer_rw(const void* q, const void* k, const IndexerArgs& ar
   if (rc) return rc;
   const int n_groups = (a.T + C::NQ - 1) / C::NQ;
   const int n_tiles = (a.S + kTileKeys - 1) / kTileKeys;
-  a.chunk_tiles = kChunkTiles;                      // same rule as the general form: at least six rounds of units
-  while (a.chunk_tiles > 8 && (int64_t)n_groups * ((n_tiles + a.chunk_tiles - 1) / a.chunk_tiles) < 6LL * sm_count())
-    a.chunk_tiles /= 2;
+  a.chunk_tiles = pick_chunk_tiles(n_groups, n_tiles);
   const int64_t n_units64 = (int64_t)n_groups * ((n_tiles + a.chunk_tiles - 1) / a.chunk_tiles);
   if (n_units64 > 0x7fffffff) return set_error(DSA_ERR_SHAPE, "indexer: too many work units");
   const int n_units = (int)n_units64;

@@ -149,3 +149,9 @@ def test_quantiser_ragged_block_counts_and_unaligned_output(n_blocks, block):
                                                        torch.cuda.current_stream().cuda_stream))
         assert torch.equal(q[off:off + n_blocks * block].cpu(), want_q.view(torch.uint8).reshape(-1)) and not q[off + n_blocks * block:].any()
         assert torch.equal(s[:n_blocks].cpu(), want_s.reshape(-1)) and float(s[n_blocks]) == 0
+
+
+@pytest.mark.parametrize("B,P,H", [(1, 1, 64), (1, 8, 64), (1, 9, 64), (1, 33, 16), (7, 66, 64), (150, 9, 64)])
+def test_paged_logits_of_calls_with_few_tiles(B, P, H):
+    """Calls too small to give every SM a unit of eight tiles: units of four, two and one tile."""
+    test_paged_logits_match_oracle(B, P, H)

@@ -198,3 +198,9 @@ def test_register_weight_form_equals_general_kernel_bitwise(T, S, window):
         b = bfull[:, :S]
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
     ops.check_status("cuda")
+
+
+@pytest.mark.parametrize("T,S,H,D", [(1, 129, 64, 128), (3, 2048, 64, 128), (130, 1000, 4, 64), (2048, 2048, 4, 64), (40, 3000, 16, 128)])
+def test_logits_of_calls_with_few_tiles(T, S, H, D):
+    """Calls too small to give every SM a unit of eight tiles: units of four, two and one tile."""
+    test_logits_match_oracle(T, S, H, D, "causal")

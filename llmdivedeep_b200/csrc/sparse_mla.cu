@@ -31,7 +31,7 @@
 // (a warp keeps about eight 512-byte requests going, whether cp.async or TMA gather4), arrivals by the copies themselves.
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137
 // cycles each; see dsa_common.cuh) and TMA gather; 3125 with warp-uniform issue; 2860 with two sets of softmax warps;
-// 2418 with sixteen and setmaxnreg; 2228 as it stands (1049 TFLOP/s).  Tried on top: the exchange by st.async (3320:
+// 2418 with sixteen and setmaxnreg; 2215 as it stands (1055 TFLOP/s).  Tried on top: the exchange by st.async (3320:
 // the stores drain slowly and clog the gather), by loads from the peer's shared memory (3560: the release at cluster
 // scope costs ~2300 cycles), a quarter of the exponentials as polynomials on the FMA pipe (+3 %: the issue slots are
 // short too).
@@ -42,6 +42,10 @@
 // block maxima through shared memory (rounded up to bf16: any common reference point is exact for a softmax); from the
 // maxima of all blocks in order every thread follows the running reference by itself, so that one set can run ahead of
 // the other; row sums stay per thread until the end.
+// Of the 71000 cycles a token takes, 54000 are its blocks; the rest is start, Q, first rows (6300), the last softmax, P.V,
+// output and the pair's exit (7500) and the relaunch (1600).  Persistent pairs that run ahead into the next token were built
+// and dropped (2710): without a panel of free shared memory Q and the output move by 16-byte accesses a row apart (7400
+// and 8000 cycles), and the two CTAs drift against each other.
 // Decode, batch 64 (a call, launch included): 105 us with eight gather warps that met at two barriers per block, 72 us with
 // eleven that never wait for one another.  Loads into registers one block ahead in place of the raw stages: 94 us (the rows
 // take about 3000 cycles to come).  The gather then costs issue slots, about as many as the softmax.
@@ -120,10 +124,6 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t cta) {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive_wait() {
-  cluster_arrive();
-  cluster_wait();
-}
 // Arrive on the peer's barrier to say "I have READ the tile".  Relaxed: a release at cluster scope costs a memory fence of
 // thousands of cycles per block, and nothing written by this thread has to become visible.  But a relaxed arrival orders
 // nothing, and straight after the loads it overtakes them -- they queue behind the gather's copies in the load/store unit,
@@ -237,7 +237,6 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   uint64_t* kv_free = bars + 54;                     // [5] P.V of the block finished: its KV buffer is free
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 59);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* last_s = const_cast<int*>(abort_flag) + 1;
   uint8_t* valid_s = reinterpret_cast<uint8_t*>(bars) + kMlaBarBytes;       // [kMlaValidRing][64] 1 = the slot of the block is in use
   uint16_t* pm_s = reinterpret_cast<uint16_t*>(valid_s + kMlaValidRing * kMlaBlk);          // block maxima, rounded up to bf16
 
@@ -258,14 +257,12 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   auto q_stage = [&](int lp) -> uint8_t* { return kv_s + kQStage + lp * kMlaQPanelBytes; };
 
   // ---- set-up, arranged so that nothing waits for anything it does not need ------------------------------------
-  // every thread requests its share of the slot list first (the scan below decides the number of key blocks) ...
-  constexpr int kScan = 4;
-  int pos[kScan];
-#pragma unroll
-  for (int u = 0; u < kScan; ++u) {
-    const int j = threadIdx.x + u * kMlaThreads;
-    pos[u] = j < k_cnt ? __ldg(idx_row + j) : -1;
-  }
+  // every warp requests the last 32 slots of the list (they decide the number of key blocks) and the gather warps their
+  // slots of the first block ...
+  const int tail_j = k_cnt - 32 + lane;
+  const int tail = tail_j >= 0 ? __ldg(idx_row + tail_j) : -1;
+  const int slot = warp >= kMlaGatherWarp0 && lane < kRawRows ? warp - kMlaGatherWarp0 + lane * kMlaGatherWarps : kMlaBlk;
+  const int slot_pos = slot < kMlaBlk && slot < k_cnt ? __ldg(idx_row + slot) : -1;
   // ... while warp 0 initialises the barriers (one per lane) and sends for Q (one panel per lane) and the MMA warp allocates
   // tensor memory
   if (warp == 0) {
@@ -278,10 +275,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       mbar_init(bars + i, count);
     }
     mbar_fence_init();
-    if (lane == 0) {
-      *abort_flag = 0;
-      *last_s = -1;
-    }
+    if (lane == 0) *abort_flag = 0;
     __syncwarp();
     if (lane == 0) mbar_expect_tx(q_full, kMlaPanels * kMlaQPanelBytes);
     __syncwarp();
@@ -296,19 +290,28 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  {  // the last usable slot decides the number of key blocks (the same number in both CTAs of the pair)
-    int last = -1;
+  // the last usable slot decides the number of key blocks (the same number in both CTAs of the pair): it is among the last 32
+  // but for short rows, where every warp looks further back
+  int nblk;
+  {
+    int end = k_cnt;
+    uint32_t hit = __ballot_sync(0xffffffffu, tail >= 0 && tail < a.S_kv);
+    while (hit == 0 && end > 32) {
+      int p[4];
 #pragma unroll
-    for (int u = 0; u < kScan; ++u)
-      if (pos[u] >= 0 && pos[u] < a.S_kv) last = threadIdx.x + u * kMlaThreads;
-    for (int j = threadIdx.x + kScan * kMlaThreads; j < k_cnt; j += kMlaThreads) {      // longer slot lists: none today (K <= 2048)
-      const int p = idx_row[j];
-      if (p >= 0 && p < a.S_kv) last = j;
+      for (int v = 0; v < 4; ++v) {                    // four looks at a time
+        const int j = end - 32 * (v + 2) + lane;
+        p[v] = j >= 0 ? __ldg(idx_row + j) : -1;
+      }
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        if (hit != 0) break;
+        end -= 32;
+        hit = __ballot_sync(0xffffffffu, p[v] >= 0 && p[v] < a.S_kv);
+      }
     }
-    if (last >= 0) atomicMax(last_s, last);
+    nblk = hit == 0 ? 0 : (end - 1 - __clz(hit)) / kMlaBlk + 1;
   }
-  __syncthreads();
-  const int nblk = (*last_s + kMlaBlk) / kMlaBlk;
   if (nblk == 0) {   // nothing selected: the output row is zero (a part: weight zero in the combine); no cluster traffic yet
     if (threadIdx.x < 128 && threadIdx.x < heads_here) {
       if (part < 0) {
@@ -333,6 +336,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   // talk to the peer (softmax) wait before their first remote access, the others only before they leave, so that the
   // round trip through the cluster barrier is off the path to the first MMA.
   cluster_arrive();
+  bool left = false;                                           // this warp has arrived at the barrier that the pair leaves through
 
   if (warp >= kMlaSoftmaxWarps) regs_dec<MlaRegs<FP8_PAGED>::kOther>();
   else regs_inc<MlaRegs<FP8_PAGED>::kSoftmax>();
@@ -404,7 +408,6 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     constexpr int kG = kMlaGatherWarps;
     bool ok = true;
     // A warp fetches every kG-th slot of a block, six at most: lane j < 6 keeps the id of slot w4 + 11 j.
-    const int slot = lane < kRawRows ? w4 + lane * kG : kMlaBlk;
     auto load_pos = [&](int blk) -> int {
       const int j = blk * kMlaBlk + slot;
       return (slot < kMlaBlk && blk < nblk && j < k_cnt) ? __ldg(idx_row + j) : -1;
@@ -417,7 +420,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // of all six rows another one.  Nobody waits for the copies here: they arrive on the block's barrier by themselves,
       // and the MMA warp orders them before the tensor core's reads (a proxy fence anywhere on the path between the two
       // will do).
-      int nxt = load_pos(0);
+      int nxt = slot_pos;
       const uint8_t* src_lat = a.kv + cta * (kMlaDvHalf * 2) + lane * 16;
       const uint8_t* src_rope = a.kv + kMlaDv * 2 + cta * 64 + (lane & 3) * 16;
       for (int i = 0; i < nblk; ++i) {
@@ -491,7 +494,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // row ids of blocks i and i+1 (which of them are used), page-table entry and position of i+2, position of i+3
       int id_cur, id_nxt, pa, ta, pb;
       {
-        const int p0 = load_pos(0), p1 = load_pos(1);
+        const int p0 = slot_pos, p1 = load_pos(1);
         pa = load_pos(2);
         pb = load_pos(3);
         const int t0 = table_entry(p0), t1 = table_entry(p1);
@@ -690,6 +693,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
+    if (ok) cluster_arrive();                          // nothing remote is left to do for this warp: the others need not wait for its output
+    left = ok;
     if (ok) ok = mbar_wait_warp(o_final, 0, abort_flag, a.status);
     // A full group of 128 heads leaves through shared memory and TMA stores: four [128 heads x 128 B] panels in the
     // (now idle) first two KV buffers, written asynchronously in whole lines.  16-byte stores from the threads -- every
@@ -754,13 +759,12 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       }
     }
     if (by_tma) {                                      // every softmax thread comes here, whatever became of its waits
-      fence_async_smem();                              // the stores below read the panels through the async proxy
-      named_bar_sync(7, 512);
-      if (threadIdx.x == 0 && !*abort_flag) {
-#pragma unroll
-        for (int pn = 0; pn < 4; ++pn)                 // x in 4-byte units: 32 per 64-column panel
-          tma_store_2d(&tmap_o, kv_s + pn * kMlaQPanelBytes, (cta * 4 + pn) * 32, t * a.H + hg * 128);
-        bulk_commit_and_wait_read();                   // the panels have been read: the CTA may go
+      // a quarter of the columns is one panel and four warps: it leaves as soon as they have written it
+      fence_async_smem();                              // the store below reads the panel through the async proxy
+      named_bar_sync(7 + quarter, 128);
+      if ((warp & 3) == 0 && elect_one() && !*abort_flag) {         // x in 4-byte units: 32 per 64-column panel
+        tma_store_2d(&tmap_o, kv_s + quarter * kMlaQPanelBytes, (cta * 4 + quarter) * 32, t * a.H + hg * 128);
+        bulk_commit_and_wait_read();                   // the panel has been read: the CTA may go
       }
     }
   }
@@ -775,7 +779,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       for (int w = 0; w < 64; ++w) __nanosleep(1000);
     __syncthreads();
   }
-  cluster_arrive_wait();          // neither CTA leaves while the other may still copy into it or arrive on its barriers
+  if (!left) cluster_arrive();
+  cluster_wait();                 // neither CTA leaves while the other may still copy into it or arrive on its barriers
   if (warp == kMlaMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem, kMlaTmemCols);

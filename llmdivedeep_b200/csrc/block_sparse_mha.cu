@@ -12,16 +12,24 @@
 //   * warps 0 and 2: TMA producers (Q and K; V).  Q [64 x 128] once per unit, then per listed key block K and
 //     V [64 x 128], each as two 128-byte-swizzled panels of 64 dims, into a 3-stage K ring and a 2-stage V ring;
 //     32 list entries are read at a time, one per lane.
-//   * warp 1: owns the tensor memory; lane 0 issues S = Q K^T (8 tcgen05.mma kind::f16, K-major
+//   * warp 1: owns the tensor memory; one elected lane issues S = Q K^T (8 tcgen05.mma kind::f16, K-major
 //     operands) into one of two score buffers, up to two blocks ahead of the softmax, and O += P V
 //     (4 MMAs; P from shared memory, V read through an MN-major descriptor, so the [key][dim] tile needs
 //     no transpose).  It polls "next K landed and its score buffer read" and "this block's P and V
-//     ready" together, so neither a late K tile nor a slow softmax leaves the tensor pipe idle.
-//   * warps 4-7: online softmax.  Scores come from tensor memory; a row (lanes 0-15 of the quadrant) is
-//     split over a lane pair -- lane r keeps columns 0-31, lane r+16 receives 32-63 by shuffle -- so all
-//     32 lanes compute; P goes to one of two shared-memory buffers as bf16 in the K-major swizzled
-//     layout; the running maximum is raised (and O rescaled in tensor memory) only when it grows by
-//     more than 8 in log2 units.
+//     ready" together, so neither a late K tile nor a slow softmax leaves the tensor pipe idle.  The role is
+//     chosen from a warp-uniform index and the lane by elect.sync: with the role from threadIdx and `lane == 0` the
+//     compiler cannot keep an MMA's descriptors in uniform registers and each issue costs over 100 cycles, more than
+//     the MMA itself.
+//   * warps 4-7: online softmax on 16 rows each.  The 16x256b form of tcgen05.ld hands every lane 16 columns of two
+//     rows, so no lane idles and nothing is moved between lanes but the four-lane maximum; P goes to one of two
+//     shared-memory buffers as bf16 through stmatrix, in the K-major swizzled layout; sums stay with the lane until
+//     the unit ends; the running maximum is raised (and O rescaled in tensor memory) only when it grows by more than
+//     8 in log2 units.  The output takes the same way out, through the P buffers, as whole 256-byte rows.
+// What bounds it: the tensor pipe (an M = 64 MMA takes as long as an M = 128 one: 8 x 50 + 4 x 64 cycles a block, two
+// CTAs share the pipe).  Measured, 24 heads, 5% of the key blocks: 16384 tokens 398 us with lane-0 issue and a
+// lane-per-row softmax (32x32b loads, 32 shuffles a block, 256-byte rows stored 16 bytes a lane), 352 us with uniform
+// issue, 265 us with the 16x256b fragments as well; 32768 tokens 1293 -> 1096 -> 901 us.  The tensor pipe alone would
+// take 183 us at 16384 tokens.
 // Every wait is bounded (dsa_common.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -64,6 +72,45 @@ __device__ __forceinline__ float bs_exp2(float x) {
   return r;
 }
 
+// An M = 64 accumulator keeps its rows in lanes 0-15 of each quadrant.  The 16x256b load spreads them over the whole warp, like
+// the fragments of mma: of every 8 columns i, lane t gets columns 2 (t % 4), + 1 of row t / 4 (registers 4 i, 4 i + 1) and of
+// row t / 4 + 8 (4 i + 2, 4 i + 3).
+__device__ __forceinline__ void bs_tmem_ld(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void bs_tmem_st(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+      "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+      "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+// 16 rows x 64 columns in those fragments, packed to bf16 pairs (w[2 i]: row t / 4, w[2 i + 1]: row t / 4 + 8), into rows
+// row0.. of a 128-byte-swizzled panel
+__device__ __forceinline__ void bs_store_rows(uint8_t* panel, int row0, int lane, const uint32_t (&w)[16]) {
+  const int r = row0 + (lane & 15);                     // lanes 0-7 / 8-15: rows of the two halves, 16-31: the next 8 columns
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    const int c = i + (lane >> 4);
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(smem_u32(panel + r * 128 + ((c ^ (r & 7)) << 4))), "r"(w[2 * i]), "r"(w[2 * i + 1]), "r"(w[2 * i + 2]), "r"(w[2 * i + 3])
+                 : "memory");
+  }
+}
+
 __global__ void __launch_bounds__(kBsThreads, 2)
 block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                         const __grid_constant__ CUtensorMap tmap_v, const BsArgs a, const int n_units) {
@@ -88,7 +135,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int nkb = a.S / kBsBlk;
   const int list_cap = a.topk;
 
@@ -96,7 +143,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
     mbar_init(o_final, 1);
-    mbar_init(o_free, 128);
+    mbar_init(o_free, 4);
     for (int i = 0; i < kBsKStages; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_free[i], 1);
@@ -106,8 +153,8 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       mbar_init(&v_free[i], 1);
       mbar_init(&pv_done[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 128);
-      mbar_init(&p_full[i], 128);
+      mbar_init(&s_free[i], 4);
+      mbar_init(&p_full[i], 4);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -196,7 +243,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc(1, 1, 0, 0, 64, kBsBlk);
       constexpr uint32_t idesc_pv = umma_idesc(1, 1, 0, 1, 64, kBsD);
       const uint64_t qdesc = umma_smem_desc(smem_u32(q_s), 16, 1024, kSwz128);
@@ -274,10 +321,8 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       }
     }
   } else if (warp >= 4) {
-    // ---------------------- softmax and output (lanes 0-15 of each warp hold rows) ----------------------
+    // ---------------------- softmax and output: 16 rows per warp, two rows (a, b) and 16 of 64 columns per lane ----------------------
     const int quad = warp - 4;
-    const bool active = lane < 16;
-    const int row = quad * 16 + (lane & 15);                  // query row of the block (lanes 16-31 shadow lanes 0-15)
     const uint32_t t_row = tmem + (uint32_t(quad * 32) << 16);
     uint32_t nq = 0, jt = 0;
     bool ok = true;
@@ -285,114 +330,128 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       const int n = unit_len(u);
       int b, h, qb;
       decode(u, b, h, qb);
-      __nv_bfloat16* orow = a.out + (((int64_t)b * a.S + qb * kBsBlk + row) * a.H + h) * kBsD;
+      // output: 16 lanes write one row's 256 bytes, two rows per instruction
+      uint8_t* out0 = reinterpret_cast<uint8_t*>(a.out + (((int64_t)b * a.S + qb * kBsBlk + quad * 16) * a.H + h) * kBsD) + (lane & 15) * 16;
+      const int64_t pitch = (int64_t)a.H * kBsD * 2;
       if (n == 0) {                                           // nothing listed: zero rows
-        if (active)
-          for (int c = 0; c < kBsD * 2 / 16; ++c) reinterpret_cast<uint4*>(orow)[c] = make_uint4(0, 0, 0, 0);
+        for (int r = lane >> 4; r < 16; r += 2) *reinterpret_cast<uint4*>(out0 + r * pitch) = make_uint4(0, 0, 0, 0);
         continue;
       }
       const int32_t* list = a.lut + (int64_t)u * a.topk;
-      float m = -CUDART_INF_F, l = 0.f;
+      float m_a = -CUDART_INF_F, m_b = -CUDART_INF_F, l_a = 0.f, l_b = 0.f;     // sums: this lane's columns only
       for (int j = 0; j < n && ok; ++j, ++jt) {
         const int kb = __ldg(list + j);                       // requested before the wait: only its validity is needed
         ok = __all_sync(0xffffffffu, mbar_wait(&s_full[jt & 1], (jt >> 1) & 1, abort_flag, a.status));
         if (!ok) break;
         tc_fence_after();
-        uint32_t sv[kBsBlk];
-        tmem_ld32(t_row + kBsColS + (jt & 1) * kBsBlk, *reinterpret_cast<uint32_t(*)[32]>(sv));
-        tmem_ld32(t_row + kBsColS + (jt & 1) * kBsBlk + 32, *reinterpret_cast<uint32_t(*)[32]>(sv + 32));
+        uint32_t sv[32];
+        bs_tmem_ld(t_row + kBsColS + (jt & 1) * kBsBlk, sv);
         tmem_wait_ld();
         tc_fence_before();
-        mbar_arrive(&s_free[jt & 1]);
-        const bool listed = kb >= 0 && kb < nkb;
-        // An M = 64 accumulator keeps its rows in lanes 0-15 of the quadrant, so lanes 16-31 would idle (and
-        // pay for 64 exponentials of garbage).  Each row is split instead: lane r keeps columns 0-31, lane
-        // r + 16 receives columns 32-63 by shuffle; maximum and sum are combined across the pair.
-        float x[kBsBlk / 2];                           // raw scores; the (positive) scale is folded into the exponent's FMA
-        float bmax = -CUDART_INF_F;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[jt & 1]);
+        if (!(kb >= 0 && kb < nkb)) {                  // a bad list entry (uniform, rare): the whole block is masked
 #pragma unroll
-        for (int i = 0; i < kBsBlk / 2; ++i) {
-          const uint32_t hi = __shfl_sync(0xffffffffu, sv[kBsBlk / 2 + i], lane & 15);
-          x[i] = __uint_as_float(active ? sv[i] : hi);
-          bmax = fmaxf(bmax, x[i]);
+          for (int i = 0; i < 32; ++i) sv[i] = __float_as_uint(-CUDART_INF_F);
         }
-        if (!listed) {                                 // a bad list entry (uniform, rare): the whole block is masked
+        float x_a = -CUDART_INF_F, x_b = -CUDART_INF_F;      // raw scores; the (positive) scale is folded into the exponent's FMA
 #pragma unroll
-          for (int i = 0; i < kBsBlk / 2; ++i) x[i] = -CUDART_INF_F;
-          bmax = -CUDART_INF_F;
+        for (int i = 0; i < 32; i += 4) {
+          x_a = fmaxf(x_a, fmaxf(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])));
+          x_b = fmaxf(x_b, fmaxf(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])));
         }
-        bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 16)) * a.scale_log2e;
-        const float m_new = fmaxf(m, bmax);
-        const bool grow = m_new - m > 8.f;             // also true when m is still -inf and m_new is finite
-        if (__any_sync(0xffffffffu, grow)) {
-          const float alpha = grow ? bs_exp2(m - m_new) : 1.f;
-          if (grow) m = m_new;
-          l *= alpha;
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {              // a row is spread over four lanes
+          x_a = fmaxf(x_a, __shfl_xor_sync(0xffffffffu, x_a, o));
+          x_b = fmaxf(x_b, __shfl_xor_sync(0xffffffffu, x_b, o));
+        }
+        x_a *= a.scale_log2e;
+        x_b *= a.scale_log2e;
+        const bool grow_a = x_a - m_a > 8.f, grow_b = x_b - m_b > 8.f;      // also true when m is still -inf and x is finite
+        if (__any_sync(0xffffffffu, grow_a || grow_b)) {
+          const float f_a = grow_a ? bs_exp2(m_a - x_a) : 1.f, f_b = grow_b ? bs_exp2(m_b - x_b) : 1.f;
+          if (grow_a) m_a = x_a;
+          if (grow_b) m_b = x_b;
+          l_a *= f_a;
+          l_b *= f_b;
           if (j > 0) {                                 // O must be quiescent: P.V of the previous block complete
             ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[(jt - 1) & 1], ((jt - 1) >> 1) & 1, abort_flag, a.status));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll 1
-            for (int c = 0; c < kBsD; c += 32) {       // lanes 0-15 scale their rows; the shadow lanes' rows are unused
+            for (int c = 0; c < kBsD; c += 64) {
               uint32_t ov[32];
-              tmem_ld32(t_row + kBsColO + c, ov);
+              bs_tmem_ld(t_row + kBsColO + c, ov);
               tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-              tmem_st32(t_row + kBsColO + c, ov);
+              for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * ((i & 2) ? f_b : f_a));
+              bs_tmem_st(t_row + kBsColO + c, ov);
             }
             tmem_wait_st();
           }
         }
-        const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
-        uint32_t pk[kBsBlk / 4];
-        float psum = 0.f;
+        const float e_a = m_a == -CUDART_INF_F ? 0.f : m_a, e_b = m_b == -CUDART_INF_F ? 0.f : m_b;
+        const uint64_t scale2 = pack_f32x2(a.scale_log2e, a.scale_log2e), ref_a = pack_f32x2(-e_a, -e_a), ref_b = pack_f32x2(-e_b, -e_b);
+        uint32_t pk[16];
+        uint64_t sum_a = 0, sum_b = 0;
 #pragma unroll
-        for (int i = 0; i < kBsBlk / 2; i += 2) {
-          const float p0 = bs_exp2(fmaf(x[i], a.scale_log2e, -m_eff)), p1 = bs_exp2(fmaf(x[i + 1], a.scale_log2e, -m_eff));
-          psum += p0 + p1;
-          pk[i >> 1] = bs_pack_bf16x2(p0, p1);
+        for (int i = 0; i < 16; ++i) {                 // word i: row a (even) or b, columns 8 (i / 2) + 2 (t % 4), + 1
+          float y0, y1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, (i & 1) ? ref_b : ref_a), y0, y1);
+          const float p0 = bs_exp2(y0), p1 = bs_exp2(y1);
+          if (i & 1) sum_b = add_f32x2(sum_b, pack_f32x2(p0, p1));
+          else sum_a = add_f32x2(sum_a, pack_f32x2(p0, p1));
+          pk[i] = bs_pack_bf16x2(p0, p1);
         }
-        psum += __shfl_xor_sync(0xffffffffu, psum, 16);
-        l += psum;
+        {
+          float s0, s1;
+          unpack_f32x2(sum_a, s0, s1);
+          l_a += s0 + s1;
+          unpack_f32x2(sum_b, s0, s1);
+          l_b += s0 + s1;
+        }
         if (jt > 1) {                                  // two P buffers: P.V of block jt-2 (of any unit) read this one
           ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[jt & 1], ((jt >> 1) - 1) & 1, abort_flag, a.status));
           if (!ok) break;
         }
-        {                                              // this lane's half row of P: 64 bytes, K-major, 128-byte swizzle
-          uint8_t* dst = p_s + (jt & 1) * kBsPanelBytes + row * 128;
-          const int c0 = (lane >> 4) * 4;              // first 16-byte chunk: columns 0-31 or 32-63
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(dst + (((c0 + c) ^ (row & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
-        }
+        bs_store_rows(p_s + (jt & 1) * kBsPanelBytes, quad * 16, lane, pk);
         fence_async_smem();                            // visible to the tensor core's reads
         tc_fence_before();
-        mbar_arrive(&p_full[jt & 1]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[jt & 1]);
       }
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_final, nq & 1, abort_flag, a.status));
       if (!ok) break;
       tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll 1
-      for (int c = 0; c < kBsD; c += 32) {
-        uint32_t ov[32];
-        tmem_ld32(t_row + kBsColO + c, ov);
-        tmem_wait_ld();
-        if (active) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 w;
-            w.x = bs_pack_bf16x2(__uint_as_float(ov[i + 0]) * inv, __uint_as_float(ov[i + 1]) * inv);
-            w.y = bs_pack_bf16x2(__uint_as_float(ov[i + 2]) * inv, __uint_as_float(ov[i + 3]) * inv);
-            w.z = bs_pack_bf16x2(__uint_as_float(ov[i + 4]) * inv, __uint_as_float(ov[i + 5]) * inv);
-            w.w = bs_pack_bf16x2(__uint_as_float(ov[i + 6]) * inv, __uint_as_float(ov[i + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c + i) = w;
-          }
+      for (int o = 1; o < 4; o <<= 1) {
+        l_a += __shfl_xor_sync(0xffffffffu, l_a, o);
+        l_b += __shfl_xor_sync(0xffffffffu, l_b, o);
+      }
+      const float inv_a = l_a > 0.f ? 1.f / l_a : 0.f, inv_b = l_b > 0.f ? 1.f / l_b : 0.f;
+      // every P has been consumed: the two P buffers take the warp's 16 rows (64 columns each) on their way out
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        uint32_t ov[32], w[16];
+        bs_tmem_ld(t_row + kBsColO + c * 64, ov);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float f = (i & 1) ? inv_b : inv_a;
+          w[i] = bs_pack_bf16x2(__uint_as_float(ov[2 * i]) * f, __uint_as_float(ov[2 * i + 1]) * f);
         }
+        bs_store_rows(p_s + c * kBsPanelBytes, quad * 16, lane, w);
       }
       tc_fence_before();
-      mbar_arrive(o_free);                             // the next unit's first P.V may overwrite O
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_free);              // the next unit's first P.V may overwrite O
+#pragma unroll
+      for (int r = 0; r < 16; r += 2) {
+        const int row = quad * 16 + r + (lane >> 4), ch = lane & 7;
+        const uint4 v = *reinterpret_cast<const uint4*>(p_s + ((lane >> 3) & 1) * kBsPanelBytes + row * 128 + ((ch ^ (row & 7)) << 4));
+        *reinterpret_cast<uint4*>(out0 + (r + (lane >> 4)) * pitch) = v;
+      }
+      __syncwarp();                                    // the rows have been read: the next unit's P may follow
       ++nq;
     }
   }

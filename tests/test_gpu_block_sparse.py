@@ -61,6 +61,18 @@ def test_large_scores_stay_finite():
     assert torch.isfinite(got).all()
 
 
+@pytest.mark.parametrize("step", [1, 3, 8])
+def test_rows_that_raise_their_maximum_at_different_blocks(step):
+    """Every ``step``-th query row meets keys that grow from block to block, the rows between them keys that shrink: one row of
+    a lane's pair is rescaled while the other keeps its maximum.  Same tolerance: the outputs are still convex sums of v."""
+    q, k, v, lut, num = _case(1, 1024, 3, 8, seed=17 + step, ragged=True)
+    lut = lut.sort(-1).values
+    u = torch.ones(128) / 128 ** 0.5
+    q = (q + (torch.arange(1024) % step == 0).float()[None, :, None, None] * 24 * u - 12 * u).bfloat16()
+    k = (k + (torch.arange(1024) // 64).float()[None, :, None, None] * 3 * u).bfloat16()
+    _check(q, k, v, lut, num, 128 ** -0.5)
+
+
 def test_bad_block_id_sets_status_and_is_skipped():
     q, k, v, lut, num = _case(1, 512, 2, 4, seed=13)
     bad = lut.clone()

@@ -204,3 +204,28 @@ def test_register_weight_form_equals_general_kernel_bitwise(T, S, window):
 def test_logits_of_calls_with_few_tiles(T, S, H, D):
     """Calls too small to give every SM a unit of eight tiles: units of four, two and one tile."""
     test_logits_match_oracle(T, S, H, D, "causal")
+
+
+@pytest.mark.parametrize("w_scale", [1e-20, 1.0, 1e28])
+def test_register_weight_form_at_the_ends_of_the_range(w_scale):
+    """The ReLU of the register-weight kernel is a saturating multiply: the largest dot products of e4m3 values (all operands
+    +-448), the smallest, zeros and NaN keys give the bits of the general kernel's max(d, 0)."""
+    from llmdivedeep_b200 import _lib
+    T, S = 70, 1500
+    q8, k8, ksc, w, ks, ke = to_dev(*indexer_inputs(T, S, 64, 128, seed=5, window="causal"))
+    w = w.float() * w_scale
+    qb, kb = q8.view(torch.uint8), k8.view(torch.uint8)
+    qb[0], kb[0] = 0x7E, 0x7E                          # 448 throughout: dot product 2.57e7
+    qb[1], kb[1] = 0xFE, 0xFE                          # -448
+    qb[2], kb[2] = 0x01, 0x01                          # the smallest subnormal
+    qb[3], kb[3] = 0, 0
+    kb[4, 7], kb[1200] = 0x7F, 0xFF                    # NaN: the dot products with these keys count as 0
+    ks, ke = torch.zeros_like(ks), torch.full_like(ke, S)
+    a = ops.fp8_mqa_logits(q8, (k8, ksc), w, ks, ke).clone()
+    b = torch.empty(T, S, dtype=torch.float32, device="cuda")
+    _lib.check(_lib.load().dsa_test_indexer_logits_general(
+        q8.data_ptr(), k8.data_ptr(), ksc.data_ptr(), w.data_ptr(), 0, ks.data_ptr(), ke.data_ptr(), b.data_ptr(), S, T, S,
+        64, 128, 1, ops.status_word("cuda").data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert float(a[:, 4].abs().max()) == 0.0 and float(a[:, 1200].abs().max()) == 0.0
+    ops.check_status("cuda")

@@ -124,14 +124,23 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t cta) {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Arrive on the peer's barrier to say "I have READ the tile".  Relaxed: a release at cluster scope costs a memory fence of
-// thousands of cycles per block, and nothing written by this thread has to become visible.  But a relaxed arrival orders
-// nothing, and straight after the loads it overtakes them -- they queue behind the gather's copies in the load/store unit,
-// and the next tile then lands on top of this one before it is read (seen: a few tokens in ten thousand).  The caller must
-// have stored or branched on a value computed from all that was loaded.  (A register-OR and warp reduction of the loaded
-// words as that value, to send the arrival earlier, cost more than it gained: 2228 -> 2280 us.)
-__device__ __forceinline__ void mbar_arrive_remote_relaxed(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrive on the peer's barrier to say "this warp has READ the tile".  Relaxed: a release at cluster scope costs a memory
+// fence of thousands of cycles per block, and nothing written by this thread has to become visible.  But a relaxed arrival
+// orders nothing, and straight after the loads it overtakes them -- they queue behind the gather's copies in the load/store
+// unit, and the next tile then lands on top of this one before it is read (seen: a few tokens in ten thousand).  So the
+// arrival takes the data as its operand: each lane gives a value computed from EVERY word that it loaded, the vote needs all
+// lanes' values, and the arrival is predicated on the vote, so that it cannot issue before the loads have returned, whatever
+// the compiler does with the code around it.  `x` comes out of fmaxf, which returns numbers or the canonical NaN: it never is
+// the bit pattern compared with (a signalling NaN), which the compiler cannot know.  (A register-OR of the loaded words
+// as that value, to send the arrival earlier, cost more than it gained: 2228 -> 2280 us.)
+__device__ __forceinline__ void mbar_arrive_remote_after(uint32_t cluster_addr, float x, bool leader) {
+  const bool seen = __any_sync(0xffffffffu, __float_as_uint(x) != 0x7f812345u);
+  if (leader)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "@p mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}"
+        ::"r"(cluster_addr), "r"(static_cast<uint32_t>(seen)) : "memory");
 }
 // this CTA's shared memory -> the peer's, completion counted on the peer's mbarrier
 __device__ __forceinline__ void bulk_copy_to_peer(uint32_t dst_cluster, const void* src, uint32_t bytes, uint32_t bar_cluster) {
@@ -627,22 +636,24 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
       }
       const uint32_t used = __ballot_sync(0xffffffffu, valid_s[(n % kMlaValidRing) * kMlaBlk + 32 * hf + lane]);
+      auto largest = [&]() {
+        float bm[4] = {s[0], s[1], s[2], s[3]};        // four independent chains
+#pragma unroll
+        for (int i = 4; i < 32; ++i) bm[i & 3] = fmaxf(bm[i & 3], s[i]);
+        return fmaxf(fmaxf(bm[0], bm[1]), fmaxf(bm[2], bm[3]));
+      };
+      const float top = largest();                     // of every value of the tile, used or not
+      float bmax = top;
       if (used != 0xffffffffu) {                       // empty slots (the tail of a short row, holes): warp-uniform
 #pragma unroll
         for (int i = 0; i < 32; ++i) s[i] = (used >> i) & 1u ? s[i] : -CUDART_INF_F;
+        bmax = largest();
       }
-      float bm[4] = {s[0], s[1], s[2], s[3]};          // four independent chains
-#pragma unroll
-      for (int i = 4; i < 32; ++i) bm[i & 3] = fmaxf(bm[i & 3], s[i]);
-      pm_of(n)[hf * 128] = static_cast<uint16_t>(bf16_bits_round_up(fmaxf(fmaxf(bm[0], bm[1]), fmaxf(bm[2], bm[3])) * a.scale_log2e));
+      pm_of(n)[hf * 128] = static_cast<uint16_t>(bf16_bits_round_up(bmax * a.scale_log2e));
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&pm_full[set * 4 + qd]);
-        // The peer may send into this stage again.  Only here: the block maximum just stored needed every value of the tile,
-        // so the loads have returned.
-        mbar_arrive_remote_relaxed(peer_xchg_free);
-        if (n + 2 < nblk) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
-      }
+      if (lane == 0) mbar_arrive(&pm_full[set * 4 + qd]);
+      mbar_arrive_remote_after(peer_xchg_free, top, lane == 0);      // the peer may send into this stage again
+      if (lane == 0 && n + 2 < nblk) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
       ok = mbar_wait_warp(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
       if (!ok) break;
       m = raise(m_prev, pair_max(pm_of(n)));

@@ -240,3 +240,46 @@ def test_decode_rounds_of_queries_with_a_split_remainder(B, H, K):
     assert float((out.float() - one.float()).abs().max()) <= MAX_ABS
     rows = [0, 1, B // 2, B - 2, B - 1]
     check(out[rows], O.sparse_mla_decode_paged(q[rows].float(), cache, table[rows], idx[rows], 0.06, round_bf16=True))
+
+
+def _holes(idx, g):
+    """Every second row: random empty slots, an empty block now and then, a tail of its own length."""
+    T, K = idx.shape
+    idx[::2].masked_fill_(torch.rand((T + 1) // 2, K, device="cuda", generator=g) < 0.2, -1)
+    idx[::4, 64:128] = -1
+    length = torch.randint(1, K + 1, (T, 1), device="cuda", generator=g)
+    idx[::2].masked_fill_(torch.arange(K, device="cuda") >= length[::2], -1)
+    return idx
+
+
+@pytest.mark.parametrize("form", ["prefill", "decode"])
+def test_ragged_lists_and_decode_repeat_bit_for_bit(form):
+    """The hand-over between the two CTAs of a pair, where the masks of holes and ragged tails come between reading a tile and
+    releasing it, and in the decode kernel: many waves of pairs, the same bits in every run, a sample against float64."""
+    g = torch.Generator(device="cuda").manual_seed(71)
+    T, H, K, P, scale = 1200, 128, 1024, 24, 192 ** -0.5
+    q = torch.randn(T, H, 576, device="cuda", generator=g).to(torch.bfloat16)
+    idx = _holes(torch.rand(T, P * 64, device="cuda", generator=g).topk(K, dim=-1).indices.int(), g)
+    if form == "prefill":
+        kv = torch.randn(P * 64, 576, device="cuda", generator=g).to(torch.bfloat16)
+        run = lambda: ops.sparse_mla_prefill(q, kv, idx, scale)
+        rows_of = lambda t, pos: kv[pos].double()
+    else:
+        records = O.pack_latent_cache(torch.randn(200 * 64, 576, generator=torch.Generator().manual_seed(72)).to(torch.bfloat16)).cuda()
+        table = torch.randint(0, 200, (T, P), device="cuda", generator=g).int()
+        run = lambda: ops.sparse_mla_decode_paged(q, records, table, idx, scale)
+
+        def rows_of(t, pos):
+            rec = records[table[t].long()[pos // 64] * 64 + pos % 64]
+            lat = rec[:, :512].contiguous().view(torch.float8_e4m3fn).float().view(-1, 4, 128)
+            lat = (lat * rec[:, 512:528].contiguous().view(torch.float32).unsqueeze(-1)).view(-1, 512).to(torch.bfloat16)
+            return torch.cat((lat, rec[:, 528:].contiguous().view(torch.bfloat16)), -1).double()
+
+    out = run()
+    for _ in range(12):
+        assert torch.equal(run(), out)
+    ops.check_status("cuda")
+    for t in range(0, T, 7):
+        rows = rows_of(t, idx[t][idx[t] >= 0].long())
+        ref = ((q[t].double() @ rows.T) * scale).softmax(-1) @ rows[:, :512] if rows.shape[0] else torch.zeros_like(out[t]).double()
+        assert float((out[t].double() - ref).abs().max()) <= MAX_ABS, t

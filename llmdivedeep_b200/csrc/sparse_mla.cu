@@ -16,10 +16,12 @@
 //   * the two partial tiles ([128 heads x 64 keys], rounded to fp16 for the way: 16 KB) are exchanged
 //     through distributed shared memory, every warp sending its own 2 KB with one bulk copy (quadrants
 //     of tensor memory without heads stand by).  Each
-//     side adds what arrives to its own unrounded fp32 partial scores and runs the whole softmax; the
-//     two sides' P may differ in the last bit of an fp16 score, which is exact for each of them: a CTA
-//     normalises its half of O by the row sums of its own P.  fp16 carries 11 significant bits: an
-//     error below the bf16 rounding of P for scores within +-65504;
+//     side adds what arrives to its own unrounded fp32 partial scores and runs the whole softmax.  The
+//     two sides' scores differ by the rounding of what was sent, so the halves of an output row come from
+//     two softmaxes: each CTA normalises its half of O by the row sums of its own P, and a part of a split
+//     list is weighted half by half.  P is off by at most scale * 2^-11 * |partial score of the peer|,
+//     relative: less than its bf16 rounding (2^-9) while scale * |partial| is below 4.  A partial beyond
+//     +-65504 saturates on the way, for the receiving side only;
 //   * P is the A operand (from tensor memory) of O_c += P V_c (4 MMAs of N = 256) with the gathered
 //     panels read through an MN-major descriptor.
 // O is rescaled in tensor memory only when the running maximum grows by more than 8 (log2 units).
@@ -112,7 +114,7 @@ struct MlaArgs {
   int n_full;                     // the first n_full queries are one unit (CTA pair) each; ...
   int n_split;                    // ... the slot list of every later one is cut into n_split parts, a unit each (decode)
   float* part_o;                  // [(T - n_full) * n_split, H, 512] fp32 normalised partial outputs
-  float* part_lse;                // [(T - n_full) * n_split, H] log2-sum-exp of each part (-inf = empty part)
+  float* part_lse;                // [(T - n_full) * n_split, 2, H] log2-sum-exp of each part as each CTA of the pair has it (-inf = empty part)
   int tma_out;                    // the output tensor map is valid: full 128-head groups leave through TMA stores
 };
 
@@ -330,7 +332,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const int64_t prow = (int64_t)part * a.H + hg * 128 + threadIdx.x;
         float4* o = reinterpret_cast<float4*>(a.part_o + prow * kMlaDv + cta * kMlaDvHalf);
         for (int c = 0; c < kMlaDvHalf / 4; ++c) o[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (cta == 0) a.part_lse[prow] = -CUDART_INF_F;
+        a.part_lse[((int64_t)part * 2 + cta) * a.H + hg * 128 + threadIdx.x] = -CUDART_INF_F;
       }
     }
     // an index that is out of range is still reported
@@ -731,8 +733,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       const float inv = l > 0.f ? 1.f / l : 0.f;
       __nv_bfloat16* orow = a.out + ((int64_t)t * a.H + hg * 128 + row) * kMlaDv + cta * kMlaDvHalf;
       const int64_t prow = (int64_t)part * a.H + hg * 128 + row;
-      if (part >= 0 && cta == 0 && quarter == 0 && row < heads_here)
-        a.part_lse[prow] = l > 0.f ? mt + log2f(l) : -CUDART_INF_F;
+      if (part >= 0 && quarter == 0 && row < heads_here)         // what this CTA's half of the columns is weighted with
+        a.part_lse[((int64_t)part * 2 + cta) * a.H + hg * 128 + row] = l > 0.f ? mt + log2f(l) : -CUDART_INF_F;
 #pragma unroll 1
       for (int c = quarter * (kMlaDvHalf / 4); c < (quarter + 1) * (kMlaDvHalf / 4); c += 32) {
         uint32_t ov[32];
@@ -798,13 +800,15 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   }
 }
 
-// out[t,h,:] = sum_s 2^(lse_s - M) o_s / sum_s 2^(lse_s - M): merges the parts of a split slot list.
+// out[t,h,:] = sum_s 2^(lse_s - M) o_s / sum_s 2^(lse_s - M): merges the parts of a split slot list, each half of the columns
+// by the sums of the CTA that computed it.
 __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a) {
   const int u = blockIdx.x, t = a.n_full + u, h = blockIdx.y;
+  const int d = threadIdx.x * 4, cta = d / kMlaDvHalf;
   float wgt[16];
   float mx = -CUDART_INF_F, den = 0.f;
   for (int sp = 0; sp < a.n_split; ++sp) {
-    wgt[sp] = a.part_lse[((int64_t)u * a.n_split + sp) * a.H + h];
+    wgt[sp] = a.part_lse[(((int64_t)u * a.n_split + sp) * 2 + cta) * a.H + h];
     mx = fmaxf(mx, wgt[sp]);
   }
   for (int sp = 0; sp < a.n_split; ++sp) {
@@ -812,7 +816,6 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a
     den += wgt[sp];
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
-  const int d = threadIdx.x * 4;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int sp = 0; sp < a.n_split; ++sp) {
     const float4 v = *reinterpret_cast<const float4*>(a.part_o + (((int64_t)u * a.n_split + sp) * a.H + h) * kMlaDv + d);
@@ -881,7 +884,7 @@ static MlaSplit mla_decode_split(int B, int H, int K) {
 }
 size_t mla_decode_workspace_bytes(int B, int H, int K) {
   const MlaSplit sp = mla_decode_split(B, H, K);
-  return (size_t)(B - sp.n_full) * sp.n_split * H * (kMlaDv + 1) * sizeof(float);
+  return (size_t)(B - sp.n_full) * sp.n_split * H * (kMlaDv + 2) * sizeof(float);
 }
 
 int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* block_table, int64_t table_stride,

@@ -283,3 +283,28 @@ def test_ragged_lists_and_decode_repeat_bit_for_bit(form):
         rows = rows_of(t, idx[t][idx[t] >= 0].long())
         ref = ((q[t].double() @ rows.T) * scale).softmax(-1) @ rows[:, :512] if rows.shape[0] else torch.zeros_like(out[t]).double()
         assert float((out[t].double() - ref).abs().max()) <= MAX_ABS, t
+
+
+def test_decode_parts_are_weighted_with_the_sums_of_their_own_half():
+    """The score of every key is about 6144 and comes from the second CTA's half of the contraction alone, so that CTA has it
+    unrounded while the other receives it in fp16 (spacing 4, two units of the scaled score).  Output columns 256.. are the
+    second CTA's: exact to bf16 whether the list is split or not, if its parts are weighted with its own sums."""
+    B, H, P, K, scale = 2, 128, 40, 2048, 0.5
+    g = torch.Generator().manual_seed(31)
+    kv = torch.randn(B * P * 64, 576, generator=g)
+    kv[:, 512:544] = 0
+    kv[:, 544:] = 24
+    cache = O.pack_latent_cache(kv.to(torch.bfloat16))
+    table = torch.randperm(B * P, generator=g).int().view(B, P)
+    idx = torch.stack([torch.randperm(P * 64, generator=g)[:K] for _ in range(B)]).int()
+    q = torch.zeros(B, H, 576)
+    q[:, :, 256:512] = torch.randn(B, H, 256, generator=g) / 2
+    q[:, :, 544:] = 8
+    q = q.to(torch.bfloat16)
+    ref = O.sparse_mla_decode_paged(q.float(), cache, table, idx, scale, round_bf16=True)[..., 256:]
+    args = (q.cuda(), cache.cuda(), table.cuda(), idx.cuda(), scale)
+    split = ops.sparse_mla_decode_paged(*args)
+    single = ops.sparse_mla_decode_paged(*args, workspace=torch.empty(16, dtype=torch.uint8, device="cuda"))
+    ops.check_status("cuda")
+    check(single[..., 256:], ref)
+    check(split[..., 256:], ref)

@@ -210,15 +210,11 @@ def topk_select(logits: torch.Tensor, k: int, ks=None, ke=None, out: Optional[to
     return out
 
 
-_workspaces = {}
-
-
 def _workspace(device, nbytes: int) -> torch.Tensor:
-    key = _dev_index(device)
-    w = _workspaces.get(key)
-    if w is None or w.numel() < nbytes:
-        _workspaces[key] = w = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{key}")
-    return w
+    """Scratch of one call, from the caching allocator of the current stream: the call's own while it enqueues its kernels
+    (another thread, even on the same stream, gets other memory), and handed on in stream order afterwards.  Nothing is kept
+    here: a buffer shared by two streams, or replaced under a captured graph, would be overwritten while it is read."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def indexer_topk(q_fp8, k_fp8, k_scale, weights, ks, ke, k: int, workspace: Optional[torch.Tensor] = None,
@@ -234,11 +230,11 @@ def indexer_topk(q_fp8, k_fp8, k_scale, weights, ks, ke, k: int, workspace: Opti
     ks = _as_i32(ks, T, "ks")
     ke = _as_i32(ke, T, "ke")
     lib = _lib.load()
+    out = _check_idx_out(out, T, k, q_fp8.device)
     if workspace is None:
         full = lib.dsa_indexer_topk_workspace_bytes(T, S)
         row = full // max(T, 1)
         workspace = _workspace(q_fp8.device, min(full, max(max_workspace_bytes, 256 * row)))
-    out = _check_idx_out(out, T, k, q_fp8.device)
     with _on(dev):
         check(lib.dsa_indexer_topk(_ptr(q_fp8), _ptr(k_fp8), _ptr(k_scale), _ptr(weights), _w_dtype(weights),
                                    _ptr(ks), _ptr(ke), T, S, H, D, k, _ptr(out), _ptr(workspace), workspace.numel(),

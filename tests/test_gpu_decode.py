@@ -155,3 +155,31 @@ def test_quantiser_ragged_block_counts_and_unaligned_output(n_blocks, block):
 def test_paged_logits_of_calls_with_few_tiles(B, P, H):
     """Calls too small to give every SM a unit of eight tiles: units of four, two and one tile."""
     test_paged_logits_match_oracle(B, P, H)
+
+
+def test_calls_without_a_workspace_on_two_streams():
+    """Split decode batches and an indexer_topk on streams of their own, none given a workspace: the results of the same calls
+    one after the other."""
+    from tests.helpers import indexer_inputs, to_dev
+    g = torch.Generator().manual_seed(5)
+    B, H, P, K = 75, 128, 10, 600                      # one query beyond a round of CTA pairs: cut into parts
+    caches = [O.pack_latent_cache(torch.randn(B * P * 64, 576, generator=g).to(torch.bfloat16)).cuda() for _ in range(2)]
+    table = torch.randperm(B * P, generator=g).int().view(B, P).cuda()
+    idx = torch.rand(B, P * 64, generator=g).topk(K, dim=-1).indices.int().cuda()
+    q = torch.randn(B, H, 576, generator=g).to(torch.bfloat16).cuda()
+    ind = to_dev(*indexer_inputs(512, 2048, 64, 128, seed=6))
+    calls = [lambda: ops.sparse_mla_decode_paged(q[:9], caches[0], table[:9], idx[:9], 0.06),
+             lambda: ops.sparse_mla_decode_paged(q, caches[1], table, idx, 0.06),
+             lambda: ops.indexer_topk(*ind, 256)]
+    want = [c() for c in calls]
+    streams = [torch.cuda.Stream() for _ in calls]
+    torch.cuda.synchronize()
+    got = [[] for _ in calls]
+    for _ in range(20):
+        for c, s, o in zip(calls, streams, got):
+            with torch.cuda.stream(s):
+                o.append(c())
+    torch.cuda.synchronize()
+    ops.check_status("cuda")
+    for w, o in zip(want, got):
+        assert all(torch.equal(x, w) for x in o)

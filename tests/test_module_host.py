@@ -1,6 +1,8 @@
 """Host-only checks of the module mirror (llmdivedeep_b200/DSA.py) and of the oracle's stage
 outputs against the reference's recorded ones: nothing here launches a kernel."""
+import contextlib
 import os
+import weakref
 
 import numpy as np
 import pytest
@@ -109,3 +111,55 @@ def test_index_share_runs_the_indexer_every_freq_layers():
     assert [layer.IndexShare(1).select(i, indexer, i) for i in range(3)] == [4, 5, 6]
     with pytest.raises(ValueError):
         layer.IndexShare(0)
+
+
+@pytest.mark.parametrize("call", ["decode", "indexer_topk"])
+def test_overlapping_calls_without_a_workspace_share_no_scratch(monkeypatch, call):
+    """A second call that starts while the first one's kernels are in flight -- here from inside the library call, as another
+    thread or stream would -- must get scratch of its own, and none may be kept once the calls are over."""
+    real_empty, spans, kept = torch.empty, [], []
+
+    class Lib:
+        def dsa_sparse_mla_decode_workspace_bytes(self, *a):
+            return 4096
+
+        def dsa_indexer_topk_workspace_bytes(self, T, S):
+            return T * S * 4
+
+        def _enter(self, ptr, nbytes):
+            spans.append((ptr, ptr + nbytes))
+            if len(spans) == 1:
+                run()
+            return 0
+
+        def dsa_sparse_mla_decode_paged(self, *a):
+            return self._enter(a[12], a[13])
+
+        def dsa_indexer_topk(self, *a):
+            return self._enter(a[13], a[14])
+
+    def empty(*a, device=None, **kw):                  # "cuda:0" lives on the CPU here
+        t = real_empty(*a, **kw)
+        if t.dtype == torch.uint8:
+            kept.append(weakref.ref(t))
+        return t
+
+    monkeypatch.setattr(torch, "empty", empty)
+    monkeypatch.setattr(ops._lib, "load", Lib)
+    monkeypatch.setattr(ops, "_need_cuda", lambda *ts: torch.device("cpu"))
+    monkeypatch.setattr(ops, "_dev_index", lambda d: 0)
+    monkeypatch.setattr(ops, "_on", lambda d: contextlib.nullcontext())
+    monkeypatch.setattr(ops, "_stream", lambda d: 0)
+    monkeypatch.setattr(ops, "status_word", lambda d: torch.zeros(1, dtype=torch.int32))
+    if call == "decode":
+        q = torch.zeros(2, 16, 576, dtype=torch.bfloat16)
+        cache, table = torch.zeros(64, 656, dtype=torch.uint8), torch.zeros(2, 1, dtype=torch.int32)
+        run = lambda: ops.sparse_mla_decode_paged(q, cache, table, torch.zeros(2, 8, dtype=torch.int32), 0.1)
+    else:
+        q8 = torch.zeros(4, 64, 128).to(torch.float8_e4m3fn)
+        ke = torch.ones(4, dtype=torch.int32)
+        run = lambda: ops.indexer_topk(q8, q8[0], torch.ones(64), torch.ones(4, 64), None, ke, 8)
+    run()
+    (a0, a1), (b0, b1) = spans
+    assert a1 > a0 and b1 > b0 and (a1 <= b0 or b1 <= a0)
+    assert kept and all(r() is None for r in kept)

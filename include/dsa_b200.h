@@ -155,10 +155,14 @@ int dsa_block_sparse_mha(const void* q_bf16, const void* k_bf16, const void* v_b
  * values; latent = e4m3 * scale is rounded to bf16 before the tensor-core math.
  *   q_bf16 [B, H, 576]; cache [num_pages*64, 656] bytes; block_table
  *   [B, table_stride] int32; idx [B, K] int32 (K <= 2048); out_bf16 [B, H, 512].
- * With few sequences the slot list of each is cut into parts that run on
- * different SMs and are merged by a second kernel; that needs `workspace` of
- * dsa_sparse_mla_decode_workspace_bytes(B, H, K) bytes (16-byte aligned).  With
- * workspace NULL or too small the call still works, one part per sequence. */
+ * Sequences run in rounds of one per pair of SMs (per group of 128 heads).  The
+ * slot lists of a partly filled last round -- every sequence of a small batch, the
+ * last B mod pairs of a larger one -- are cut into up to eight parts that run on
+ * different SMs and are merged by a second kernel in fp32, so that a row's last
+ * bits depend on the batch it is computed in.  The parts need `workspace` (16-byte
+ * aligned): dsa_sparse_mla_decode_workspace_bytes(B, H, K) bytes are enough for
+ * every batch of up to B sequences.  A smaller workspace holds fewer parts; with
+ * NULL, or less than two parts a sequence, the call works with one. */
 size_t dsa_sparse_mla_decode_workspace_bytes(int B, int H, int K);
 int dsa_sparse_mla_decode_paged(const void* q_bf16, const void* cache, const int32_t* block_table,
                                 int64_t table_stride, const int32_t* idx, void* out_bf16, int B, int H, int K,

@@ -874,17 +874,20 @@ int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx,
 // take as long as a full one.  The queries of that round are cut into parts that share its pairs: as many as fit, at most
 // eight, of at least 256 slots.  More parts than that lose: every part pays the set-up again and writes an fp32 partial
 // output that the combine kernel reads back.  Batch 160 (two rounds and twelve queries in six parts each): 174 -> 156 us.
-struct MlaSplit { int n_full, n_split; };
-static MlaSplit mla_decode_split(int B, int H, int K) {
-  int pairs = sm_count() / (2 * ((H + 127) / 128));
-  if (pairs < 1) pairs = 1;
-  const int rest = B % pairs;
-  const int ns = rest == 0 ? 1 : min(min(8, K / 256), pairs / rest);
-  return ns > 1 ? MlaSplit{B - rest, ns} : MlaSplit{B, 1};
-}
+static int mla_pairs(int H) { return max(1, sm_count() / (2 * ((H + 127) / 128))); }
+static int mla_parts_per_query(int rest, int pairs, int K) { return rest == 0 ? 1 : max(1, min(min(8, K / 256), pairs / rest)); }
+static size_t mla_part_bytes(int H) { return (size_t)H * (kMlaDv + 2) * sizeof(float); }
+// Enough for every batch of up to B queries.  The need of a batch goes up and down with the queries of its last round (128
+// heads, 2048 slots, 148 SMs: 64 parts for 8 queries, 74 for 37, none for 38 or for 74), and a serving loop runs smaller
+// batches in the buffer that it made for its largest.
 size_t mla_decode_workspace_bytes(int B, int H, int K) {
-  const MlaSplit sp = mla_decode_split(B, H, K);
-  return (size_t)(B - sp.n_full) * sp.n_split * H * (kMlaDv + 2) * sizeof(float);
+  const int pairs = mla_pairs(H);
+  int parts = 0;
+  for (int rest = 1; rest < pairs && rest <= B; ++rest) {
+    const int ns = mla_parts_per_query(rest, pairs, K);
+    if (ns > 1) parts = max(parts, rest * ns);
+  }
+  return parts * mla_part_bytes(H);
 }
 
 int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* block_table, int64_t table_stride,
@@ -892,14 +895,19 @@ int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* bl
                              float scale, void* workspace, size_t workspace_bytes, int32_t* status,
                              cudaStream_t stream) {
   MlaArgs a{};
-  const MlaSplit sp = mla_decode_split(B, H, K);
+  const int pairs = mla_pairs(H), rest = B % pairs;
+  int ns = mla_parts_per_query(rest, pairs, K);
+  if (ns > 1) {                                        // a smaller workspace: as many parts as it holds
+    const size_t fit = workspace ? workspace_bytes / mla_part_bytes(H) / rest : 0;
+    if (fit < (size_t)ns) ns = fit > 1 ? (int)fit : 1;
+  }
   a.n_full = B;
   a.n_split = 1;
-  if (sp.n_split > 1 && workspace && workspace_bytes >= mla_decode_workspace_bytes(B, H, K)) {
-    a.n_full = sp.n_full;
-    a.n_split = sp.n_split;
+  if (ns > 1) {
+    a.n_full = B - rest;
+    a.n_split = ns;
     a.part_o = static_cast<float*>(workspace);
-    a.part_lse = a.part_o + (size_t)(B - sp.n_full) * sp.n_split * H * kMlaDv;
+    a.part_lse = a.part_o + (size_t)rest * ns * H * kMlaDv;
   }
   a.cache = static_cast<const uint8_t*>(cache);
   a.block_table = block_table;

@@ -78,3 +78,23 @@ def test_cpu_tensors_are_refused():
     x = torch.zeros(2, 8)
     with pytest.raises(_lib.DsaError):
         ops.topk_select(x, 2)
+
+
+@pytest.mark.parametrize("H,K", [(16, 2048), (128, 2048), (128, 700), (200, 1024), (128, 511)])
+def test_decode_workspace_serves_every_smaller_batch(lib, H, K):
+    """A buffer made for a batch holds the parts of every batch up to it (148 SMs here: there is no GPU to ask), and never
+    more than one part per pair of SMs."""
+    pairs = 148 // (2 * -(-H // 128))
+    part = H * 514 * 4
+
+    def parts(b):
+        rest = b % pairs
+        ns = min(8, K // 256, pairs // rest) if rest else 1
+        return rest * ns if ns > 1 else 0
+
+    most = 0
+    for b in range(1, 300):
+        most = max(most, parts(b))
+        assert lib.dsa_sparse_mla_decode_workspace_bytes(b, H, K) == most * part <= pairs * part
+    from llmdivedeep_b200.layer import DecodeWorkspace
+    assert DecodeWorkspace(64, H, 4096, K, "cpu").mla_ws.numel() >= max(parts(b) for b in range(1, 65)) * part

@@ -183,3 +183,28 @@ def test_calls_without_a_workspace_on_two_streams():
     ops.check_status("cuda")
     for w, o in zip(want, got):
         assert all(torch.equal(x, w) for x in o)
+
+
+def test_smaller_batches_in_the_workspace_of_a_larger_one():
+    """The parts of every batch fit the buffer made for the largest: the bits of the call with scratch of its own.  Buffers of
+    fewer parts give fewer parts, and the same result within the merge's rounding."""
+    B, H, P, K = 64, 128, 34, 2048
+    g = torch.Generator().manual_seed(64)
+    cache = O.pack_latent_cache(torch.randn(B * P * 64, 576, generator=g).to(torch.bfloat16)).cuda()
+    table = torch.randperm(B * P, generator=g).int().view(B, P).cuda()
+    idx = torch.rand(B, P * 64, generator=g).topk(K, dim=-1).indices.int().cuda()
+    q = torch.randn(B, H, 576, generator=g).to(torch.bfloat16).cuda()
+    ws = layer.DecodeWorkspace(B, H, P * 64, K, "cuda").mla_ws
+    for b in (1, 7, 12, 23, 37, 38, 64):
+        args = (q[:b], cache, table[:b], idx[:b], 0.06)
+        own = ops.sparse_mla_decode_paged(*args)
+        assert torch.equal(ops.sparse_mla_decode_paged(*args, workspace=ws), own)
+        assert torch.equal(ops.sparse_mla_decode_paged(*args, workspace=ws), own)
+        whole = ops.sparse_mla_decode_paged(*args, workspace=ws[:16])
+        for parts in (1, 2, 3, 5):                     # per query; poison behind what such a buffer may use
+            small = torch.full((b * parts * H * 514 * 4 + 4096,), 7, dtype=torch.uint8, device="cuda")
+            out = ops.sparse_mla_decode_paged(*args, workspace=small[: b * parts * H * 514 * 4 + 100])
+            assert bool((small[b * parts * H * 514 * 4:] == 7).all())
+            assert float((out.float() - whole.float()).abs().max()) <= 2e-2
+            assert not torch.isnan(out).any()
+    ops.check_status("cuda")

@@ -308,3 +308,31 @@ def test_decode_parts_are_weighted_with_the_sums_of_their_own_half():
     ops.check_status("cuda")
     check(single[..., 256:], ref)
     check(split[..., 256:], ref)
+
+
+@pytest.mark.parametrize("form", ["prefill", "decode"])
+@pytest.mark.parametrize("K", [32, 33, 64, 700, 929, 1000, 1824, 2048])
+def test_last_used_slot_anywhere_in_the_list(form, K):
+    """The last used slot decides how many blocks a row walks: at both ends of the list, around its last 32 slots and around
+    the 896 slots that the threads of a CTA look at together; alone, and behind holes."""
+    last = sorted({p for p in (0, 31, 32, 63, 64, 863, 864, 895, 896, 897, 1791, 1792, K - 66, K - 34, K - 33, K - 32, K - 31, K - 1)
+                   if 0 <= p < K})
+    g = torch.Generator().manual_seed(K)
+    T, H, P = 2 * len(last) + 1, 16, 34
+    idx = torch.full((T, K), -1, dtype=torch.int32)
+    for i, p in enumerate(last):                       # row T - 1 stays empty
+        idx[2 * i, p] = 5 + i
+        idx[2 * i + 1, :p + 1] = torch.randperm(P * 64, generator=g)[:p + 1].int()
+        idx[2 * i + 1, 1:p:3] = -1
+    q = torch.randn(T, H, 576, generator=g).to(torch.bfloat16)
+    kv = torch.randn(P * 64, 576, generator=g).to(torch.bfloat16)
+    if form == "prefill":
+        out = ops.sparse_mla_prefill(q.cuda(), kv.cuda(), idx.cuda(), 0.06)
+        ref = O.sparse_mla(q.float(), kv.float(), idx, 0.06)
+    else:                                              # T < 74: the lists are cut into parts
+        cache, table = O.pack_latent_cache(kv), torch.arange(P, dtype=torch.int32).repeat(T, 1)
+        out = ops.sparse_mla_decode_paged(q.cuda(), cache.cuda(), table.cuda(), idx.cuda(), 0.06)
+        ref = O.sparse_mla_decode_paged(q.float(), cache, table, idx, 0.06, round_bf16=True)
+    ops.check_status("cuda")
+    check(out, ref)
+    assert float(out[T - 1].float().abs().max()) == 0.0

@@ -32,12 +32,12 @@
 
 namespace dsa {
 
-constexpr int kTileKeys = 128;         // keys per MMA (M); a paged work tile is two of these, see tile_keys()
+constexpr int kTileKeys = 128;         // keys per MMA (M); a paged work tile is four of these, see tile_keys()
 constexpr int kChunkTiles = 64;        // most key tiles per work unit (launches with few units use fewer)
 constexpr int kPageTokens = 64;
 // Keys per pipeline tile.  The paged (decode) form has one query token per sequence, so a 128-key tile is little
-// work (64 accumulator columns) against the fixed cost of its barrier hand-offs: it moves 256 keys (four pages)
-// per tile, as two M=128 MMAs into adjacent accumulator columns.
+// work (64 accumulator columns) against the fixed cost of its barrier hand-offs: it moves 512 keys (eight pages)
+// per tile, as four M=128 MMAs into adjacent accumulator columns.
 template <bool PAGED>
 __host__ __device__ constexpr int tile_keys() { return PAGED ? 4 * kTileKeys : kTileKeys; }
 

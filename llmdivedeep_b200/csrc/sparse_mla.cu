@@ -83,11 +83,13 @@ struct MlaRegs {                                   // decode's gather converts i
   static constexpr int kSoftmax = FP8_PAGED ? 88 : 96, kOther = FP8_PAGED ? 48 : 40;
   static_assert(512 * kSoftmax + 384 * kOther <= 896 * 72, "more registers than the launch has");
 };
+constexpr int kMlaMaxK = 2048;                     // slots of a list
 constexpr int kMlaThreads = 896, kMlaSoftmaxWarps = 16, kMlaMmaWarp = 16, kMlaGatherWarp0 = 17, kMlaGatherWarps = 11;
 template <int R>
 __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+constexpr int kMlaLooks = (kMlaMaxK + kMlaThreads - 1) / kMlaThreads;
 constexpr int kMlaBarBytes = 512;                  // mbarriers and a few words
 constexpr int kMlaPairBytes = 4 * 2 * 128 * 2;     // block maxima: [block mod 4][key half][head], bf16
 constexpr int kMlaSmemBytes = kMlaBufs * kMlaKBytes + 2 * kMlaXBytes + kMlaBarBytes +
@@ -275,6 +277,12 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const int tail = tail_j >= 0 ? __ldg(idx_row + tail_j) : -1;
   const int slot = warp >= kMlaGatherWarp0 && lane < kRawRows ? warp - kMlaGatherWarp0 + lane * kMlaGatherWarps : kMlaBlk;
   const int slot_pos = slot < kMlaBlk && slot < k_cnt ? __ldg(idx_row + slot) : -1;
+  int look[kMlaLooks];                                         // ... and every thread its share of the whole list
+#pragma unroll
+  for (int u = 0; u < kMlaLooks; ++u) {
+    const int j = threadIdx.x + u * kMlaThreads;
+    look[u] = j < k_cnt - 32 ? __ldg(idx_row + j) : -1;
+  }
   // ... while warp 0 initialises the barriers (one per lane) and sends for Q (one panel per lane) and the MMA warp allocates
   // tensor memory
   if (warp == 0) {
@@ -306,19 +314,18 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   __syncthreads();
   tc_fence_after();
   // The last usable slot decides the number of key blocks (the same number in both CTAs of the pair).  It is among the last 32
-  // but for short rows (the first 2048 of every prompt): there the threads look at the whole list at once, one load latency
-  // whatever its length.  Rows 0-295, K = 2048, 128 heads: 103 us with every warp walking back 128 slots a turn, 55 us so.
+  // but for short rows (the first 2048 of every prompt): there the shares of all threads decide.  Rows 0-295, K = 2048, 128
+  // heads: 103 us with every warp walking back 128 slots a turn, 55 with the shares requested here, 50 with them under way
+  // since the start (full rows pay nothing for it: 4096 x 2048 keys 2280 us without, 2255 with).
   int nblk;
   {
     const uint32_t hit = __ballot_sync(0xffffffffu, tail >= 0 && tail < a.S_kv);
     int last = k_cnt - 1 - __clz(hit);
     if (hit == 0) {                                    // the same answer in every warp
       last = -1;
-#pragma unroll 3
-      for (int j = threadIdx.x; j < k_cnt - 32; j += kMlaThreads) {
-        const int p = __ldg(idx_row + j);
-        if (p >= 0 && p < a.S_kv) last = j;
-      }
+#pragma unroll
+      for (int u = 0; u < kMlaLooks; ++u)
+        if (look[u] >= 0 && look[u] < a.S_kv) last = threadIdx.x + u * kMlaThreads;
       last = __reduce_max_sync(0xffffffffu, last);
       if (lane == 0 && last >= 0) atomicMax(last_s, last);
       __syncthreads();
@@ -836,6 +843,7 @@ int make_tmap_2d_bytes(CUtensorMap* m, const void* base, uint64_t rows, uint64_t
 template <bool FP8_PAGED>
 static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaStream_t stream) {
   if (args.T == 0 || args.H == 0) return DSA_OK;
+  if (args.K > kMlaMaxK) return set_error(DSA_ERR_SHAPE, "sparse_mla: K (%d) exceeds %d", args.K, kMlaMaxK);
   MlaArgs a = args;
   CUtensorMap tq, to;
   int rc = make_tmap_2d_bytes(&tq, q, (uint64_t)a.T * a.H, kMlaDqk * 2, kMlaDqk * 2, 128, 128);

@@ -835,15 +835,22 @@ int make_tmap_2d_u8(CUtensorMap* m, const void* base, uint64_t rows, uint32_t ro
 
 // Key tiles per work unit.  Units are dealt to the CTAs round-robin: keep at least six rounds of them so that the last,
 // partly filled round costs little, by cutting the key range finer when there are few query blocks -- down to eight tiles,
-// below which a unit's own start shows.  A call that would leave SMs without a unit goes on cutting, to single tiles if need
-// be: a start on an idle SM costs nothing (2048 rows x 2048 keys of 4 heads x 64: 32 units of eight tiles took 63.0 us, 30.7 with 256 units of one;
-// one sequence of 2000 tokens, paged: one unit 9.8 us, four 6.0; seven of 33000: 63 units 15.0 us, 119 units 12.0).
+// below which a unit's own start shows.  A call that leaves SMs without a unit is cut further, to where the longest CTA has
+// least to do: its rounds times a unit's tiles plus one, which is about what a start costs.  Measured over 472 calls of 1 to
+// 2048 rows and 60 to 131072 keys at every cut, this is within 1 % of the best cut on average and nowhere slower than eight
+// tiles; cutting on until every SM has a unit was up to 18 % slower (257 rows x 2000 keys, 64 heads: 130 units of eight tiles
+// 11.8 us, 260 of four 13.1).  2048 rows x 2000 keys of 4 heads x 64: 32 units of eight tiles 51.6 us, 128 of two 18.7; paged,
+// one sequence of 2000 tokens: one unit 9.6 us, four 6.0; seven of 33000: 63 units 14.9 us, 119 units 10.5, 231 units 11.8.
 static int pick_chunk_tiles(int n_qblocks, int n_tiles) {
   auto units = [&](int chunk) { return (int64_t)n_qblocks * ((n_tiles + chunk - 1) / chunk); };
   int chunk = kChunkTiles;
   while (chunk > 8 && units(chunk) < 6LL * sm_count()) chunk /= 2;
-  while (chunk > 1 && units(chunk) < sm_count()) chunk /= 2;
-  return chunk;
+  if (units(chunk) >= sm_count()) return chunk;
+  auto cost = [&](int c) { return (units(c) + sm_count() - 1) / sm_count() * ((c < n_tiles ? c : n_tiles) + 1); };
+  int best = chunk;
+  for (int c = chunk / 2; c >= 1; c /= 2)
+    if (cost(c) < cost(best)) best = c;
+  return best;
 }
 
 template <int H, int D, int NQ, bool PAGED, int QB, int EPI>

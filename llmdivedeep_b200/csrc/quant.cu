@@ -11,69 +11,78 @@
 
 namespace dsa {
 
-// 16 consecutive values per thread, in 16-byte loads.
-template <typename T>
-__device__ __forceinline__ void load16(const T* __restrict__ src, float (&v)[16]) {
+// V (4 or 16) consecutive values per thread, in loads of 16 bytes (4 bf16 values: 8).
+template <int V, typename T>
+__device__ __forceinline__ void load_values(const T* __restrict__ src, float (&v)[V]) {
   if constexpr (sizeof(T) == 2) {
+    uint32_t w[V / 2];
+    if constexpr (V == 4) {
+      const uint2 raw = __ldg(reinterpret_cast<const uint2*>(src));
+      w[0] = raw.x; w[1] = raw.y;
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + h);
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {                    // bf16 -> fp32: the value is the upper half of the word
-        v[8 * h + 2 * i] = __uint_as_float(w[i] << 16);
-        v[8 * h + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      for (int h = 0; h < V / 8; ++h) {
+        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + h);
+        w[4 * h] = raw.x; w[4 * h + 1] = raw.y; w[4 * h + 2] = raw.z; w[4 * h + 3] = raw.w;
       }
+    }
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {                  // bf16 -> fp32: the value is the upper half of the word
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
   } else {
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int h = 0; h < V / 4; ++h) {
       const float4 raw = __ldg(reinterpret_cast<const float4*>(src) + h);
       v[4 * h] = raw.x; v[4 * h + 1] = raw.y; v[4 * h + 2] = raw.z; v[4 * h + 3] = raw.w;
     }
   }
 }
-// The scale of the block that LANES neighbouring lanes hold, and this thread's 16 values as e4m3.
-template <int LANES>
-__device__ __forceinline__ float quant16(const float (&v)[16], uint4& out) {
+// The scale of the block that LANES neighbouring lanes hold, and this thread's V values as e4m3.
+template <int LANES, int V>
+__device__ __forceinline__ float quant_values(const float (&v)[V], uint32_t (&w)[V / 4]) {
   float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  for (int i = 0; i < V; ++i) amax = fmaxf(amax, fabsf(v[i]));
 #pragma unroll
   for (int o = LANES / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   const float sc = __fdiv_rn(fmaxf(amax, 1e-6f), 448.f);
-  uint32_t w[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < V / 4; ++i) {
     const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * i], sc), __fdiv_rn(v[4 * i + 1], sc)), __NV_SATFINITE, __NV_E4M3);
     const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * i + 2], sc), __fdiv_rn(v[4 * i + 3], sc)), __NV_SATFINITE, __NV_E4M3);
     w[i] = lo | (hi << 16);
   }
-  out = make_uint4(w[0], w[1], w[2], w[3]);
   return sc;
 }
 
-// BLOCK / 16 threads per block of BLOCK values: three (two) shuffle steps instead of five, 16 bytes per load and store.
-// Bound by issue (the IEEE divisions) from a few thousand blocks on, by the launch below.
-// [32768, 64, 128] bf16: 253 us with one warp per block and 8-byte loads, 173 us so (4.7 TB/s = 0.72 of measured HBM).
-template <typename T, int BLOCK>
+// BLOCK / V threads per block of BLOCK values.  V = 16: three (two) shuffle steps instead of five, 16 bytes per load and
+// store; bound by issue (the IEEE divisions).  [32768, 64, 128] bf16: 253 us with one warp per block and 8-byte loads, 176 us so
+// (4.6 TB/s).  V = 4 for calls that are over in two or three microseconds: a thread's sixteen divisions in a row are then what
+// takes the time (100 blocks of 128 bf16 values 1.65 us, 1.9 with V = 16; 4800 blocks of fp32 2.3 and 2.6, of bf16 2.35 and 2.2).
+template <typename T, int BLOCK, int V>
 __global__ void __launch_bounds__(256) fp8_quant_kernel(const T* __restrict__ x, int64_t n_blocks,
                                                         uint8_t* __restrict__ q, float* __restrict__ scale, const int q_aligned) {
-  constexpr int LANES = BLOCK / 16;
+  constexpr int LANES = BLOCK / V;
   const int64_t n = n_blocks * LANES, stride = (int64_t)gridDim.x * blockDim.x;
   // whole warps stay together for the shuffles: the loop runs over warps' first threads
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
     const int64_t i = i0 + (threadIdx.x & 31);
-    float v[16] = {};
-    if (i < n) load16<T>(x + i * 16, v);
-    uint4 w;
-    const float sc = quant16<LANES>(v, w);
+    float v[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = 1.f;            // lanes past the end: dividing zeros takes the slow way, 2 us for the warp
+    if (i < n) load_values<V>(x + i * V, v);
+    uint32_t w[V / 4];
+    const float sc = quant_values<LANES, V>(v, w);
     if (i < n) {
-      if (q_aligned) {
-        reinterpret_cast<uint4*>(q)[i] = w;
+      uint32_t* o = reinterpret_cast<uint32_t*>(q) + i * (V / 4);
+      if constexpr (V == 4) {
+        *o = w[0];
+      } else if (q_aligned) {
+        *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
       } else {                                         // the caller's q starts on a 4-byte boundary only
-        uint32_t* o = reinterpret_cast<uint32_t*>(q) + i * 4;
-        o[0] = w.x; o[1] = w.y; o[2] = w.z; o[3] = w.w;
+        o[0] = w[0]; o[1] = w[1]; o[2] = w[2]; o[3] = w[3];
       }
       if (i % LANES == 0) scale[i / LANES] = sc;
     }
@@ -104,10 +113,10 @@ __global__ void __launch_bounds__(256) pack_latent_kernel(const T* __restrict__ 
       }
     }
     float v[16];
-    load16<T>(src + lane * 16, v);
-    uint4 w;
-    const float sc = quant16<8>(v, w);
-    reinterpret_cast<uint4*>(dst)[lane] = w;
+    load_values<16>(src + lane * 16, v);
+    uint32_t w[4];
+    const float sc = quant_values<8, 16>(v, w);
+    reinterpret_cast<uint4*>(dst)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
     if ((lane & 7) == 0) reinterpret_cast<float*>(dst + 512)[lane >> 3] = sc;
     if (lane < 8) reinterpret_cast<uint4*>(dst + 528)[lane] = rope;
   }
@@ -212,23 +221,26 @@ int rope_fp8_quant_launch(const void* x, int64_t n_rows, int head_dim, int rope_
   return check_launch("rope_fp8_quant");
 }
 
+template <typename T, int BLOCK>
+static void launch_fp8_quant(const void* x, int64_t n_blocks, void* q, float* scale, cudaStream_t stream) {
+  const int al = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+  const bool small = n_blocks * (BLOCK / 16) < (int64_t)sm_count() * (sizeof(T) == 2 ? 256 : 512);
+  const int64_t want = (n_blocks * (BLOCK / (small ? 4 : 16)) + 255) / 256, most = (int64_t)sm_count() * 16;
+  const int grid = (int)(want < most ? want : most);
+  const T* xt = static_cast<const T*>(x);
+  uint8_t* qt = static_cast<uint8_t*>(q);
+  if (small) fp8_quant_kernel<T, BLOCK, 4><<<grid, 256, 0, stream>>>(xt, n_blocks, qt, scale, al);
+  else fp8_quant_kernel<T, BLOCK, 16><<<grid, 256, 0, stream>>>(xt, n_blocks, qt, scale, al);
+}
+
 int fp8_quant_launch(const void* x, int x_is_bf16, int64_t n_blocks, int block, void* q, float* scale,
                      cudaStream_t stream) {
   if (n_blocks == 0) return DSA_OK;
-  const int64_t want = (n_blocks * (block / 16) + 255) / 256;
-  const int grid = (int)(want < (int64_t)sm_count() * 16 ? want : (int64_t)sm_count() * 16);
-  uint8_t* qo = static_cast<uint8_t*>(q);
-  const int al = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
-  if (block == 128 && x_is_bf16)
-    fp8_quant_kernel<__nv_bfloat16, 128><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), n_blocks, qo, scale, al);
-  else if (block == 128)
-    fp8_quant_kernel<float, 128><<<grid, 256, 0, stream>>>(static_cast<const float*>(x), n_blocks, qo, scale, al);
-  else if (block == 64 && x_is_bf16)
-    fp8_quant_kernel<__nv_bfloat16, 64><<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), n_blocks, qo, scale, al);
-  else if (block == 64)
-    fp8_quant_kernel<float, 64><<<grid, 256, 0, stream>>>(static_cast<const float*>(x), n_blocks, qo, scale, al);
-  else
-    return set_error(DSA_ERR_SHAPE, "fp8_quant: block size %d not supported (64 or 128)", block);
+  if (block == 128 && x_is_bf16) launch_fp8_quant<__nv_bfloat16, 128>(x, n_blocks, q, scale, stream);
+  else if (block == 128) launch_fp8_quant<float, 128>(x, n_blocks, q, scale, stream);
+  else if (block == 64 && x_is_bf16) launch_fp8_quant<__nv_bfloat16, 64>(x, n_blocks, q, scale, stream);
+  else if (block == 64) launch_fp8_quant<float, 64>(x, n_blocks, q, scale, stream);
+  else return set_error(DSA_ERR_SHAPE, "fp8_quant: block size %d not supported (64 or 128)", block);
   return check_launch("fp8_quant");
 }
 

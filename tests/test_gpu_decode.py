@@ -208,3 +208,18 @@ def test_smaller_batches_in_the_workspace_of_a_larger_one():
             assert float((out.float() - whole.float()).abs().max()) <= 2e-2
             assert not torch.isnan(out).any()
     ops.check_status("cuda")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("block", [64, 128])
+def test_quantiser_around_the_change_of_values_per_thread(block, dtype):
+    """Few blocks take four values a thread, many sixteen: the oracle's bytes and scales on both sides of the line, with zero
+    blocks among them."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    line = sms * (256 if dtype == torch.bfloat16 else 512) // (block // 16)
+    x = torch.randn(line + 1, block, generator=torch.Generator().manual_seed(block)).to(dtype)
+    x[::37] = 0
+    want_q, want_s = O.fp8_quant_per_block(x, block)
+    for n in (line - 1, line, line + 1):
+        q, s = ops.fp8_quant_per_block(x[:n].cuda(), block)
+        assert torch.equal(q.view(torch.uint8).cpu(), want_q[:n].view(torch.uint8)) and torch.equal(s.cpu().reshape(-1), want_s[:n].reshape(-1))

@@ -256,7 +256,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
 
   const int cta = blockIdx.x & 1, peer = cta ^ 1;              // rank in the cluster = V half = contraction part
   const int unit = blockIdx.x >> 1;
-  const int part = unit - a.n_full;                            // >= 0: a part of a split slot list
+  const int part = FP8_PAGED ? unit - a.n_full : -1;           // >= 0: a part of a split slot list (prefill's are never cut)
   const int n_split = part < 0 ? 1 : a.n_split, t = part < 0 ? unit : a.n_full + part / n_split, split = part < 0 ? 0 : part % n_split;
   const int hg = blockIdx.z;
   const int warp = warp_index(), lane = threadIdx.x & 31;

@@ -547,8 +547,8 @@ __global__ void fill_masked_kernel(const IndexerArgs a) {
 // ReLU is a multiply with saturation to [0, 1]: max(d, 0) would go to the ALU pipe at half rate, this goes to the FMA pipe
 // and, like max, turns a NaN into 0.  A dot product of 128 e4m3 pairs is at most 128 x 448^2 < 2^25 and at least 2^-18 when
 // it is not 0, so 2^-25 d is exact and never saturates above; the score takes the factor back at the end, exactly too unless
-// its terms are below 2^-101.  4096 x 65536: 2598 -> 2423 us (ncu before: ALU pipe 58 %, FMA pipe 18 %, issue slots 64 %); a
-// quarter of the columns left to the ALU 2432, half of them 2611.
+// its terms are below 2^-101.  4096 x 65536: 2595 -> 2410 us in short runs at full clock, 2850 -> 2735 under the power cap (ncu: ALU
+// pipe 58 -> 21 %, FMA pipe 18 -> 39 %, issue slots 64 -> 68 %); a quarter of the columns left to the ALU 2432, half of them 2611.
 constexpr float kReluScale = 0x1p-25f;
 struct RwCfg {
   static constexpr int H = 64, D = 128, NQ = 4, N = 256, KSTEPS = 4;

@@ -33,7 +33,10 @@
 // (a warp keeps about eight 512-byte requests going, whether cp.async or TMA gather4), arrivals by the copies themselves.
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137
 // cycles each; see dsa_common.cuh) and TMA gather; 3125 with warp-uniform issue; 2860 with two sets of softmax warps;
-// 2418 with sixteen and setmaxnreg; 2215 as it stands (1055 TFLOP/s).  Tried on top: the exchange by st.async (3320:
+// 2418 with sixteen and setmaxnreg; 2215 with this gather; 2266 as it stands, the exchange stage released by the data (1031
+// TFLOP/s; short runs at full clock -- at the power cap, 1600 MHz, 2607 against 3565).  That is N(0,1) data, whose maxima never
+// raise the reference by 8; q scaled by 2, 4 and 8 takes 2550, 2935 and 3030 us (first form 3635 to 3767): with scores that
+// wide some lane of a quadrant makes its warps rescale O in most blocks, on the way from the softmax to P.V.  Tried on top: the exchange by st.async (3320:
 // the stores drain slowly and clog the gather), by loads from the peer's shared memory (3560: the release at cluster
 // scope costs ~2300 cycles), a quarter of the exponentials as polynomials on the FMA pipe (+3 %: the issue slots are
 // short too).

@@ -1,7 +1,7 @@
 """dsa_sparse_mla_prefill / dsa_sparse_mla_decode_paged (through the C ABI) against the CPU oracle.
 
-Floating point: bf16 inputs, bf16 tensor-core products with fp32 accumulation, the two halves
-of every score rounded to fp16 between the CTAs of a pair, P rounded to bf16, bf16 output.  Tolerance (the one stated for this path): max-abs 2e-2 and mean-abs 2e-3
+Floating point: bf16 inputs, bf16 tensor-core products with fp32 accumulation, the other CTA's
+half of every score rounded to fp16 on its way between the pair, P rounded to bf16, bf16 output.  Tolerance (the one stated for this path): max-abs 2e-2 and mean-abs 2e-3
 against the oracle's fp32 computation on the same bf16 inputs.
 """
 import pytest
@@ -63,8 +63,8 @@ def test_large_scores_trigger_rescaling():
     kv = kv.to(torch.bfloat16)
     idx = torch.arange(K, dtype=torch.int32).repeat(T, 1)
     # scale 0.2: logits reach +-20 and the block maximum climbs by ~25 log2 units along the list (several rescales).
-    # The two halves of a score cross the CTA pair as fp16 (11 significant bits each), so the error of a logit grows
-    # with scale * |score|; DSA's own scale is 576^-0.5 or 192^-0.5, five to three times smaller than this one.
+    # The other CTA's half of a score arrives as fp16 (11 significant bits), so the error of a logit grows with
+    # scale * |score|; DSA's own scale is 576^-0.5 or 192^-0.5, five to three times smaller than this one.
     out = ops.sparse_mla_prefill(q.cuda(), kv.cuda(), idx.cuda(), 0.2)
     check(out, O.sparse_mla(q.float(), kv.float(), idx, 0.2))
 
@@ -135,7 +135,7 @@ def test_decode_paged_matches_oracle(B, H, P, K):
 
 def test_decode_holes_and_odd_block_counts():
     """Holes inside the slot list (empty slots are zero-filled rows with a cleared validity bit) and slot lists of one,
-    three and five 64-key blocks: the gather alternates between two raw stages and two sets of rope registers."""
+    three and five 64-key blocks: a gather warp alternates between two raw stages of its own."""
     for K in (40, 130, 300):
         g = torch.Generator().manual_seed(K)
         B, H, P = 3, 128, 6

@@ -342,7 +342,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       float m_a = -CUDART_INF_F, m_b = -CUDART_INF_F, l_a = 0.f, l_b = 0.f;     // sums: this lane's columns only
       for (int j = 0; j < n && ok; ++j, ++jt) {
         const int kb = __ldg(list + j);                       // requested before the wait: only its validity is needed
-        ok = __all_sync(0xffffffffu, mbar_wait(&s_full[jt & 1], (jt >> 1) & 1, abort_flag, a.status));
+        ok = mbar_wait_warp(&s_full[jt & 1], (jt >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         tc_fence_after();
         uint32_t sv[32];
@@ -376,7 +376,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           l_a *= f_a;
           l_b *= f_b;
           if (j > 0) {                                 // O must be quiescent: P.V of the previous block complete
-            ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[(jt - 1) & 1], ((jt - 1) >> 1) & 1, abort_flag, a.status));
+            ok = mbar_wait_warp(&pv_done[(jt - 1) & 1], ((jt - 1) >> 1) & 1, abort_flag, a.status);
             if (!ok) break;
             tc_fence_after();
 #pragma unroll 1
@@ -412,7 +412,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           l_b += s0 + s1;
         }
         if (jt > 1) {                                  // two P buffers: P.V of block jt-2 (of any unit) read this one
-          ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[jt & 1], ((jt >> 1) - 1) & 1, abort_flag, a.status));
+          ok = mbar_wait_warp(&pv_done[jt & 1], ((jt >> 1) - 1) & 1, abort_flag, a.status);
           if (!ok) break;
         }
         bs_store_rows(p_s + (jt & 1) * kBsPanelBytes, quad * 16, lane, pk);
@@ -421,7 +421,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[jt & 1]);
       }
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(o_final, nq & 1, abort_flag, a.status));
+      if (ok) ok = mbar_wait_warp(o_final, nq & 1, abort_flag, a.status);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll

@@ -72,8 +72,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Wait for `parity` on `bar`, giving up after `limit` polls.  Returns false (after
 // flagging) when the wait expired or another role already aborted.
+template <int UNROLL = 1>
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 int* status, uint32_t limit) {
+#pragma unroll UNROLL
   for (uint32_t i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if (i > kFastSpins) {
@@ -90,9 +92,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_limit(bar, parity, abort_flag, status, kSpinLimit);
 }
 
-// the same for a whole warp whose lanes all come here: one answer for all of them
+// The same for a whole warp whose lanes all come here: one answer for all of them.  The first look stands before the loop, so
+// that a wait which finds its phase complete costs a poll, a vote and a branch and leaves nothing to test behind it; with the
+// loop alone (which the compiler unrolls by four at every place) the indexer takes 2379 us for 4096 x 65536 instead of 2204, the
+// sparse MLA of 16 heads 1239 instead of 1183 (4096 x 2048 keys), block-sparse attention 247 instead of 244.
+template <int UNROLL = 1>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_limit<UNROLL>(bar, parity, abort_flag, status, kSpinLimit));
 }
 // ---- TMA (tiled bulk tensor copies, global -> this CTA's shared memory) ----
 __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, int y, uint64_t* bar) {

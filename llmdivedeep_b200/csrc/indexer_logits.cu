@@ -375,7 +375,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       int qb, nb, t_lo, t_hi;
       if (!unit_tiles<NQ, QB, PAGED>(a, u, n_qblocks, n_groups, qb, nb, t_lo, t_hi)) continue;
       const int ub = nu & 1;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status));
+      const bool ok = mbar_wait_warp(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
       if (!ok) break;
       float* wd = w_s + ub * QB * C::N;
       int2* wind = win_s + ub * C::NTOK;
@@ -432,7 +432,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       int qb, nb, t_lo, t_hi;
       if (!unit_tiles<NQ, QB, PAGED>(a, u, n_qblocks, n_groups, qb, nb, t_lo, t_hi)) continue;
       const int ub = nu & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&w_full[ub], (nu >> 1) & 1, abort_flag, a.status));
+      ok = mbar_wait_warp(&w_full[ub], (nu >> 1) & 1, abort_flag, a.status);
       if (!ok) break;
       // k_scale of the tile AHEAD tiles on travels global -> shared asynchronously into this thread's own slot
       // (paged: its cache row comes from the page rows the stager wrote, so it is a single fetch)
@@ -474,7 +474,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           const int2* my_win = win_s + ub * C::NTOK + b * NQ;
           float* grp_base = a.logits + (int64_t)g * NQ * a.ld;   // 32-bit offsets from here: NQ * ld < 2^31
           const int n_tok = min(NQ, a.T - g * NQ);
-          ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[stage], n_mine & 1, abort_flag, a.status));
+          ok = mbar_wait_warp(&acc_full[stage], n_mine & 1, abort_flag, a.status);
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
@@ -683,7 +683,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       int g, nb, t_lo, t_hi;
       if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
       const int ub = nu & 1;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status));
+      const bool ok = mbar_wait_warp(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
       if (!ok) break;
       float* wd = w_s + ub * C::N;
       const int t0 = g * C::NQ;
@@ -723,7 +723,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       int g, nb, t_lo, t_hi;
       if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
       const int ub = nu & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&w_full[ub], (nu >> 1) & 1, abort_flag, a.status));
+      ok = mbar_wait_warp(&w_full[ub], (nu >> 1) & 1, abort_flag, a.status);
       if (!ok) break;
       uint64_t wreg[C::H / 2];                   // this token's 64 head weights as 32 packed pairs, for the whole unit
       {
@@ -746,7 +746,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         // tile's work to arrive (the array is L2-resident), and nothing is carried from tile to tile
         const int s = kt * kTileKeys + row;              // key position
         const float kscale = s < a.S ? __ldg(a.k_scale + s) : 0.f;
-        ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[stage], (it >> 1) & 1, abort_flag, a.status));
+        ok = mbar_wait_warp(&acc_full[stage], (it >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         tc_fence_after();
         const uint32_t t_acc = t_lane + stage * C::N;

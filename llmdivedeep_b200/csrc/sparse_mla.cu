@@ -372,7 +372,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     {
       constexpr uint32_t idesc_qk = umma_idesc(1, 1, 0, 0, 128, kMlaBlk);
       constexpr uint32_t idesc_pv = umma_idesc(1, 1, 0, 1, 128, kMlaDvHalf);
-      bool ok = mbar_wait_warp(q_moved, 0, abort_flag, a.status);
+      bool ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);
       const uint64_t kdesc0 = umma_smem_desc(smem_u32(kv_s), 16, 1024, kSwz128);
       const uint64_t vdesc0 = umma_smem_desc(smem_u32(kv_s), kMlaKPanelBytes, 1024, kSwz128);
       const uint64_t rdesc0 = umma_smem_desc(smem_u32(kv_s + kMlaRopeOff), 16, 512, kSwz64);
@@ -414,13 +414,13 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // time for.  (Whatever is ready first, by polling three barriers: the same speed, and every look costs ~100 cycles.)
       for (int n = 0; n < nblk + 2 && ok; ++n) {
         if (n < nblk) {
-          ok = mbar_wait_warp(&kv_full[n % NB], (n / NB) & 1, abort_flag, a.status);
-          if (ok && n > 0) ok = mbar_wait_warp(s_free, (n - 1) & 1, abort_flag, a.status);
+          ok = mbar_wait_warp<4>(&kv_full[n % NB], (n / NB) & 1, abort_flag, a.status);
+          if (ok && n > 0) ok = mbar_wait_warp<4>(s_free, (n - 1) & 1, abort_flag, a.status);
           if (!ok) break;
           issue_qk(n);
         }
         if (n >= 2) {
-          ok = mbar_wait_warp(p_full, n & 1, abort_flag, a.status);
+          ok = mbar_wait_warp<4>(p_full, n & 1, abort_flag, a.status);
           if (!ok) break;
           pv_mmas(n - 2);
         }
@@ -455,8 +455,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
           id = -1;
         }
         nxt = load_pos(i + 1);
-        if (i == kQBuf0) ok = mbar_wait_warp(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
-        if (i >= NB) ok = mbar_wait_warp(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
+        if (i == kQBuf0) ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
+        if (i >= NB) ok = mbar_wait_warp<4>(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
         mark(i, id >= 0);
         uint8_t* dst = kv_s + kvb * kMlaKBytes;
@@ -534,8 +534,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         pa = pb;
         ta = table_entry(pa);
         pb = load_pos(i + 4);
-        if (i == kQBuf0) ok = mbar_wait_warp(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
-        if (i >= NB) ok = mbar_wait_warp(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
+        if (i == kQBuf0) ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
+        if (i >= NB) ok = mbar_wait_warp<4>(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
         mark(i, id_cur >= 0);
         id_cur = id_nxt;
@@ -573,7 +573,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const uint32_t peer_xchg_free = mapa_u32(smem_u32(xchg_free + warp), peer);
     const uint32_t peer_recv_full = mapa_u32(smem_u32(recv_full + warp), peer);
     float m = -CUDART_INF_F, l = 0.f;                  // m: reference of the last block seen; l: this thread's keys only
-    bool ok = mbar_wait_warp(q_full, 0, abort_flag, a.status);
+    bool ok = mbar_wait_warp<4>(q_full, 0, abort_flag, a.status);
     if (ok) {
       // this head's row of the five Q panels, swizzled shared memory -> packed bf16 pairs in tensor memory: the ten
       // half-panels (64 B) are dealt to the four threads of the head
@@ -609,7 +609,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     for (int n = qd < n_quad ? set : nblk; n < nblk && ok; n += 2) {
       const uint32_t ph = (n >> 1) & 1;
       uint32_t sv[32];                                 // this CTA's partial scores
-      ok = mbar_wait_warp(&s_full[set], ph, abort_flag, a.status);
+      ok = mbar_wait_warp<4>(&s_full[set], ph, abort_flag, a.status);
       if (!ok) break;
       tc_fence_after();
       tmem_ld32(t_row + kColS + 32 * hf, sv);
@@ -618,7 +618,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);              // the next block's scores may overwrite S now
       if (n > 0) {                                     // the peer has read block n-1: both stages are free
-        ok = mbar_wait_warp(&xchg_free[warp ^ 8], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mbar_wait_warp<4>(&xchg_free[warp ^ 8], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
       }
 #pragma unroll
@@ -632,13 +632,13 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       __syncwarp();
       // the reference of the block before, from that block's maxima: every thread follows the whole sequence by itself
       if (n > 0) {
-        ok = mbar_wait_warp(&pm_full[(set ^ 1) * 4 + qd], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mbar_wait_warp<4>(&pm_full[(set ^ 1) * 4 + qd], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
       }
       const float m_own = m;                           // what l is relative to
       if (n > 0) m = raise(m, pair_max(pm_of(n - 1)));
       const float m_prev = m;
-      ok = mbar_wait_warp(&recv_full[warp], ph, abort_flag, a.status);
+      ok = mbar_wait_warp<4>(&recv_full[warp], ph, abort_flag, a.status);
       if (!ok) break;
       float s[32];                                     // raw scores; the (positive) scale is folded into the exponent's FMA
 #pragma unroll
@@ -669,14 +669,14 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (lane == 0) mbar_arrive(&pm_full[set * 4 + qd]);
       mbar_arrive_remote_after(peer_xchg_free, top, lane == 0);      // the peer may send into this stage again
       if (lane == 0 && n + 2 < nblk) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
-      ok = mbar_wait_warp(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
+      ok = mbar_wait_warp<4>(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
       if (!ok) break;
       m = raise(m_prev, pair_max(pm_of(n)));
       if (m != m_own) l = m_own == -CUDART_INF_F ? 0.f : l * fast_exp2(m_own - m);
       bool waited_pv = n == 0;
       if (__any_sync(0xffffffffu, m != m_prev) && n > 0) {
         // O must be quiescent: P.V of the previous block has to be complete.  This thread scales its half of the columns.
-        ok = mbar_wait_warp(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mbar_wait_warp<4>(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         waited_pv = true;
         tc_fence_after();
@@ -709,7 +709,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         l += e + o;
       }
       if (!waited_pv) {                                // P is single-buffered: P.V of the previous block must be done
-        ok = mbar_wait_warp(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mbar_wait_warp<4>(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         tc_fence_after();
       }
@@ -721,7 +721,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
     if (ok) cluster_arrive();                          // nothing remote is left to do for this warp: the others need not wait for its output
     left = ok;
-    if (ok) ok = mbar_wait_warp(o_final, 0, abort_flag, a.status);
+    if (ok) ok = mbar_wait_warp<4>(o_final, 0, abort_flag, a.status);
     // A full group of 128 heads leaves through shared memory and TMA stores: four [128 heads x 128 B] panels in the
     // (now idle) first two KV buffers, written asynchronously in whole lines.  16-byte stores from the threads -- every
     // lane its own 1 KB-strided row -- cost about 4 % of the kernel.

@@ -646,35 +646,35 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
+    // The warp walks its loop as a whole and elects a lane for the instructions (dsa_common.cuh): 4096 x 65536 2222 -> 2173 us.
     constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, kTileKeys, C::N);
     uint32_t it = 0, nu = 0;
     for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
       int g, nb, t_lo, t_hi;
       if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
       const int qs = nu & 1;
-      bool ok = true;
-      if (lane == 0) {
-        ok = mbar_wait(&q_full[qs], (nu >> 1) & 1, abort_flag, a.status);
-        const uint64_t qdesc = umma_smem_desc(smem_u32(q_s + qs * C::Q_TILE_BYTES), 16, C::SBO, kSwz128);
-        for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
-          const int st = it % C::STAGES, acc = it & 1;
-          ok = mbar_wait(&k_full[st], (it / C::STAGES) & 1, abort_flag, a.status) &&
-               mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag, a.status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t kdesc = umma_smem_desc(smem_u32(k_s + st * C::K_TILE_BYTES), 16, C::SBO, kSwz128);
+      bool ok = mbar_wait_warp(&q_full[qs], (nu >> 1) & 1, abort_flag, a.status);
+      const uint64_t qdesc = umma_smem_desc(smem_u32(q_s + qs * C::Q_TILE_BYTES), 16, C::SBO, kSwz128);
+      for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
+        const int st = it % C::STAGES, acc = it & 1;
+        ok = mbar_wait_warp(&k_full[st], (it / C::STAGES) & 1, abort_flag, a.status) &&
+             mbar_wait_warp(&acc_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag, a.status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t kdesc = umma_smem_desc(smem_u32(k_s + st * C::K_TILE_BYTES), 16, C::SBO, kSwz128);
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < C::KSTEPS; ++k)
             umma_f8(tmem_base + acc * C::N, kdesc + (k * 32 >> 4), qdesc + (k * 32 >> 4), idesc, k > 0);
           umma_commit(&acc_full[acc]);
           umma_commit(&k_empty[st]);
         }
-        if (ok) umma_commit(&q_empty[qs]);
+        __syncwarp();
       }
-      ++nu;
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      it = __shfl_sync(0xffffffffu, it, 0);
       if (!ok) break;
+      if (elect_one()) umma_commit(&q_empty[qs]);
+      __syncwarp();
+      ++nu;
     }
   } else if (warp == 2) {
     // ------------------- stager: head weights and windows of the next unit -------------------

@@ -368,7 +368,7 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         }
         x_a *= a.scale_log2e;
         x_b *= a.scale_log2e;
-        const bool grow_a = x_a - m_a > 8.f, grow_b = x_b - m_b > 8.f;      // also true when m is still -inf and x is finite
+        const bool grow_a = x_a - m_a > kMaxRaise, grow_b = x_b - m_b > kMaxRaise;      // also true when m is still -inf and x is finite
         if (__any_sync(0xffffffffu, grow_a || grow_b)) {
           const float f_a = grow_a ? bs_exp2(m_a - x_a) : 1.f, f_b = grow_b ? bs_exp2(m_b - x_b) : 1.f;
           if (grow_a) m_a = x_a;
@@ -394,23 +394,18 @@ block_sparse_mha_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const float e_a = m_a == -CUDART_INF_F ? 0.f : m_a, e_b = m_b == -CUDART_INF_F ? 0.f : m_b;
         const uint64_t scale2 = pack_f32x2(a.scale_log2e, a.scale_log2e), ref_a = pack_f32x2(-e_a, -e_a), ref_b = pack_f32x2(-e_b, -e_b);
         uint32_t pk[16];
-        uint64_t sum_a = 0, sum_b = 0;
+        float sa0 = 0.f, sa1 = 0.f, sb0 = 0.f, sb1 = 0.f;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {                 // word i: row a (even) or b, columns 8 (i / 2) + 2 (t % 4), + 1
           float y0, y1;
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, (i & 1) ? ref_b : ref_a), y0, y1);
           const float p0 = bs_exp2(y0), p1 = bs_exp2(y1);
-          if (i & 1) sum_b = add_f32x2(sum_b, pack_f32x2(p0, p1));
-          else sum_a = add_f32x2(sum_a, pack_f32x2(p0, p1));
           pk[i] = bs_pack_bf16x2(p0, p1);
+          if (i & 1) add_bf16x2(pk[i], sb0, sb1);
+          else add_bf16x2(pk[i], sa0, sa1);
         }
-        {
-          float s0, s1;
-          unpack_f32x2(sum_a, s0, s1);
-          l_a += s0 + s1;
-          unpack_f32x2(sum_b, s0, s1);
-          l_b += s0 + s1;
-        }
+        l_a += sa0 + sa1;
+        l_b += sb0 + sb1;
         if (jt > 1) {                                  // two P buffers: P.V of block jt-2 (of any unit) read this one
           ok = mbar_wait_warp(&pv_done[jt & 1], ((jt >> 1) - 1) & 1, abort_flag, a.status);
           if (!ok) break;

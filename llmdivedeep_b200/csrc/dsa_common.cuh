@@ -19,6 +19,12 @@ enum : int {
   kStatusBadIndex = 2,        // a gathered index / page id was out of range (access skipped)
 };
 
+// By how much (log2 units) the scores of a row may exceed the softmax reference before it is raised.  Raising it rescales the
+// output accumulator in tensor memory between a softmax and its P.V, so it should be rare: P and the sums are then at most 2^32
+// and 2^43, as precise as near 1, and the accumulator overflows only where values beyond 2^84 are averaged.  With 8, 16, 24, 32
+// and 64, sparse MLA, 128 heads, 4096 x 2048 keys: q x 4 2943, 2580, 2237, 2216, 2236 us, q x 8 3040, 2945, 2853, 2567, 2206
+// (q x 1: 2210 to 2228 with all of them).
+constexpr float kMaxRaise = 32.f;
 constexpr uint32_t kFastSpins = 1u << 12;
 constexpr uint32_t kSpinLimit = 1u << 24;   // ~1 s with the back-off below
 
@@ -252,6 +258,12 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+
+// a pair of bf16 values added to a pair of fp32 values
+__device__ __forceinline__ void add_bf16x2(uint32_t v, float& x, float& y) {
+  asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, u, %1;\n\t}"
+      : "+f"(x), "+f"(y) : "r"(v));
 }
 
 // named barrier among `count` threads (ids 1..15; 0 is __syncthreads)

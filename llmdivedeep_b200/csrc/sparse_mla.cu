@@ -24,7 +24,10 @@
 //     +-65504 saturates on the way, for the receiving side only;
 //   * P is the A operand (from tensor memory) of O_c += P V_c (4 MMAs of N = 256) with the gathered
 //     panels read through an MN-major descriptor.
-// O is rescaled in tensor memory only when the running maximum grows by more than 8 (log2 units).
+// O is rescaled in tensor memory only when the running maximum grows by more than kMaxRaise (32 log2 units).  The row sums add up P as
+// it was rounded for the tensor core, so that the rounding of a key that dominates its row cancels in the quotient: error against
+// float64 2.16e-3 -> 2.11e-3 at q x 1, 2.40e-3 -> 2.04e-3 at q x 4 (of the tree before: sums of the unrounded P, reference raised
+// by 8), for 0.5 % of the time.
 //
 // What bounds it: the time a KV buffer is held.  A block's rows are needed from the scores to P.V, with the exchange
 // and the softmax in between; that round trip (gather 2400 cycles, scores 1000, exchange + softmax 3600, P.V with its
@@ -33,10 +36,10 @@
 // (a warp keeps about eight 512-byte requests going, whether cp.async or TMA gather4), arrivals by the copies themselves.
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137
 // cycles each; see dsa_common.cuh) and TMA gather; 3125 with warp-uniform issue; 2860 with two sets of softmax warps;
-// 2418 with sixteen and setmaxnreg; 2215 with this gather; 2266 as it stands, the exchange stage released by the data (1031
-// TFLOP/s; short runs at full clock -- at the power cap, 1600 MHz, 2607 against 3565).  That is N(0,1) data, whose maxima never
-// raise the reference by 8; q scaled by 2, 4 and 8 takes 2550, 2935 and 3030 us (first form 3635 to 3767): with scores that
-// wide some lane of a quadrant makes its warps rescale O in most blocks, on the way from the softmax to P.V.  Tried on top: the exchange by st.async (3320:
+// 2418 with sixteen and setmaxnreg; 2215 with this gather; 2266 with the exchange stage released by the data; 2180 with waits that
+// look once before they loop (1071 TFLOP/s; short runs at full clock -- at the power cap, 1600 MHz, 2530 against 3565).  q scaled by 2
+// and 4 takes the same; by 8, where maxima do outgrow the reference, 2570 us (with the reference raised by 8: 2550, 2935 and
+// 3030 us).  Tried on top: the exchange by st.async (3320:
 // the stores drain slowly and clog the gather), by loads from the peer's shared memory (3560: the release at cluster
 // scope costs ~2300 cycles), a quarter of the exponentials as polynomials on the FMA pipe (+3 %: the issue slots are
 // short too).
@@ -92,6 +95,11 @@ template <int R>
 __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+// Waits here loop unrolled by four: with the compact loop decode is 7 % slower (batch 64 68.6 us against 64.2, both with the first
+// look in front) and prefill the same.
+__device__ __forceinline__ bool mla_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  return mbar_wait_warp<4>(bar, parity, abort_flag, status);
+}
 constexpr int kMlaLooks = (kMlaMaxK + kMlaThreads - 1) / kMlaThreads;
 constexpr int kMlaBarBytes = 512;                  // mbarriers and a few words
 constexpr int kMlaPairBytes = 4 * 2 * 128 * 2;     // block maxima: [block mod 4][key half][head], bf16
@@ -372,7 +380,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     {
       constexpr uint32_t idesc_qk = umma_idesc(1, 1, 0, 0, 128, kMlaBlk);
       constexpr uint32_t idesc_pv = umma_idesc(1, 1, 0, 1, 128, kMlaDvHalf);
-      bool ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);
+      bool ok = mla_wait(q_moved, 0, abort_flag, a.status);
       const uint64_t kdesc0 = umma_smem_desc(smem_u32(kv_s), 16, 1024, kSwz128);
       const uint64_t vdesc0 = umma_smem_desc(smem_u32(kv_s), kMlaKPanelBytes, 1024, kSwz128);
       const uint64_t rdesc0 = umma_smem_desc(smem_u32(kv_s + kMlaRopeOff), 16, 512, kSwz64);
@@ -414,13 +422,13 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // time for.  (Whatever is ready first, by polling three barriers: the same speed, and every look costs ~100 cycles.)
       for (int n = 0; n < nblk + 2 && ok; ++n) {
         if (n < nblk) {
-          ok = mbar_wait_warp<4>(&kv_full[n % NB], (n / NB) & 1, abort_flag, a.status);
-          if (ok && n > 0) ok = mbar_wait_warp<4>(s_free, (n - 1) & 1, abort_flag, a.status);
+          ok = mla_wait(&kv_full[n % NB], (n / NB) & 1, abort_flag, a.status);
+          if (ok && n > 0) ok = mla_wait(s_free, (n - 1) & 1, abort_flag, a.status);
           if (!ok) break;
           issue_qk(n);
         }
         if (n >= 2) {
-          ok = mbar_wait_warp<4>(p_full, n & 1, abort_flag, a.status);
+          ok = mla_wait(p_full, n & 1, abort_flag, a.status);
           if (!ok) break;
           pv_mmas(n - 2);
         }
@@ -455,8 +463,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
           id = -1;
         }
         nxt = load_pos(i + 1);
-        if (i == kQBuf0) ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
-        if (i >= NB) ok = mbar_wait_warp<4>(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
+        if (i == kQBuf0) ok = mla_wait(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
+        if (i >= NB) ok = mla_wait(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
         mark(i, id >= 0);
         uint8_t* dst = kv_s + kvb * kMlaKBytes;
@@ -534,8 +542,8 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
         pa = pb;
         ta = table_entry(pa);
         pb = load_pos(i + 4);
-        if (i == kQBuf0) ok = mbar_wait_warp<4>(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
-        if (i >= NB) ok = mbar_wait_warp<4>(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
+        if (i == kQBuf0) ok = mla_wait(q_moved, 0, abort_flag, a.status);   // from here on the buffers held Q
+        if (i >= NB) ok = mla_wait(&kv_free[kvb], ((i / NB) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
         mark(i, id_cur >= 0);
         id_cur = id_nxt;
@@ -573,7 +581,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const uint32_t peer_xchg_free = mapa_u32(smem_u32(xchg_free + warp), peer);
     const uint32_t peer_recv_full = mapa_u32(smem_u32(recv_full + warp), peer);
     float m = -CUDART_INF_F, l = 0.f;                  // m: reference of the last block seen; l: this thread's keys only
-    bool ok = mbar_wait_warp<4>(q_full, 0, abort_flag, a.status);
+    bool ok = mla_wait(q_full, 0, abort_flag, a.status);
     if (ok) {
       // this head's row of the five Q panels, swizzled shared memory -> packed bf16 pairs in tensor memory: the ten
       // half-panels (64 B) are dealt to the four threads of the head
@@ -601,7 +609,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const uint32_t peer_recv = mapa_u32(smem_u32(recv), peer);
     // block maxima, four blocks deep: a warp may be two blocks behind its partner, never four (P.V orders them)
     auto pm_of = [&](int blk) -> uint16_t* { return pm_s + (blk & 3) * 256 + row; };      // [key half][head]
-    auto raise = [&](float m_old, float bmax) { return bmax - m_old > 8.f ? bmax : m_old; };   // -inf - -inf: stays
+    auto raise = [&](float m_old, float bmax) { return bmax - m_old > kMaxRaise ? bmax : m_old; };   // -inf - -inf: stays
     auto pair_max = [&](const uint16_t* pm) {
       return fmaxf(__uint_as_float(uint32_t(pm[0]) << 16), __uint_as_float(uint32_t(pm[128]) << 16));
     };
@@ -609,7 +617,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     for (int n = qd < n_quad ? set : nblk; n < nblk && ok; n += 2) {
       const uint32_t ph = (n >> 1) & 1;
       uint32_t sv[32];                                 // this CTA's partial scores
-      ok = mbar_wait_warp<4>(&s_full[set], ph, abort_flag, a.status);
+      ok = mla_wait(&s_full[set], ph, abort_flag, a.status);
       if (!ok) break;
       tc_fence_after();
       tmem_ld32(t_row + kColS + 32 * hf, sv);
@@ -618,7 +626,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);              // the next block's scores may overwrite S now
       if (n > 0) {                                     // the peer has read block n-1: both stages are free
-        ok = mbar_wait_warp<4>(&xchg_free[warp ^ 8], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mla_wait(&xchg_free[warp ^ 8], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
       }
 #pragma unroll
@@ -632,13 +640,13 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       __syncwarp();
       // the reference of the block before, from that block's maxima: every thread follows the whole sequence by itself
       if (n > 0) {
-        ok = mbar_wait_warp<4>(&pm_full[(set ^ 1) * 4 + qd], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mla_wait(&pm_full[(set ^ 1) * 4 + qd], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
       }
       const float m_own = m;                           // what l is relative to
       if (n > 0) m = raise(m, pair_max(pm_of(n - 1)));
       const float m_prev = m;
-      ok = mbar_wait_warp<4>(&recv_full[warp], ph, abort_flag, a.status);
+      ok = mla_wait(&recv_full[warp], ph, abort_flag, a.status);
       if (!ok) break;
       float s[32];                                     // raw scores; the (positive) scale is folded into the exponent's FMA
 #pragma unroll
@@ -669,14 +677,14 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (lane == 0) mbar_arrive(&pm_full[set * 4 + qd]);
       mbar_arrive_remote_after(peer_xchg_free, top, lane == 0);      // the peer may send into this stage again
       if (lane == 0 && n + 2 < nblk) mbar_expect_tx(&recv_full[warp], kMlaXWarp);
-      ok = mbar_wait_warp<4>(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
+      ok = mla_wait(&pm_full[set * 4 + qd], ph, abort_flag, a.status);
       if (!ok) break;
       m = raise(m_prev, pair_max(pm_of(n)));
       if (m != m_own) l = m_own == -CUDART_INF_F ? 0.f : l * fast_exp2(m_own - m);
       bool waited_pv = n == 0;
       if (__any_sync(0xffffffffu, m != m_prev) && n > 0) {
         // O must be quiescent: P.V of the previous block has to be complete.  This thread scales its half of the columns.
-        ok = mbar_wait_warp<4>(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mla_wait(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         waited_pv = true;
         tc_fence_after();
@@ -694,22 +702,18 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
       const float m_eff = (m == -CUDART_INF_F) ? 0.f : m;
       uint32_t pk[16];
       const uint64_t scale2 = pack_f32x2(a.scale_log2e, a.scale_log2e), m2 = pack_f32x2(-m_eff, -m_eff);
-      uint64_t ps[2] = {0, 0};                         // sums of the even and odd keys, two chains each
+      float ps[4] = {0.f, 0.f, 0.f, 0.f};              // sums of the even and odd keys, two chains each
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         float x0, x1;
         unpack_f32x2(fma_f32x2(pack_f32x2(s[i], s[i + 1]), scale2, m2), x0, x1);
         const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-        ps[(i >> 1) & 1] = add_f32x2(ps[(i >> 1) & 1], pack_f32x2(p0, p1));
         pk[i >> 1] = pack_bf16x2(p0, p1);
+        add_bf16x2(pk[i >> 1], ps[i & 2], ps[(i & 2) + 1]);
       }
-      {
-        float e, o;
-        unpack_f32x2(add_f32x2(ps[0], ps[1]), e, o);
-        l += e + o;
-      }
+      l += (ps[0] + ps[1]) + (ps[2] + ps[3]);
       if (!waited_pv) {                                // P is single-buffered: P.V of the previous block must be done
-        ok = mbar_wait_warp<4>(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+        ok = mla_wait(&pv_done[set ^ 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
         if (!ok) break;
         tc_fence_after();
       }
@@ -721,7 +725,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
     if (ok) cluster_arrive();                          // nothing remote is left to do for this warp: the others need not wait for its output
     left = ok;
-    if (ok) ok = mbar_wait_warp<4>(o_final, 0, abort_flag, a.status);
+    if (ok) ok = mla_wait(o_final, 0, abort_flag, a.status);
     // A full group of 128 heads leaves through shared memory and TMA stores: four [128 heads x 128 B] panels in the
     // (now idle) first two KV buffers, written asynchronously in whole lines.  16-byte stores from the threads -- every
     // lane its own 1 KB-strided row -- cost about 4 % of the kernel.

@@ -874,8 +874,12 @@ static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaSt
   return check_launch("sparse_mla");
 }
 
+int sparse_mla_few_launch(const void* q, const void* kv, const int32_t* idx, void* out, int T, int H, int S_kv, int K,
+                          float scale, int32_t* status, cudaStream_t stream);
+
 int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx, void* out, int T, int H, int S_kv,
                               int K, float scale, int32_t* status, cudaStream_t stream) {
+  if (H <= 32) return sparse_mla_few_launch(q, kv, idx, out, T, H, S_kv, K, scale, status, stream);
   MlaArgs a{};
   a.kv = static_cast<const uint8_t*>(kv);
   a.idx = idx;

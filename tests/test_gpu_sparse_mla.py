@@ -336,3 +336,39 @@ def test_last_used_slot_anywhere_in_the_list(form, K):
     ops.check_status("cuda")
     check(out, ref)
     assert float(out[T - 1].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("H", [1, 8, 15, 16, 17, 31, 32])
+@pytest.mark.parametrize("T,K", [(1, 1), (5, 64), (150, 65), (200, 177), (160, 2048)])
+def test_prefill_of_few_heads(H, T, K):
+    """Up to 32 heads go through the kernel with scores and output transposed (tiles of 16 and 32 heads): head counts around the
+    tiles, blocks and their remainders, more tokens than CTAs, holes, empty lists, scores wide enough to raise the references.
+    (The kernel of more heads sends partial scores as fp16: its bound at q x 8 also holds 2^-11 |partial| of the scores.)"""
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + T + K)
+    S, scale = 2500, 192 ** -0.5
+    kv = torch.randn(S, 576, device="cuda", generator=g).to(torch.bfloat16)
+    for wide in (1, 8):
+        q = (torch.randn(T, H, 576, device="cuda", generator=g) * wide).to(torch.bfloat16)
+        idx = _holes(torch.rand(T, S, device="cuda", generator=g).topk(K, dim=-1).indices.int(), g)
+        idx[T // 2] = -1
+        out = ops.sparse_mla_prefill(q, kv, idx, scale)
+        assert torch.equal(ops.sparse_mla_prefill(q, kv, idx, scale), out)
+        # a row does not depend on the call's other rows
+        assert torch.equal(ops.sparse_mla_prefill(q[-1:].contiguous(), kv, idx[-1:].contiguous(), scale), out[-1:])
+        ops.check_status("cuda")
+        rows = kv[idx.clamp_min(0).long()].double()
+        s = (torch.bmm(q.double(), rows.transpose(1, 2)) * scale).masked_fill((idx < 0).unsqueeze(1), float("-inf"))
+        ref = torch.bmm(s.softmax(-1).nan_to_num(0.0), rows[..., :512])
+        # bf16 P and outputs: 2^-9 of the largest value each (|v| < 6), and their sums
+        assert float((out.double() - ref).abs().max()) <= 6 * 2 ** -8 + 2 ** -9
+
+
+def test_prefill_of_few_heads_flags_positions_out_of_range():
+    q, kv, idx = make(9, 16, 300, 130, seed=4, causal=False)
+    bad = idx.clone()
+    bad[3, 70], bad[8, 129] = 300, 2 ** 31 - 1
+    out = ops.sparse_mla_prefill(q.cuda(), kv.cuda(), bad.cuda(), 0.06)
+    with pytest.raises(ops.DsaError, match="out of range"):
+        ops.check_status("cuda")
+    skipped = torch.where(bad >= 300, torch.full_like(bad, -1), bad)
+    check(out, O.sparse_mla(q.float(), kv.float(), skipped, 0.06))

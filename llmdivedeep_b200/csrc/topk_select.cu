@@ -1,29 +1,31 @@
 // Per-row top-k by radix select (sm_100a).  Stands in for the torch.topk calls at
 // sparse_attn/DSA.py:361, 567 and 675-676 of the reference.
 //
-// One CTA per row.  fp32 values are mapped to order-preserving 32-bit keys and
-// the k-th largest key is found digit by digit (12 + 12 + 8 bits):
-//   1. histogram the top 12 key bits of the row (shared-memory atomics), suffix-
-//      scan the bins to find the bin holding the k-th largest element;
-//   2. if that bin holds more than 2048 elements, repeat on the next digit over
-//      the row (only rows with tightly clustered values need this);
-//   3. one ordered pass over the row writes every element above the threshold
-//      bin straight to the output and stages the threshold bin's elements
-//      ("candidates") in shared memory, in column order;
-//   4. the remaining digits are resolved on the staged candidates, and a final
-//      ordered compaction emits candidates above the exact k-th key plus the
-//      first `need` candidates equal to it -- ties go to the lower column.
-// Compaction uses block prefix sums, never atomics, so the output is
-// bit-identical from run to run.  The row is read from HBM once; the second
-// read hits L2 (a 131072-column row is 512 KB).
-//
-// Long rows first try a single pass: a sample of the row (one 128-float block in
-// every 16 or more) is ranked in shared memory, a threshold a few standard
-// deviations below the sample's estimate of the k-th value is taken from it, and one
-// ordered pass stages every element at or above that threshold (at most 4096) as a
-// candidate; step 4 then runs on the candidates alone.  If the staged count turns
-// out below k or above 4096 the row falls back to steps 1-4, so the result never
-// depends on the sample.
+// One CTA per row.  fp32 values are mapped to order-preserving 32-bit keys.  Three ways to the same set (ties: lower column):
+//   * direct (rows of at most 8188 columns): the row stays in registers.  One histogram of 2048 equal bins over its range of
+//     VALUES -- they spread, where the leading bits of the keys pile up on a few exponents -- gives the bin of the k-th value;
+//     what lies above it leaves in column order, the bin's own few elements are ranked against one another.
+//   * sampled (longer rows): a sample of the row (one 128-float block in every 16, more of a row below 32768 columns) is ranked by the
+//     same kind of histogram, a threshold a few standard deviations below the sample's estimate of the k-th value is taken
+//     from it, and one ordered pass stages every element at or above it (at most 4096) and counts it by bins as it does; the
+//     select then reads the candidates once.
+//   * two passes, for what the others give up (a staged count that misses [k, 4096], infinities or NaN in the range, more than 256
+//     elements in the threshold bin, long unaligned rows): the k-th key digit by digit (12 + 12 + 8 bits):
+//       1. histogram the top 12 key bits of the row (shared-memory atomics), suffix-
+//          scan the bins to find the bin holding the k-th largest element;
+//       2. if that bin holds more than 2048 elements, repeat on the next digit over
+//          the row (only rows with tightly clustered values need this);
+//       3. one ordered pass over the row writes every element above the threshold
+//          bin straight to the output and stages the threshold bin's elements
+//          ("candidates") in shared memory, in column order;
+//       4. the remaining digits are resolved on the staged candidates, and a final
+//          ordered compaction emits candidates above the exact k-th key plus the
+//          first `need` candidates equal to it.
+// Compaction uses block prefix sums, never atomics, and no order depends on the number of threads, so a row's output is
+// the same from run to run and whatever the number of rows of the call.
+// What bounds it: latency, of the barriers between a row's steps.  us, against the form before (digit passes behind the sample, two
+// passes below 16384 columns), k = 2048: 7 rows of up to 33000 columns 13.5 -> 8.7, 64 x 131072 21.2 -> 13.3, 160 x 9000 15.0 -> 10.4, 2048 x 16384
+// causal 104 -> 71, 4096 x 32768 213 -> 172, 4096 x 131072 453 -> 400, 3000 x 3000 30 -> 19; 2048 x 2048, k = 256 42 -> 21.
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -33,30 +35,42 @@
 
 namespace dsa {
 
-constexpr int kTopkThreads = 512;
-constexpr int kTopkWarps = kTopkThreads / 32;
 constexpr int kDigitBits = 12;
-constexpr int kBins = 1 << kDigitBits;
-constexpr int kBinsPerThread = kBins / kTopkThreads;   // 8
+constexpr int kBins = 1 << kDigitBits;                 // digit passes
+constexpr int kLinBins = 2048;                         // one-pass histograms over a range of values
 constexpr int kCand = 2048;                            // two-pass path: largest threshold bin staged
-constexpr int kCandPerThread = kCand / kTopkThreads;   // 4
-constexpr int kCandS = 4096;                           // sampled path: candidate capacity
-constexpr int kCandSPerThread = kCandS / kTopkThreads; // 8
+constexpr int kCandS = 4096;                           // candidates that the sampled path may stage
+constexpr int kDirectChunk = 4096;
+constexpr int kDirectRow = 2 * kDirectChunk - 4;       // longest row without sample and staging (it may start three columns into a float4)
+constexpr int kTieCap = 256;                           // elements of the threshold bin that are ranked by counting
 constexpr int kSampleBlock = 128;                      // floats per sampled block (one float4 per lane)
 constexpr int kSampleMaxBlocks = 64;                   // at most 8192 sampled values
-constexpr int kSamplePerThread = kSampleMaxBlocks / kTopkWarps * 4;   // 16
-constexpr int kSampleMinRow = 16384;
-constexpr int kRun = 32;                               // sampled path: contiguous columns per thread per chunk
-constexpr int kChunkRun = kTopkThreads * kRun;                   // shorter rows take the two-pass path
+constexpr int kSampleWant = 16;                        // blocks wanted where a block in 16 gives fewer
+constexpr int kRun = 32;                               // sampled path: columns per thread per chunk
 constexpr int kVec = 4;
-constexpr int kEltPerThread = 16;                      // final pass: 4 x float4, contiguous
-constexpr int kChunkHist = kTopkThreads * kVec;        // histogram pass: coalesced float4
-constexpr int kChunkFinal = kTopkThreads * kEltPerThread;
+constexpr int kEltPerThread = 16;                      // two-pass path, final pass: 4 x float4, contiguous
 
 __device__ __forceinline__ uint32_t order_key(float x) {
   const uint32_t u = __float_as_uint(x);
   return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
 }
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float(key ^ (static_cast<uint32_t>(static_cast<int32_t>(~key) >> 31) | 0x80000000u));
+}
+
+// A range of values cut into kLinBins equal bins, counted from the top.  (hi - x) and its product with a positive factor are
+// monotone in floating point, so the bins order elements as their keys do; what lies above hi falls into bin 0, what lies below
+// the range into the last.  A NaN with the sign bit clear has the largest key and falls into bin 0, one with the sign bit set
+// must not come here.
+struct LinBins {
+  float hi, scale;
+  __device__ __forceinline__ bool set(float top, float bottom) {       // false: no usable range (all equal, infinite, NaN)
+    hi = top;
+    scale = static_cast<float>(kLinBins) / (top - bottom);
+    return top > bottom && scale > 0.f && scale < CUDART_INF_F;
+  }
+  __device__ __forceinline__ int of(float x) const { return max(0, min(kLinBins - 1, __float2int_rz((hi - x) * scale))); }
+};
 
 // hist and cand_key share storage: candidate keys are copied to registers (followed by a block
 // barrier) before the histogram is next cleared, and the histogram is dead while candidates are staged.
@@ -66,46 +80,53 @@ struct alignas(16) TopkSmem {
     uint32_t cand_key[kCandS];
   };
   int32_t cand_idx[kCandS];
-  uint32_t warp_tot[2][kTopkWarps];
+  union {
+    uint32_t lin[kLinBins];
+    struct { uint32_t key[kTieCap]; int32_t col[kTieCap]; } tie;       // the threshold bin's elements
+  };
+  uint32_t warp_tot[2][32];
   uint32_t bin, need, cnt;
 };
 static_assert(kBins == kCandS, "hist and cand_key are one array");
 
-__device__ __forceinline__ void zero_hist(TopkSmem& sm) {
-  uint4* h4 = reinterpret_cast<uint4*>(sm.hist);
+template <int TH, int BINS>
+__device__ __forceinline__ void zero_bins(uint32_t* hist) {
+  uint4* h4 = reinterpret_cast<uint4*>(hist);
 #pragma unroll
-  for (int b = threadIdx.x; b < kBins / 4; b += kTopkThreads) h4[b] = make_uint4(0u, 0u, 0u, 0u);
+  for (int b = threadIdx.x; b < BINS / 4; b += TH) h4[b] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Block-wide: given hist[], find the bin b with  sum(hist[b+1..]) < need <= sum(hist[b..]).
-// Leaves bin / need (remaining within the bin) / cnt (= hist[b]) in shared memory.
-__device__ __forceinline__ void find_threshold_bin(TopkSmem& sm, uint32_t need) {
+// Block-wide: given hist[], find the bin b with  sum(hist[b+1..]) < need <= sum(hist[b..]), or with FROM_TOP counting from bin 0:
+// sum(hist[..b-1]) < need <= sum(hist[..b]).  Leaves bin / need (remaining within the bin) / cnt (= hist[b]) in shared memory.
+template <int TH, int BINS, bool FROM_TOP>
+__device__ __forceinline__ void find_threshold_bin(TopkSmem& sm, const uint32_t* hist, uint32_t need) {
+  constexpr int PER = BINS / TH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t h[kBinsPerThread];
+  const int b0 = (FROM_TOP ? tid : TH - 1 - tid) * PER;  // threads in the order of the count
+  uint32_t h[PER];
   uint32_t mine = 0;
 #pragma unroll
-  for (int j = 0; j < kBinsPerThread; j += 4) {
-    const uint4 q = *reinterpret_cast<const uint4*>(&sm.hist[tid * kBinsPerThread + j]);
-    h[j] = q.x; h[j + 1] = q.y; h[j + 2] = q.z; h[j + 3] = q.w;
-    mine += q.x + q.y + q.z + q.w;
+  for (int j = 0; j < PER; ++j) {
+    h[j] = hist[FROM_TOP ? b0 + j : b0 + PER - 1 - j];
+    mine += h[j];
   }
-  uint32_t v = mine;                     // suffix-inclusive scan inside the warp
+  uint32_t v = mine;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const uint32_t nb = __shfl_down_sync(0xffffffffu, v, off);
-    if (lane + off < 32) v += nb;
+    const uint32_t nb = __shfl_up_sync(0xffffffffu, v, off);
+    if (lane >= off) v += nb;
   }
-  if (lane == 0) sm.warp_tot[0][warp] = v;
+  if (lane == 31) sm.warp_tot[0][warp] = v;
   __syncthreads();
-  uint32_t above = 0;
-  for (int w2 = warp + 1; w2 < kTopkWarps; ++w2) above += sm.warp_tot[0][w2];
-  const uint32_t incl = v + above;       // elements in bins >= first bin of this thread
-  uint32_t cum = incl - mine;            // elements in bins above this thread's
+  uint32_t wt = lane < warp ? sm.warp_tot[0][lane] : 0u;               // warps before this one
+  wt = __reduce_add_sync(0xffffffffu, wt);
+  const uint32_t incl = v + wt;
+  uint32_t cum = incl - mine;
   if (cum < need && need <= incl) {
 #pragma unroll
-    for (int j = kBinsPerThread - 1; j >= 0; --j) {
+    for (int j = 0; j < PER; ++j) {
       if (cum < need && cum + h[j] >= need) {
-        sm.bin = tid * kBinsPerThread + j;
+        sm.bin = FROM_TOP ? b0 + j : b0 + PER - 1 - j;
         sm.need = need - cum;
         sm.cnt = h[j];
       }
@@ -117,6 +138,7 @@ __device__ __forceinline__ void find_threshold_bin(TopkSmem& sm, uint32_t need) 
 
 // Exclusive block prefix of a packed (lo16, hi16) counter pair; also returns the block total.
 // `buf` alternates between calls so one __syncthreads per call is enough.
+template <int TH>
 __device__ __forceinline__ uint32_t block_exclusive_scan(TopkSmem& sm, uint32_t packed, int buf, uint32_t& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t incl = packed;
@@ -127,28 +149,21 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(TopkSmem& sm, uint32_t 
   }
   if (lane == 31) sm.warp_tot[buf][warp] = incl;
   __syncthreads();
-  uint32_t wt = lane < kTopkWarps ? sm.warp_tot[buf][lane] : 0u;
-  uint32_t winc = wt;
-#pragma unroll
-  for (int o = 1; o < kTopkWarps; o <<= 1) {
-    const uint32_t nb = __shfl_up_sync(0xffffffffu, winc, o);
-    if (lane >= o) winc += nb;
-  }
-  total = __shfl_sync(0xffffffffu, winc, kTopkWarps - 1);
-  const uint32_t before = __shfl_sync(0xffffffffu, winc - wt, warp);
-  return incl - packed + before;
+  const uint32_t wt = lane < TH / 32 ? sm.warp_tot[buf][lane] : 0u;
+  total = __reduce_add_sync(0xffffffffu, wt);          // the halves do not carry into each other: counts stay below 2^16
+  return incl - packed + __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
 }
 
 // Digit passes over keys held in registers (bit j of `valid` says whether ck[j] counts): refines
 // (prefix, pbits, need) 12 bits at a time until `stop_bits` key bits are decided.  Ends on a block barrier.
-template <int NPT>
+template <int TH, int NPT>
 __device__ __forceinline__ void digit_passes(TopkSmem& sm, const uint32_t (&ck)[NPT], uint32_t valid, uint32_t& prefix,
                                              int& pbits, uint32_t& need, int stop_bits) {
   while (pbits < stop_bits) {
     const int dbits = min(kDigitBits, 32 - pbits);
     const int shift = 32 - pbits - dbits;
     const uint32_t dmask = (1u << dbits) - 1u;
-    zero_hist(sm);
+    zero_bins<TH, kBins>(sm.hist);
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
@@ -156,7 +171,7 @@ __device__ __forceinline__ void digit_passes(TopkSmem& sm, const uint32_t (&ck)[
       if (((valid >> j) & 1u) && match) atomicAdd(&sm.hist[(ck[j] >> shift) & dmask], 1u);
     }
     __syncthreads();
-    find_threshold_bin(sm, need);
+    find_threshold_bin<TH, kBins, false>(sm, sm.hist, need);
     prefix = (pbits == 0 ? 0u : (prefix << dbits)) | sm.bin;
     need = sm.need;
     pbits += dbits;
@@ -166,7 +181,7 @@ __device__ __forceinline__ void digit_passes(TopkSmem& sm, const uint32_t (&ck)[
 
 // Ordered emission of staged candidates (thread t holds candidates [t*NPT, t*NPT+NPT) in column order):
 // those above the exact k-th key `kth` go to o[n_above...], the first `need` equal to it fill the tail.
-template <int NPT>
+template <int TH, int NPT>
 __device__ __forceinline__ void emit_candidates(TopkSmem& sm, const uint32_t (&ck)[NPT], uint32_t valid, uint32_t kth,
                                                 uint32_t need, uint32_t n_above, int k, int32_t* __restrict__ o) {
   const int tid = threadIdx.x;
@@ -179,7 +194,7 @@ __device__ __forceinline__ void emit_candidates(TopkSmem& sm, const uint32_t (&c
     }
   }
   uint32_t total;
-  const uint32_t excl = block_exclusive_scan(sm, __popc(fgt) | (__popc(feq) << 16), 0, total);
+  const uint32_t excl = block_exclusive_scan<TH>(sm, __popc(fgt) | (__popc(feq) << 16), 0, total);
   uint32_t pg = n_above + (excl & 0xffffu);
   uint32_t pe = excl >> 16;
 #pragma unroll
@@ -204,7 +219,7 @@ __device__ __forceinline__ bool at_or_above(float v, uint32_t tfb) {
   return NEG ? (u <= tfb) : (static_cast<int32_t>(u) >= static_cast<int32_t>(tfb));
 }
 
-// One 16384-column chunk of the sampled pass: warp w owns columns [w*1024, w*1024+1024) of the chunk and
+// One chunk (32 columns a thread) of the sampled pass: warp w owns columns [w*1024, w*1024+1024) of the chunk and
 // reads them as 8 coalesced float4 rows.  Returns the hit flags of this lane, bit q*4+e for column
 // wbase + q*128 + lane*4 + e.
 template <bool NEG>
@@ -235,234 +250,298 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* __restrict__ x, int
   return fc;
 }
 
-__device__ __forceinline__ uint32_t stage_hits(TopkSmem& sm, const float* __restrict__ x, int wbase, int lane,
-                                               uint32_t fc, uint32_t pc) {
+__device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* __restrict__ x, int wbase, int lane, uint32_t fc,
+                                           uint32_t pc, const LinBins& bins) {
   while (fc) {                               // few bits set: reload the hits (L1) rather than keep 32 values
     const int j = __ffs(fc) - 1;
     fc &= fc - 1;
     const int col = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
-    sm.cand_key[pc] = order_key(__ldg(x + col));
+    const float v = __ldg(x + col);
+    sm.cand_key[pc] = order_key(v);
     sm.cand_idx[pc] = col;
+    atomicAdd(&sm.lin[bins.of(v)], 1u);
     ++pc;
   }
-  return pc;
 }
 
-// The ordered pass of the sampled path: stages every element with key >= thr, two chunks per block scan.
-// Candidates end up in a fixed order (chunk, thread, column) that does not depend on timing.
+// The ordered pass of the sampled path: stages every element with key >= thr, two chunks per block scan, and counts them by
+// bins.  Candidates end up in a fixed order (1024 columns, lane, column) that does not depend on timing or on TH.
 // Returns the staged count, or 0xffffffff once it would exceed the capacity (uniform over the block).
-template <bool NEG>
-__device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t tfb) {
+template <int TH, bool NEG>
+__device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t tfb,
+                                              const LinBins& bins) {
+  constexpr int CHUNK = TH * kRun;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int base = lo & ~(kVec - 1);
-  const int n_pairs = (hi - base + 2 * kChunkRun - 1) / (2 * kChunkRun);
+  const int n_pairs = (hi - base + 2 * CHUNK - 1) / (2 * CHUNK);
   uint32_t staged = 0;
   for (int c = 0; c < n_pairs; ++c) {
-    const int wb0 = base + (2 * c) * kChunkRun + warp * (kRun * 32);
-    const int wb1 = wb0 + kChunkRun;
+    const int wb0 = base + (2 * c) * CHUNK + warp * (kRun * 32);
+    const int wb1 = wb0 + CHUNK;
     const uint32_t f0 = chunk_flags<NEG>(x, wb0, lane, lo, hi, tfb);
     const uint32_t f1 = chunk_flags<NEG>(x, wb1, lane, lo, hi, tfb);
     uint32_t total;
-    const uint32_t excl = block_exclusive_scan(sm, __popc(f0) | (__popc(f1) << 16), c & 1, total);
+    const uint32_t excl = block_exclusive_scan<TH>(sm, __popc(f0) | (__popc(f1) << 16), c & 1, total);
     const uint32_t t0 = total & 0xffffu, t1 = total >> 16;
     if (staged + t0 + t1 > (uint32_t)kCandS) return 0xffffffffu;   // every thread sees the same totals
-    stage_hits(sm, x, wb0, lane, f0, staged + (excl & 0xffffu));
-    stage_hits(sm, x, wb1, lane, f1, staged + t0 + (excl >> 16));
+    stage_hits(sm, x, wb0, lane, f0, staged + (excl & 0xffffu), bins);
+    stage_hits(sm, x, wb1, lane, f1, staged + t0 + (excl >> 16), bins);
     staged += t0 + t1;
   }
   __syncthreads();
   return staged;
 }
 
-// Emission for the sampled path, whose candidates are not in column order: candidates above the exact k-th
-// key `kth` first, then `need` of those equal to it -- the ones in the lowest columns, found by a second
-// radix select on the column numbers when there are more ties than wanted.
-template <int NPT>
-__device__ __forceinline__ void emit_unordered(TopkSmem& sm, const uint32_t (&ck)[NPT], uint32_t valid, uint32_t kth,
-                                               uint32_t need, int k, int32_t* __restrict__ o) {
-  const int tid = threadIdx.x;
-  uint32_t fgt = 0, feq = 0;
+// The k largest of a set of elements that sm.lin counts by `bins` (complete, a barrier behind it), in CHUNKS chunks: each(c, ck,
+// col) gives thread t's elements of a chunk (keys and columns; returns which of them count), in a fixed order over chunks,
+// threads and elements.  One look for the threshold bin; what lies above it leaves in that order, the bin's own few elements are
+// ranked against one another (ties: lower column first).  Returns false, for all threads alike and with nothing written, when
+// the bin holds too many.
+template <int TH, int NPT, int CHUNKS, typename Each>
+__device__ __forceinline__ bool select_by_bins(TopkSmem& sm, const LinBins& bins, int k, int32_t* __restrict__ o, const Each& each) {
+  find_threshold_bin<TH, kLinBins, true>(sm, sm.lin, (uint32_t)k);
+  const int b = sm.bin;
+  const uint32_t need = sm.need, cnt = sm.cnt, n_above = k - need;
+  if (cnt > (uint32_t)kTieCap) return false;
+  uint32_t pg = 0, pe = 0;                                // emitted and ranked elements of the chunks before
 #pragma unroll
-  for (int j = 0; j < NPT; ++j) {
-    if ((valid >> j) & 1u) {
-      fgt |= (uint32_t)(ck[j] > kth) << j;
-      feq |= (uint32_t)(ck[j] == kth) << j;
+  for (int c = 0; c < CHUNKS; ++c) {
+    uint32_t ck[NPT];
+    int32_t col[NPT];
+    const uint32_t valid = each(c, ck, col);
+    uint32_t fgt = 0, feq = 0;
+#pragma unroll
+    for (int j = 0; j < NPT; ++j) {
+      if ((valid >> j) & 1u) {
+        const int bj = bins.of(key_value(ck[j]));
+        fgt |= (uint32_t)(bj < b) << j;
+        feq |= (uint32_t)(bj == b) << j;
+      }
     }
+    uint32_t total;
+    const uint32_t excl = block_exclusive_scan<TH>(sm, __popc(fgt) | (__popc(feq) << 16), (c & 1) ^ 1, total);
+    uint32_t p = pg + (excl & 0xffffu), q = pe + (excl >> 16);
+#pragma unroll
+    for (int j = 0; j < NPT; ++j) {
+      if (fgt & (1u << j)) o[p++] = col[j];
+      if (feq & (1u << j)) {
+        sm.tie.key[q] = ck[j];
+        sm.tie.col[q++] = col[j];
+      }
+    }
+    pg += total & 0xffffu;
+    pe += total >> 16;
   }
-  uint32_t total;
-  uint32_t excl = block_exclusive_scan(sm, __popc(fgt) | (__popc(feq) << 16), 0, total);
-  uint32_t tkey[NPT];                         // complement of the column: lowest column = largest key
-#pragma unroll
-  for (int j = 0; j < NPT; ++j) tkey[j] = ~static_cast<uint32_t>(sm.cand_idx[tid * NPT + j]);
-  uint32_t pg = excl & 0xffffu;
-#pragma unroll
-  for (int j = 0; j < NPT; ++j)
-    if (fgt & (1u << j)) o[pg++] = static_cast<int32_t>(~tkey[j]);
-  if ((total >> 16) > need) {                 // uniform: more ties than wanted, keep the lowest columns
-    uint32_t prefix = 0, need2 = need;
-    int pbits = 0;
-    __syncthreads();                          // the scan above is done with warp_tot before hist work starts
-    digit_passes<NPT>(sm, tkey, feq, prefix, pbits, need2, 32);
-#pragma unroll
-    for (int j = 0; j < NPT; ++j)
-      if (tkey[j] < prefix) feq &= ~(1u << j);
-    excl = block_exclusive_scan(sm, __popc(feq) << 16, 1, total);
+  __syncthreads();
+  if (threadIdx.x < cnt) {
+    const uint32_t key = sm.tie.key[threadIdx.x];
+    const int32_t c = sm.tie.col[threadIdx.x];
+    uint32_t rank = 0;
+    for (uint32_t i = 0; i < cnt; ++i) {
+      const uint32_t ki = sm.tie.key[i];
+      rank += ki > key || (ki == key && sm.tie.col[i] < c);
+    }
+    if (rank < need) o[n_above + rank] = c;
   }
-  uint32_t pe = k - need + (excl >> 16);
-#pragma unroll
-  for (int j = 0; j < NPT; ++j)
-    if (feq & (1u << j)) o[pe++] = static_cast<int32_t>(~tkey[j]);
+  return true;
 }
 
-// The threshold of the sampled pass: the key a few standard deviations below the sample's estimate of the k-th value.
-// Returns false (for every thread of the block alike) when the geometry of the row rules the sampled pass out.  The
-// result depends on the row alone, so every CTA that evaluates it for one row gets the same key.
+// The threshold of the sampled pass: a value a few standard deviations below the sample's estimate of the k-th, and the bins
+// that its candidates are counted by.  Returns false (for every thread of the block alike) when the row rules the sampled pass
+// out.  The result depends on the row alone, not on TH.  Leaves sm.lin zeroed (a barrier has to follow).
+template <int TH>
 __device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, int k,
-                                                 uint32_t& thr_out) {
+                                                 float& thr_out, LinBins& bins_out) {
+  constexpr int NPT = kSampleMaxBlocks / (TH / 32) * 4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = hi - lo;
   const int first = (lo + kVec - 1) & ~(kVec - 1);
   const int nblk = (hi - first) / kSampleBlock;
-  const int sb = max(16, (nblk + kSampleMaxBlocks - 1) / kSampleMaxBlocks);   // one block sampled in every sb
-  const int mblk = nblk / sb;
+  // one block sampled in every sb: one in 16, fewer of a very long row, more of a short one
+  const int sb = max(min(16, nblk / kSampleWant), (nblk + kSampleMaxBlocks - 1) / kSampleMaxBlocks);
+  const int mblk = sb > 0 ? nblk / sb : 0;
   const int m = mblk * kSampleBlock;
   const float frac = (float)m / (float)n;
   const float mu = (float)k * frac;                       // top-k elements expected inside the sample
   const float rf = ceilf(mu + 4.f * sqrtf(mu) + 2.f);     // rank taken: about 4 sigma below the k-th value
   if (m < 1024 || rf > (float)m || rf > 0.8f * (float)kCandS * frac) return false;
 
-  // ---- sample: up to 4 blocks per warp, one float4 per lane -----------------------
-  uint32_t skey[kSamplePerThread];
-  uint32_t svalid = 0;
+  uint32_t skey[NPT];
+  uint32_t svalid = 0, kmax = 0, kmin = 0xffffffffu;
 #pragma unroll
-  for (int i = 0; i < kSamplePerThread / 4; ++i) {
-    const int j = warp + kTopkWarps * i;
+  for (int i = 0; i < NPT / 4; ++i) {
+    const int j = warp + TH / 32 * i;
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < mblk) {
+    const bool in = j < mblk;
+    if (in) {
       f = __ldg(reinterpret_cast<const float4*>(x + first + (j * sb + sb / 2) * kSampleBlock + lane * kVec));
       svalid |= 0xFu << (4 * i);
     }
     skey[4 * i + 0] = order_key(f.x); skey[4 * i + 1] = order_key(f.y);
     skey[4 * i + 2] = order_key(f.z); skey[4 * i + 3] = order_key(f.w);
-  }
-  // The rf-th largest sample key, to 4096 key steps, in one histogram pass: bins count down from a
-  // base near the top of the sample (the smallest of the warps' maxima, which one outlier cannot move),
-  // so the digits are mantissa bits and spread over the bins.  Keys more than 2^24 steps below the base
-  // are left out; if fewer than rf keys remain the generic digit passes take over.
-  uint32_t wmax = 0;
+    if (in) {
 #pragma unroll
-  for (int j = 0; j < kSamplePerThread; ++j)
-    if ((svalid >> j) & 1u) wmax = max(wmax, skey[j]);
-  wmax = __reduce_max_sync(0xffffffffu, wmax);
-  if (lane == 0) sm.warp_tot[0][warp] = (svalid != 0u) ? wmax : 0xffffffffu;
-  if (tid == 0) sm.bin = 0xffffffffu;
-  zero_hist(sm);
-  __syncthreads();
-  const uint32_t key_base = __reduce_min_sync(0xffffffffu, lane < kTopkWarps ? sm.warp_tot[0][lane] : 0xffffffffu);
-#pragma unroll
-  for (int j = 0; j < kSamplePerThread; ++j) {
-    if ((svalid >> j) & 1u) {
-      if (skey[j] >= key_base) {
-        atomicAdd(&sm.hist[kBins - 1], 1u);
-      } else {
-        const uint32_t q = (key_base - skey[j] - 1u) >> 12;
-        if (q < (uint32_t)(kBins - 1)) atomicAdd(&sm.hist[kBins - 2 - q], 1u);
+      for (int e = 0; e < 4; ++e) {
+        kmax = max(kmax, skey[4 * i + e]);
+        kmin = min(kmin, skey[4 * i + e]);
       }
     }
   }
-  __syncthreads();
-  uint32_t prefix = 0, need = (uint32_t)rf;
-  int pbits = 0;
-  find_threshold_bin(sm, need);
-  uint32_t thr;
-  if (sm.bin != 0xffffffffu) {
-    const uint32_t below = (uint32_t)(kBins - 1 - sm.bin) << 12;       // lower edge of the bin, in key steps below the base
-    thr = key_base > below ? key_base - below : 0u;
-    __syncthreads();
-  } else {
-    __syncthreads();
-    digit_passes<kSamplePerThread>(sm, skey, svalid, prefix, pbits, need, 24);
-    thr = prefix << 8;                                    // lower edge of the 24-bit bin of the sample's rf-th key
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  if (lane == 0) {
+    sm.warp_tot[0][warp] = kmax;
+    sm.warp_tot[1][warp] = kmin;
   }
+  zero_bins<TH, kLinBins>(sm.lin);
+  __syncthreads();
+  kmax = __reduce_max_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[0][lane] : 0u);
+  kmin = __reduce_min_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[1][lane] : 0xffffffffu);
+  const float top = key_value(kmax), bottom = key_value(kmin);
+  LinBins bins;
+  if (!bins.set(top, bottom)) return false;               // a NaN makes it false too, whatever its sign
+#pragma unroll
+  for (int j = 0; j < NPT; ++j)
+    if ((svalid >> j) & 1u) atomicAdd(&sm.lin[bins.of(key_value(skey[j]))], 1u);
+  __syncthreads();
+  find_threshold_bin<TH, kLinBins, true>(sm, sm.lin, (uint32_t)rf);
+  const float thr = top - (float)(sm.bin + 1) * ((top - bottom) * (1.f / kLinBins));     // the bin's lower edge, give or take a rounding
+  zero_bins<TH, kLinBins>(sm.lin);                        // for the candidates (all have read the counts)
   thr_out = thr;
-  return true;
+  return bins_out.set(top, thr);
 }
 
-// One ordered pass over columns [lo, hi) of the row: stages everything whose key is at or above thr.
+// One ordered pass over columns [lo, hi) of the row: stages everything whose key is at or above thr's.
 // Returns the staged count, or 0xffffffff once it would exceed the capacity (uniform over the block).
-__device__ __forceinline__ uint32_t stage_above(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t thr) {
+template <int TH>
+__device__ __forceinline__ uint32_t stage_above(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t thr,
+                                                const LinBins& bins) {
   const bool neg = (thr & 0x80000000u) == 0u;             // the threshold is a negative float
   const uint32_t tfb = neg ? ~thr : (thr ^ 0x80000000u);  // its bits as a float
-  return neg ? stage_row<true>(sm, x, lo, hi, tfb) : stage_row<false>(sm, x, lo, hi, tfb);
-}
-
-// The exact k-th key among `staged` candidates (all with key >= thr, in any order) and the output.
-// Offsets d = key - thr are >= 0; when all are below 2^24 (floats within a few binades of the
-// threshold) two 12-bit passes over d << 8 settle it, and their digits are mantissa bits, which
-// spread over the histogram instead of piling onto a few exponent bins.
-__device__ __forceinline__ void select_among_staged(TopkSmem& sm, uint32_t staged, uint32_t thr, int k,
-                                                    int32_t* __restrict__ o) {
-  const int tid = threadIdx.x;
-  uint32_t prefix, need;
-  int pbits;
-  uint32_t ck[kCandSPerThread];
-  uint32_t valid = 0;
-  int wide = 0;
-#pragma unroll
-  for (int j = 0; j < kCandSPerThread; ++j) {
-    const uint32_t a = tid * kCandSPerThread + j;
-    const bool ok = a < staged;
-    ck[j] = ok ? sm.cand_key[a] - thr : 0u;
-    valid |= (uint32_t)ok << j;
-    wide |= (ck[j] >> 24) != 0u;
-  }
-  wide = __syncthreads_or(wide);                           // also: keys are in registers, hist may reuse the storage
-  prefix = 0; pbits = 0; need = (uint32_t)k;
-  uint32_t kth_off;
-  if (!wide) {
-#pragma unroll
-    for (int j = 0; j < kCandSPerThread; ++j) ck[j] <<= 8;
-    digit_passes<kCandSPerThread>(sm, ck, valid, prefix, pbits, need, 24);
-    kth_off = prefix << 8;
-  } else {
-    digit_passes<kCandSPerThread>(sm, ck, valid, prefix, pbits, need, 32);
-    kth_off = prefix;
-  }
-  emit_unordered<kCandSPerThread>(sm, ck, valid, kth_off, need, k, o);
+  return neg ? stage_row<TH, true>(sm, x, lo, hi, tfb, bins) : stage_row<TH, false>(sm, x, lo, hi, tfb, bins);
 }
 
 // Single pass over a long row, steered by a sample.  Returns false (for every thread of the block alike)
 // when the row has to take the two-pass path: geometry out of range, or the staged count missed [k, 4096].
 // Needs 16-byte aligned rows.
+template <int TH>
 __device__ __forceinline__ bool sampled_single_pass(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, int k,
                                                     int32_t* __restrict__ o) {
-  uint32_t thr;
-  if (!sample_threshold(sm, x, lo, hi, k, thr)) return false;
-  const uint32_t staged = stage_above(sm, x, lo, hi, thr);
+  constexpr int NPT = kCandS / TH;
+  float thr;
+  LinBins bins;
+  if (!sample_threshold<TH>(sm, x, lo, hi, k, thr, bins)) return false;
+  const uint32_t staged = stage_above<TH>(sm, x, lo, hi, order_key(thr), bins);
   if (staged == 0xffffffffu || staged < (uint32_t)k) return false;   // missed [k, capacity]: two-pass path
-  select_among_staged(sm, staged, thr, k, o);
-  return true;
+  return select_by_bins<TH, NPT, 1>(sm, bins, k, o, [&](int, uint32_t(&ck)[NPT], int32_t(&col)[NPT]) {
+    uint32_t valid = 0;
+#pragma unroll
+    for (int j = 0; j < NPT; j += 4) {
+      const uint32_t a = threadIdx.x * NPT + j;
+      const uint4 q = *reinterpret_cast<const uint4*>(&sm.cand_key[a]);
+      const int4 c = *reinterpret_cast<const int4*>(&sm.cand_idx[a]);
+      ck[j] = q.x; ck[j + 1] = q.y; ck[j + 2] = q.z; ck[j + 3] = q.w;
+      col[j] = c.x; col[j + 1] = c.y; col[j + 2] = c.z; col[j + 3] = c.w;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) valid |= (uint32_t)(a + e < staged) << (j + e);
+    }
+    return valid;
+  });
+}
+
+// A row of at most CHUNKS x 4096 - 4 columns, without a sample or staging: it stays in registers, chunks of 4096 columns, thread
+// order = column order.  Returns false, for all threads alike, when the values have no usable range (infinities, NaN, all equal)
+// or the threshold bin holds too many: the two-pass path settles those.
+template <int TH, int CHUNKS>
+__device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* __restrict__ x, bool vec, int lo, int hi, int k,
+                                           int32_t* __restrict__ o) {
+  constexpr int NPT = kDirectChunk / TH;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = (lo & ~(kVec - 1)) + tid * NPT;
+  auto used = [&](int c, int j) { return i0 + c * kDirectChunk + j >= lo && i0 + c * kDirectChunk + j < hi; };
+  uint32_t key[CHUNKS][NPT], kmax = 0, kmin = 0xffffffffu;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const float* xc = x + c * kDirectChunk;
+#pragma unroll
+    for (int j = 0; j < NPT; j += kVec) {
+      float v[kVec] = {0.f, 0.f, 0.f, 0.f};
+      if (vec) {                                          // a float4 that starts below hi lies inside the row's allocation
+        if (i0 + c * kDirectChunk + j < hi) {
+          const float4 f = __ldg(reinterpret_cast<const float4*>(xc + i0 + j));
+          v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
+          if (used(c, j + e)) v[e] = __ldg(xc + i0 + j + e);
+      }
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) key[c][j + e] = order_key(v[e]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+    for (int j = 0; j < NPT; ++j)
+      if (used(c, j)) {
+        kmax = max(kmax, key[c][j]);
+        kmin = min(kmin, key[c][j]);
+      }
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  if (lane == 0) {
+    sm.warp_tot[0][warp] = kmax;
+    sm.warp_tot[1][warp] = kmin;
+  }
+  zero_bins<TH, kLinBins>(sm.lin);
+  __syncthreads();
+  kmax = __reduce_max_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[0][lane] : 0u);
+  kmin = __reduce_min_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[1][lane] : 0xffffffffu);
+  LinBins bins;
+  if (!bins.set(key_value(kmax), key_value(kmin))) return false;       // a NaN makes it false too, whatever its sign
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+    for (int j = 0; j < NPT; ++j)
+      if (used(c, j)) atomicAdd(&sm.lin[bins.of(key_value(key[c][j]))], 1u);
+  __syncthreads();
+  return select_by_bins<TH, NPT, CHUNKS>(sm, bins, k, o, [&](int c, uint32_t(&ck)[NPT], int32_t(&col)[NPT]) {
+    uint32_t valid = 0;
+#pragma unroll
+    for (int j = 0; j < NPT; ++j) {
+      ck[j] = key[c][j];
+      col[j] = i0 + c * kDirectChunk + j;
+      valid |= (uint32_t)used(c, j) << j;
+    }
+    return valid;
+  });
 }
 
 // One row, one CTA: the whole selection.
+template <int TH>
 __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__ logits, int64_t ld,
                                          const int32_t* __restrict__ ks, const int32_t* __restrict__ ke, int S, int k,
-                                         int32_t* __restrict__ out, int sample, int row) {
+                                         int32_t* __restrict__ out, int one_pass, int row) {
+  constexpr int kChunkHist = TH * kVec, kChunkFinal = TH * kEltPerThread, kCandPerThread = kCand / TH;
   const int tid = threadIdx.x;
   const int lo = ks ? max(ks[row], 0) : 0;
   const int hi = ke ? min(ke[row], S) : S;
   const int n = max(hi - lo, 0);
   int32_t* o = out + (int64_t)row * k;
   if (n <= k) {
-    for (int j = tid; j < k; j += kTopkThreads) o[j] = j < n ? lo + j : -1;
+    for (int j = tid; j < k; j += TH) o[j] = j < n ? lo + j : -1;
     return;
   }
   const float* x = logits + (int64_t)row * ld;
   const bool vec = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && (ld % kVec == 0);
   const int base = lo & ~(kVec - 1);           // chunk origin: multiple of 4, <= lo
 
-  if (vec && n >= kSampleMinRow && sample) {
-    if (sampled_single_pass(sm, x, lo, hi, k, o)) return;
+  if (one_pass && (n <= kDirectRow || vec)) {
+    if (n <= kDirectChunk - 4 ? direct_row<TH, 1>(sm, x, vec, lo, hi, k, o)
+        : n <= kDirectRow     ? direct_row<TH, 2>(sm, x, vec, lo, hi, k, o)
+                              : sampled_single_pass<TH>(sm, x, lo, hi, k, o))
+      return;
     __syncthreads();
   }
 
@@ -476,7 +555,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
     const int dbits = min(kDigitBits, 32 - pbits);
     const int shift = 32 - pbits - dbits;
     const uint32_t dmask = (1u << dbits) - 1u;
-    for (int b = tid; b < kBins; b += kTopkThreads) sm.hist[b] = 0;
+    for (int b = tid; b < kBins; b += TH) sm.hist[b] = 0;
     __syncthreads();
     if (vec) {
       // interior float4s need no window test; the (at most two) edge float4s do
@@ -513,13 +592,13 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     } else {
-      for (int i = lo + tid; i < hi; i += kTopkThreads) {
+      for (int i = lo + tid; i < hi; i += TH) {
         const uint32_t key = order_key(__ldg(x + i));
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     }
     __syncthreads();
-    find_threshold_bin(sm, need);
+    find_threshold_bin<TH, kBins, false>(sm, sm.hist, need);
     prefix = (pbits == 0 ? 0u : (prefix << dbits)) | sm.bin;
     need = sm.need;
     cnt = sm.cnt;
@@ -562,7 +641,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
     }
     const uint32_t packed = __popc(fsel) | (__popc(fcand) << 16);
     uint32_t total;
-    const uint32_t excl = block_exclusive_scan(sm, packed, c & 1, total);
+    const uint32_t excl = block_exclusive_scan<TH>(sm, packed, c & 1, total);
     if (fsel | fcand) {
       uint32_t ps = base_sel + (excl & 0xffffu);
       uint32_t pc = base_cand + (excl >> 16);
@@ -597,29 +676,29 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
     valid |= (uint32_t)(a < cnt) << j;
   }
   __syncthreads();                                      // keys are in registers: hist may reuse the storage
-  digit_passes<kCandPerThread>(sm, ck, valid, prefix, pbits, need, 32);
+  digit_passes<TH, kCandPerThread>(sm, ck, valid, prefix, pbits, need, 32);
   // prefix is now the exact k-th largest key; `need` of the candidates equal to it are wanted.
   // Output layout: [0, n_above) above the bin, then candidates > key, then the `need` tied ones.
-  emit_candidates<kCandPerThread>(sm, ck, valid, prefix, need, n_above, k, o);
+  emit_candidates<TH, kCandPerThread>(sm, ck, valid, prefix, need, n_above, k, o);
 }
 
-__global__ void __launch_bounds__(kTopkThreads, 3)
+template <int TH, int PER_SM>
+__global__ void __launch_bounds__(TH, PER_SM)
 topk_select_kernel(const float* __restrict__ logits, int64_t ld, const int32_t* __restrict__ ks,
-                   const int32_t* __restrict__ ke, int T, int S, int k, int32_t* __restrict__ out, int sample) {
+                   const int32_t* __restrict__ ke, int S, int k, int32_t* __restrict__ out, int one_pass) {
   __shared__ TopkSmem sm;
-  topk_row(sm, logits, ld, ks, ke, S, k, out, sample, blockIdx.x);
+  topk_row<TH>(sm, logits, ld, ks, ke, S, k, out, one_pass, blockIdx.x);
 }
 
 // sample = 0 forces the two-pass path on every row (the test hook that pits the two paths against each other)
 int topk_select_launch(const float* logits, int64_t ld, const int32_t* ks, const int32_t* ke, int T, int S, int k,
                        int32_t* out, int sample, cudaStream_t stream) {
   if (T == 0 || k == 0) return DSA_OK;
-  // (Tried for few long rows, i.e. decode: a cluster of four CTAs per row, each staging a quarter of the columns and
-  // CTA 0 collecting the candidates through distributed shared memory.  Same output, order included, and 22.2 us
-  // against 23.0 for 64 rows of 131072.  In cycles per row: one CTA spends 5600 on the sample and threshold, 22200 on
-  // the staging pass, 9900 on the exact select and the output; the cluster 6100 + 7100 + 10800, but also 3500 in its
-  // two cluster barriers and 4100 pulling ~2100 candidates across.)
-  topk_select_kernel<<<T, kTopkThreads, 0, stream>>>(logits, ld, ks, ke, T, S, k, out, sample);
+  // Up to one row per SM a row has 1024 threads, beyond that 512, three rows to an SM: 7 rows of up to 33000 columns 11.0 us with 512,
+  // 8.9 with 1024, 64 x 131072 18.5 and 13.3; 160 x 9000 11.5 and 15.5, 4096 x 32768 175 and 283.  (256 threads, five rows to an SM:
+  // 4096 x 32768 207, 2048 x 2048 21.5.)
+  if (T <= sm_count()) topk_select_kernel<1024, 1><<<T, 1024, 0, stream>>>(logits, ld, ks, ke, S, k, out, sample);
+  else topk_select_kernel<512, 3><<<T, 512, 0, stream>>>(logits, ld, ks, ke, S, k, out, sample);
   return check_launch("topk_select");
 }
 

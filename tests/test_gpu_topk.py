@@ -178,3 +178,48 @@ def _sets_equal_with_ties(x, idx, k):
         tied = (row == kth).nonzero().flatten()[: k - above.numel()]
         want = torch.cat([above, tied]).sort().values
         assert torch.equal(idx[t].long().sort().values, want), f"row {t}"
+
+
+@pytest.mark.parametrize("n", [257, 2047, 4092, 4093, 4096, 4097, 8188, 8189, 8192, 12000, 16384])
+@pytest.mark.parametrize("k", [1, 256, 2048])
+def test_row_lengths_around_the_changes_of_path(n, k):
+    """Rows kept in registers (one and two chunks of 4096 columns), read again, or staged behind a sample: lengths at the edges,
+    windows that start inside a float4, calls of few rows (a larger CTA) and of many.  Sets against torch.topk with the tie rule,
+    the same output, order included, whatever the number of rows, and against the two-pass path."""
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    rows = [torch.randn(n + 3, device=DEV, generator=g), torch.randn(n + 3, device=DEV, generator=g).exp() * -1,
+            torch.randint(0, 50, (n + 3,), device=DEV, generator=g).float(), torch.full((n + 3,), -1.5, device=DEV),
+            1e30 * torch.randn(n + 3, device=DEV, generator=g) ** 9]
+    x = torch.zeros(len(rows), (n + 6) // 4 * 4, device=DEV)
+    x[:, :n + 3] = torch.stack(rows)
+    for lo in (0, 1, 3):
+        ks = torch.full((len(rows),), lo, dtype=torch.int32, device=DEV)
+        ke = ks + n
+        a = ops.topk_select(x, min(k, n), ks, ke)
+        _sets_equal_with_ties(x[:, lo:lo + n], a - lo, min(k, n))
+        assert torch.equal(a.sort(1).values, _two_pass(x, min(k, n), ks, ke).sort(1).values)
+        many = ops.topk_select(x.repeat(40, 1), min(k, n), ks.repeat(40), ke.repeat(40))
+        assert torch.equal(many[:len(rows)], a) and torch.equal(many[-len(rows):], a)
+
+
+@pytest.mark.parametrize("n", [3000, 6000, 9000, 40000])
+def test_nan_and_infinities_keep_the_order_of_the_bits(n):
+    """A NaN counts by its bits: above +inf with the sign bit clear, below -inf with it set; the oracle is the order-preserving
+    map of the bit patterns to integers, lower column first among equals."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = torch.randn(6, n, device=DEV, generator=g)
+    nan = torch.tensor([0x7fc00000, -0x400000], dtype=torch.int32, device=DEV).view(torch.float32)
+    x[0, 5::97] = nan[0]
+    x[1, 7::89] = nan[1]
+    x[2, 11::101] = float("inf")
+    x[3, 3::2] = float("-inf")
+    x[4, ::3], x[4, 1::3] = nan[1], nan[0]
+    x[5, 0] = 3e38
+    bits = x.view(torch.int32).long()
+    key = torch.where(bits < 0, -(bits & 0x7fffffff) - 1, bits)
+    for k in (40, 2048):
+        got = ops.topk_select(x, k)
+        assert torch.equal(got, ops.topk_select(x.repeat(60, 1), k)[:6])
+        for t in range(6):
+            want = sorted(range(n), key=lambda c, kt=key[t].tolist(): (-kt[c], c))[:k]
+            assert sorted(got[t].tolist()) == sorted(want), (t, k)

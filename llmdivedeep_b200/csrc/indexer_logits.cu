@@ -839,14 +839,26 @@ int make_tmap_2d_u8(CUtensorMap* m, const void* base, uint64_t rows, uint32_t ro
 // least to do: its rounds times a unit's tiles plus one, which is about what a start costs.  Measured over 472 calls of 1 to
 // 2048 rows and 60 to 131072 keys at every cut, this is within 1 % of the best cut on average and nowhere slower than eight
 // tiles; cutting on until every SM has a unit was up to 18 % slower (257 rows x 2000 keys, 64 heads: 130 units of eight tiles
-// 11.8 us, 260 of four 13.1).  2048 rows x 2000 keys of 4 heads x 64: 32 units of eight tiles 51.6 us, 128 of two 18.7; paged,
-// one sequence of 2000 tokens: one unit 9.6 us, four 6.0; seven of 33000: 63 units 14.9 us, 119 units 10.5, 231 units 11.8.
+// 11.8 us, 260 of four 13.1).  2048 rows x 2000 keys of 4 heads x 64: 32 units of eight tiles 51.6 us, 128 of two 18.7.
+// Paged calls (512 keys a tile, a unit's page ids fetched three tiles ahead): the sequences' lengths are not known here and often
+// differ by half, so the units stay small enough for the round-robin to even them out -- four tiles while that gives every SM
+// two, else the unit of at most eight tiles that leaves the longest CTA least to do.  us against eight tiles and more: 64
+// sequences of 65536 to 131072 tokens 172 -> 151 (all of 131072: the same), 160 of 4500 to 9000 41.6 -> 39.4, 12 of up to 131072 42.3 -> 38.4, 20 of
+// up to 20000 15.2 -> 13.3 (six tiles).
+template <bool PAGED>
 static int pick_chunk_tiles(int n_qblocks, int n_tiles) {
   auto units = [&](int chunk) { return (int64_t)n_qblocks * ((n_tiles + chunk - 1) / chunk); };
+  auto cost = [&](int c) { return (units(c) + sm_count() - 1) / sm_count() * ((c < n_tiles ? c : n_tiles) + 1); };
+  if (PAGED) {
+    if (units(4) >= 2LL * sm_count()) return 4;
+    int best = 8;
+    for (int c = 7; c >= 1; --c)
+      if (cost(c) < cost(best)) best = c;
+    return best;
+  }
   int chunk = kChunkTiles;
   while (chunk > 8 && units(chunk) < 6LL * sm_count()) chunk /= 2;
   if (units(chunk) >= sm_count()) return chunk;
-  auto cost = [&](int c) { return (units(c) + sm_count() - 1) / sm_count() * ((c < n_tiles ? c : n_tiles) + 1); };
   int best = chunk;
   for (int c = chunk / 2; c >= 1; c /= 2)
     if (cost(c) < cost(best)) best = c;
@@ -867,7 +879,7 @@ static int launch_indexer(const void* q, const void* k, const IndexerArgs& args,
   const int n_groups = (a.T + NQ - 1) / NQ;
   const int n_qblocks = (n_groups + QB - 1) / QB;
   const int n_tiles = (a.S + C::TILE_KEYS - 1) / C::TILE_KEYS;
-  a.chunk_tiles = pick_chunk_tiles(n_qblocks, n_tiles);
+  a.chunk_tiles = pick_chunk_tiles<PAGED>(n_qblocks, n_tiles);
   const int n_chunks = (n_tiles + a.chunk_tiles - 1) / a.chunk_tiles;
   const int64_t n_units64 = (int64_t)n_qblocks * n_chunks;
   if (n_units64 > 0x7fffffff) return set_error(DSA_ERR_SHAPE, "indexer: too many work units");
@@ -895,7 +907,7 @@ static int launch_indexer_rw(const void* q, const void* k, const IndexerArgs& ar
   if (rc) return rc;
   const int n_groups = (a.T + C::NQ - 1) / C::NQ;
   const int n_tiles = (a.S + kTileKeys - 1) / kTileKeys;
-  a.chunk_tiles = pick_chunk_tiles(n_groups, n_tiles);
+  a.chunk_tiles = pick_chunk_tiles<false>(n_groups, n_tiles);
   const int64_t n_units64 = (int64_t)n_groups * ((n_tiles + a.chunk_tiles - 1) / a.chunk_tiles);
   if (n_units64 > 0x7fffffff) return set_error(DSA_ERR_SHAPE, "indexer: too many work units");
   const int n_units = (int)n_units64;

@@ -223,3 +223,23 @@ def test_quantiser_around_the_change_of_values_per_thread(block, dtype):
     for n in (line - 1, line, line + 1):
         q, s = ops.fp8_quant_per_block(x[:n].cuda(), block)
         assert torch.equal(q.view(torch.uint8).cpu(), want_q[:n].view(torch.uint8)) and torch.equal(s.cpu().reshape(-1), want_s[:n].reshape(-1))
+
+
+@pytest.mark.parametrize("B,P,lens", [(1, 3, "full"), (3, 130, "ragged"), (40, 141, "ragged"), (64, 300, "ragged"), (160, 60, "full"), (300, 20, "short")])
+def test_paged_scan_units_cover_every_context(B, P, lens):
+    """The cut of the paged scan into units (four tiles, or what leaves the longest CTA least to do): every position of every
+    context scored, against the contiguous kernel on the same keys."""
+    g = torch.Generator(device="cuda").manual_seed(B + P)
+    k8, ksc = ops.fp8_quant_per_block(torch.randn(B * P * 64, 128, device="cuda", generator=g), 128)
+    table = torch.randperm(B * P, device="cuda", generator=g).int().view(B, P)
+    lo = {"full": P * 64, "ragged": P * 32, "short": 1}[lens]
+    ctx = torch.randint(lo, P * 64 + 1, (B,), device="cuda", generator=g).int()
+    q8, _ = ops.fp8_quant_per_block(torch.randn(B, 64, 128, device="cuda", generator=g), 128)
+    w = torch.randn(B, 64, device="cuda", generator=g)
+    got = ops.fp8_paged_mqa_logits(q8, w, k8, ksc, table, ctx, P * 64)
+    ops.check_status("cuda")
+    for b in sorted({0, B // 2, B - 1}):
+        rows = (table[b].long().unsqueeze(1) * 64 + torch.arange(64, device="cuda")).flatten()
+        n = int(ctx[b])
+        one = ops.fp8_mqa_logits(q8[b:b + 1], (k8.view(torch.uint8)[rows].view(ops.FP8), ksc[rows]), w[b:b + 1], None, ctx[b:b + 1].clone())
+        assert torch.allclose(got[b, :n], one[0, :n], rtol=1e-5, atol=1e-5)

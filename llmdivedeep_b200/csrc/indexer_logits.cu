@@ -555,6 +555,10 @@ struct RwCfg {
   static constexpr int K_TILE_BYTES = kTileKeys * D, Q_TILE_BYTES = N * D;
   static constexpr int STAGES = 6;
   static constexpr int EPI_WG = 4, EPI_WARPS = 16, THREADS = 128 + EPI_WG * 128;
+  // 96 registers a thread at launch; an epilogue thread holds 64 weights and two chunks of 16 columns.  Eight more from the other
+  // four warps end its spills: 4096 x 65536 2205 -> 2148 us (112 and 32: 2180, the others spill).
+  static constexpr int REGS_EPI = 104, REGS_OTHER = 64;
+  static_assert(512 * REGS_EPI + 128 * REGS_OTHER <= THREADS * 96, "more registers than the launch has");
   static constexpr uint32_t SBO = 8 * D;
   static constexpr int SMEM_BYTES = 1024 + STAGES * K_TILE_BYTES + 2 * Q_TILE_BYTES + 2 * N * 4 + 2 * NQ * 8 + 256;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -612,105 +616,109 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
-    uint32_t it = 0, nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
-      int g, nb, t_lo, t_hi;
-      if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
-      const int qs = nu & 1;
-      bool ok = true;
-      if (lane == 0) {
-        ok = mbar_wait(&q_empty[qs], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
-        if (ok) {
-          mbar_expect_tx(&q_full[qs], C::Q_TILE_BYTES);
-          tma_load_2d(q_s + qs * C::Q_TILE_BYTES, &tmap_q, 0, g * C::N, &q_full[qs]);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REGS_OTHER));
+    if (warp == 0) {
+      // ------------------------------ TMA producer ------------------------------
+      uint32_t it = 0, nu = 0;
+      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+        int g, nb, t_lo, t_hi;
+        if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
+        const int qs = nu & 1;
+        bool ok = true;
+        if (lane == 0) {
+          ok = mbar_wait(&q_empty[qs], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
+          if (ok) {
+            mbar_expect_tx(&q_full[qs], C::Q_TILE_BYTES);
+            tma_load_2d(q_s + qs * C::Q_TILE_BYTES, &tmap_q, 0, g * C::N, &q_full[qs]);
+          }
+          for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
+            const int st = it % C::STAGES;
+            ok = mbar_wait(&k_empty[st], ((it / C::STAGES) & 1) ^ 1, abort_flag, a.status);
+            if (!ok) break;
+            mbar_expect_tx(&k_full[st], C::K_TILE_BYTES);
+            tma_load_2d(k_s + st * C::K_TILE_BYTES, &tmap_k, 0, kt * kTileKeys, &k_full[st]);
+          }
         }
-        for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
-          const int st = it % C::STAGES;
-          ok = mbar_wait(&k_empty[st], ((it / C::STAGES) & 1) ^ 1, abort_flag, a.status);
-          if (!ok) break;
-          mbar_expect_tx(&k_full[st], C::K_TILE_BYTES);
-          tma_load_2d(k_s + st * C::K_TILE_BYTES, &tmap_k, 0, kt * kTileKeys, &k_full[st]);
-        }
-      }
-      ++nu;
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      it = __shfl_sync(0xffffffffu, it, 0);
-      if (!ok) break;
-    }
-    if (lane == 0 && *abort_flag) {               // on abort, give copies already in flight a bounded chance to land
-      for (int st = 0; st < C::STAGES; ++st)
-        for (uint32_t spin = 0; spin < (1u << 16) && !mbar_try_wait(&k_full[st], 0) && !mbar_try_wait(&k_full[st], 1); ++spin) {
-        }
-    }
-  } else if (warp == 1) {
-    // ------------------------------- MMA issuer -------------------------------
-    // The warp walks its loop as a whole and elects a lane for the instructions (dsa_common.cuh): 4096 x 65536 2222 -> 2173 us.
-    constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, kTileKeys, C::N);
-    uint32_t it = 0, nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
-      int g, nb, t_lo, t_hi;
-      if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
-      const int qs = nu & 1;
-      bool ok = mbar_wait_warp(&q_full[qs], (nu >> 1) & 1, abort_flag, a.status);
-      const uint64_t qdesc = umma_smem_desc(smem_u32(q_s + qs * C::Q_TILE_BYTES), 16, C::SBO, kSwz128);
-      for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
-        const int st = it % C::STAGES, acc = it & 1;
-        ok = mbar_wait_warp(&k_full[st], (it / C::STAGES) & 1, abort_flag, a.status) &&
-             mbar_wait_warp(&acc_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag, a.status);
+        ++nu;
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        it = __shfl_sync(0xffffffffu, it, 0);
         if (!ok) break;
-        tc_fence_after();
-        const uint64_t kdesc = umma_smem_desc(smem_u32(k_s + st * C::K_TILE_BYTES), 16, C::SBO, kSwz128);
-        if (elect_one()) {
-#pragma unroll
-          for (int k = 0; k < C::KSTEPS; ++k)
-            umma_f8(tmem_base + acc * C::N, kdesc + (k * 32 >> 4), qdesc + (k * 32 >> 4), idesc, k > 0);
-          umma_commit(&acc_full[acc]);
-          umma_commit(&k_empty[st]);
+      }
+      if (lane == 0 && *abort_flag) {               // on abort, give copies already in flight a bounded chance to land
+        for (int st = 0; st < C::STAGES; ++st)
+          for (uint32_t spin = 0; spin < (1u << 16) && !mbar_try_wait(&k_full[st], 0) && !mbar_try_wait(&k_full[st], 1); ++spin) {
+          }
+      }
+    } else if (warp == 1) {
+      // ------------------------------- MMA issuer -------------------------------
+      // The warp walks its loop as a whole and elects a lane for the instructions (dsa_common.cuh): 4096 x 65536 2222 -> 2173 us.
+      constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, kTileKeys, C::N);
+      uint32_t it = 0, nu = 0;
+      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+        int g, nb, t_lo, t_hi;
+        if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
+        const int qs = nu & 1;
+        bool ok = mbar_wait_warp(&q_full[qs], (nu >> 1) & 1, abort_flag, a.status);
+        const uint64_t qdesc = umma_smem_desc(smem_u32(q_s + qs * C::Q_TILE_BYTES), 16, C::SBO, kSwz128);
+        for (int kt = t_lo; kt < t_hi && ok; ++kt, ++it) {
+          const int st = it % C::STAGES, acc = it & 1;
+          ok = mbar_wait_warp(&k_full[st], (it / C::STAGES) & 1, abort_flag, a.status) &&
+               mbar_wait_warp(&acc_empty[acc], ((it >> 1) & 1) ^ 1, abort_flag, a.status);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t kdesc = umma_smem_desc(smem_u32(k_s + st * C::K_TILE_BYTES), 16, C::SBO, kSwz128);
+          if (elect_one()) {
+  #pragma unroll
+            for (int k = 0; k < C::KSTEPS; ++k)
+              umma_f8(tmem_base + acc * C::N, kdesc + (k * 32 >> 4), qdesc + (k * 32 >> 4), idesc, k > 0);
+            umma_commit(&acc_full[acc]);
+            umma_commit(&k_empty[st]);
+          }
+          __syncwarp();
+        }
+        if (!ok) break;
+        if (elect_one()) umma_commit(&q_empty[qs]);
+        __syncwarp();
+        ++nu;
+      }
+    } else if (warp == 2) {
+      // ------------------- stager: head weights and windows of the next unit -------------------
+      uint32_t nu = 0;
+      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+        int g, nb, t_lo, t_hi;
+        if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
+        const int ub = nu & 1;
+        const bool ok = mbar_wait_warp(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
+        if (!ok) break;
+        float* wd = w_s + ub * C::N;
+        const int t0 = g * C::NQ;
+        for (int c = lane; c < C::N; c += 32) {
+          const int t = t0 + c / C::H;
+          float wvv = 0.f;
+          if (t < a.T) {
+            const int64_t off = (int64_t)t * C::H + (c % C::H);
+            wvv = a.w_is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.w)[off])
+                              : reinterpret_cast<const float*>(a.w)[off];
+          }
+          wd[c] = wvv;
+        }
+        if (lane < C::NQ) {
+          const int t = t0 + lane;
+          int s0 = 0, s1 = 0;
+          if (t < a.T) {
+            s0 = a.ks ? max(a.ks[t], 0) : 0;
+            s1 = min(a.ke[t], a.S);
+          }
+          win_s[ub * C::NQ + lane] = make_int2(s0, max(s1 - s0, 0));
         }
         __syncwarp();
+        if (lane == 0) mbar_arrive(&w_full[ub]);
+        ++nu;
       }
-      if (!ok) break;
-      if (elect_one()) umma_commit(&q_empty[qs]);
-      __syncwarp();
-      ++nu;
     }
-  } else if (warp == 2) {
-    // ------------------- stager: head weights and windows of the next unit -------------------
-    uint32_t nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
-      int g, nb, t_lo, t_hi;
-      if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
-      const int ub = nu & 1;
-      const bool ok = mbar_wait_warp(&w_empty[ub], ((nu >> 1) & 1) ^ 1, abort_flag, a.status);
-      if (!ok) break;
-      float* wd = w_s + ub * C::N;
-      const int t0 = g * C::NQ;
-      for (int c = lane; c < C::N; c += 32) {
-        const int t = t0 + c / C::H;
-        float wvv = 0.f;
-        if (t < a.T) {
-          const int64_t off = (int64_t)t * C::H + (c % C::H);
-          wvv = a.w_is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.w)[off])
-                            : reinterpret_cast<const float*>(a.w)[off];
-        }
-        wd[c] = wvv;
-      }
-      if (lane < C::NQ) {
-        const int t = t0 + lane;
-        int s0 = 0, s1 = 0;
-        if (t < a.T) {
-          s0 = a.ks ? max(a.ks[t], 0) : 0;
-          s1 = min(a.ke[t], a.S);
-        }
-        win_s[ub * C::NQ + lane] = make_int2(s0, max(s1 - s0, 0));
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&w_full[ub]);
-      ++nu;
-    }
-  } else if (warp >= 4) {
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REGS_EPI));
     // ------------- epilogue: warpgroup = query token of the group, thread = key of the tile -------------
     const int ew = warp - 4;
     const int tok = ew >> 2;                     // token within the group = 64-column slice of the accumulator

@@ -169,6 +169,14 @@ int dsa_sparse_mla_decode_paged(const void* q_bf16, const void* cache, const int
                                 int num_pages, int max_ctx, float scale, void* workspace, size_t workspace_bytes,
                                 int32_t* status, void* stream);
 
+/* One decode step: dsa_indexer_logits_paged, dsa_topk_select over [0, ctx_len) and dsa_sparse_mla_decode_paged with the arguments
+ * of those calls, for hosts whose calls cost as much as the kernels.  The caches may have different numbers of pages. */
+int dsa_decode_step(const void* q_fp8, const void* w, int w_dtype, const void* kcache, const float* kscale, int k_pages,
+                    const int32_t* block_table, int64_t table_stride, const int32_t* ctx_len, float* logits, int64_t ld_logits,
+                    int B, int idx_heads, int idx_dim, int max_ctx, int k, int32_t* idx, const void* q_bf16, const void* latent,
+                    int latent_pages, void* out_bf16, int H, float scale, void* workspace, size_t workspace_bytes,
+                    int32_t* status, void* stream);
+
 /* dsa_indexer_topk without a caller-supplied workspace.  No counterpart in the
  * reference: it exists for hosts that cannot allocate device memory at the call
  * site (a runtime that owns the whole device heap and forbids allocation inside

@@ -40,6 +40,9 @@ SIGNATURES = {
     "dsa_sparse_mla_decode_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "dsa_sparse_mla_decode_paged": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int,
                                             c_int, c_int, c_int, c_float, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "dsa_decode_step": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int64,
+                                c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_float,
+                                c_void_p, c_size_t, c_void_p, c_void_p]),
     "dsa_test_indexer_logits_general": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                 c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                                 c_void_p]),

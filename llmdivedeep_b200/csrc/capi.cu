@@ -229,6 +229,19 @@ int dsa_sparse_mla_decode_paged(const void* q_bf16, const void* cache, const int
                                   max_ctx, scale, workspace, workspace_bytes, status, static_cast<cudaStream_t>(stream));
 }
 
+int dsa_decode_step(const void* q_fp8, const void* w, int w_dtype, const void* kcache, const float* kscale, int k_pages,
+                    const int32_t* block_table, int64_t table_stride, const int32_t* ctx_len, float* logits, int64_t ld_logits,
+                    int B, int idx_heads, int idx_dim, int max_ctx, int k, int32_t* idx, const void* q_bf16, const void* latent,
+                    int latent_pages, void* out_bf16, int H, float scale, void* workspace, size_t workspace_bytes,
+                    int32_t* status, void* stream) {
+  int rc = dsa_indexer_logits_paged(q_fp8, w, w_dtype, kcache, kscale, block_table, table_stride, ctx_len, logits, ld_logits, B,
+                                    idx_heads, idx_dim, k_pages, max_ctx, status, stream);
+  if (!rc) rc = dsa_topk_select(logits, ld_logits, nullptr, ctx_len, B, max_ctx, k, idx, stream);
+  if (!rc) rc = dsa_sparse_mla_decode_paged(q_bf16, latent, block_table, table_stride, idx, out_bf16, B, H, k, latent_pages, max_ctx,
+                                            scale, workspace, workspace_bytes, status, stream);
+  return rc;
+}
+
 size_t dsa_sparse_mla_decode_workspace_bytes(int B, int H, int K) {
   if (B <= 0 || H <= 0 || K <= 0) return 0;
   return mla_decode_workspace_bytes(B, H, K);

@@ -368,21 +368,24 @@ class HostPrefillPipeline:
 LATENT_TOKEN_BYTES = 656          # 512 e4m3 latent values, 4 fp32 group scales, 64 bf16 rope values
 
 
-@torch.no_grad()
 def pack_latent_cache(kv: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Latent KV rows [N, 576] (bf16 or fp32, CUDA) -> records of the paged FP8 latent cache, uint8
     [N, 656]: the 512 latent values as e4m3 with one fp32 scale per 128 values (the indexer quantiser's
     rule, sparse_attn/DSA.py:121-124: scale = max(absmax, 1e-6) / 448), then the 64 rope values as bf16.
     This is the write side of the cache sparse_mla_decode_paged reads; rows go to
     cache[block_table[b, pos // 64] * 64 + pos % 64]."""
-    N = kv.shape[0]
     if kv.dim() != 2 or kv.shape[1] != 576:
         raise ops.DsaError(f"latent KV must be [N, 576], got {tuple(kv.shape)}")
+    records = ops.pack_latent_records(kv, out)
+    return _pack_by_parts(kv, out) if records is None else records
+
+
+@torch.no_grad()
+def _pack_by_parts(kv: torch.Tensor, out: Optional[torch.Tensor]) -> torch.Tensor:
+    """pack_latent_cache for other types, strides or alignments: the quantiser and three copies."""
+    N = kv.shape[0]
     if out is None:
         out = torch.empty(N, LATENT_TOKEN_BYTES, dtype=torch.uint8, device=kv.device)
-    if ops.pack_latent_records(kv, out):
-        return out
-    # other types, strides or alignments: the quantiser and three copies
     q8, scale = ops.fp8_quant_per_block(kv[:, :512].contiguous(), 128)      # [N,512] e4m3, [N,4] fp32
     out[:, :512] = q8.view(torch.uint8)
     out[:, 512:528] = scale.contiguous().view(torch.uint8).view(N, 16)
@@ -411,6 +414,9 @@ def dsa_decode_step(q_idx_fp8, w, kcache, kscale, block_table, ctx_len, q, laten
     context, sparse MLA over the paged FP8 latent cache.  Returns (idx, out) views of ``ws``."""
     B = q.shape[0]
     idx, out = ws.idx[:B], ws.out[:B]
+    if ops.decode_step(q_idx_fp8, w, kcache, kscale, block_table, ctx_len, q, latent_cache, softmax_scale, ws.max_ctx, ws.logits, idx, out,
+                       ws.mla_ws):
+        return idx, out
     logits = ops.fp8_paged_mqa_logits(q_idx_fp8, w, kcache, kscale, block_table, ctx_len, ws.max_ctx, out=ws.logits)
     ops.topk_select(logits, ws.k, None, ctx_len, out=idx)
     ops.sparse_mla_decode_paged(q, latent_cache, block_table, idx, softmax_scale, ws.max_ctx, out=out, workspace=ws.mla_ws)

@@ -333,6 +333,39 @@ def sparse_mla_decode_paged(q, cache, block_table, idx, scale: float, max_ctx: O
     return out
 
 
+def decode_step(q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, scale: float, max_ctx: int, logits, idx, out,
+                workspace) -> bool:
+    """fp8_paged_mqa_logits, topk_select and sparse_mla_decode_paged into the given buffers (logits [>=B, >=max_ctx], idx [B,k],
+    out [B,H,512]) as one library call.  Returns False, with nothing done, unless every tensor is of the plain form that the
+    three wrappers pass on as it is -- they convert or refuse the others."""
+    dev = q.device
+    i = dev.index
+    if dev.type != "cuda" or q.dim() != 3 or q_fp8.dim() != 3 or block_table.dim() != 2 or idx.dim() != 2:
+        return False
+    for t in (q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, idx, out, workspace):
+        if t.get_device() != i or not t.is_contiguous():
+            return False
+    B, H, dq = q.shape
+    Bi, Hi, D = q_fp8.shape
+    if (B == 0 or Bi != B or dq != 576 or tuple(weights.shape) != (B, Hi) or kcache.dim() != 2 or kcache.shape[1] != D or kcache.shape[0] % 64
+            or kscale.dim() != 1 or kscale.shape[0] != kcache.shape[0] or block_table.shape[0] != B or ctx_len.numel() != B
+            or cache.dim() != 2 or cache.shape[1] != 656 or cache.shape[0] % 64 or idx.shape[0] != B or tuple(out.shape) != (B, H, 512)
+            or logits.get_device() != i or logits.dim() != 2 or logits.shape[0] < B or logits.shape[1] < max_ctx or logits.stride(1) != 1):
+        return False
+    if (q_fp8.dtype != FP8 or kcache.dtype != FP8 or kscale.dtype != torch.float32 or block_table.dtype != torch.int32
+            or ctx_len.dtype != torch.int32 or q.dtype != torch.bfloat16 or cache.dtype != torch.uint8 or idx.dtype != torch.int32
+            or out.dtype != torch.bfloat16 or logits.dtype != torch.float32 or workspace.dtype != torch.uint8
+            or weights.dtype not in (torch.float32, torch.bfloat16)):
+        return False
+    with _on(dev):
+        check(_lib.load().dsa_decode_step(
+            q_fp8.data_ptr(), weights.data_ptr(), _w_dtype(weights), kcache.data_ptr(), kscale.data_ptr(), kcache.shape[0] // 64,
+            block_table.data_ptr(), block_table.stride(0), ctx_len.data_ptr(), logits.data_ptr(), max(logits.stride(0), max_ctx), B, Hi, D,
+            max_ctx, idx.shape[1], idx.data_ptr(), q.data_ptr(), cache.data_ptr(), cache.shape[0] // 64, out.data_ptr(), H, float(scale),
+            workspace.data_ptr(), workspace.numel(), status_word(dev).data_ptr(), _stream(dev)))
+    return True
+
+
 class HostIndexerPipeline:
     """indexer_topk for inputs and outputs that live in (pinned) host memory.
 
@@ -469,29 +502,34 @@ def fp8_quant_per_block(x: torch.Tensor, block_size: int = 128):
     x = x.contiguous()
     nb = last // block_size
     n_blocks = x.numel() // block_size
-    q = torch.empty(x.shape, dtype=FP8, device=x.device)
-    scale = torch.empty(n_blocks, dtype=torch.float32, device=x.device)
+    q = torch.empty(x.shape, dtype=FP8, device=dev)
+    scale = torch.empty(x.shape[:-1] if nb == 1 else (*x.shape[:-1], nb), dtype=torch.float32, device=dev)
     lib = _lib.load()
     with _on(dev):
-        check(lib.dsa_fp8_quant_per_block(_ptr(x), 1 if x.dtype == torch.bfloat16 else 0, n_blocks, block_size,
-                                          _ptr(q), _ptr(scale), _stream(dev)))
-    return q, (scale.view(x.shape[:-1]) if nb == 1 else scale.view(*x.shape[:-1], nb))
+        check(lib.dsa_fp8_quant_per_block(x.data_ptr(), 1 if x.dtype == torch.bfloat16 else 0, n_blocks, block_size,
+                                          q.data_ptr(), scale.data_ptr(), _stream(dev)))
+    return q, scale
 
 
-def pack_latent_records(kv: torch.Tensor, out: torch.Tensor) -> bool:
-    """Latent rows [N, 576] -> cache records uint8 [N, 656] in one kernel.  Takes bf16 or fp32 rows with unit column
-    stride and dense records, everything 16-byte aligned; returns False, having done nothing, for any other call."""
+def pack_latent_records(kv: torch.Tensor, out: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """Latent rows [N, 576] -> cache records uint8 [N, 656] in one kernel, into ``out`` (None: a new tensor).  Takes bf16 or fp32
+    rows with unit column stride and dense records, everything 16-byte aligned; returns None, having done nothing, for any other
+    call."""
+    dev = kv.device
     N = kv.shape[0]
-    if (not kv.is_cuda or kv.dtype not in (torch.bfloat16, torch.float32) or out.dtype != torch.uint8 or out.device != kv.device
-            or tuple(out.shape) != (N, 656) or not out.is_contiguous()):
-        return False
+    if dev.type != "cuda" or kv.dtype not in (torch.bfloat16, torch.float32):
+        return None
     rs, cs = kv.stride()
-    if N and (cs != 1 or (N > 1 and (rs < 576 or rs * kv.element_size() % 16)) or (kv.data_ptr() | out.data_ptr()) % 16):
-        return False
-    lib = _lib.load()
-    with _on(kv.device):
-        check(lib.dsa_pack_latent_cache(_ptr(kv), 1 if kv.dtype == torch.bfloat16 else 0, rs, N, _ptr(out), _stream(kv.device)))
-    return True
+    if N and (cs != 1 or (N > 1 and (rs < 576 or rs * kv.element_size() % 16)) or kv.data_ptr() % 16):
+        return None
+    if out is None:
+        out = torch.empty(N, 656, dtype=torch.uint8, device=dev)
+    elif (out.dtype != torch.uint8 or out.device != dev or tuple(out.shape) != (N, 656) or not out.is_contiguous()
+          or (N and out.data_ptr() % 16)):
+        return None
+    with _on(dev):
+        check(_lib.load().dsa_pack_latent_cache(kv.data_ptr(), 1 if kv.dtype == torch.bfloat16 else 0, rs, N, out.data_ptr(), _stream(dev)))
+    return out
 
 
 def rope_fp8_quant(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rope_dim: int, interleave: bool,

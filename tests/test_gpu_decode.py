@@ -243,3 +243,32 @@ def test_paged_scan_units_cover_every_context(B, P, lens):
         n = int(ctx[b])
         one = ops.fp8_mqa_logits(q8[b:b + 1], (k8.view(torch.uint8)[rows].view(ops.FP8), ksc[rows]), w[b:b + 1], None, ctx[b:b + 1].clone())
         assert torch.allclose(got[b, :n], one[0, :n], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("B,heads,w_dtype", [(1, 128, torch.float32), (5, 64, torch.bfloat16), (80, 16, torch.float32)])
+def test_one_call_decode_step_equals_the_three_calls(B, heads, w_dtype):
+    """layer.dsa_decode_step makes one library call for tensors of the plain form and three wrapper calls for others (here: a
+    strided block table): the same selection and the same bits, in a workspace made for more sequences too."""
+    g = torch.Generator(device="cuda").manual_seed(B)
+    P, k = 40, 512
+    n = B * P * 64
+    kc, ksc = ops.fp8_quant_per_block(torch.randn(n, 128, device="cuda", generator=g), 128)
+    lat = layer.pack_latent_cache(torch.randn(n, 576, device="cuda", generator=g).bfloat16())
+    table = torch.randperm(B * P, device="cuda", generator=g).int().view(B, P)
+    ctx = torch.randint(300, P * 64 + 1, (B,), device="cuda", generator=g).int()
+    q8, qs = ops.fp8_quant_per_block(torch.randn(B, 64, 128, device="cuda", generator=g), 128)
+    w = (torch.randn(B, 64, device="cuda", generator=g) * qs).to(w_dtype)
+    q = torch.randn(B, heads, 576, device="cuda", generator=g).bfloat16()
+    strided = torch.zeros(B, P + 3, dtype=torch.int32, device="cuda")[:, :P]
+    strided.copy_(table)
+    got = []
+    for tab, room in ((table, B), (strided, B), (table, B + 3)):
+        ws = layer.DecodeWorkspace(room, heads, P * 64, k, "cuda")
+        idx, out = layer.dsa_decode_step(q8, w, kc, ksc, tab, ctx, q, lat, 0.07, ws)
+        got.append((idx.clone(), out.clone()))
+    ops.check_status("cuda")
+    for idx, out in got[1:]:
+        assert torch.equal(idx, got[0][0])
+    assert torch.equal(got[1][1], got[0][1]) and torch.equal(got[2][1], got[0][1])
+    with pytest.raises(ops.DsaError):
+        layer.dsa_decode_step(q8, w, kc, ksc, table, ctx.long(), q, lat, 0.07, layer.DecodeWorkspace(B, heads, P * 64, k, "cuda"))

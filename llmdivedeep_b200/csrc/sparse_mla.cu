@@ -907,15 +907,8 @@ int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx,
 // take as long as a full one.  The queries of that round are cut into parts that share its pairs: as many as fit, at most
 // eight, of at least 256 slots.  More parts than that lose: every part pays the set-up again and writes an fp32 partial
 // output that the combine kernel reads back.  Batch 160 (two rounds and twelve queries in six parts each): 174 -> 156 us.
-// But for so few queries that they leave twelve pairs each: there the latency of a part's blocks counts, and up to sixteen
-// parts of 128 slots are faster.  us in eight / sixteen (six queries: twelve) parts, 128 heads, 2048 slots: one query 22.1 / 19.4, two
-// 22.4 / 19.9, four 23.5 / 21.5, six 24.1 / 23.0; seven in ten parts 24.4 / 24.9.
 static int mla_pairs(int H) { return max(1, sm_count() / (2 * ((H + 127) / 128))); }
-static int mla_parts_per_query(int rest, int pairs, int K) {
-  if (rest == 0) return 1;
-  const int fine = min(min(kMlaMaxParts, (K + 127) / 128), pairs / rest);
-  return fine >= 12 ? fine : max(1, min(min(8, K / 256), pairs / rest));
-}
+static int mla_parts_per_query(int rest, int pairs, int K) { return rest == 0 ? 1 : max(1, min(min(8, K / 256), pairs / rest)); }
 static size_t mla_part_bytes(int H) { return (size_t)H * (kMlaDv + 2) * sizeof(float); }
 // Enough for every batch of up to B queries.  The need of a batch goes up and down with the queries of its last round (128
 // heads, 2048 slots, 148 SMs: 64 parts for 8 queries, 74 for 37, none for 38 or for 74), and a serving loop runs smaller

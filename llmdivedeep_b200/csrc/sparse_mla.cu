@@ -89,7 +89,7 @@ struct MlaRegs {                                   // decode's gather converts i
   static constexpr int kSoftmax = FP8_PAGED ? 88 : 96, kOther = FP8_PAGED ? 48 : 40;
   static_assert(512 * kSoftmax + 384 * kOther <= 896 * 72, "more registers than the launch has");
 };
-constexpr int kMlaMaxParts = 16;                   // parts of a split list
+constexpr int kMlaMaxParts = 8;                    // parts of a split list
 constexpr int kMlaMaxK = 2048;                     // slots of a list
 constexpr int kMlaThreads = 896, kMlaSoftmaxWarps = 16, kMlaMmaWarp = 16, kMlaGatherWarp0 = 17, kMlaGatherWarps = 11;
 template <int R>
@@ -820,32 +820,31 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
 
 // out[t,h,:] = sum_s 2^(lse_s - M) o_s / sum_s 2^(lse_s - M): merges the parts of a split slot list, each half of the columns
 // by the sums of the CTA that computed it.
-// PARTS: the most that n_split may be.  A query in eight parts: 4.8 us with loads behind the weights' loop, 3.6 so.
-template <int PARTS>
+// A query in eight parts: 4.8 us with loads behind the weights' loop, 3.6 so.
 __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a) {
   const int u = blockIdx.x, t = a.n_full + u, h = blockIdx.y;
   const int d = threadIdx.x * 4, cta = d / kMlaDvHalf;
   // every load is requested before any is used: a part's weight and values do not wait for one another
-  float wgt[PARTS];
-  float4 v[PARTS];
+  float wgt[kMlaMaxParts];
+  float4 v[kMlaMaxParts];
 #pragma unroll
-  for (int sp = 0; sp < PARTS; ++sp) {
+  for (int sp = 0; sp < kMlaMaxParts; ++sp) {
     const int64_t p = (int64_t)u * a.n_split + sp;
     wgt[sp] = sp < a.n_split ? a.part_lse[(p * 2 + cta) * a.H + h] : -CUDART_INF_F;
     v[sp] = sp < a.n_split ? *reinterpret_cast<const float4*>(a.part_o + (p * a.H + h) * kMlaDv + d) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float mx = -CUDART_INF_F, den = 0.f;
 #pragma unroll
-  for (int sp = 0; sp < PARTS; ++sp) mx = fmaxf(mx, wgt[sp]);
+  for (int sp = 0; sp < kMlaMaxParts; ++sp) mx = fmaxf(mx, wgt[sp]);
 #pragma unroll
-  for (int sp = 0; sp < PARTS; ++sp) {
+  for (int sp = 0; sp < kMlaMaxParts; ++sp) {
     wgt[sp] = (mx == -CUDART_INF_F) ? 0.f : exp2f(wgt[sp] - mx);
     den += wgt[sp];
   }
   const float inv = den > 0.f ? 1.f / den : 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int sp = 0; sp < PARTS; ++sp) {
+  for (int sp = 0; sp < kMlaMaxParts; ++sp) {
     acc.x += wgt[sp] * v[sp].x; acc.y += wgt[sp] * v[sp].y; acc.z += wgt[sp] * v[sp].z; acc.w += wgt[sp] * v[sp].w;
   }
   uint2 o;
@@ -880,8 +879,7 @@ static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaSt
   const int n_parts = a.T - a.n_full;
   const dim3 grid(2 * (a.n_full + n_parts * a.n_split), 1, (a.H + 127) / 128);
   kern<<<grid, kMlaThreads, smem_bytes, stream>>>(tq, to, a);
-  if (n_parts > 0 && a.n_split <= 8) sparse_mla_combine_kernel<8><<<dim3(n_parts, a.H), 128, 0, stream>>>(a);
-  else if (n_parts > 0) sparse_mla_combine_kernel<kMlaMaxParts><<<dim3(n_parts, a.H), 128, 0, stream>>>(a);
+  if (n_parts > 0) sparse_mla_combine_kernel<<<dim3(n_parts, a.H), 128, 0, stream>>>(a);
   return check_launch("sparse_mla");
 }
 
@@ -908,7 +906,7 @@ int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx,
 // eight, of at least 256 slots.  More parts than that lose: every part pays the set-up again and writes an fp32 partial
 // output that the combine kernel reads back.  Batch 160 (two rounds and twelve queries in six parts each): 174 -> 156 us.
 static int mla_pairs(int H) { return max(1, sm_count() / (2 * ((H + 127) / 128))); }
-static int mla_parts_per_query(int rest, int pairs, int K) { return rest == 0 ? 1 : max(1, min(min(8, K / 256), pairs / rest)); }
+static int mla_parts_per_query(int rest, int pairs, int K) { return rest == 0 ? 1 : max(1, min(min(kMlaMaxParts, K / 256), pairs / rest)); }
 static size_t mla_part_bytes(int H) { return (size_t)H * (kMlaDv + 2) * sizeof(float); }
 // Enough for every batch of up to B queries.  The need of a batch goes up and down with the queries of its last round (128
 // heads, 2048 slots, 148 SMs: 64 parts for 8 queries, 74 for 37, none for 38 or for 74), and a serving loop runs smaller

@@ -140,6 +140,31 @@ __device__ __forceinline__ bool unit_tiles(const IndexerArgs& a, int u, int n_qb
   return t_lo < t_hi;
 }
 
+// The stager's part: head weights of tokens t0.. (COUNT of them, H to a token, zeros past the last) into shared memory.  All of a
+// lane's loads are requested before the first is stored: one by one they cost a unit's start a load latency each.  4 heads x 64, 2048
+// rows x 2048 keys 17.8 -> 15.4 us, 300 x 300 11.8 -> 9.5; 64 heads x 128, 64 x 2048 6.7 -> 5.6, 257 x 20011 58.2 -> 57.3.
+template <int COUNT, int H>
+__device__ __forceinline__ void stage_weights(const IndexerArgs& a, int t0, int lane, float* __restrict__ dst) {
+  constexpr int ROUNDS = (COUNT + 31) / 32, BATCH = ROUNDS < 16 ? ROUNDS : 16;
+  const int64_t off = (int64_t)t0 * H;                 // the tokens' weights are contiguous
+  const int64_t left = (int64_t)(a.T - t0) * H < COUNT ? (int64_t)(a.T - t0) * H : COUNT;
+#pragma unroll 1
+  for (int c0 = lane; c0 < COUNT; c0 += 32 * BATCH) {
+    float v[BATCH];
+    if (a.w_is_bf16) {
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i)
+        v[i] = c0 + 32 * i < left ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.w)[off + c0 + 32 * i]) : 0.f;
+    } else {
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) v[i] = c0 + 32 * i < left ? reinterpret_cast<const float*>(a.w)[off + c0 + 32 * i] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i)
+      if (c0 + 32 * i < COUNT) dst[c0 + 32 * i] = v[i];
+  }
+}
+
 // One thread = one key.  Walks NCOLS accumulator columns starting at column COL0 of
 // its TMEM lane.  Weights of chunk c+1 and its TMEM load are both requested before
 // the math of chunk c, in that order: shared-memory loads queue behind a TMEM load
@@ -380,16 +405,8 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       float* wd = w_s + ub * QB * C::N;
       int2* wind = win_s + ub * C::NTOK;
       const int t0 = qb * QB * NQ;
-      for (int c = lane; c < QB * C::N; c += 32) {
-        const int t = t0 + c / H;
-        float wvv = 0.f;
-        if (t < a.T) {
-          const int64_t off = (int64_t)t * H + (c % H);
-          wvv = a.w_is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.w)[off])
-                            : reinterpret_cast<const float*>(a.w)[off];
-        }
-        wd[c] = wvv;
-      }
+      stage_weights<QB * C::N, H>(a, t0, lane, wd);
+#pragma unroll
       for (int j = lane; j < C::NTOK; j += 32) {
         const int t = t0 + j;
         int s0 = 0, s1 = 0;
@@ -693,16 +710,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         if (!ok) break;
         float* wd = w_s + ub * C::N;
         const int t0 = g * C::NQ;
-        for (int c = lane; c < C::N; c += 32) {
-          const int t = t0 + c / C::H;
-          float wvv = 0.f;
-          if (t < a.T) {
-            const int64_t off = (int64_t)t * C::H + (c % C::H);
-            wvv = a.w_is_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.w)[off])
-                              : reinterpret_cast<const float*>(a.w)[off];
-          }
-          wd[c] = wvv;
-        }
+        stage_weights<C::N, C::H>(a, t0, lane, wd);
         if (lane < C::NQ) {
           const int t = t0 + lane;
           int s0 = 0, s1 = 0;

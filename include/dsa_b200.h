@@ -71,6 +71,12 @@ int dsa_rope_fp8_quant(const void* x_bf16, int64_t n_rows, int head_dim, int rop
                        const float* cos_table, const float* sin_table, int64_t n_pos, void* q_fp8, float* scale,
                        void* stream);
 
+/* The same, and with gate_bf16 [n_rows] the scorer's weights of the rows as well: gate_out[r] =
+ * ((float(gate[r]) * gate_mul0) * scale[r]) * gate_mul1 in fp32, every product rounded (sparse_attn/DSA.py:327-331, 505-511). */
+int dsa_rope_fp8_quant_gated(const void* x_bf16, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
+                             const float* cos_table, const float* sin_table, int64_t n_pos, void* q_fp8, float* scale,
+                             const void* gate_bf16, float gate_mul0, float gate_mul1, float* gate_out, void* stream);
+
 /* Lightning-indexer logits, contiguous keys.
  *   logits[t, s] = k_scale[s] * sum_h w[t,h] * relu(q[t,h,:] . k[s,:])  for ks[t] <= s < ke[t].
  * Stands in for deep_gemm.fp8_mqa_logits(q_fp8, (k_fp8, k_scale), w, ks, ke) as

@@ -72,9 +72,9 @@ def _fold(w: torch.Tensor, q_scale: torch.Tensor, head_dim: int) -> torch.Tensor
     return (w.float() * qs.float() * head_dim ** -0.5).contiguous()
 
 
-def _score_topk(q_fp8, k_fp8, k_scale, w_eff, ks, ke, k: int) -> torch.Tensor:
+def _score_topk(q_fp8, k_fp8, k_scale, w_eff, ks, ke, k: int, dtype: torch.dtype = torch.int64) -> torch.Tensor:
     ksc = k_scale if k_scale.dim() == 1 else k_scale.squeeze(-1)
-    return ops.indexer_topk(q_fp8.contiguous(), k_fp8.contiguous(), ksc.contiguous(), w_eff, ks, ke, k).long()
+    return ops.indexer_topk(q_fp8.contiguous(), k_fp8.contiguous(), ksc.contiguous(), w_eff, ks, ke, k).to(dtype)
 
 
 # ---- dense / block-sparse registration hooks (reference: sparse_attn/DSA.py:139-249) -------------
@@ -236,28 +236,43 @@ class DsaIndexer(nn.Module):
         rd, il = self.spec.rope_head_dim, self.spec.rope_interleave
         return _rope_head(q, rd, q.shape[0], il), _rope_head(k, rd, k.shape[0], il)
 
-    def _rope_quant(self, x: torch.Tensor, n_pos: int, rows_per_pos: int):
-        """RoPE on the first rope_head_dim values of every head row, then the per-row FP8 quantiser: one fused kernel
-        for bf16 rows of one FP8 block (its bytes and scales equal the eager chain's), the eager chain otherwise."""
-        rd, il = self.spec.rope_head_dim, self.spec.rope_interleave
+    def _rope_quant(self, x: torch.Tensor, n_pos: int, rows_per_pos: int, gate: Optional[torch.Tensor] = None):
+        """RoPE on the first rope_head_dim values of every head row, then the per-row FP8 quantiser, and for q the scorer's
+        weights from the rows' head gates (straight from weights_proj): one fused kernel for bf16 rows of one FP8 block (its
+        results equal the eager chain's bit for bit), the eager chain otherwise."""
+        sp = self.spec
+        rd, il = sp.rope_head_dim, sp.rope_interleave
         if x.dtype == torch.bfloat16 and x.shape[-1] == self._quant_block() and x.shape[-1] in (64, 128):
             cos, sin = _rope_cossin(n_pos, rd, x.device)
-            return ops.rope_fp8_quant(x, cos, sin, rd, il, rows_per_pos)
-        return fp8_quant_per_block(_rope_head(x, rd, n_pos, il), self._quant_block())
+            if gate is None or gate.dtype == torch.bfloat16:
+                return ops.rope_fp8_quant(x, cos, sin, rd, il, rows_per_pos, gate, (sp.index_n_heads ** -0.5, sp.index_head_dim ** -0.5))
+            q8, scale = ops.rope_fp8_quant(x, cos, sin, rd, il, rows_per_pos)
+        else:
+            q8, scale = fp8_quant_per_block(_rope_head(x, rd, n_pos, il), self._quant_block())
+        return (q8, scale) if gate is None else (q8, scale, _fold(gate.float() * sp.index_n_heads ** -0.5, scale, sp.index_head_dim))
 
-    def _select(self, q, k, w, ke, topk: int) -> torch.Tensor:
-        """q [T,H,D], k [T_kv,D] straight from the projections (before RoPE), head gates w, windows ke."""
-        q_fp8, q_scale = self._rope_quant(q, q.shape[0], q.shape[1])
+    def _select(self, q, k, gate, ke, topk: int, dtype: torch.dtype, w: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """q [T,H,D], k [T_kv,D], head gates [T,H] straight from the projections (before RoPE), windows [0, ke).  With w, the
+        gates as projections() returns them, `gate` is not used."""
+        if w is None:
+            q_fp8, _, w = self._rope_quant(q, q.shape[0], q.shape[1], gate)
+        else:
+            q_fp8, q_scale = self._rope_quant(q, q.shape[0], q.shape[1])
+            w = _fold(w, q_scale, self.spec.index_head_dim)
         k_fp8, k_scale = self._rope_quant(k, k.shape[0], 1)
-        ks = torch.zeros_like(ke)
-        return _score_topk(q_fp8, k_fp8, k_scale, _fold(w, q_scale, self.spec.index_head_dim), ks, ke, topk)
+        return _score_topk(q_fp8, k_fp8, k_scale, w, None, ke, topk, dtype)
 
     @torch.no_grad()
-    def forward(self, x, q_lora_a):
-        q, k, w = self.projections(x, q_lora_a)
+    def forward(self, x, q_lora_a, index_dtype: torch.dtype = torch.int64):
         T = x.shape[0]
+        gate = w = None
+        if getattr(self.projections, "__func__", None) is DsaIndexer.projections:
+            q = self.wq_b(q_lora_a).view(T, self.spec.index_n_heads, self.spec.index_head_dim)
+            k, gate = self.k_norm(self.wk(x)), self.weights_proj(x)
+        else:                                              # a subclass's own
+            q, k, w = self.projections(x, q_lora_a)
         ke = torch.arange(1, T + 1, dtype=torch.int32, device=x.device)
-        return self._select(q, k, w, ke, min(self.spec.index_topk, T))
+        return self._select(q, k, gate, ke, min(self.spec.index_topk, T), index_dtype, w)
 
 
 class C4Compressor(nn.Module):
@@ -289,6 +304,5 @@ class Dsv4Indexer(DsaIndexer):
         T_kv = T // cr
         q = self.wq_b(q_lora_a).view(T, self.spec.index_n_heads, self.spec.index_head_dim)
         k = self.k_norm(self.compressor(x))
-        w = self.weights_proj(x).float() * self.spec.index_n_heads ** -0.5
         ke = ((torch.arange(1, T + 1, device=x.device) + cr - 1) // cr).to(torch.int32)
-        return self._select(q, k, w, ke, min(self.spec.index_topk // cr, T_kv))
+        return self._select(q, k, self.weights_proj(x), ke, min(self.spec.index_topk // cr, T_kv), torch.int64)

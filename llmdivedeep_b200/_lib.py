@@ -24,6 +24,8 @@ SIGNATURES = {
     "dsa_pack_latent_cache": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p]),
     "dsa_rope_fp8_quant": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p,
                                    c_void_p, c_void_p]),
+    "dsa_rope_fp8_quant_gated": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int64, c_void_p,
+                                         c_void_p, c_void_p, c_float, c_float, c_void_p, c_void_p]),
     "dsa_indexer_logits": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                    c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "dsa_indexer_logits_paged": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int64,

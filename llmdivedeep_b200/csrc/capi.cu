@@ -65,7 +65,8 @@ int fp8_quant_launch(const void* x, int x_is_bf16, int64_t n_blocks, int block, 
                      cudaStream_t stream);
 int pack_latent_launch(const void* kv, int kv_is_bf16, int64_t row_stride, int64_t n, void* rec, cudaStream_t stream);
 int rope_fp8_quant_launch(const void* x, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
-                          const float* cos_t, const float* sin_t, void* q, float* scale, cudaStream_t stream);
+                          const float* cos_t, const float* sin_t, void* q, float* scale, const void* gate, float mul0,
+                          float mul1, float* gate_out, cudaStream_t stream);
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
@@ -272,14 +273,15 @@ int dsa_pack_latent_cache(const void* kv, int kv_dtype, int64_t row_stride, int6
   return pack_latent_launch(kv, kv_dtype == DSA_X_BF16, row_stride, n_tokens, records, static_cast<cudaStream_t>(stream));
 }
 
-int dsa_rope_fp8_quant(const void* x_bf16, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
-                       const float* cos_table, const float* sin_table, int64_t n_pos, void* q_fp8, float* scale,
-                       void* stream) {
+int dsa_rope_fp8_quant_gated(const void* x_bf16, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
+                             const float* cos_table, const float* sin_table, int64_t n_pos, void* q_fp8, float* scale,
+                             const void* gate_bf16, float gate_mul0, float gate_mul1, float* gate_out, void* stream) {
   g_err[0] = 0;
   if (n_rows < 0 || n_pos < 0) return set_error(DSA_ERR_SHAPE, "rope_fp8_quant: negative size");
   if (n_rows == 0) return DSA_OK;
   if (!x_bf16 || !cos_table || !sin_table || !q_fp8 || !scale) return set_error(DSA_ERR_ARG, "rope_fp8_quant: NULL pointer argument");
   if (head_dim != 64 && head_dim != 128) return set_error(DSA_ERR_SHAPE, "rope_fp8_quant: head dim %d, only 64 and 128 are built", head_dim);
+  if (gate_bf16 && !gate_out) return set_error(DSA_ERR_ARG, "rope_fp8_quant: NULL pointer argument");
   // the rotated part is made of whole lanes (head_dim / 32 values each) and, in the halves form, of two equal lane groups
   const int per = head_dim / 32;
   if (rope_dim <= 0 || rope_dim > head_dim || rope_dim % (2 * per)) return set_error(DSA_ERR_SHAPE, "rope_fp8_quant: rope_dim %d does not fit head dim %d", rope_dim, head_dim);
@@ -289,7 +291,14 @@ int dsa_rope_fp8_quant(const void* x_bf16, int64_t n_rows, int head_dim, int rop
                      (long long)n_rows, rows_per_pos, (long long)n_pos);
   if (!aligned16(x_bf16) || (reinterpret_cast<uintptr_t>(q_fp8) & 3)) return set_error(DSA_ERR_ALIGN, "rope_fp8_quant: x must be 16-byte and q_fp8 4-byte aligned");
   return rope_fp8_quant_launch(x_bf16, n_rows, head_dim, rope_dim, interleave, rows_per_pos, cos_table, sin_table, q_fp8, scale,
-                               static_cast<cudaStream_t>(stream));
+                               gate_bf16, gate_mul0, gate_mul1, gate_out, static_cast<cudaStream_t>(stream));
+}
+
+int dsa_rope_fp8_quant(const void* x_bf16, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
+                       const float* cos_table, const float* sin_table, int64_t n_pos, void* q_fp8, float* scale,
+                       void* stream) {
+  return dsa_rope_fp8_quant_gated(x_bf16, n_rows, head_dim, rope_dim, interleave, rows_per_pos, cos_table, sin_table, n_pos, q_fp8, scale,
+                                  nullptr, 0.f, 0.f, nullptr, stream);
 }
 
 static const int kMinChunkRows = 256;

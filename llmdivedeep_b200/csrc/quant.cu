@@ -132,11 +132,22 @@ __global__ void __launch_bounds__(256) pack_latent_kernel(const T* __restrict__ 
 //   interleaved (GPT-J):  the same on (even, odd) pairs, result rounded to bf16 (the reference writes it into a
 //                         tensor of x's dtype).
 // Row r belongs to position r / rows_per_pos (query rows: heads per token; key rows: 1).  One warp per row.
+// With `gate`, the head gates of the rows become the scorer's weights on the way: ((float(gate) * mul0) * scale) * mul1, every
+// product rounded as the eager chain rounds it (sparse_attn/DSA.py:327-331, 505-511).
+constexpr int kRopeV = 8;                              // values per thread of the wide form
+struct RopeGate {
+  const __nv_bfloat16* gate;                           // [n_rows], or null
+  float* out;
+  float mul0, mul1;
+  __device__ __forceinline__ float fold(int64_t row, float scale) const {
+    return __fmul_rn(__fmul_rn(__fmul_rn(__bfloat162float(gate[row]), mul0), scale), mul1);
+  }
+};
 template <int BLOCK, bool INTERLEAVE>
 __global__ void __launch_bounds__(256) rope_fp8_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t n_rows, int rope_dim,
                                                              int rows_per_pos, const float* __restrict__ cos_t,
                                                              const float* __restrict__ sin_t, uint8_t* __restrict__ q,
-                                                             float* __restrict__ scale) {
+                                                             float* __restrict__ scale, const RopeGate g) {
   constexpr int PER = BLOCK / 32;
   const int lane = threadIdx.x & 31;
   const int half = rope_dim >> 1;
@@ -153,7 +164,7 @@ __global__ void __launch_bounds__(256) rope_fp8_quant_kernel(const __nv_bfloat16
       const __nv_bfloat162 p0 = *reinterpret_cast<const __nv_bfloat162*>(src);
       v[0] = __low2float(p0); v[1] = __high2float(p0);
     }
-    const int64_t pos = b / rows_per_pos;
+    const int64_t pos = static_cast<uint32_t>(b) / static_cast<uint32_t>(rows_per_pos);      // 2^32 rows do not fit the device's memory
     const float* cr = cos_t + pos * half;
     const float* sr = sin_t + pos * half;
     const int d0 = lane * PER;                          // first dim of this lane
@@ -200,23 +211,100 @@ __global__ void __launch_bounds__(256) rope_fp8_quant_kernel(const __nv_bfloat16
     } else {
       reinterpret_cast<uint16_t*>(q + b * BLOCK)[lane] = (uint16_t)packed;
     }
-    if (lane == 0) scale[b] = sc;
+    if (lane == 0) {
+      scale[b] = sc;
+      if (g.gate) g.out[b] = g.fold(b, sc);
+    }
+  }
+}
+
+// The same with eight values per thread, BLOCK / 8 threads per row: 16-byte loads, fewer shuffle steps.  [3000, 64, 128] 41.1 us with a
+// warp per row, 37.1 so (the quantiser alone 16.2).  Sixteen values, as that one has them, need 78 registers here: no faster.
+template <int BLOCK, bool INTERLEAVE>
+__global__ void __launch_bounds__(256) rope_fp8_quant_wide_kernel(const __nv_bfloat16* __restrict__ x, int64_t n_rows, int rope_dim,
+                                                                  int rows_per_pos, const float* __restrict__ cos_t,
+                                                                  const float* __restrict__ sin_t, uint8_t* __restrict__ q,
+                                                                  float* __restrict__ scale, const RopeGate g) {
+  constexpr int V = kRopeV, LANES = BLOCK / V;
+  const int lane = threadIdx.x & 31, half = rope_dim >> 1;
+  const int d0 = (lane & (LANES - 1)) * V;             // first dim of this lane
+  const bool rotated = d0 < rope_dim, first = d0 < half;
+  const int64_t n = n_rows * LANES, stride = (int64_t)gridDim.x * blockDim.x;
+  // whole warps stay together for the shuffles: the loop runs over warps' first threads
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
+    const int64_t i = i0 + lane, row = i / LANES;
+    float v[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = 1.f;            // lanes past the end: dividing zeros takes the slow way
+    if (i < n) load_values<V>(x + i * V, v);
+    const int64_t pos = i < n ? static_cast<uint32_t>(row) / static_cast<uint32_t>(rows_per_pos) : 0;
+    if constexpr (INTERLEAVE) {
+      if (rotated) {
+#pragma unroll
+        for (int j = 0; j < V; j += 2) {
+          const float c = __ldg(cos_t + pos * half + ((d0 + j) >> 1)), s = __ldg(sin_t + pos * half + ((d0 + j) >> 1));
+          const float e = __fsub_rn(__fmul_rn(v[j], c), __fmul_rn(v[j + 1], s));
+          const float o = __fadd_rn(__fmul_rn(v[j], s), __fmul_rn(v[j + 1], c));
+          v[j] = __bfloat162float(__float2bfloat16_rn(e));
+          v[j + 1] = __bfloat162float(__float2bfloat16_rn(o));
+        }
+      }
+    } else {
+      // the other half of the pair is half / V lanes away; every lane takes part in the shuffle
+      float c[V], s[V];
+      const float4* cr = reinterpret_cast<const float4*>(cos_t + pos * half + (first ? d0 : d0 - half));
+      const float4* sr = reinterpret_cast<const float4*>(sin_t + pos * half + (first ? d0 : d0 - half));
+#pragma unroll
+      for (int j = 0; j < V; j += 4) {
+        const float4 c4 = rotated ? __ldg(cr + j / 4) : make_float4(1.f, 1.f, 1.f, 1.f), s4 = rotated ? __ldg(sr + j / 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        c[j] = c4.x; c[j + 1] = c4.y; c[j + 2] = c4.z; c[j + 3] = c4.w;
+        s[j] = s4.x; s[j + 1] = s4.y; s[j + 2] = s4.z; s[j + 3] = s4.w;
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float other = __shfl_xor_sync(0xffffffffu, v[j], half / V);
+        const float s1 = first ? -s[j] : s[j];         // x1 c - x2 s and x2 c + x1 s: the same roundings
+        if (rotated) v[j] = __fadd_rn(__fmul_rn(v[j], c[j]), __fmul_rn(other, s1));
+      }
+    }
+    uint32_t w[V / 4];
+    const float sc = quant_values<LANES, V>(v, w);
+    if (i < n) {
+      *reinterpret_cast<uint2*>(q + i * V) = make_uint2(w[0], w[1]);
+      if ((lane & (LANES - 1)) == 0) {
+        scale[row] = sc;
+        if (g.gate) g.out[row] = g.fold(row, sc);
+      }
+    }
   }
 }
 
 int rope_fp8_quant_launch(const void* x, int64_t n_rows, int head_dim, int rope_dim, int interleave, int rows_per_pos,
-                          const float* cos_t, const float* sin_t, void* q, float* scale, cudaStream_t stream) {
+                          const float* cos_t, const float* sin_t, void* q, float* scale, const void* gate, float mul0,
+                          float mul1, float* gate_out, cudaStream_t stream) {
   if (n_rows == 0) return DSA_OK;
-  const int64_t want = (n_rows + 7) / 8;
-  const int grid = (int)(want < (int64_t)sm_count() * 16 ? want : (int64_t)sm_count() * 16);
+  if (head_dim != 64 && head_dim != 128) return set_error(DSA_ERR_SHAPE, "rope_fp8_quant: head dim %d not supported (64 or 128)", head_dim);
   const __nv_bfloat16* xi = static_cast<const __nv_bfloat16*>(x);
   uint8_t* qo = static_cast<uint8_t*>(q);
-#define DSA_ROPE_CASE(B, I) rope_fp8_quant_kernel<B, I><<<grid, 256, 0, stream>>>(xi, n_rows, rope_dim, rows_per_pos, cos_t, sin_t, qo, scale)
-  if (head_dim == 128 && interleave) DSA_ROPE_CASE(128, true);
-  else if (head_dim == 128) DSA_ROPE_CASE(128, false);
-  else if (head_dim == 64 && interleave) DSA_ROPE_CASE(64, true);
-  else if (head_dim == 64) DSA_ROPE_CASE(64, false);
-  else return set_error(DSA_ERR_SHAPE, "rope_fp8_quant: head dim %d not supported (64 or 128)", head_dim);
+  const RopeGate g{static_cast<const __nv_bfloat16*>(gate), gate_out, mul0, mul1};
+  // Eight values a thread where the rotated part is made of whole threads (whole pairs of them), the addresses allow its accesses
+  // and the call is not over in two microseconds anyway (a thread's divisions in a row are then what takes the time).
+  const bool wide = rope_dim % (interleave ? kRopeV : 2 * kRopeV) == 0 && n_rows * (head_dim / kRopeV) >= (int64_t)sm_count() * 512 &&
+                    ((reinterpret_cast<uintptr_t>(q) & 7) | ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15)) == 0;
+  const int64_t want = wide ? (n_rows * (head_dim / kRopeV) + 255) / 256 : (n_rows + 7) / 8, most = (int64_t)sm_count() * 16;
+  const int grid = (int)(want < most ? want : most);
+#define DSA_ROPE_CASE(K, B, I) K<B, I><<<grid, 256, 0, stream>>>(xi, n_rows, rope_dim, rows_per_pos, cos_t, sin_t, qo, scale, g)
+#define DSA_ROPE_CASES(K)                                     \
+  if (head_dim == 128 && interleave) DSA_ROPE_CASE(K, 128, true); \
+  else if (head_dim == 128) DSA_ROPE_CASE(K, 128, false);     \
+  else if (interleave) DSA_ROPE_CASE(K, 64, true);            \
+  else DSA_ROPE_CASE(K, 64, false)
+  if (wide) {
+    DSA_ROPE_CASES(rope_fp8_quant_wide_kernel);
+  } else {
+    DSA_ROPE_CASES(rope_fp8_quant_kernel);
+  }
+#undef DSA_ROPE_CASES
 #undef DSA_ROPE_CASE
   return check_launch("rope_fp8_quant");
 }

@@ -71,10 +71,13 @@ class DSALayer(nn.Module):
     def stages(self, x: torch.Tensor) -> dict:
         """forward() with every intermediate kept: q_lora, the indexer's selection (int32, -1 = unused
         slot), the attention operands and the output."""
+        from . import DSA
         x = x.to(self.dtype)
         T = x.shape[0]
         q_lora = self.q_a(x)
-        idx = self.indexer(x, q_lora).to(torch.int32)
+        # the kernels' own int32 positions, without the way through the int64 that the reference's indexer returns
+        own = type(self.indexer).forward is DSA.DsaIndexer.forward
+        idx = (self.indexer(x, q_lora, index_dtype=torch.int32) if own else self.indexer(x, q_lora)).to(torch.int32)
         q = self.wq(q_lora).view(T, self.n_heads, 576)
         kv = self.wkv(x)
         out = self.attn(q, kv, idx)

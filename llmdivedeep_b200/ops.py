@@ -533,12 +533,14 @@ def pack_latent_records(kv: torch.Tensor, out: Optional[torch.Tensor]) -> Option
 
 
 def rope_fp8_quant(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rope_dim: int, interleave: bool,
-                   rows_per_pos: int = 1):
+                   rows_per_pos: int = 1, gate: Optional[torch.Tensor] = None, gate_mul: tuple = (1.0, 1.0)):
     """RoPE on the first ``rope_dim`` values of every head row followed by the per-row FP8 quantiser, one kernel
     (DsaIndexer.rope + fp8_quant_per_block, sparse_attn/DSA.py:513-524, 530-531).  x bf16 [..., head_dim] with
     head_dim 64 or 128; cos / sin fp32 [positions, rope_dim / 2]; the row with flat index r sits at position
-    r // rows_per_pos.  Returns (q float8_e4m3fn like x, scale fp32 x.shape[:-1]), bit-identical to the eager chain."""
-    dev = _need_cuda(x, cos, sin)
+    r // rows_per_pos.  Returns (q float8_e4m3fn like x, scale fp32 x.shape[:-1]), bit-identical to the eager chain.
+    With ``gate`` (bf16, x.shape[:-1]) also the scorer's weights (gate.float() * gate_mul[0]) * scale * gate_mul[1]
+    (sparse_attn/DSA.py:327-331, 505-511), fp32, from the same kernel."""
+    dev = _need_cuda(x, cos, sin, gate)
     if x.dtype != torch.bfloat16 or cos.dtype != torch.float32 or sin.dtype != torch.float32:
         raise DsaError("rope_fp8_quant takes bf16 x and fp32 cos / sin tables")
     D = x.shape[-1]
@@ -548,8 +550,14 @@ def rope_fp8_quant(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, rope_d
     n_rows = x.numel() // D
     q = torch.empty(x.shape, dtype=FP8, device=x.device)
     scale = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
+    w = None
+    if gate is not None:
+        if gate.dtype != torch.bfloat16 or gate.shape != x.shape[:-1]:
+            raise DsaError(f"gate must be bf16 {tuple(x.shape[:-1])}, got {gate.dtype} {tuple(gate.shape)}")
+        gate, w = gate.contiguous(), torch.empty_like(scale)
     lib = _lib.load()
     with _on(dev):
-        check(lib.dsa_rope_fp8_quant(_ptr(x), n_rows, D, rope_dim, int(bool(interleave)), rows_per_pos, _ptr(cos), _ptr(sin),
-                                     cos.shape[0], _ptr(q), _ptr(scale), _stream(dev)))
-    return q, scale
+        check(lib.dsa_rope_fp8_quant_gated(_ptr(x), n_rows, D, rope_dim, int(bool(interleave)), rows_per_pos, _ptr(cos), _ptr(sin),
+                                           cos.shape[0], _ptr(q), _ptr(scale), _ptr(gate), float(gate_mul[0]), float(gate_mul[1]),
+                                           _ptr(w), _stream(dev)))
+    return (q, scale) if w is None else (q, scale, w)

@@ -160,3 +160,22 @@ def test_fused_rope_quantiser_refuses_bad_shapes():
         ops.rope_fp8_quant(x, t, t, 48, False)            # 24 dims per half = 6 lanes: not a power of two
     with pytest.raises(ops.DsaError):
         ops.rope_fp8_quant(x, t[:2, :16].contiguous(), t[:2, :16].contiguous(), 32, False)   # 4 rows, 2 positions
+
+
+@pytest.mark.parametrize("D,rope", [(128, 64), (128, 128), (128, 32), (64, 64), (64, 32), (64, 8)])
+@pytest.mark.parametrize("interleave", [False, True])
+@pytest.mark.parametrize("T,H", [(1, 1), (37, 4), (300, 64), (1501, 64)])
+def test_rope_quant_and_gates_equal_the_eager_chain(D, rope, interleave, T, H):
+    """The fused kernel (a warp per row for small calls, eight values a thread for large ones, rope widths that do not fill threads)
+    against RoPE, quantiser and gate folding as separate torch operations: bytes, scales and weights bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(T + H + D + rope)
+    x = torch.randn(T, H, D, device="cuda", generator=g).bfloat16()
+    x[0, 0] = 0
+    gate = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    cos, sin = DSA._rope_cossin(T, rope, x.device)
+    q8, scale, w = ops.rope_fp8_quant(x, cos, sin, rope, interleave, H, gate, (H ** -0.5, D ** -0.5))
+    eq, es = DSA.fp8_quant_per_block(DSA._rope_head(x, rope, T, interleave), D)
+    assert torch.equal(q8.view(torch.uint8), eq.view(torch.uint8)) and torch.equal(scale, es)
+    assert torch.equal(w, DSA._fold(gate.float() * H ** -0.5, es, D))
+    again = ops.rope_fp8_quant(x, cos, sin, rope, interleave, H)
+    assert torch.equal(again[0].view(torch.uint8), eq.view(torch.uint8)) and torch.equal(again[1], es)

@@ -15,9 +15,11 @@
 //     number of blocks) and for positions out of range, and sends for Q.
 //   * warps 6-21: gather, four rows of a block each, by cp.async that arrive on the block's barrier by themselves.  The latent
 //     rows lie in a ring of panel pairs (128 dims of 64 keys), freed one by one as P.V has read them, the rope panels in another.
-// 2048 tokens x 2048 of 16384 keys, 16 heads: 985 -> 610 us (a gather of 7.9 TB/s); 4096 tokens 1938 -> 1180; 2048 tokens x 256 keys
-// 276 -> 138.  32 heads: 992 -> 804.  64 heads as one N = 64 tile were built too: Q takes the room of a third block, 1127 us
-// against 1051 for the pair kernel, which therefore keeps them.
+// What bounds it: the tensor pipe, whose 52 MMAs a block cost 47 cycles each whatever their N (2450 cycles; the gather alone would
+// take 1900).  us before (the pair kernel) and now: 16 heads, 2048 tokens x 2048 of 16384 keys 985 -> 571, 4096 tokens 1938 -> 1105, 2048
+// tokens x 256 keys 276 -> 92; 32 heads 992 -> 705.  Tried: 128 keys a score tile (fewer MMAs, but then 1 1/4 blocks fit and the
+// gather waits for P.V: 835 against 607); 64 heads as one N = 64 tile (Q takes the room of a block: 1127 against 1051 for the pair
+// kernel, which therefore keeps them); the output put off until the next token's first P is on its way (spills: 668 against 610).
 // Every wait is bounded (dsa_common.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -445,7 +447,17 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
 #pragma unroll
         for (int i = 0; i < NH; ++i) *reinterpret_cast<float2*>(sum_s + warp * N + 8 * i + 2 * lane) = make_float2(l[2 * i], l[2 * i + 1]);
       }
-      ok = all_meet() && mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+      ok = all_meet();
+      if (!ok) break;
+      // a head's quotient is taken once, into this warp's row of the other half (taken by every thread for every tile: 48 -> 85 us
+      // for 2048 tokens x 64 keys)
+      float* inv_s = max_s + ((n + 1) & 1) * 4 * N + warp * N;
+      if (lane < N) {
+        const float sum = (sum_s[lane] + sum_s[N + lane]) + (sum_s[2 * N + lane] + sum_s[3 * N + lane]);
+        inv_s[lane] = sum > 0.f ? 1.f / sum : 0.f;
+      }
+      __syncwarp();
+      ok = mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
       if (!ok) break;
       tc_fence_after();
       const int even = (lane & 1) ^ 1;
@@ -456,9 +468,9 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
         const int h0 = c & (N - 1);
         float inv[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float sum = (sum_s[h0 + i] + sum_s[N + h0 + i]) + (sum_s[2 * N + h0 + i] + sum_s[3 * N + h0 + i]);
-          inv[i] = sum > 0.f ? 1.f / sum : 0.f;
+        for (int i = 0; i < 16; i += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(inv_s + h0 + i);
+          inv[i] = f.x; inv[i + 1] = f.y; inv[i + 2] = f.z; inv[i + 3] = f.w;
         }
         tmem_wait_ld();
         // two neighbouring dims to a word: the even lane takes the pair of the even head, the odd lane that of the odd one

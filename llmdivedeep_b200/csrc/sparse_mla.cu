@@ -439,6 +439,9 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     // ----------------------------- gather of the selected rows -----------------------------
     const int w4 = warp - kMlaGatherWarp0;
     constexpr int kG = kMlaGatherWarps;
+    // Five of a warp's six slots are always within the block: said so, prefill of 128 heads takes 2160 us instead of 2202 (4096 x 2048
+    // keys), of 64 heads 1988 instead of 2044.  (Decode gains nothing.)
+    if constexpr (!FP8_PAGED) __builtin_assume(w4 < kG);
     bool ok = true;
     // A warp fetches every kG-th slot of a block, six at most: lane j < 6 keeps the id of slot w4 + 11 j.
     auto load_pos = [&](int blk) -> int {

@@ -107,6 +107,18 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait_limit<UNROLL>(bar, parity, abort_flag, status, kSpinLimit));
 }
+// ---- kernels that start under the end of the one before -------------------------
+// In a launch with the programmatic-serialisation attribute a kernel may start when every block of the one before has called
+// launch_dependents; what that one has written is visible after grid_wait (which returns at once in an ordinary launch).
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The pointer that comes back is the one to read through: loads through it cannot move before the wait, nor be taken for
+// loads of memory that does not change while the kernel runs.
+template <typename T>
+__device__ __forceinline__ T* grid_wait(T* p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+  return p;
+}
+
 // ---- TMA (tiled bulk tensor copies, global -> this CTA's shared memory) ----
 __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, int y, uint64_t* bar) {
   asm volatile(

@@ -11,6 +11,21 @@ namespace dsa {
 int set_error(int code, const char* fmt, ...);
 // cudaGetLastError() after a launch; no synchronisation.
 int check_launch(const char* what);
+// A launch that, with `overlapped`, may start under the end of the kernel before it on the stream (griddepcontrol in both).
+template <typename... Params, typename... Args>
+inline void launch_after(int overlapped, void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlapped ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);          // its error is the launch check's
+}
 // Multiprocessor count of the current device (cached per device).
 int sm_count();
 

@@ -251,6 +251,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  if constexpr (PAGED) launch_dependents();
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::STAGES; ++i) {
       mbar_init(&k_full[i], 1);

@@ -240,7 +240,9 @@ __device__ __forceinline__ uint4 e4m3x8_to_bf16(uint2 raw, float sc) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-template <bool FP8_PAGED>
+// OVERLAPPED: a launch that may start under the end of the top-k's (decode of few sequences; in the others its loads and their
+// place cost 2 %: batch 148 122.3 -> 124.9 us).
+template <bool FP8_PAGED, bool OVERLAPPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMlaThreads, 1)
 sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
                   const __grid_constant__ CUtensorMap tmap_o, const MlaArgs a) {
@@ -286,19 +288,27 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
   auto q_stage = [&](int lp) -> uint8_t* { return kv_s + kQStage + lp * kMlaQPanelBytes; };
 
   // ---- set-up, arranged so that nothing waits for anything it does not need ------------------------------------
-  // every warp requests the last 32 slots of the list (they decide the number of key blocks) and the gather warps their
-  // slots of the first block ...
+  // every warp requests the last 32 slots of the list (they decide the number of key blocks), the gather warps their slots of the
+  // first block and every thread its share of the whole list.  A kernel that started under the top-k's end reads it
+  // after the wait for that, and by loads that may not be served from before; its set-up comes first.
+  if constexpr (OVERLAPPED) launch_dependents();
+  int tail = -1, slot_pos = -1;
+  int look[kMlaLooks];
   const int tail_j = k_cnt - 32 + lane;
-  const int tail = tail_j >= 0 ? __ldg(idx_row + tail_j) : -1;
   const int slot = warp >= kMlaGatherWarp0 && lane < kRawRows ? warp - kMlaGatherWarp0 + lane * kMlaGatherWarps : kMlaBlk;
-  const int slot_pos = slot < kMlaBlk && slot < k_cnt ? __ldg(idx_row + slot) : -1;
-  int look[kMlaLooks];                                         // ... and every thread its share of the whole list
+  auto list_at = [&](int j) { return OVERLAPPED ? idx_row[j] : __ldg(idx_row + j); };
+  auto request_list = [&]() {
+    if constexpr (OVERLAPPED) idx_row = grid_wait(idx_row);
+    tail = tail_j >= 0 ? list_at(tail_j) : -1;
+    slot_pos = slot < kMlaBlk && slot < k_cnt ? list_at(slot) : -1;
 #pragma unroll
-  for (int u = 0; u < kMlaLooks; ++u) {
-    const int j = threadIdx.x + u * kMlaThreads;
-    look[u] = j < k_cnt - 32 ? __ldg(idx_row + j) : -1;
-  }
-  // ... while warp 0 initialises the barriers (one per lane) and sends for Q (one panel per lane) and the MMA warp allocates
+    for (int u = 0; u < kMlaLooks; ++u) {
+      const int j = threadIdx.x + u * kMlaThreads;
+      look[u] = j < k_cnt - 32 ? list_at(j) : -1;
+    }
+  };
+  if constexpr (!OVERLAPPED) request_list();
+  // Meanwhile warp 0 initialises the barriers (one per lane) and sends for Q (one panel per lane) and the MMA warp allocates
   // tensor memory
   if (warp == 0) {
     for (int i = lane; i < 59; i += 32) {
@@ -325,6 +335,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tmem_alloc(tmem_slot, kMlaTmemCols);
     tmem_relinquish();
   }
+  if constexpr (OVERLAPPED) request_list();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -449,7 +460,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
     // A warp fetches every kG-th slot of a block, six at most: lane j < 6 keeps the id of slot w4 + 11 j.
     auto load_pos = [&](int blk) -> int {
       const int j = blk * kMlaBlk + slot;
-      return (slot < kMlaBlk && blk < nblk && j < k_cnt) ? __ldg(idx_row + j) : -1;
+      return (slot < kMlaBlk && blk < nblk && j < k_cnt) ? list_at(j) : -1;
     };
     auto mark = [&](int blk, bool used) {
       if (slot < kMlaBlk) valid_s[(blk % kMlaValidRing) * kMlaBlk + slot] = used;
@@ -845,6 +856,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // by the sums of the CTA that computed it.
 // A query in eight parts: 4.8 us with loads behind the weights' loop, 3.6 so.
 __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a) {
+  const float *lse = grid_wait(a.part_lse), *part = a.part_o;
   const int u = blockIdx.x, t = a.n_full + u, h = blockIdx.y;
   const int d = threadIdx.x * 4, cta = d / kMlaDvHalf;
   // every load is requested before any is used: a part's weight and values do not wait for one another
@@ -853,8 +865,8 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a
 #pragma unroll
   for (int sp = 0; sp < kMlaMaxParts; ++sp) {
     const int64_t p = (int64_t)u * a.n_split + sp;
-    wgt[sp] = sp < a.n_split ? a.part_lse[(p * 2 + cta) * a.H + h] : -CUDART_INF_F;
-    v[sp] = sp < a.n_split ? *reinterpret_cast<const float4*>(a.part_o + (p * a.H + h) * kMlaDv + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    wgt[sp] = sp < a.n_split ? lse[(p * 2 + cta) * a.H + h] : -CUDART_INF_F;
+    v[sp] = sp < a.n_split ? *reinterpret_cast<const float4*>(part + (p * a.H + h) * kMlaDv + d) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   float mx = -CUDART_INF_F, den = 0.f;
 #pragma unroll
@@ -879,7 +891,7 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a
 int make_tmap_2d_bytes(CUtensorMap* m, const void* base, uint64_t rows, uint64_t inner_bytes, uint64_t row_pitch,
                        uint32_t box_bytes, uint32_t box_rows);
 
-template <bool FP8_PAGED>
+template <bool FP8_PAGED, bool OVERLAPPED>
 static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaStream_t stream) {
   if (args.T == 0 || args.H == 0) return DSA_OK;
   if (args.K > kMlaMaxK) return set_error(DSA_ERR_SHAPE, "sparse_mla: K (%d) exceeds %d", args.K, kMlaMaxK);
@@ -895,14 +907,14 @@ static int launch_mla(const void* q, const void* kv, const MlaArgs& args, cudaSt
     if ((rc = make_tmap_2d_bytes(&to, a.out, (uint64_t)a.T * a.H, kMlaDv * 2, kMlaDv * 2, 128, 128))) return rc;
     a.tma_out = 1;
   }
-  auto kern = sparse_mla_kernel<FP8_PAGED>;
+  auto kern = sparse_mla_kernel<FP8_PAGED, OVERLAPPED>;
   constexpr int smem_bytes = FP8_PAGED ? kMlaSmemDecode : kMlaSmemBytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess)
     return set_error(DSA_ERR_CUDA, "sparse_mla: cannot raise dynamic shared memory to %d", smem_bytes);
   const int n_parts = a.T - a.n_full;
   const dim3 grid(2 * (a.n_full + n_parts * a.n_split), 1, (a.H + 127) / 128);
-  kern<<<grid, kMlaThreads, smem_bytes, stream>>>(tq, to, a);
-  if (n_parts > 0) sparse_mla_combine_kernel<<<dim3(n_parts, a.H), 128, 0, stream>>>(a);
+  launch_after(OVERLAPPED, kern, grid, kMlaThreads, smem_bytes, stream, tq, to, a);
+  if (n_parts > 0) launch_after(OVERLAPPED, sparse_mla_combine_kernel, dim3(n_parts, a.H), 128, 0, stream, a);
   return check_launch("sparse_mla");
 }
 
@@ -921,7 +933,7 @@ int sparse_mla_prefill_launch(const void* q, const void* kv, const int32_t* idx,
   a.status = status;
   a.n_full = T;
   a.n_split = 1;
-  return launch_mla<false>(q, kv, a, stream);
+  return launch_mla<false, false>(q, kv, a, stream);
 }
 
 // A CTA pair per query fills the GPU in rounds of (SMs / 2 / head groups) queries; the last, partly filled round would
@@ -946,7 +958,7 @@ size_t mla_decode_workspace_bytes(int B, int H, int K) {
 
 int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* block_table, int64_t table_stride,
                              const int32_t* idx, void* out, int B, int H, int K, int num_pages, int max_ctx,
-                             float scale, void* workspace, size_t workspace_bytes, int32_t* status,
+                             float scale, void* workspace, size_t workspace_bytes, int32_t* status, int overlapped,
                              cudaStream_t stream) {
   MlaArgs a{};
   const int pairs = mla_pairs(H), rest = B % pairs;
@@ -972,7 +984,7 @@ int sparse_mla_decode_launch(const void* q, const void* cache, const int32_t* bl
   a.num_phys_rows = num_pages * kLatentPage;
   a.scale_log2e = scale * 1.4426950408889634f;
   a.status = status;
-  return launch_mla<true>(q, nullptr, a, stream);
+  return overlapped ? launch_mla<true, true>(q, nullptr, a, stream) : launch_mla<true, false>(q, nullptr, a, stream);
 }
 
 }  // namespace dsa

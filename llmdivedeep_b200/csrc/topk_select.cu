@@ -58,6 +58,10 @@ __device__ __forceinline__ float key_value(uint32_t key) {
   return __uint_as_float(key ^ (static_cast<uint32_t>(static_cast<int32_t>(~key) >> 31) | 0x80000000u));
 }
 
+// a plain load: the logits may have been written while this kernel was already running
+template <typename T>
+__device__ __forceinline__ T load_now(const T* p) { return *p; }
+
 // A range of values cut into kLinBins equal bins, counted from the top.  (hi - x) and its product with a positive factor are
 // monotone in floating point, so the bins order elements as their keys do; what lies above hi falls into bin 0, what lies below
 // the range into the last.  A NaN with the sign bit clear has the largest key and falls into bin 0, one with the sign bit set
@@ -223,13 +227,13 @@ __device__ __forceinline__ bool at_or_above(float v, uint32_t tfb) {
 // reads them as 8 coalesced float4 rows.  Returns the hit flags of this lane, bit q*4+e for column
 // wbase + q*128 + lane*4 + e.
 template <bool NEG>
-__device__ __forceinline__ uint32_t chunk_flags(const float* __restrict__ x, int wbase, int lane, int lo, int hi,
+__device__ __forceinline__ uint32_t chunk_flags(const float* x, int wbase, int lane, int lo, int hi,
                                                 uint32_t tfb) {
   uint32_t fc = 0;
   if (wbase >= lo && wbase + kRun * 32 <= hi) {
 #pragma unroll
     for (int q = 0; q < kRun / kVec; ++q) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(x + wbase + q * 128 + lane * kVec));
+      const float4 f = load_now(reinterpret_cast<const float4*>(x + wbase + q * 128 + lane * kVec));
       if (at_or_above<NEG>(f.x, tfb)) fc |= 1u << (q * 4 + 0);
       if (at_or_above<NEG>(f.y, tfb)) fc |= 1u << (q * 4 + 1);
       if (at_or_above<NEG>(f.z, tfb)) fc |= 1u << (q * 4 + 2);
@@ -239,7 +243,7 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* __restrict__ x, int
     for (int q = 0; q < kRun / kVec; ++q) {
       const int i = wbase + q * 128 + lane * kVec;
       if (i < hi && i + kVec > lo) {         // a float4 that starts below hi lies inside the row's allocation
-        const float4 f = __ldg(reinterpret_cast<const float4*>(x + i));
+        const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
         const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
         for (int e2 = 0; e2 < kVec; ++e2)
@@ -250,13 +254,13 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* __restrict__ x, int
   return fc;
 }
 
-__device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* __restrict__ x, int wbase, int lane, uint32_t fc,
+__device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* x, int wbase, int lane, uint32_t fc,
                                            uint32_t pc, const LinBins& bins) {
   while (fc) {                               // few bits set: reload the hits (L1) rather than keep 32 values
     const int j = __ffs(fc) - 1;
     fc &= fc - 1;
     const int col = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
-    const float v = __ldg(x + col);
+    const float v = load_now(x + col);
     sm.cand_key[pc] = order_key(v);
     sm.cand_idx[pc] = col;
     atomicAdd(&sm.lin[bins.of(v)], 1u);
@@ -268,7 +272,7 @@ __device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* __restrict
 // bins.  Candidates end up in a fixed order (1024 columns, lane, column) that does not depend on timing or on TH.
 // Returns the staged count, or 0xffffffff once it would exceed the capacity (uniform over the block).
 template <int TH, bool NEG>
-__device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t tfb,
+__device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* x, int lo, int hi, uint32_t tfb,
                                               const LinBins& bins) {
   constexpr int CHUNK = TH * kRun;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -350,7 +354,7 @@ __device__ __forceinline__ bool select_by_bins(TopkSmem& sm, const LinBins& bins
 // that its candidates are counted by.  Returns false (for every thread of the block alike) when the row rules the sampled pass
 // out.  The result depends on the row alone, not on TH.  Leaves sm.lin zeroed (a barrier has to follow).
 template <int TH>
-__device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, int k,
+__device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* x, int lo, int hi, int k,
                                                  float& thr_out, LinBins& bins_out) {
   constexpr int NPT = kSampleMaxBlocks / (TH / 32) * 4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -374,7 +378,7 @@ __device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* __re
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool in = j < mblk;
     if (in) {
-      f = __ldg(reinterpret_cast<const float4*>(x + first + (j * sb + sb / 2) * kSampleBlock + lane * kVec));
+      f = load_now(reinterpret_cast<const float4*>(x + first + (j * sb + sb / 2) * kSampleBlock + lane * kVec));
       svalid |= 0xFu << (4 * i);
     }
     skey[4 * i + 0] = order_key(f.x); skey[4 * i + 1] = order_key(f.y);
@@ -414,7 +418,7 @@ __device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* __re
 // One ordered pass over columns [lo, hi) of the row: stages everything whose key is at or above thr's.
 // Returns the staged count, or 0xffffffff once it would exceed the capacity (uniform over the block).
 template <int TH>
-__device__ __forceinline__ uint32_t stage_above(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, uint32_t thr,
+__device__ __forceinline__ uint32_t stage_above(TopkSmem& sm, const float* x, int lo, int hi, uint32_t thr,
                                                 const LinBins& bins) {
   const bool neg = (thr & 0x80000000u) == 0u;             // the threshold is a negative float
   const uint32_t tfb = neg ? ~thr : (thr ^ 0x80000000u);  // its bits as a float
@@ -425,7 +429,7 @@ __device__ __forceinline__ uint32_t stage_above(TopkSmem& sm, const float* __res
 // when the row has to take the two-pass path: geometry out of range, or the staged count missed [k, 4096].
 // Needs 16-byte aligned rows.
 template <int TH>
-__device__ __forceinline__ bool sampled_single_pass(TopkSmem& sm, const float* __restrict__ x, int lo, int hi, int k,
+__device__ __forceinline__ bool sampled_single_pass(TopkSmem& sm, const float* x, int lo, int hi, int k,
                                                     int32_t* __restrict__ o) {
   constexpr int NPT = kCandS / TH;
   float thr;
@@ -453,7 +457,7 @@ __device__ __forceinline__ bool sampled_single_pass(TopkSmem& sm, const float* _
 // order = column order.  Returns false, for all threads alike, when the values have no usable range (infinities, NaN, all equal)
 // or the threshold bin holds too many: the two-pass path settles those.
 template <int TH, int CHUNKS>
-__device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* __restrict__ x, bool vec, int lo, int hi, int k,
+__device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* x, bool vec, int lo, int hi, int k,
                                            int32_t* __restrict__ o) {
   constexpr int NPT = kDirectChunk / TH;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -468,13 +472,13 @@ __device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* __restrict
       float v[kVec] = {0.f, 0.f, 0.f, 0.f};
       if (vec) {                                          // a float4 that starts below hi lies inside the row's allocation
         if (i0 + c * kDirectChunk + j < hi) {
-          const float4 f = __ldg(reinterpret_cast<const float4*>(xc + i0 + j));
+          const float4 f = load_now(reinterpret_cast<const float4*>(xc + i0 + j));
           v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
         }
       } else {
 #pragma unroll
         for (int e = 0; e < kVec; ++e)
-          if (used(c, j + e)) v[e] = __ldg(xc + i0 + j + e);
+          if (used(c, j + e)) v[e] = load_now(xc + i0 + j + e);
       }
 #pragma unroll
       for (int e = 0; e < kVec; ++e) key[c][j + e] = order_key(v[e]);
@@ -520,7 +524,7 @@ __device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* __restrict
 
 // One row, one CTA: the whole selection.
 template <int TH>
-__device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__ logits, int64_t ld,
+__device__ __forceinline__ void topk_row(TopkSmem& sm, const float* logits, int64_t ld,
                                          const int32_t* __restrict__ ks, const int32_t* __restrict__ ke, int S, int k,
                                          int32_t* __restrict__ out, int one_pass, int row) {
   constexpr int kChunkHist = TH * kVec, kChunkFinal = TH * kEltPerThread, kCandPerThread = kCand / TH;
@@ -564,7 +568,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
       if (pbits == 0) {
 #pragma unroll 4
         for (int i = first_full + tid * kVec; i < last_full; i += kChunkHist) {
-          const float4 f = __ldg(reinterpret_cast<const float4*>(x + i));
+          const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
           atomicAdd(&sm.hist[order_key(f.x) >> shift], 1u);
           atomicAdd(&sm.hist[order_key(f.y) >> shift], 1u);
           atomicAdd(&sm.hist[order_key(f.z) >> shift], 1u);
@@ -574,7 +578,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
         const int pshift = 32 - pbits;
 #pragma unroll 4
         for (int i = first_full + tid * kVec; i < last_full; i += kChunkHist) {
-          const float4 f = __ldg(reinterpret_cast<const float4*>(x + i));
+          const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
           const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -588,12 +592,12 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
       const int n_tail = last_full >= first_full ? hi - last_full : 0;
       if (tid < n_head + n_tail) {
         const int i = tid < n_head ? lo + tid : last_full + (tid - n_head);
-        const uint32_t key = order_key(__ldg(x + i));
+        const uint32_t key = order_key(load_now(x + i));
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     } else {
       for (int i = lo + tid; i < hi; i += TH) {
-        const uint32_t key = order_key(__ldg(x + i));
+        const uint32_t key = order_key(load_now(x + i));
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     }
@@ -622,13 +626,13 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
 #pragma unroll
         for (int q = 0; q < kEltPerThread / kVec; ++q) {
           // a float4 that starts below hi lies inside the row's allocation (ld % 4 == 0)
-          const float4 f = (i0 + q * kVec < hi) ? __ldg(reinterpret_cast<const float4*>(x + i0 + q * kVec))
+          const float4 f = (i0 + q * kVec < hi) ? load_now(reinterpret_cast<const float4*>(x + i0 + q * kVec))
                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
           v[q * 4 + 0] = f.x; v[q * 4 + 1] = f.y; v[q * 4 + 2] = f.z; v[q * 4 + 3] = f.w;
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kEltPerThread; ++j) v[j] = (i0 + j >= lo && i0 + j < hi) ? __ldg(x + i0 + j) : 0.f;
+        for (int j = 0; j < kEltPerThread; ++j) v[j] = (i0 + j >= lo && i0 + j < hi) ? load_now(x + i0 + j) : 0.f;
       }
       const bool interior = (i0 >= lo) && (i0 + kEltPerThread <= hi);
 #pragma unroll
@@ -684,21 +688,25 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* __restrict__
 
 template <int TH, int PER_SM>
 __global__ void __launch_bounds__(TH, PER_SM)
-topk_select_kernel(const float* __restrict__ logits, int64_t ld, const int32_t* __restrict__ ks,
+topk_select_kernel(const float* logits, int64_t ld, const int32_t* __restrict__ ks,
                    const int32_t* __restrict__ ke, int S, int k, int32_t* __restrict__ out, int one_pass) {
   __shared__ TopkSmem sm;
+  launch_dependents();
+  logits = grid_wait(logits);
   topk_row<TH>(sm, logits, ld, ks, ke, S, k, out, one_pass, blockIdx.x);
 }
 
 // sample = 0 forces the two-pass path on every row (the test hook that pits the two paths against each other)
 int topk_select_launch(const float* logits, int64_t ld, const int32_t* ks, const int32_t* ke, int T, int S, int k,
-                       int32_t* out, int sample, cudaStream_t stream) {
+                       int32_t* out, int sample, int overlapped, cudaStream_t stream) {
   if (T == 0 || k == 0) return DSA_OK;
   // Up to one row per SM a row has 1024 threads, beyond that 512, three rows to an SM: 7 rows of up to 33000 columns 11.0 us with 512,
   // 8.9 with 1024, 64 x 131072 18.5 and 13.3; 160 x 9000 11.5 and 15.5, 4096 x 32768 175 and 283.  (256 threads, five rows to an SM:
   // 4096 x 32768 207, 2048 x 2048 21.5.)
-  if (T <= sm_count()) topk_select_kernel<1024, 1><<<T, 1024, 0, stream>>>(logits, ld, ks, ke, S, k, out, sample);
-  else topk_select_kernel<512, 3><<<T, 512, 0, stream>>>(logits, ld, ks, ke, S, k, out, sample);
+  if (T <= sm_count())
+    launch_after(overlapped, topk_select_kernel<1024, 1>, dim3(T), 1024, 0, stream, logits, ld, ks, ke, S, k, out, sample);
+  else
+    launch_after(overlapped, topk_select_kernel<512, 3>, dim3(T), 512, 0, stream, logits, ld, ks, ke, S, k, out, sample);
   return check_launch("topk_select");
 }
 

@@ -272,3 +272,43 @@ def test_one_call_decode_step_equals_the_three_calls(B, heads, w_dtype):
     assert torch.equal(got[1][1], got[0][1]) and torch.equal(got[2][1], got[0][1])
     with pytest.raises(ops.DsaError):
         layer.dsa_decode_step(q8, w, kc, ksc, table, ctx.long(), q, lat, 0.07, layer.DecodeWorkspace(B, heads, P * 64, k, "cuda"))
+
+
+@pytest.mark.parametrize("B,heads", [(1, 128), (6, 64), (24, 128), (25, 128)])
+def test_overlapping_kernels_of_steps_in_a_row(B, heads):
+    """Up to 24 sequences each kernel of a step may start under the one before: many steps back to back on two sets of inputs in one
+    workspace, eager and from a graph, equal those of the three separate calls."""
+    g = torch.Generator(device="cuda").manual_seed(B)
+    P, k = 60, 1024
+    n = B * P * 64
+    sets = []
+    for _ in range(2):
+        kc, ksc = ops.fp8_quant_per_block(torch.randn(n, 128, device="cuda", generator=g), 128)
+        lat = layer.pack_latent_cache(torch.randn(n, 576, device="cuda", generator=g).bfloat16())
+        table = torch.randperm(B * P, device="cuda", generator=g).int().view(B, P)
+        ctx = torch.randint(1200, P * 64 + 1, (B,), device="cuda", generator=g).int()
+        q8, qs = ops.fp8_quant_per_block(torch.randn(B, 64, 128, device="cuda", generator=g), 128)
+        w = torch.randn(B, 64, device="cuda", generator=g) * qs
+        q = torch.randn(B, heads, 576, device="cuda", generator=g).bfloat16()
+        lg = ops.fp8_paged_mqa_logits(q8, w, kc, ksc, table, ctx, P * 64)
+        idx = ops.topk_select(lg, k, None, ctx)
+        sets.append(((q8, w, kc, ksc, table, ctx, q, lat), idx, ops.sparse_mla_decode_paged(q, lat, table, idx, 0.07, P * 64)))
+    ws = layer.DecodeWorkspace(B, heads, P * 64, k, "cuda")
+    got = []
+    for i in range(60):
+        idx, out = layer.dsa_decode_step(*sets[i % 2][0], 0.07, ws)
+        got.append((idx.clone(), out.clone()))
+    ops.check_status("cuda")
+    for i, (idx, out) in enumerate(got):
+        assert torch.equal(idx, sets[i % 2][1]) and torch.equal(out, sets[i % 2][2]), i
+    outs = [torch.empty_like(ws.out) for _ in range(20)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for i, o in enumerate(outs):
+            o.copy_(layer.dsa_decode_step(*sets[i % 2][0], 0.07, ws)[1])
+    for _ in range(3):
+        for o in outs:
+            o.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, sets[i % 2][2]) for i, o in enumerate(outs))

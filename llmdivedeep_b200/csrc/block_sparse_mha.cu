@@ -24,12 +24,12 @@
 //     rows, so no lane idles and nothing is moved between lanes but the four-lane maximum; P goes to one of two
 //     shared-memory buffers as bf16 through stmatrix, in the K-major swizzled layout; sums stay with the lane until
 //     the unit ends; the running maximum is raised (and O rescaled in tensor memory) only when it grows by more than
-//     8 in log2 units.  The output takes the same way out, through the P buffers, as whole 256-byte rows.
+//     kMaxRaise (32 log2 units).  The output takes the same way out, through the P buffers, as whole 256-byte rows.
 // What bounds it: the tensor pipe (an M = 64 MMA takes as long as an M = 128 one: 8 x 50 + 4 x 64 cycles a block, two
 // CTAs share the pipe).  Measured, 24 heads, 5% of the key blocks, the public call: 16384 tokens 380 us with lane-0 issue and
 // a lane-per-row softmax (32x32b loads, 32 shuffles a block, 256-byte rows stored 16 bytes a lane), 352 us with uniform
-// issue, 253 us with the 16x256b fragments as well, all in short runs at full clock; in long loops at the power cap
-// 396 -> 292 us (1870 and 1610 MHz).  32768 tokens 1290 -> 900, and 1373 -> 1039 us.  The tensor pipe alone would take
+// issue, 253 us with the 16x256b fragments as well (246 with the later raise), all in short runs at full clock; in long loops at the power cap
+// 396 -> 288 us (1870 and 1610 MHz).  32768 tokens 1290 -> 900, and 1373 -> 1039 us.  The tensor pipe alone would take
 // 183 us at 16384 tokens and full clock.
 // Every wait is bounded (dsa_common.cuh).
 #include <cuda.h>

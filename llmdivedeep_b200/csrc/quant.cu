@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) rope_fp8_quant_kernel(const __nv_bfloat16
 }
 
 // The same with eight values per thread, BLOCK / 8 threads per row: 16-byte loads, fewer shuffle steps.  [3000, 64, 128] 41.1 us with a
-// warp per row, 37.1 so (the quantiser alone 16.2).  Sixteen values, as that one has them, need 78 registers here: no faster.
+// warp per row, 31.0 so (the quantiser alone 16.2).  Sixteen values, as that one has them, need 78 registers here: no faster.
 template <int BLOCK, bool INTERLEAVE>
 __global__ void __launch_bounds__(256) rope_fp8_quant_wide_kernel(const __nv_bfloat16* __restrict__ x, int64_t n_rows, int rope_dim,
                                                                   int rows_per_pos, const float* __restrict__ cos_t,

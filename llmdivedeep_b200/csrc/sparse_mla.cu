@@ -37,7 +37,8 @@
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137
 // cycles each; see dsa_common.cuh) and TMA gather; 3125 with warp-uniform issue; 2860 with two sets of softmax warps;
 // 2418 with sixteen and setmaxnreg; 2215 with this gather; 2266 with the exchange stage released by the data; 2180 with waits that
-// look once before they loop (1071 TFLOP/s; short runs at full clock -- at the power cap, 1600 MHz, 2530 against 3565).  q scaled by 2
+// look once before they loop; 2140 with the gather's bounds known to the compiler and no zero-fill arithmetic where a warp's slots
+// are all in use (1091 TFLOP/s; short runs at full clock -- at the power cap, 1600 MHz, 2500 against 3565).  At 2180, q scaled by 2
 // and 4 takes the same; by 8, where maxima do outgrow the reference, 2570 us (with the reference raised by 8: 2550, 2935 and
 // 3030 us).  Tried on top: the exchange by st.async (3320:
 // the stores drain slowly and clog the gather), by loads from the peer's shared memory (3560: the release at cluster

@@ -31,7 +31,7 @@
 //
 // What bounds it: the time a KV buffer is held.  A block's rows are needed from the scores to P.V, with the exchange
 // and the softmax in between; that round trip (gather 2400 cycles, scores 1000, exchange + softmax 3600, P.V with its
-// queueing 1700), divided by five buffers, is the ~1900 cycles a block takes, against 1400 of tensor pipe.  Everything
+// queueing 1700), divided by five buffers, is the ~1700 cycles a block takes, against 1400 of tensor pipe.  Everything
 // below therefore shortens the trip: sixteen softmax warps in two sets that take alternate blocks, eleven gather warps
 // (a warp keeps about eight 512-byte requests going, whether cp.async or TMA gather4), arrivals by the copies themselves.
 // 4096 tokens x 2048 keys: 3594 us with eight softmax warps in lockstep, MMAs issued from a lane-dependent branch (~137

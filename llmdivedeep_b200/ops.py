@@ -337,7 +337,8 @@ def decode_step(q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, 
                 workspace) -> bool:
     """fp8_paged_mqa_logits, topk_select and sparse_mla_decode_paged into the given buffers (logits [>=B, >=max_ctx], idx [B,k],
     out [B,H,512]) as one library call.  Returns False, with nothing done, unless every tensor is of the plain form that the
-    three wrappers pass on as it is -- they convert or refuse the others."""
+    three wrappers pass on as it is -- they convert or refuse the others.  Rows of logits that are closer together than max_ctx
+    (expanded, overlapping) are among those: the kernel would write past them."""
     dev = q.device
     i = dev.index
     if dev.type != "cuda" or q.dim() != 3 or q_fp8.dim() != 3 or block_table.dim() != 2 or idx.dim() != 2:
@@ -350,7 +351,8 @@ def decode_step(q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, 
     if (B == 0 or Bi != B or dq != 576 or tuple(weights.shape) != (B, Hi) or kcache.dim() != 2 or kcache.shape[1] != D or kcache.shape[0] % 64
             or kscale.dim() != 1 or kscale.shape[0] != kcache.shape[0] or block_table.shape[0] != B or ctx_len.numel() != B
             or cache.dim() != 2 or cache.shape[1] != 656 or cache.shape[0] % 64 or idx.shape[0] != B or tuple(out.shape) != (B, H, 512)
-            or logits.get_device() != i or logits.dim() != 2 or logits.shape[0] < B or logits.shape[1] < max_ctx or logits.stride(1) != 1):
+            or logits.get_device() != i or logits.dim() != 2 or logits.shape[0] < B or logits.shape[1] < max_ctx or logits.stride(1) != 1
+            or logits.stride(0) < max_ctx):
         return False
     if (q_fp8.dtype != FP8 or kcache.dtype != FP8 or kscale.dtype != torch.float32 or block_table.dtype != torch.int32
             or ctx_len.dtype != torch.int32 or q.dtype != torch.bfloat16 or cache.dtype != torch.uint8 or idx.dtype != torch.int32
@@ -360,7 +362,7 @@ def decode_step(q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, 
     with _on(dev):
         check(_lib.load().dsa_decode_step(
             q_fp8.data_ptr(), weights.data_ptr(), _w_dtype(weights), kcache.data_ptr(), kscale.data_ptr(), kcache.shape[0] // 64,
-            block_table.data_ptr(), block_table.stride(0), ctx_len.data_ptr(), logits.data_ptr(), max(logits.stride(0), max_ctx), B, Hi, D,
+            block_table.data_ptr(), block_table.stride(0), ctx_len.data_ptr(), logits.data_ptr(), logits.stride(0), B, Hi, D,
             max_ctx, idx.shape[1], idx.data_ptr(), q.data_ptr(), cache.data_ptr(), cache.shape[0] // 64, out.data_ptr(), H, float(scale),
             workspace.data_ptr(), workspace.numel(), status_word(dev).data_ptr(), _stream(dev)))
     return True

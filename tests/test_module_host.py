@@ -163,3 +163,49 @@ def test_overlapping_calls_without_a_workspace_share_no_scratch(monkeypatch, cal
     (a0, a1), (b0, b1) = spans
     assert a1 > a0 and b1 > b0 and (a1 <= b0 or b1 <= a0)
     assert kept and all(r() is None for r in kept)
+
+class _OnGpu(torch.Tensor):
+    """A host tensor that says it lives on cuda:0: enough for the checks that a wrapper makes before it calls the library."""
+    device = property(lambda self: torch.device("cuda", 0))
+    is_cuda = property(lambda self: True)
+
+    def get_device(self):
+        return 0
+
+
+def _decode_step_call(monkeypatch, B=4, max_ctx=1024, k=256, heads=2):
+    """Arguments of ops.decode_step in its plain form (tiny caches), and the list that a stand-in for the library fills."""
+    calls = []
+
+    class Lib:
+        def dsa_decode_step(self, *args):
+            calls.append(args)
+            return 0
+
+    monkeypatch.setattr(ops._lib, "load", Lib)
+    monkeypatch.setattr(ops, "_on", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(ops, "_stream", lambda dev: 0)
+    monkeypatch.setattr(ops, "status_word", lambda dev: torch.zeros(1, dtype=torch.int32))
+    pages = max_ctx // 64
+    args = dict(q_fp8=torch.zeros(B, 64, 128).to(ops.FP8), weights=torch.zeros(B, 64), kcache=torch.zeros(64, 128).to(ops.FP8),
+                kscale=torch.zeros(64), block_table=torch.zeros(B, pages, dtype=torch.int32),
+                ctx_len=torch.full((B,), max_ctx, dtype=torch.int32), q=torch.zeros(B, heads, 576, dtype=torch.bfloat16),
+                cache=torch.zeros(64, 656, dtype=torch.uint8), logits=torch.zeros(B + 1, max_ctx), idx=torch.zeros(B, k, dtype=torch.int32),
+                out=torch.zeros(B, heads, 512, dtype=torch.bfloat16), workspace=torch.zeros(16, dtype=torch.uint8))
+    return {n: t.as_subclass(_OnGpu) for n, t in args.items()}, dict(scale=0.07, max_ctx=max_ctx), calls
+
+
+@pytest.mark.parametrize("B", [1, 4])
+def test_decode_step_passes_on_the_row_pitch_that_its_logits_have(monkeypatch, B):
+    """Rows further apart than max_ctx are passed on with their pitch; rows closer together than that (an expanded or overlapping
+    buffer) would be written past their storage and go to the wrappers, which refuse them."""
+    args, rest, calls = _decode_step_call(monkeypatch, B)
+    assert ops.decode_step(**args, **rest) and len(calls) == 1
+    pitch = 10                                                  # position of ld_logits in the C signature
+    assert calls[0][pitch - 1] == args["logits"].data_ptr() and calls[0][pitch] == 1024
+    wide = torch.zeros(B, 1500).as_subclass(_OnGpu)
+    assert ops.decode_step(**{**args, "logits": wide}, **rest) and calls[1][pitch] == 1500
+    for stride in (0, 256, 1023):
+        bad = torch.zeros(1024 + stride * B).as_strided((B, 1024), (stride, 1))
+        assert not ops.decode_step(**{**args, "logits": bad.as_subclass(_OnGpu)}, **rest)
+    assert len(calls) == 2

@@ -337,11 +337,12 @@ def decode_step(q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, 
                 workspace) -> bool:
     """fp8_paged_mqa_logits, topk_select and sparse_mla_decode_paged into the given buffers (logits [>=B, >=max_ctx], idx [B,k],
     out [B,H,512]) as one library call.  Returns False, with nothing done, unless every tensor is of the plain form that the
-    three wrappers pass on as it is -- they convert or refuse the others.  Rows of logits that are closer together than max_ctx
+    three wrappers pass on as it is -- they convert or refuse the others, and make scratch that is None.  Rows of logits that are closer together than max_ctx
     (expanded, overlapping) are among those: the kernel would write past them."""
     dev = q.device
     i = dev.index
-    if dev.type != "cuda" or q.dim() != 3 or q_fp8.dim() != 3 or block_table.dim() != 2 or idx.dim() != 2:
+    if (logits is None or workspace is None or dev.type != "cuda" or q.dim() != 3 or q_fp8.dim() != 3 or block_table.dim() != 2
+            or idx.dim() != 2):
         return False
     for t in (q_fp8, weights, kcache, kscale, block_table, ctx_len, q, cache, idx, out, workspace):
         if t.get_device() != i or not t.is_contiguous():

@@ -209,3 +209,10 @@ def test_decode_step_passes_on_the_row_pitch_that_its_logits_have(monkeypatch, B
         bad = torch.zeros(1024 + stride * B).as_strided((B, 1024), (stride, 1))
         assert not ops.decode_step(**{**args, "logits": bad.as_subclass(_OnGpu)}, **rest)
     assert len(calls) == 2
+
+
+@pytest.mark.parametrize("missing", ["logits", "workspace"])
+def test_decode_step_leaves_absent_scratch_to_the_wrappers(monkeypatch, missing):
+    """The wrappers allocate a logits buffer or a split workspace that is None; the one library call needs both."""
+    args, rest, calls = _decode_step_call(monkeypatch)
+    assert ops.decode_step(**{**args, missing: None}, **rest) is False and not calls

@@ -107,6 +107,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait_limit<UNROLL>(bar, parity, abort_flag, status, kSpinLimit));
 }
+
+// Whether another role has given up, for a warp whose lanes all come here: one answer for all of them (the flag may be raised
+// between two lanes' reads, and a warp that left its loop lane by lane would hang in the next vote).
+__device__ __forceinline__ bool aborted_warp(volatile int* abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }
+
 // ---- kernels that start under the end of the one before -------------------------
 // In a launch with the programmatic-serialisation attribute a kernel may start when every block of the one before has called
 // launch_dependents; what that one has written is visible after grid_wait (which returns at once in an ordinary launch).

@@ -286,7 +286,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const int pidx = warp == 0 ? 0 : 1;
     int* my_pages = pages_s + pidx * C::PAGES * kChunkTiles;
     uint32_t it = 0, nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+    for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
       int qb, nb, t_lo, t_hi;
       if (!unit_tiles<NQ, QB, PAGED>(a, u, n_qblocks, n_groups, qb, nb, t_lo, t_hi)) continue;
       const int qs = nu & 1;
@@ -357,7 +357,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     // ------------------------------- MMA issuer -------------------------------
     constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, kTileKeys, C::N);
     uint32_t it = 0, it2 = 0, nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+    for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
       int qb, nb, t_lo, t_hi;
       if (!unit_tiles<NQ, QB, PAGED>(a, u, n_qblocks, n_groups, qb, nb, t_lo, t_hi)) continue;
       const int qs = nu & 1;
@@ -397,7 +397,7 @@ indexer_logits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   } else if (warp == 2) {
     // ------------------- stager: head weights and windows per unit -------------------
     uint32_t nu = 0;
-    for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+    for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
       int qb, nb, t_lo, t_hi;
       if (!unit_tiles<NQ, QB, PAGED>(a, u, n_qblocks, n_groups, qb, nb, t_lo, t_hi)) continue;
       const int ub = nu & 1;
@@ -639,7 +639,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     if (warp == 0) {
       // ------------------------------ TMA producer ------------------------------
       uint32_t it = 0, nu = 0;
-      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+      for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
         int g, nb, t_lo, t_hi;
         if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
         const int qs = nu & 1;
@@ -673,7 +673,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       // The warp walks its loop as a whole and elects a lane for the instructions (dsa_common.cuh): 4096 x 65536 2222 -> 2173 us.
       constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, kTileKeys, C::N);
       uint32_t it = 0, nu = 0;
-      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+      for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
         int g, nb, t_lo, t_hi;
         if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
         const int qs = nu & 1;
@@ -703,7 +703,7 @@ indexer_logits_rw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     } else if (warp == 2) {
       // ------------------- stager: head weights and windows of the next unit -------------------
       uint32_t nu = 0;
-      for (int u = blockIdx.x; u < n_units && !*abort_flag; u += gridDim.x) {
+      for (int u = blockIdx.x; u < n_units && !aborted_warp(abort_flag); u += gridDim.x) {
         int g, nb, t_lo, t_hi;
         if (!unit_tiles<C::NQ, 1, false>(a, u, n_groups, n_groups, g, nb, t_lo, t_hi)) continue;
         const int ub = nu & 1;

@@ -243,7 +243,7 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
           ++pv;
           idle = 0;
         } else if (++idle > kFastSpins) {
-          if (idle > kSpinLimit || *abort_flag) {
+          if (idle > kSpinLimit || aborted_warp(abort_flag)) {      // the same for all lanes: they leave together
             *abort_flag = 1;
             if (a.status) atomicCAS(a.status, kStatusOk, kStatusWaitTimeout);
             ok = false;
@@ -251,7 +251,6 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
           }
           __nanosleep(40);
         }
-        ok = __all_sync(0xffffffffu, ok);
       }
       n = end;
       ++nq;

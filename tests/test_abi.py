@@ -98,3 +98,12 @@ def test_decode_workspace_serves_every_smaller_batch(lib, H, K):
         assert lib.dsa_sparse_mla_decode_workspace_bytes(b, H, K) == most * part <= pairs * part
     from llmdivedeep_b200.layer import DecodeWorkspace
     assert DecodeWorkspace(64, H, 4096, K, "cpu").mla_ws.numel() >= max(parts(b) for b in range(1, 65)) * part
+
+
+def test_a_warp_leaves_its_loops_as_a_whole():
+    """The abort flag may be raised between two lanes' reads of it.  A loop that a whole warp walks, with votes and shuffles of all
+    lanes inside, therefore asks for it by a vote; only single threads, and threads behind a block barrier, read it plainly."""
+    csrc = os.path.join(ROOT, "llmdivedeep_b200", "csrc")
+    for name in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
+        for i, line in enumerate(open(os.path.join(csrc, name)), 1):
+            assert not re.search(r"(for \(.*&& !|\|\| )\*abort_flag", line), f"{name}:{i}: {line.strip()}"

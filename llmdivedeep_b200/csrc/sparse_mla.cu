@@ -857,7 +857,7 @@ sparse_mla_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // by the sums of the CTA that computed it.
 // A query in eight parts: 4.8 us with loads behind the weights' loop, 3.6 so.
 __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const MlaArgs a) {
-  const float *lse = grid_wait(a.part_lse), *part = a.part_o;
+  const float *lse = grid_wait(a.part_lse), *part = grid_wait(a.part_o);      // the second returns at once
   const int u = blockIdx.x, t = a.n_full + u, h = blockIdx.y;
   const int d = threadIdx.x * 4, cta = d / kMlaDvHalf;
   // every load is requested before any is used: a part's weight and values do not wait for one another

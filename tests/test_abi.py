@@ -107,3 +107,10 @@ def test_a_warp_leaves_its_loops_as_a_whole():
     for name in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
         for i, line in enumerate(open(os.path.join(csrc, name)), 1):
             assert not re.search(r"(for \(.*&& !|\|\| )\*abort_flag", line), f"{name}:{i}: {line.strip()}"
+
+
+def test_the_combine_kernel_reads_the_parts_through_its_wait():
+    """It may start while the parts are still being written: loads through the raw pointers could move in front of the wait."""
+    src = open(os.path.join(ROOT, "llmdivedeep_b200", "csrc", "sparse_mla.cu")).read()
+    body = re.search(r"sparse_mla_combine_kernel\(const MlaArgs a\) \{(.*?)\n\}", src, flags=re.S).group(1)
+    assert body.count("a.part_") == body.count("grid_wait(a.part_") == 2

@@ -75,9 +75,10 @@ class DSALayer(nn.Module):
         x = x.to(self.dtype)
         T = x.shape[0]
         q_lora = self.q_a(x)
-        # the kernels' own int32 positions, without the way through the int64 that the reference's indexer returns
-        own = type(self.indexer).forward is DSA.DsaIndexer.forward
-        idx = (self.indexer(x, q_lora, index_dtype=torch.int32) if own else self.indexer(x, q_lora)).to(torch.int32)
+        # the kernels' own int32 positions, without the way through the int64 that the reference's indexer returns, where nobody
+        # else stands on that way
+        ix = self.indexer
+        idx = (ix(x, q_lora, index_dtype=torch.int32) if DSA.called_plainly(ix) else ix(x, q_lora)).to(torch.int32)
         q = self.wq(q_lora).view(T, self.n_heads, 576)
         kv = self.wkv(x)
         out = self.attn(q, kv, idx)

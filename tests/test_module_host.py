@@ -216,3 +216,50 @@ def test_decode_step_leaves_absent_scratch_to_the_wrappers(monkeypatch, missing)
     """The wrappers allocate a logits buffer or a split workspace that is None; the one library call needs both."""
     args, rest, calls = _decode_step_call(monkeypatch)
     assert ops.decode_step(**{**args, missing: None}, **rest) is False and not calls
+
+
+def _host_layer(monkeypatch, T=5):
+    """A DSALayer whose selection and attention are stand-ins on the host, and the dtypes that the two were asked for / given."""
+    from llmdivedeep_b200 import layer
+    seen = {}
+
+    def select(self, q, k, gate, ke, topk, dtype, w=None):
+        seen["selected"], seen["w"] = dtype, w
+        return torch.zeros(T, topk, dtype=dtype)
+
+    monkeypatch.setattr(DSA.DsaIndexer, "_select", select)
+    m = layer.DSALayer(hidden_size=32, q_lora_rank=16, index_n_heads=2, n_heads=1, index_topk=3, seed=0)
+    m.attn.forward = lambda q, kv, idx: seen.setdefault("attended", idx)
+    return m, torch.zeros(T, 32), seen
+
+
+def test_layer_takes_its_own_indexers_positions_without_a_detour(monkeypatch):
+    m, x, seen = _host_layer(monkeypatch)
+    assert m.stages(x)["idx"].dtype == torch.int32 and seen["selected"] == torch.int32
+
+
+@pytest.mark.parametrize("where", ["instance", "class"])
+def test_layer_calls_a_replaced_indexer_forward_with_two_arguments(monkeypatch, where):
+    m, x, seen = _host_layer(monkeypatch)
+    if where == "instance":
+        m.indexer.forward = lambda x, q_lora: torch.full((5, 3), 7)
+    else:
+        monkeypatch.setattr(DSA.DsaIndexer, "forward", lambda self, x, q_lora: torch.full((5, 3), 7))
+    assert torch.equal(m.stages(x)["idx"], torch.full((5, 3), 7, dtype=torch.int32)) and seen["attended"].dtype == torch.int32
+
+
+@pytest.mark.parametrize("scope", ["module", "global", "pre"])
+def test_hooks_on_the_layers_indexer_see_its_int64_positions(monkeypatch, scope):
+    m, x, seen = _host_layer(monkeypatch)
+    outs, ins = [], []
+    if scope == "module":
+        h = m.indexer.register_forward_hook(lambda mod, args, out: outs.append(out.dtype))
+    elif scope == "global":
+        h = torch.nn.modules.module.register_module_forward_hook(lambda mod, args, out: outs.append(out.dtype) if mod is m.indexer else None)
+    else:
+        h = m.indexer.register_forward_pre_hook(lambda mod, args, kwargs: ins.append(kwargs), with_kwargs=True)
+    try:
+        assert m.stages(x)["idx"].dtype == torch.int32
+    finally:
+        h.remove()
+    assert outs == ([] if scope == "pre" else [torch.int64]) and ins == ([{}] if scope == "pre" else [])

@@ -266,16 +266,16 @@ class DsaIndexer(nn.Module):
     def forward(self, x, q_lora_a, index_dtype: torch.dtype = torch.int64):
         T = x.shape[0]
         gate = w = None
-        if getattr(self.projections, "__func__", None) is DsaIndexer.projections:
+        if getattr(self.projections, "__func__", None) is _OWN_PROJECTIONS:
             q = self.wq_b(q_lora_a).view(T, self.spec.index_n_heads, self.spec.index_head_dim)
             k, gate = self.k_norm(self.wk(x)), self.weights_proj(x)
-        else:                                              # a subclass's own
+        else:                                              # a subclass's, an instance's, or put on the class
             q, k, w = self.projections(x, q_lora_a)
         ke = torch.arange(1, T + 1, dtype=torch.int32, device=x.device)
         return self._select(q, k, gate, ke, min(self.spec.index_topk, T), index_dtype, w)
 
 
-_OWN_FORWARD = DsaIndexer.forward
+_OWN_FORWARD, _OWN_PROJECTIONS = DsaIndexer.forward, DsaIndexer.projections
 
 
 def called_plainly(indexer: nn.Module) -> bool:

@@ -263,3 +263,12 @@ def test_hooks_on_the_layers_indexer_see_its_int64_positions(monkeypatch, scope)
     finally:
         h.remove()
     assert outs == ([] if scope == "pre" else [torch.int64]) and ins == ([{}] if scope == "pre" else [])
+
+
+def test_projections_replaced_on_the_class_are_called(monkeypatch):
+    """As those of a subclass or an instance are."""
+    m, x, seen = _host_layer(monkeypatch)
+    w = torch.full((5, 2), 0.25)
+    monkeypatch.setattr(DSA.DsaIndexer, "projections", lambda self, x, q_lora: (torch.zeros(5, 2, 64), torch.zeros(5, 64), w))
+    m.stages(x)
+    assert seen["w"] is w

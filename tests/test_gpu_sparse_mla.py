@@ -4,6 +4,10 @@ Floating point: bf16 inputs, bf16 tensor-core products with fp32 accumulation, t
 half of every score rounded to fp16 on its way between the pair, P rounded to bf16, bf16 output.  Tolerance (the one stated for this path): max-abs 2e-2 and mean-abs 2e-3
 against the oracle's fp32 computation on the same bf16 inputs.
 """
+import math
+import os
+import re
+
 import pytest
 import torch
 
@@ -372,3 +376,70 @@ def test_prefill_of_few_heads_flags_positions_out_of_range():
         ops.check_status("cuda")
     skipped = torch.where(bad >= 300, torch.full_like(bad, -1), bad)
     check(out, O.sparse_mla(q.float(), kv.float(), skipped, 0.06))
+
+
+def _climbing(T, H, K, seed):
+    """Rows whose scores climb from block to block of the list by far more than the softmax reference may lag.  In log2 units
+    the blocks lie at 0, 31.5, 33, 66, 97.5, ...: where the reference is raised, the block before may still have a third of
+    the new one's weight, so that the factor shows in the output.  A head takes them once, by half, not at all, or backwards.
+    The levels (half-integers up to 1408 before the scale) come from the second CTA's rope dims, the random part from the
+    first CTA's latent values: the level is exact in fp16 on its way between the two."""
+    g = torch.Generator().manual_seed(seed)
+    level = [0.0]
+    for b in range((K - 1) // 64):
+        level.append(level[-1] + 2 * (31.5, 1.5, 33.0)[b % 3])
+    scale = 0.5 * math.log(2.0)                                # log2 units are half the raw score
+    kv = torch.randn(K, 576, generator=g)
+    lv = torch.tensor(level).repeat_interleave(64)[:K]
+    kv[:, 512:] = 0
+    kv[:, 544], kv[:, 545] = torch.div(lv, 8, rounding_mode="floor"), lv % 8
+    q = torch.zeros(T, H, 576)
+    q[:, :, :256] = torch.randn(T, H, 256, generator=g) / 16
+    c = torch.tensor([1.0, 0.5, 1.0, 0.0, 1.0, -1.0]).repeat(H)[:H]
+    q[:, :, 544], q[:, :, 545] = 8 * c, c
+    idx = torch.empty(T, K, dtype=torch.int32)
+    for t in range(T):
+        for b in range(0, K, 64):
+            n = min(64, K - b)
+            idx[t, b:b + n] = b + torch.randperm(n, generator=g).int()
+    return q.to(torch.bfloat16), kv.to(torch.bfloat16), idx, scale
+
+
+def _raises(q, kv, idx, scale, first=0, last=None):
+    """How often the reference of each row and head is raised after its first block, walking slots [first, last)."""
+    src = open(os.path.join(os.path.dirname(ops.__file__), "csrc", "dsa_common.cuh")).read()
+    lag = float(re.search(r"kMaxRaise = ([0-9.]+)f", src).group(1))
+    s = torch.einsum("thd,tkd->thk", q.float(), kv.float()[idx.long()])[..., first:last] * (scale / math.log(2.0))
+    m, n = torch.full(s.shape[:2], -math.inf), torch.zeros(s.shape[:2], dtype=torch.int32)
+    for b in range(0, s.shape[2], 64):
+        top = s[..., b:b + 64].amax(-1)
+        up = top - m > lag
+        n += up if b else 0
+        m = torch.where(up, top, m)
+    return n
+
+
+@pytest.mark.parametrize("H,K", [(64, 1024), (128, 2048), (200, 700), (16, 2048), (32, 1000), (7, 321)])
+def test_prefill_scores_that_outgrow_the_reference_many_times(H, K):
+    q, kv, idx, scale = _climbing(3, H, K, seed=H + K)
+    assert int(_raises(q, kv, idx, scale)[:, 0].min()) >= 2
+    out = ops.sparse_mla_prefill(q.cuda(), kv.cuda(), idx.cuda(), scale)
+    ops.check_status("cuda")
+    check(out, O.sparse_mla(q.float(), kv.float(), idx, scale))
+
+
+@pytest.mark.parametrize("H", [64, 128, 200])
+@pytest.mark.parametrize("form", ["split", "whole"])
+def test_decode_scores_that_outgrow_the_reference_many_times(form, H):
+    """In a list that one pair walks, and in the parts of a split one (256 slots: the reference is raised in each)."""
+    B, K = 2, 2048
+    q, kv, idx, scale = _climbing(B, H, K, seed=H)
+    for first in range(0, K, 256):
+        assert int(_raises(q, kv, idx, scale, first, first + 256)[:, 0].min()) >= 1
+    assert int(_raises(q, kv, idx, scale)[:, 0].min()) >= 2
+    cache = O.pack_latent_cache(kv)
+    table = torch.arange(K // 64, dtype=torch.int32).repeat(B, 1)
+    ws = torch.empty(16, dtype=torch.uint8, device="cuda") if form == "whole" else None
+    out = ops.sparse_mla_decode_paged(q.cuda(), cache.cuda(), table.cuda(), idx.cuda(), scale, workspace=ws)
+    ops.check_status("cuda")
+    check(out, O.sparse_mla_decode_paged(q.float(), cache, table, idx, scale, round_bf16=True))

@@ -380,7 +380,7 @@ def pack_latent_cache(kv: torch.Tensor, out: Optional[torch.Tensor] = None) -> t
     cache[block_table[b, pos // 64] * 64 + pos % 64]."""
     if kv.dim() != 2 or kv.shape[1] != 576:
         raise ops.DsaError(f"latent KV must be [N, 576], got {tuple(kv.shape)}")
-    records = ops.pack_latent_records(kv, out)
+    records = ops.packed_latent_records(kv, out)
     return _pack_by_parts(kv, out) if records is None else records
 
 

@@ -514,7 +514,12 @@ def fp8_quant_per_block(x: torch.Tensor, block_size: int = 128):
     return q, scale
 
 
-def pack_latent_records(kv: torch.Tensor, out: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+def pack_latent_records(kv: torch.Tensor, out: torch.Tensor) -> bool:
+    """packed_latent_records into the given records; whether it took the call."""
+    return packed_latent_records(kv, out) is not None
+
+
+def packed_latent_records(kv: torch.Tensor, out: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """Latent rows [N, 576] -> cache records uint8 [N, 656] in one kernel, into ``out`` (None: a new tensor).  Takes bf16 or fp32
     rows with unit column stride and dense records, everything 16-byte aligned; returns None, having done nothing, for any other
     call."""

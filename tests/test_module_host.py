@@ -272,3 +272,21 @@ def test_projections_replaced_on_the_class_are_called(monkeypatch):
     monkeypatch.setattr(DSA.DsaIndexer, "projections", lambda self, x, q_lora: (torch.zeros(5, 2, 64), torch.zeros(5, 64), w))
     m.stages(x)
     assert seen["w"] is w
+
+
+def test_pack_latent_records_answers_yes_or_no(monkeypatch):
+    """Into the caller's records: True once the kernel has the call, False, with nothing done, for rows that it does not take."""
+    calls = []
+
+    class Lib:
+        def dsa_pack_latent_cache(self, *args):
+            calls.append(args)
+            return 0
+
+    monkeypatch.setattr(ops._lib, "load", Lib)
+    monkeypatch.setattr(ops, "_on", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(ops, "_stream", lambda dev: 0)
+    kv = torch.zeros(2, 576, dtype=torch.bfloat16).as_subclass(_OnGpu)
+    out = torch.zeros(2, 656, dtype=torch.uint8).as_subclass(_OnGpu)
+    assert ops.pack_latent_records(kv, out) is True and len(calls) == 1
+    assert ops.pack_latent_records(kv.half(), out) is False and ops.pack_latent_records(kv, out[:1]) is False and len(calls) == 1

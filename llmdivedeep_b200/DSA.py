@@ -244,7 +244,7 @@ class DsaIndexer(nn.Module):
         rd, il = sp.rope_head_dim, sp.rope_interleave
         if x.dtype == torch.bfloat16 and x.shape[-1] == self._quant_block() and x.shape[-1] in (64, 128):
             cos, sin = _rope_cossin(n_pos, rd, x.device)
-            if gate is None or gate.dtype == torch.bfloat16:
+            if gate is None or (gate.dtype == torch.bfloat16 and gate.shape == x.shape[:-1]):     # others broadcast
                 return ops.rope_fp8_quant(x, cos, sin, rd, il, rows_per_pos, gate, (sp.index_n_heads ** -0.5, sp.index_head_dim ** -0.5))
             q8, scale = ops.rope_fp8_quant(x, cos, sin, rd, il, rows_per_pos)
         else:

@@ -290,3 +290,23 @@ def test_pack_latent_records_answers_yes_or_no(monkeypatch):
     out = torch.zeros(2, 656, dtype=torch.uint8).as_subclass(_OnGpu)
     assert ops.pack_latent_records(kv, out) is True and len(calls) == 1
     assert ops.pack_latent_records(kv.half(), out) is False and ops.pack_latent_records(kv, out[:1]) is False and len(calls) == 1
+
+
+@pytest.mark.parametrize("gates", [(5, 1), (1, 2), (5, 2)])
+def test_gates_shared_by_heads_or_rows_broadcast(monkeypatch, gates):
+    """A replaced weights_proj may give one gate for all heads (or rows): folded by torch, as every gate once was; the kernel
+    takes one for each."""
+    taken = []
+
+    def kernel(x, cos, sin, rd, il, rows, gate=None, mul=None):
+        taken.append(gate is not None)
+        out = x.to(ops.FP8), torch.full(x.shape[:-1], 2.0)
+        return out if gate is None else (*out, torch.zeros(x.shape[:-1]))
+
+    monkeypatch.setattr(ops, "rope_fp8_quant", kernel)
+    ix = DSA.DsaIndexer(DSA.IndexerSpec("t", 32, 16, 2, 64, 32, 3), dtype=torch.bfloat16)
+    x, gate = torch.randn(5, 2, 64).bfloat16(), torch.randn(gates).bfloat16()
+    w = ix._rope_quant(x, 5, 2, gate)[2]
+    assert taken == [gates == (5, 2)]
+    if gates != (5, 2):
+        assert torch.equal(w, gate.float() * 2 ** -0.5 * torch.full((5, 2), 2.0) * 64 ** -0.5)

@@ -271,12 +271,6 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 // a pair of bf16 values added to a pair of fp32 values
 __device__ __forceinline__ void add_bf16x2(uint32_t v, float& x, float& y) {
   asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, u, %1;\n\t}"

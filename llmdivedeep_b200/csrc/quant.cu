@@ -11,7 +11,7 @@
 
 namespace dsa {
 
-// V (4 or 16) consecutive values per thread, in loads of 16 bytes (4 bf16 values: 8).
+// V (4, 8 or 16) consecutive values per thread, in loads of 16 bytes (4 bf16 values: 8).
 template <int V, typename T>
 __device__ __forceinline__ void load_values(const T* __restrict__ src, float (&v)[V]) {
   if constexpr (sizeof(T) == 2) {

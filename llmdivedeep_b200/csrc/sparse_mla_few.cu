@@ -4,10 +4,10 @@
 //   O^T [512 dims x N heads] += V^T P^T (four M = 128 tiles, 4 K-steps over a block's 64 keys; V^T is the gathered latent rows
 //                                        read through an MN-major descriptor, so nothing is transposed in memory)
 // N is 16 or 32.  In the other kernel 16 heads fill an eighth of a 128-row tile that costs the tensor pipe as much as a full
-// one, and the two CTAs of a pair exchange tiles that are mostly empty.  Here a CTA does a token by itself and the gather
-// bounds it: every row of the list crosses from L2 once, 1152 bytes, to 148 SMs.
-// Persistent CTAs, one per SM, each walking units (token, head group) with running counters, so that the gather and the scores
-// of the next token run under the last softmax and the output of this one.
+// one, and the two CTAs of a pair exchange tiles that are mostly empty.  Here a CTA does a token by itself: every row of the list
+// crosses from L2 once, 1152 bytes, to 148 SMs.
+// Persistent CTAs, one per SM, each walking tokens with running counters, so that the gather and the scores of the next token run
+// under the last softmax and the output of this one.
 //   * warps 0-3: softmax and output.  An M = 64 accumulator keeps its rows in lanes 0-15 of each quadrant: a warp has 16 keys and
 //     reads them with 16x256b loads, two keys and two heads of every eight to a lane.  Block maxima go over the lanes by three
 //     shuffles and over the warps through shared memory; P leaves through stmatrix.trans as [head][key] rows, the K-major B operand.
@@ -35,7 +35,6 @@ struct FewArgs {
   const int32_t* idx;             // [T, K] selected key positions (negative = empty)
   __nv_bfloat16* out;             // [T, H, 512]
   int T, H, K, S_kv;
-  int groups;                     // head groups of N
   float scale_log2e;
   int* status;
 };
@@ -135,8 +134,8 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // A unit is (token, head group).  Every role walks u = blockIdx.x, + gridDim.x, ... with running counters: nu units, n blocks,
-  // nq units with blocks.
+  // A unit is a token.  Every role walks u = blockIdx.x, + gridDim.x, ... with running counters: nu units, n blocks, nq units
+  // with blocks.
   auto unit_blocks = [&](uint32_t nu, bool& ok) -> int {     // number of blocks of the CTA's nu-th unit; the warp's reading frees the slot
     ok = mbar_wait_warp(&tok_full[nu % kFewTokRing], (nu / kFewTokRing) & 1, abort_flag, a.status);
     const int nb = ok ? tok_s[nu % kFewTokRing] : 0;
@@ -150,8 +149,7 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
     uint32_t nu = 0, nq = 0;
     bool ok = true;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
-      const int t = u / a.groups, hg = u - t * a.groups;
-      const int32_t* row = a.idx + (int64_t)t * a.K;
+      const int32_t* row = a.idx + (int64_t)u * a.K;
       int last = -1;
       for (int j0 = 0; j0 < a.K; j0 += 512) {
 #pragma unroll
@@ -176,7 +174,7 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
       if (!ok) break;
       if (lane == 0) mbar_expect_tx(q_full, C::Q_BYTES);
       __syncwarp();
-      if (lane < 9) tma_load_2d(q_s + lane * N * 128, &tmap_q, lane * 32, t * a.H + hg * N, q_full);   // x in 4-byte units
+      if (lane < 9) tma_load_2d(q_s + lane * N * 128, &tmap_q, lane * 32, u * a.H, q_full);   // x in 4-byte units
       ++nq;
     }
   } else if (warp == kFewMmaWarp) {
@@ -263,7 +261,7 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
     // lane group g of eight has the id of row r0 + g; requested a block ahead, across units too
     auto load_id = [&](int u, int blk) -> int {
       const int j = blk * kFewBlk + r0 + (lane >> 3);
-      return u < n_units && j < a.K ? __ldg(a.idx + (int64_t)(u / a.groups) * a.K + j) : -1;
+      return u < n_units && j < a.K ? __ldg(a.idx + (int64_t)u * a.K + j) : -1;
     };
     int nxt = load_id(blockIdx.x, 0);
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
@@ -315,12 +313,11 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
       return mbar_wait_warp(meet, met++ & 1, abort_flag, a.status);
     };
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
-      const int t = u / a.groups, hg = u - t * a.groups, heads = min(N, a.H - hg * N);
-      __nv_bfloat16* out = a.out + ((int64_t)t * a.H + hg * N) * kFewDv;
+      __nv_bfloat16* out = a.out + (int64_t)u * a.H * kFewDv;
       const int nb = unit_blocks(nu, ok);
       if (!ok) break;
       if (nb == 0) {                                   // nothing selected: zero rows
-        for (int i = warp * 32 + lane; i < heads * (kFewDv / 8); i += kFewSoftmaxWarps * 32)
+        for (int i = warp * 32 + lane; i < a.H * (kFewDv / 8); i += kFewSoftmaxWarps * 32)
           reinterpret_cast<uint4*>(out)[i] = make_uint4(0, 0, 0, 0);
         continue;
       }
@@ -479,7 +476,7 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
           const float x0 = __uint_as_float(ov[i]) * inv[i], x1 = __uint_as_float(ov[i + 1]) * inv[i + 1];
           const float y = __shfl_xor_sync(0xffffffffu, even ? x1 : x0, 1);
           const int h = i + (lane & 1);
-          if (h0 + h < heads) *reinterpret_cast<uint32_t*>(o + h * kFewDv) = even ? few_pack(x0, y) : few_pack(y, x1);
+          if (h0 + h < a.H) *reinterpret_cast<uint32_t*>(o + h * kFewDv) = even ? few_pack(x0, y) : few_pack(y, x1);
         }
       }
       tc_fence_before();
@@ -511,13 +508,11 @@ static int launch_few(const void* q, const FewArgs& args, cudaStream_t stream) {
   CUtensorMap tq;
   const int rc = make_tmap_2d_bytes(&tq, q, (uint64_t)a.T * a.H, kFewRowBytes, kFewRowBytes, 128, N);
   if (rc) return rc;
-  a.groups = (a.H + N - 1) / N;
-  const int64_t units = (int64_t)a.T * a.groups;
+  if (a.H > N) return set_error(DSA_ERR_SHAPE, "sparse_mla: %d heads in a kernel for %d", a.H, N);
   auto kern = sparse_mla_few_kernel<N>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
     return set_error(DSA_ERR_CUDA, "sparse_mla: cannot raise dynamic shared memory to %d", C::SMEM);
-  const int grid = units < sm_count() ? (int)units : sm_count();
-  kern<<<grid, kFewThreads, C::SMEM, stream>>>(tq, a, (int)units);
+  kern<<<a.T < sm_count() ? a.T : sm_count(), kFewThreads, C::SMEM, stream>>>(tq, a, a.T);
   return check_launch("sparse_mla");
 }
 

@@ -58,10 +58,6 @@ __device__ __forceinline__ float key_value(uint32_t key) {
   return __uint_as_float(key ^ (static_cast<uint32_t>(static_cast<int32_t>(~key) >> 31) | 0x80000000u));
 }
 
-// a plain load: the logits may have been written while this kernel was already running
-template <typename T>
-__device__ __forceinline__ T load_now(const T* p) { return *p; }
-
 // A range of values cut into kLinBins equal bins, counted from the top.  (hi - x) and its product with a positive factor are
 // monotone in floating point, so the bins order elements as their keys do; what lies above hi falls into bin 0, what lies below
 // the range into the last.  A NaN with the sign bit clear has the largest key and falls into bin 0, one with the sign bit set
@@ -233,7 +229,7 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* x, int wbase, int l
   if (wbase >= lo && wbase + kRun * 32 <= hi) {
 #pragma unroll
     for (int q = 0; q < kRun / kVec; ++q) {
-      const float4 f = load_now(reinterpret_cast<const float4*>(x + wbase + q * 128 + lane * kVec));
+      const float4 f = *reinterpret_cast<const float4*>(x + wbase + q * 128 + lane * kVec);
       if (at_or_above<NEG>(f.x, tfb)) fc |= 1u << (q * 4 + 0);
       if (at_or_above<NEG>(f.y, tfb)) fc |= 1u << (q * 4 + 1);
       if (at_or_above<NEG>(f.z, tfb)) fc |= 1u << (q * 4 + 2);
@@ -243,7 +239,7 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* x, int wbase, int l
     for (int q = 0; q < kRun / kVec; ++q) {
       const int i = wbase + q * 128 + lane * kVec;
       if (i < hi && i + kVec > lo) {         // a float4 that starts below hi lies inside the row's allocation
-        const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
+        const float4 f = *reinterpret_cast<const float4*>(x + i);
         const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
         for (int e2 = 0; e2 < kVec; ++e2)
@@ -260,7 +256,7 @@ __device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* x, int wba
     const int j = __ffs(fc) - 1;
     fc &= fc - 1;
     const int col = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
-    const float v = load_now(x + col);
+    const float v = x[col];
     sm.cand_key[pc] = order_key(v);
     sm.cand_idx[pc] = col;
     atomicAdd(&sm.lin[bins.of(v)], 1u);
@@ -378,7 +374,7 @@ __device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* x, i
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool in = j < mblk;
     if (in) {
-      f = load_now(reinterpret_cast<const float4*>(x + first + (j * sb + sb / 2) * kSampleBlock + lane * kVec));
+      f = *reinterpret_cast<const float4*>(x + first + (j * sb + sb / 2) * kSampleBlock + lane * kVec);
       svalid |= 0xFu << (4 * i);
     }
     skey[4 * i + 0] = order_key(f.x); skey[4 * i + 1] = order_key(f.y);
@@ -472,13 +468,13 @@ __device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* x, bool ve
       float v[kVec] = {0.f, 0.f, 0.f, 0.f};
       if (vec) {                                          // a float4 that starts below hi lies inside the row's allocation
         if (i0 + c * kDirectChunk + j < hi) {
-          const float4 f = load_now(reinterpret_cast<const float4*>(xc + i0 + j));
+          const float4 f = *reinterpret_cast<const float4*>(xc + i0 + j);
           v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
         }
       } else {
 #pragma unroll
         for (int e = 0; e < kVec; ++e)
-          if (used(c, j + e)) v[e] = load_now(xc + i0 + j + e);
+          if (used(c, j + e)) v[e] = xc[i0 + j + e];
       }
 #pragma unroll
       for (int e = 0; e < kVec; ++e) key[c][j + e] = order_key(v[e]);
@@ -568,7 +564,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* logits, int6
       if (pbits == 0) {
 #pragma unroll 4
         for (int i = first_full + tid * kVec; i < last_full; i += kChunkHist) {
-          const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
+          const float4 f = *reinterpret_cast<const float4*>(x + i);
           atomicAdd(&sm.hist[order_key(f.x) >> shift], 1u);
           atomicAdd(&sm.hist[order_key(f.y) >> shift], 1u);
           atomicAdd(&sm.hist[order_key(f.z) >> shift], 1u);
@@ -578,7 +574,7 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* logits, int6
         const int pshift = 32 - pbits;
 #pragma unroll 4
         for (int i = first_full + tid * kVec; i < last_full; i += kChunkHist) {
-          const float4 f = load_now(reinterpret_cast<const float4*>(x + i));
+          const float4 f = *reinterpret_cast<const float4*>(x + i);
           const float v[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -592,12 +588,12 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* logits, int6
       const int n_tail = last_full >= first_full ? hi - last_full : 0;
       if (tid < n_head + n_tail) {
         const int i = tid < n_head ? lo + tid : last_full + (tid - n_head);
-        const uint32_t key = order_key(load_now(x + i));
+        const uint32_t key = order_key(x[i]);
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     } else {
       for (int i = lo + tid; i < hi; i += TH) {
-        const uint32_t key = order_key(load_now(x + i));
+        const uint32_t key = order_key(x[i]);
         if (pbits == 0 || (key >> (32 - pbits)) == prefix) atomicAdd(&sm.hist[(key >> shift) & dmask], 1u);
       }
     }
@@ -626,13 +622,13 @@ __device__ __forceinline__ void topk_row(TopkSmem& sm, const float* logits, int6
 #pragma unroll
         for (int q = 0; q < kEltPerThread / kVec; ++q) {
           // a float4 that starts below hi lies inside the row's allocation (ld % 4 == 0)
-          const float4 f = (i0 + q * kVec < hi) ? load_now(reinterpret_cast<const float4*>(x + i0 + q * kVec))
+          const float4 f = (i0 + q * kVec < hi) ? *reinterpret_cast<const float4*>(x + i0 + q * kVec)
                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
           v[q * 4 + 0] = f.x; v[q * 4 + 1] = f.y; v[q * 4 + 2] = f.z; v[q * 4 + 3] = f.w;
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kEltPerThread; ++j) v[j] = (i0 + j >= lo && i0 + j < hi) ? load_now(x + i0 + j) : 0.f;
+        for (int j = 0; j < kEltPerThread; ++j) v[j] = (i0 + j >= lo && i0 + j < hi) ? x[i0 + j] : 0.f;
       }
       const bool interior = (i0 >= lo) && (i0 + kEltPerThread <= hi);
 #pragma unroll
@@ -692,7 +688,7 @@ topk_select_kernel(const float* logits, int64_t ld, const int32_t* __restrict__ 
                    const int32_t* __restrict__ ke, int S, int k, int32_t* __restrict__ out, int one_pass) {
   __shared__ TopkSmem sm;
   launch_dependents();
-  logits = grid_wait(logits);
+  logits = grid_wait(logits);                            // read by plain loads: they may have been written while this kernel ran
   topk_row<TH>(sm, logits, ld, ks, ke, S, k, out, one_pass, blockIdx.x);
 }
 

@@ -7,7 +7,10 @@
 // one, and the two CTAs of a pair exchange tiles that are mostly empty.  Here a CTA does a token by itself: every row of the list
 // crosses from L2 once, 1152 bytes, to 148 SMs.
 // Persistent CTAs, one per SM, each walking tokens with running counters, so that the gather and the scores of the next token run
-// under the last softmax and the output of this one.
+// under the last softmax and the output of this one.  A list of more than four blocks is taken in two halves, each with a softmax
+// reference, row sums and an output accumulator of its own, merged at the end: where a call has at most one token for every two
+// SMs, a cluster of two CTAs takes a half each and 256 dims of the merge, and the bits of a row are the same as when one CTA
+// takes both (they must not depend on the size of the call: rows are dealt to ranks).
 //   * warps 0-3: softmax and output.  An M = 64 accumulator keeps its rows in lanes 0-15 of each quadrant: a warp has 16 keys and
 //     reads them with 16x256b loads, two keys and two heads of every eight to a lane.  Block maxima go over the lanes by three
 //     shuffles and over the warps through shared memory; P leaves through stmatrix.trans as [head][key] rows, the K-major B operand.
@@ -16,10 +19,16 @@
 //   * warps 6-21: gather, four rows of a block each, by cp.async that arrive on the block's barrier by themselves.  The latent
 //     rows lie in a ring of panel pairs (128 dims of 64 keys), freed one by one as P.V has read them, the rope panels in another.
 // What bounds it: the tensor pipe, whose 52 MMAs a block cost 47 cycles each whatever their N (2450 cycles; the gather alone would
-// take 1900).  us before (the pair kernel) and now: 16 heads, 2048 tokens x 2048 of 16384 keys 985 -> 571, 4096 tokens 1938 -> 1105, 2048
-// tokens x 256 keys 276 -> 92; 32 heads 992 -> 705.  Tried: 128 keys a score tile (fewer MMAs, but then 1 1/4 blocks fit and the
-// gather waits for P.V: 835 against 607); 64 heads as one N = 64 tile (Q takes the room of a block: 1127 against 1051 for the pair
-// kernel, which therefore keeps them); the output put off until the next token's first P is on its way (spills: 668 against 610).
+// take 1900); in calls of few tokens the chain of one list.  us, keys of 16384: the kernel for many heads, this one with a list in
+// one piece (and read 16 slots a lane at a time for its end), as it is now.
+//   16 heads, 2048 keys: 1 token 33.9, 52.2, 25.5; 74 tokens 36.4, 53.1, 27.0; 148 tokens 71.5, 54.0, 44.1; 2048 tokens 1090, 566, 548
+//             256 keys:  1 token 9.9, 10.9, 9.5;   74 tokens 11.0, 11.3, 9.9;  2048 tokens 272, 91, 86
+//   32 heads, 2048 keys: 1 token 34.1, 61.7, 29.8; 74 tokens 36.6, 62.5, 31.6; 148 tokens 71.6, 63.5, 53.2; 2048 tokens 1090, 701, 680
+//             256 keys:  1 token 10.1, 12.5, 11.1; 74 tokens 11.0, 13.0, 11.6; 2048 tokens 281, 117, 117
+// (At 256 keys and up to 74 tokens 17 to 32 heads stay up to 10 % behind; halves of two blocks end that and cost 10 % at 2048 tokens.)
+// Tried: 128 keys a score tile (fewer MMAs, but then 1 1/4 blocks fit and the gather waits for P.V: 835 against 607); 64 heads as
+// one N = 64 tile (Q takes the room of a block: 1127 against 1051 for the pair kernel, which therefore keeps them); the output put
+// off until the next token's first P is on its way (spills: 668 against 610).
 // Every wait is bounded (dsa_common.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -47,6 +56,10 @@ constexpr int kFewPanel = kFewBlk * 128;               // 64 keys x 64 dims, 128
 constexpr int kFewRowBytes = 1152, kFewDv = 512;
 constexpr int kFewValidRing = 8;
 constexpr int kFewTokRing = 4;
+constexpr int kFewWhole = 4;                           // lists of more blocks than this are taken in two halves (below, the merge costs what they save)
+// Slots of a list that a lane looks at together, without a branch.  With 16, and one for a bad position, the look was most of a
+// call's start: 16 heads, 148 tokens x 2048 keys 54.0 -> 44.1 us.
+constexpr int kFewLook = 32;
 
 template <int N>
 struct FewCfg {
@@ -56,8 +69,8 @@ struct FewCfg {
   static constexpr int Q_BYTES = 9 * N * 128, P_BYTES = N * 128;
   static constexpr int BAR_BYTES = 512;
   static constexpr int SMEM = PAIRS * 2 * kFewPanel + ROPES * kFewPanel + Q_BYTES + PBUFS * P_BYTES + BAR_BYTES + kFewValidRing * kFewBlk +
-                              2 * kFewSoftmaxWarps * N * 4;
-  static constexpr uint32_t COL_O = 0, COL_S = 4 * N, COLS = COL_S + 2 * N <= 256 ? 256 : 512;
+                              6 * kFewSoftmaxWarps * N * 4;
+  static constexpr uint32_t COL_O = 0, COL_S = 8 * N, COLS = COL_S + 2 * N <= 256 ? 256 : 512;      // O of two halves
   static_assert(SMEM <= 232448 && COL_S + 2 * N <= COLS, "budget of one CTA");
 };
 
@@ -85,7 +98,51 @@ __device__ __forceinline__ void few_cp_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-template <int N>
+// The weights of the two halves' outputs, from their row sums and references (log2 units).
+__device__ __forceinline__ void few_weights(float l0, float m0, float l1, float m1, float& w0, float& w1) {
+  const float top = fmaxf(m0, m1);
+  const float f0 = m0 == -CUDART_INF_F ? 0.f : few_exp2(m0 - top), f1 = m1 == -CUDART_INF_F ? 0.f : few_exp2(m1 - top);
+  const float den = __fadd_rn(__fmul_rn(f0, l0), __fmul_rn(f1, l1));
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  w0 = __fmul_rn(f0, inv);
+  w1 = __fmul_rn(f1, inv);
+}
+__device__ __forceinline__ float few_ld_peer(uint32_t addr) {
+  float x;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
+  return x;
+}
+__device__ __forceinline__ uint32_t mapa_peer(uint32_t addr, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void few_ld_weights(const float* src, float (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) {
+    const float4 f = *reinterpret_cast<const float4*>(src + i);
+    w[i] = f.x; w[i + 1] = f.y; w[i + 2] = f.z; w[i + 3] = f.w;
+  }
+}
+// 16 heads from h0 on of the dims d0 + lane of a token's output: two neighbouring dims to a word, the even lane takes the pair
+// of the even head, the odd lane that of the odd one.
+__device__ __forceinline__ void few_store(__nv_bfloat16* out, int heads, int h0, int d0, int lane, const float (&x)[16]) {
+  const bool even = !(lane & 1);
+  __nv_bfloat16* o = out + (int64_t)h0 * kFewDv + d0 + (lane & ~1);
+#pragma unroll
+  for (int i = 0; i < 16; i += 2) {
+    const float y = __shfl_xor_sync(0xffffffffu, even ? x[i + 1] : x[i], 1);
+    const int h = i + (lane & 1);
+    if (h0 + h < heads) *reinterpret_cast<uint32_t*>(o + h * kFewDv) = even ? few_pack(x[i], y) : few_pack(y, x[i + 1]);
+  }
+}
+// every thread of both CTAs; what was written before is seen after
+__device__ __forceinline__ void few_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// PAIR: a cluster of two CTAs to a token, each with one half of its list.
+template <int N, bool PAIR>
 __global__ void __launch_bounds__(kFewThreads, 1)
 sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs a, const int n_units) {
   using C = FewCfg<N>;
@@ -114,6 +171,8 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
   // [2][4 warps][N] block maxima by block parity.  The half that the block does not use is free: a warp's row of it takes the
   // factors of a rescale, and all of it the row sums at the end of a unit.
   float* max_s = reinterpret_cast<float*>(valid_s + kFewValidRing * kFewBlk);
+  float* half_s = max_s + 2 * kFewSoftmaxWarps * N;    // [row sums, references][4 warps][N] of the first half (PAIR: of this CTA's)
+  float* wgt_s = half_s + 2 * kFewSoftmaxWarps * N;    // [4 warps][2][N] weights of the halves' outputs
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   if (warp == 0) {
@@ -134,8 +193,15 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // A unit is a token.  Every role walks u = blockIdx.x, + gridDim.x, ... with running counters: nu units, n blocks, nq units
-  // with blocks.
+  // A unit is a token.  Every role walks u = blockIdx.x, + gridDim.x, ... (PAIR: one unit) with running counters: nu units, n
+  // blocks, nq units with blocks.  Blocks [b0, b1) of a list are this CTA's; from first_half(nb) on, a list has its second
+  // softmax state and output.
+  const int rank = PAIR ? blockIdx.x & 1 : 0, u0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, du = PAIR ? n_units : gridDim.x;
+  auto first_half = [](int nb) { return nb > kFewWhole ? (nb + 1) / 2 : nb; };
+  auto my_blocks = [&](int nb, int& b0, int& b1) {
+    b0 = PAIR && rank ? first_half(nb) : 0;
+    b1 = PAIR && !rank ? first_half(nb) : nb;
+  };
   auto unit_blocks = [&](uint32_t nu, bool& ok) -> int {     // number of blocks of the CTA's nu-th unit; the warp's reading frees the slot
     ok = mbar_wait_warp(&tok_full[nu % kFewTokRing], (nu / kFewTokRing) & 1, abort_flag, a.status);
     const int nb = ok ? tok_s[nu % kFewTokRing] : 0;
@@ -148,19 +214,22 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
     // ------------- the last used slot of every list (it decides the number of blocks), and Q -------------
     uint32_t nu = 0, nq = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
+    for (int u = u0; u < n_units && ok; u += du, ++nu) {
       const int32_t* row = a.idx + (int64_t)u * a.K;
-      int last = -1;
-      for (int j0 = 0; j0 < a.K; j0 += 512) {
+      int last = -1, top = -1;
+#pragma unroll 1
+      for (int j0 = lane; j0 < a.K; j0 += 32 * kFewLook) {      // all of a lane's loads are requested before the first is looked at
+        int id[kFewLook];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int j = j0 + i * 32 + lane;
-          const int id = j < a.K ? __ldg(row + j) : -1;
-          if (id >= 0 && id < a.S_kv) last = j;
-          if (id >= a.S_kv && a.status) atomicCAS(a.status, kStatusOk, kStatusBadIndex);
+        for (int i = 0; i < kFewLook; ++i) id[i] = j0 + i * 32 < a.K ? __ldg(row + j0 + i * 32) : -1;
+#pragma unroll
+        for (int i = 0; i < kFewLook; ++i) {
+          if (id[i] >= 0 && id[i] < a.S_kv) last = j0 + i * 32;
+          top = max(top, id[i]);
         }
       }
       last = __reduce_max_sync(0xffffffffu, last);
+      if (top >= a.S_kv && a.status) atomicCAS(a.status, kStatusOk, kStatusBadIndex);
       const int nb = (last + kFewBlk) / kFewBlk;
       ok = mbar_wait_warp(&tok_free[nu % kFewTokRing], ((nu / kFewTokRing) & 1) ^ 1, abort_flag, a.status);
       if (!ok) break;
@@ -169,7 +238,9 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
         mbar_arrive(&tok_full[nu % kFewTokRing]);
       }
       __syncwarp();
-      if (nb == 0) continue;
+      int b0, b1;
+      my_blocks(nb, b0, b1);
+      if (b0 == b1) continue;
       ok = mbar_wait_warp(q_free, (nq & 1) ^ 1, abort_flag, a.status);
       if (!ok) break;
       if (lane == 0) mbar_expect_tx(q_full, C::Q_BYTES);
@@ -189,14 +260,16 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
     constexpr uint64_t kPair = (2 * kFewPanel) >> 4, kOne = kFewPanel >> 4, kQPanel = (N * 128) >> 4;
     uint32_t nu = 0, nq = 0, n = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
+    for (int u = u0; u < n_units && ok; u += du, ++nu) {
       const int nb = unit_blocks(nu, ok);
       if (!ok) break;
-      if (nb == 0) continue;
+      int b0, b1;
+      my_blocks(nb, b0, b1);
+      if (b0 == b1) continue;
       ok = mbar_wait_warp(q_full, nq & 1, abort_flag, a.status);
       if (!ok) break;
-      const uint32_t end = n + nb;
-      uint32_t qk = n, pv = n, idle = 0;
+      const uint32_t end = n + (b1 - b0), half = PAIR ? end : n + first_half(nb);
+      uint32_t qk = n, pv = n, begun = n, d_o = tmem + C::COL_O, idle = 0;      // begun: first block of the half
       // Whatever is ready first: the scores of the next block, at most two ahead of P.V (whose P says that the score buffer
       // has been read), or P.V of the oldest (whose P, for a unit's first block, says that the last unit's O has been read).
       while (pv < end) {
@@ -232,13 +305,16 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
               const uint64_t vd = vdesc + slot * kPair;
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks)           // 16 keys: 16 rows x 128 B further into each panel, 32 B along P's rows
-                umma_f16_ss(tmem + C::COL_O + mt * N, vd + ks * (2048 >> 4), pd + 2 * ks, idesc_pv, pv != n || ks != 0);
+                umma_f16_ss(d_o + mt * N, vd + ks * (2048 >> 4), pd + 2 * ks, idesc_pv, pv != begun || ks != 0);
               umma_commit(&pair_free[slot]);
             }
             umma_commit(&pv_done[pv & 1]);
           }
           __syncwarp();
-          ++pv;
+          if (++pv == half) {
+            begun = half;
+            d_o += 4 * N;
+          }
           idle = 0;
         } else if (++idle > kFastSpins) {
           if (idle > kSpinLimit || aborted_warp(abort_flag)) {      // the same for all lanes: they leave together
@@ -263,14 +339,17 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
       const int j = blk * kFewBlk + r0 + (lane >> 3);
       return u < n_units && j < a.K ? __ldg(a.idx + (int64_t)u * a.K + j) : -1;
     };
-    int nxt = load_id(blockIdx.x, 0);
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
+    const int guess = PAIR && rank ? first_half((a.K + kFewBlk - 1) / kFewBlk) : 0;      // before the list's end is known
+    int nxt = load_id(u0, guess);
+    for (int u = u0; u < n_units && ok; u += du, ++nu) {
       const int nb = unit_blocks(nu, ok);
       if (!ok) break;
-      if (nb == 0) nxt = load_id(u + gridDim.x, 0);
-      for (int j = 0; j < nb; ++j, ++n) {
+      int b0, b1;
+      my_blocks(nb, b0, b1);
+      if (PAIR ? b0 != guess : nb == 0) nxt = PAIR ? load_id(u, b0) : load_id(u + du, 0);
+      for (int j = b0; j < b1; ++j, ++n) {
         const int id = nxt < a.S_kv ? nxt : -1;        // -1 = empty slot; bad positions are flagged by the warp that read the list
-        nxt = j + 1 < nb ? load_id(u, j + 1) : load_id(u + gridDim.x, 0);
+        nxt = j + 1 < b1 ? load_id(u, j + 1) : load_id(u + du, 0);
         {
           const uint32_t slot = n % C::ROPES;
           if (n >= C::ROPES) ok = mbar_wait_warp(&rope_free[slot], (n / C::ROPES - 1) & 1, abort_flag, a.status);
@@ -312,171 +391,216 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
       if (lane == 0) mbar_arrive(meet);
       return mbar_wait_warp(meet, met++ & 1, abort_flag, a.status);
     };
-    for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++nu) {
-      __nv_bfloat16* out = a.out + (int64_t)u * a.H * kFewDv;
+    // this warp's row: heads 8 i + 2 (lane % 4), + 1 of every thread's values
+    auto put_row = [&](float* row, const float(&v)[2 * NH]) {
+      if (lane < 4) {
+#pragma unroll
+        for (int i = 0; i < NH; ++i) *reinterpret_cast<float2*>(row + 8 * i + 2 * lane) = make_float2(v[2 * i], v[2 * i + 1]);
+      }
+    };
+    auto sum_lanes = [&](float(&l)[2 * NH]) {          // over the lanes that share a head
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < 2 * NH; ++i) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+    };
+    for (int u = u0; u < n_units && ok; u += du, ++nu) {
       const int nb = unit_blocks(nu, ok);
       if (!ok) break;
-      if (nb == 0) {                                   // nothing selected: zero rows
-        for (int i = warp * 32 + lane; i < a.H * (kFewDv / 8); i += kFewSoftmaxWarps * 32)
-          reinterpret_cast<uint4*>(out)[i] = make_uint4(0, 0, 0, 0);
+      int b0, b1;
+      my_blocks(nb, b0, b1);
+      if (b0 == b1) {                                  // nothing selected: zero rows (or no second half)
+        for (int i = warp * 32 + lane; nb == 0 && rank == 0 && i < a.H * (kFewDv / 8); i += kFewSoftmaxWarps * 32)
+          reinterpret_cast<uint4*>(a.out + (int64_t)u * a.H * kFewDv)[i] = make_uint4(0, 0, 0, 0);
         continue;
       }
       float m[2 * NH], l[2 * NH];                      // heads 8 i + 2 (lane % 4), + 1: references (log2), sums over this thread's keys
 #pragma unroll
       for (int i = 0; i < 2 * NH; ++i) { m[i] = -CUDART_INF_F; l[i] = 0.f; }
-      for (int j = 0; j < nb; ++j, ++n) {
-        ok = mbar_wait_warp(&s_full[n & 1], (n >> 1) & 1, abort_flag, a.status);
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t sv[4 * NH];
-#pragma unroll
-        for (int i = 0; i < NH; i += 2) few_ld_s(t_row + C::COL_S + (n & 1) * N + 8 * i, *reinterpret_cast<uint32_t(*)[8]>(&sv[4 * i]));
-        const uint8_t* valid = valid_s + (n % kFewValidRing) * kFewBlk + 16 * warp + (lane >> 2);
-        const bool va = valid[0], vb = valid[8];
-        tmem_wait_ld();
-        tc_fence_before();
-        float s[4 * NH], bm[2 * NH];
-#pragma unroll
-        for (int i = 0; i < NH; ++i) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            s[4 * i + e] = va ? __uint_as_float(sv[4 * i + e]) : -CUDART_INF_F;
-            s[4 * i + 2 + e] = vb ? __uint_as_float(sv[4 * i + 2 + e]) : -CUDART_INF_F;
-            bm[2 * i + e] = fmaxf(s[4 * i + e], s[4 * i + 2 + e]);
-          }
-        }
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1)
-#pragma unroll
-          for (int i = 0; i < 2 * NH; ++i) bm[i] = fmaxf(bm[i], __shfl_xor_sync(0xffffffffu, bm[i], o));
-        float* mx = max_s + (n & 1) * 4 * N;
-        if (lane < 4) {
-#pragma unroll
-          for (int i = 0; i < NH; ++i) *reinterpret_cast<float2*>(mx + warp * N + 8 * i + 2 * lane) = make_float2(bm[2 * i], bm[2 * i + 1]);
-        }
-        ok = all_meet();
-        if (!ok) break;
-        bool grown = false;
-        float f[2 * NH];
-#pragma unroll
-        for (int i = 0; i < NH; ++i) {
-          float2 b = make_float2(-CUDART_INF_F, -CUDART_INF_F);
-#pragma unroll
-          for (int w = 0; w < kFewSoftmaxWarps; ++w) {
-            const float2 x = *reinterpret_cast<const float2*>(mx + w * N + 8 * i + 2 * (lane & 3));
-            b.x = fmaxf(b.x, x.x);
-            b.y = fmaxf(b.y, x.y);
-          }
-          const float bx[2] = {b.x * a.scale_log2e, b.y * a.scale_log2e};
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float m_old = m[2 * i + e];
-            const bool up = bx[e] - m_old > kMaxRaise;  // also true when m is still -inf and the maximum finite
-            f[2 * i + e] = up ? few_exp2(m_old - bx[e]) : 1.f;
-            if (up) m[2 * i + e] = bx[e];
-            grown |= up;
-          }
-        }
-        if (__any_sync(0xffffffffu, grown)) {          // the same in all four warps
-#pragma unroll
-          for (int i = 0; i < 2 * NH; ++i) l[i] *= f[i];
-          if (j > 0) {                                 // O must be quiescent: P.V of the block before complete
-            ok = mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
-            if (!ok) break;
-            tc_fence_after();
-            float* fac = max_s + ((n + 1) & 1) * 4 * N + warp * N;
-            if (lane < 4) {
-#pragma unroll
-              for (int i = 0; i < NH; ++i) *reinterpret_cast<float2*>(fac + 8 * i + 2 * lane) = make_float2(f[2 * i], f[2 * i + 1]);
-            }
-            __syncwarp();
-#pragma unroll 1
-            for (int c = 0; c < 4 * N; c += 16) {
-              uint32_t ov[16];
-              tmem_ld16(t_row + C::COL_O + c, ov);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * fac[(c & (N - 1)) + i]);
-              tmem_st16(t_row + C::COL_O + c, ov);
-            }
-            tmem_wait_st();
-            __syncwarp();
-          }
-        }
-        uint32_t pk[2 * NH];                           // [group of eight heads][keys t / 4, t / 4 + 8]: two heads each
-#pragma unroll
-        for (int i = 0; i < NH; ++i) {
-          const float m0 = m[2 * i] == -CUDART_INF_F ? 0.f : m[2 * i], m1 = m[2 * i + 1] == -CUDART_INF_F ? 0.f : m[2 * i + 1];
-          const float p0 = few_exp2(fmaf(s[4 * i], a.scale_log2e, -m0)), p1 = few_exp2(fmaf(s[4 * i + 1], a.scale_log2e, -m1));
-          const float p2 = few_exp2(fmaf(s[4 * i + 2], a.scale_log2e, -m0)), p3 = few_exp2(fmaf(s[4 * i + 3], a.scale_log2e, -m1));
-          pk[2 * i] = few_pack(p0, p1);
-          pk[2 * i + 1] = few_pack(p2, p3);
-          add_bf16x2(pk[2 * i], l[2 * i], l[2 * i + 1]);
-          add_bf16x2(pk[2 * i + 1], l[2 * i], l[2 * i + 1]);
-        }
-        if (n >= C::PBUFS) {                           // that P buffer has been read
-          ok = mbar_wait_warp(&pv_done[(n - C::PBUFS) & 1], ((n - C::PBUFS) >> 1) & 1, abort_flag, a.status);
+      uint32_t begun = n, stop = n + (PAIR ? b1 - b0 : first_half(nb)), t_o = t_row + C::COL_O;
+      while (true) {                                   // over the halves
+        for (; n != stop; ++n) {
+          ok = mbar_wait_warp(&s_full[n & 1], (n >> 1) & 1, abort_flag, a.status);
           if (!ok) break;
-        }
-        // transposed on the way: row = head, 16-byte chunk = eight keys
-        uint8_t* p = p_s + (n % C::PBUFS) * C::P_BYTES;
+          tc_fence_after();
+          uint32_t sv[4 * NH];
 #pragma unroll
-        for (int i = 0; i < NH; i += 2) {
-          const int h = 8 * (i + (lane >> 4)) + (lane & 7), ch = 2 * warp + ((lane >> 3) & 1);
-          asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
-                       ::"r"(smem_u32(p + h * 128 + ((ch ^ (h & 7)) << 4))), "r"(pk[2 * i]), "r"(pk[2 * i + 1]), "r"(pk[2 * i + 2]), "r"(pk[2 * i + 3])
-                       : "memory");
+          for (int i = 0; i < NH; i += 2) few_ld_s(t_row + C::COL_S + (n & 1) * N + 8 * i, *reinterpret_cast<uint32_t(*)[8]>(&sv[4 * i]));
+          const uint8_t* valid = valid_s + (n % kFewValidRing) * kFewBlk + 16 * warp + (lane >> 2);
+          const bool va = valid[0], vb = valid[8];
+          tmem_wait_ld();
+          tc_fence_before();
+          float s[4 * NH], bm[2 * NH];
+#pragma unroll
+          for (int i = 0; i < NH; ++i) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              s[4 * i + e] = va ? __uint_as_float(sv[4 * i + e]) : -CUDART_INF_F;
+              s[4 * i + 2 + e] = vb ? __uint_as_float(sv[4 * i + 2 + e]) : -CUDART_INF_F;
+              bm[2 * i + e] = fmaxf(s[4 * i + e], s[4 * i + 2 + e]);
+            }
+          }
+#pragma unroll
+          for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < 2 * NH; ++i) bm[i] = fmaxf(bm[i], __shfl_xor_sync(0xffffffffu, bm[i], o));
+          float* mx = max_s + (n & 1) * 4 * N;
+          put_row(mx + warp * N, bm);
+          ok = all_meet();
+          if (!ok) break;
+          bool grown = false;
+          float f[2 * NH];
+#pragma unroll
+          for (int i = 0; i < NH; ++i) {
+            float2 b = make_float2(-CUDART_INF_F, -CUDART_INF_F);
+#pragma unroll
+            for (int w = 0; w < kFewSoftmaxWarps; ++w) {
+              const float2 x = *reinterpret_cast<const float2*>(mx + w * N + 8 * i + 2 * (lane & 3));
+              b.x = fmaxf(b.x, x.x);
+              b.y = fmaxf(b.y, x.y);
+            }
+            const float bx[2] = {b.x * a.scale_log2e, b.y * a.scale_log2e};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float m_old = m[2 * i + e];
+              const bool up = bx[e] - m_old > kMaxRaise;  // also true when m is still -inf and the maximum finite
+              f[2 * i + e] = up ? few_exp2(m_old - bx[e]) : 1.f;
+              if (up) m[2 * i + e] = bx[e];
+              grown |= up;
+            }
+          }
+          if (__any_sync(0xffffffffu, grown)) {          // the same in all four warps
+#pragma unroll
+            for (int i = 0; i < 2 * NH; ++i) l[i] *= f[i];
+            if (n != begun) {                            // O must be quiescent: P.V of the block before complete
+              ok = mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
+              if (!ok) break;
+              tc_fence_after();
+              float* fac = max_s + ((n + 1) & 1) * 4 * N + warp * N;
+              put_row(fac, f);
+              __syncwarp();
+#pragma unroll 1
+              for (int c = 0; c < 4 * N; c += 16) {
+                uint32_t ov[16];
+                tmem_ld16(t_o + c, ov);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * fac[(c & (N - 1)) + i]);
+                tmem_st16(t_o + c, ov);
+              }
+              tmem_wait_st();
+              __syncwarp();
+            }
+          }
+          uint32_t pk[2 * NH];                           // [group of eight heads][keys t / 4, t / 4 + 8]: two heads each
+#pragma unroll
+          for (int i = 0; i < NH; ++i) {
+            const float m0 = m[2 * i] == -CUDART_INF_F ? 0.f : m[2 * i], m1 = m[2 * i + 1] == -CUDART_INF_F ? 0.f : m[2 * i + 1];
+            const float p0 = few_exp2(fmaf(s[4 * i], a.scale_log2e, -m0)), p1 = few_exp2(fmaf(s[4 * i + 1], a.scale_log2e, -m1));
+            const float p2 = few_exp2(fmaf(s[4 * i + 2], a.scale_log2e, -m0)), p3 = few_exp2(fmaf(s[4 * i + 3], a.scale_log2e, -m1));
+            pk[2 * i] = few_pack(p0, p1);
+            pk[2 * i + 1] = few_pack(p2, p3);
+            add_bf16x2(pk[2 * i], l[2 * i], l[2 * i + 1]);
+            add_bf16x2(pk[2 * i + 1], l[2 * i], l[2 * i + 1]);
+          }
+          if (n >= C::PBUFS) {                           // that P buffer has been read
+            ok = mbar_wait_warp(&pv_done[(n - C::PBUFS) & 1], ((n - C::PBUFS) >> 1) & 1, abort_flag, a.status);
+            if (!ok) break;
+          }
+          // transposed on the way: row = head, 16-byte chunk = eight keys
+          uint8_t* p = p_s + (n % C::PBUFS) * C::P_BYTES;
+#pragma unroll
+          for (int i = 0; i < NH; i += 2) {
+            const int h = 8 * (i + (lane >> 4)) + (lane & 7), ch = 2 * warp + ((lane >> 3) & 1);
+            asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+                         ::"r"(smem_u32(p + h * 128 + ((ch ^ (h & 7)) << 4))), "r"(pk[2 * i]), "r"(pk[2 * i + 1]), "r"(pk[2 * i + 2]), "r"(pk[2 * i + 3])
+                         : "memory");
+          }
+          fence_async_smem();                            // visible to the tensor core's reads
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[n & 1]);
         }
-        fence_async_smem();                            // visible to the tensor core's reads
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[n & 1]);
+        if (PAIR || !ok || nb <= kFewWhole || t_o != t_row + C::COL_O) break;
+        // the first half's sums and references, read after the unit's last meeting
+        sum_lanes(l);
+        put_row(half_s + warp * N, l);
+        put_row(half_s + (kFewSoftmaxWarps + warp) * N, m);
+#pragma unroll
+        for (int i = 0; i < 2 * NH; ++i) { m[i] = -CUDART_INF_F; l[i] = 0.f; }
+        begun = n;
+        stop = n + nb / 2;
+        t_o += 4 * N;
       }
       if (!ok) break;
-      // row sums: over the lanes that share a head, then over the warps
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1)
-#pragma unroll
-        for (int i = 0; i < 2 * NH; ++i) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+      __nv_bfloat16* out = a.out + (int64_t)u * a.H * kFewDv;
+      // row sums over the warps
+      const bool halves = nb > kFewWhole;
       float* sum_s = max_s + (n & 1) * 4 * N;
-      if (lane < 4) {
-#pragma unroll
-        for (int i = 0; i < NH; ++i) *reinterpret_cast<float2*>(sum_s + warp * N + 8 * i + 2 * lane) = make_float2(l[2 * i], l[2 * i + 1]);
-      }
+      sum_lanes(l);
+      put_row(sum_s + warp * N, l);
+      float* wgt = wgt_s + warp * 2 * N;
+      if (halves) put_row(wgt + N, m);
       ok = all_meet();
       if (!ok) break;
-      // a head's quotient is taken once, into this warp's row of the other half (taken by every thread for every tile: 48 -> 85 us
-      // for 2048 tokens x 64 keys)
-      float* inv_s = max_s + ((n + 1) & 1) * 4 * N + warp * N;
+      // a head's weights are computed once (a quotient by every thread for every tile: 48 -> 85 us for 2048 tokens x 64 keys)
       if (lane < N) {
-        const float sum = (sum_s[lane] + sum_s[N + lane]) + (sum_s[2 * N + lane] + sum_s[3 * N + lane]);
-        inv_s[lane] = sum > 0.f ? 1.f / sum : 0.f;
+        auto over_warps = [&](const float* r) { return (r[lane] + r[N + lane]) + (r[2 * N + lane] + r[3 * N + lane]); };
+        const float sum = over_warps(sum_s);
+        if (!halves) {
+          wgt[lane] = sum > 0.f ? 1.f / sum : 0.f;
+        } else if constexpr (PAIR) {                   // for the peer, which merges the other 256 dims
+          half_s[lane] = sum;
+          half_s[N + lane] = wgt[N + lane];
+        } else {
+          float w0, w1;
+          few_weights(over_warps(half_s), half_s[(kFewSoftmaxWarps + warp) * N + lane], sum, wgt[N + lane], w0, w1);
+          wgt[lane] = w0;
+          wgt[N + lane] = w1;
+        }
       }
       __syncwarp();
       ok = mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, a.status);
       if (!ok) break;
       tc_fence_after();
-      const int even = (lane & 1) ^ 1;
+      if (PAIR && halves) {
+        // the peer's two tiles of 128 dims, [tile][head][dim], where the (idle) panels were
+        float* give = reinterpret_cast<float*>(pair_s) + warp * 32 + lane;
 #pragma unroll 1
-      for (int c = 0; c < 4 * N; c += 16) {            // 16 heads of this lane's dim of a 128-dim tile
-        uint32_t ov[16];
-        tmem_ld16(t_row + C::COL_O + c, ov);
-        const int h0 = c & (N - 1);
-        float inv[16];
+        for (int c = 0; c < 2 * N; c += 16) {
+          uint32_t ov[16];
+          tmem_ld16(t_row + C::COL_O + (rank ^ 1) * 2 * N + c, ov);
+          tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          const float4 f = *reinterpret_cast<const float4*>(inv_s + h0 + i);
-          inv[i] = f.x; inv[i + 1] = f.y; inv[i + 2] = f.z; inv[i + 3] = f.w;
+          for (int i = 0; i < 16; ++i) give[(c + i) * 128] = __uint_as_float(ov[i]);
         }
-        tmem_wait_ld();
-        // two neighbouring dims to a word: the even lane takes the pair of the even head, the odd lane that of the odd one
-        __nv_bfloat16* o = out + (int64_t)h0 * kFewDv + (c / N) * 128 + warp * 32 + (lane & ~1);
+      } else if (!halves) {
+#pragma unroll 1
+        for (int c = 0; c < 4 * N; c += 16) {          // 16 heads of this lane's dim of a 128-dim tile
+          uint32_t ov[16];
+          tmem_ld16(t_row + C::COL_O + c, ov);
+          float w[16], x[16];
+          few_ld_weights(wgt + (c & (N - 1)), w);
+          tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const float x0 = __uint_as_float(ov[i]) * inv[i], x1 = __uint_as_float(ov[i + 1]) * inv[i + 1];
-          const float y = __shfl_xor_sync(0xffffffffu, even ? x1 : x0, 1);
-          const int h = i + (lane & 1);
-          if (h0 + h < a.H) *reinterpret_cast<uint32_t*>(o + h * kFewDv) = even ? few_pack(x0, y) : few_pack(y, x1);
+          for (int i = 0; i < 16; ++i) x[i] = __fmul_rn(__uint_as_float(ov[i]), w[i]);
+          few_store(out, a.H, c & (N - 1), (c / N) * 128 + warp * 32, lane, x);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < 4 * N; c += 16) {
+          uint32_t ov[16], ow[16];
+          tmem_ld16(t_row + C::COL_O + c, ov);
+          tmem_ld16(t_row + C::COL_O + 4 * N + c, ow);
+          float w[16], x[16];
+          few_ld_weights(wgt + (c & (N - 1)), w);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __fmul_rn(__uint_as_float(ov[i]), w[i]);
+          few_ld_weights(wgt + N + (c & (N - 1)), w);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __fmaf_rn(__uint_as_float(ow[i]), w[i], x[i]);
+          few_store(out, a.H, c & (N - 1), (c / N) * 128 + warp * 32, lane, x);
         }
       }
       tc_fence_before();
@@ -485,6 +609,44 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
   }
 
   __syncwarp();
+  if constexpr (PAIR) {
+    few_cluster_sync();                                // both halves are complete, and what they give one another is written
+    const int nb = tok_s[0];
+    if (warp < kFewSoftmaxWarps && nb > kFewWhole && !aborted_warp(abort_flag)) {
+      const uint32_t t_o = tmem + (uint32_t(warp * 32) << 16) + C::COL_O + rank * 2 * N;
+      float* wgt = wgt_s + warp * 2 * N;
+      if (lane < N) {
+        const uint32_t peer = mapa_peer(smem_u32(half_s + lane), rank ^ 1);
+        const float l = half_s[lane], m = half_s[N + lane], lp = few_ld_peer(peer), mp = few_ld_peer(peer + 4 * N);
+        float w0, w1;
+        few_weights(rank ? lp : l, rank ? mp : m, rank ? l : lp, rank ? m : mp, w0, w1);
+        wgt[lane] = w0;
+        wgt[N + lane] = w1;
+      }
+      __syncwarp();
+      const uint32_t taken = mapa_peer(smem_u32(reinterpret_cast<float*>(pair_s) + warp * 32 + lane), rank ^ 1);
+#pragma unroll 1
+      for (int c = 0; c < 2 * N; c += 16) {
+        uint32_t ov[16];
+        float x[16];
+        tmem_ld16(t_o + c, ov);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = few_ld_peer(taken + (c + i) * 512);
+        float w0[16], w1[16];
+        few_ld_weights(wgt + (c & (N - 1)), w0);
+        few_ld_weights(wgt + N + (c & (N - 1)), w1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float mine = __uint_as_float(ov[i]);
+          x[i] = __fmaf_rn(rank ? mine : x[i], w1[i], __fmul_rn(rank ? x[i] : mine, w0[i]));
+        }
+        few_store(a.out + (int64_t)u0 * a.H * kFewDv, a.H, c & (N - 1), (2 * rank + c / N) * 128 + warp * 32, lane, x);
+      }
+    }
+    __syncwarp();
+    few_cluster_sync();                                // the peer has read what this CTA gave it
+  }
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {                                   // a wait gave up: let the copies in flight land (bounded)
@@ -501,19 +663,37 @@ sparse_mla_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const FewArgs 
 int make_tmap_2d_bytes(CUtensorMap* m, const void* base, uint64_t rows, uint64_t inner_bytes, uint64_t row_pitch,
                        uint32_t box_bytes, uint32_t box_rows);
 
-template <int N>
-static int launch_few(const void* q, const FewArgs& args, cudaStream_t stream) {
+template <int N, bool PAIR>
+static int launch_few(const void* q, const FewArgs& a, cudaStream_t stream) {
   using C = FewCfg<N>;
-  FewArgs a = args;
+  if (a.H > N) return set_error(DSA_ERR_SHAPE, "sparse_mla: %d heads in a kernel for %d", a.H, N);
   CUtensorMap tq;
   const int rc = make_tmap_2d_bytes(&tq, q, (uint64_t)a.T * a.H, kFewRowBytes, kFewRowBytes, 128, N);
   if (rc) return rc;
-  if (a.H > N) return set_error(DSA_ERR_SHAPE, "sparse_mla: %d heads in a kernel for %d", a.H, N);
-  auto kern = sparse_mla_few_kernel<N>;
+  auto kern = sparse_mla_few_kernel<N, PAIR>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
     return set_error(DSA_ERR_CUDA, "sparse_mla: cannot raise dynamic shared memory to %d", C::SMEM);
-  kern<<<a.T < sm_count() ? a.T : sm_count(), kFewThreads, C::SMEM, stream>>>(tq, a, a.T);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(PAIR ? 2 * a.T : min(a.T, sm_count()));
+  cfg.blockDim = dim3(kFewThreads);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, tq, a, a.T);          // its error is the launch check's
   return check_launch("sparse_mla");
+}
+
+// Two CTAs to a token where that takes one round of them and lists may have two halves (2048 keys, 16 heads: 74 tokens 27.0
+// us, 148 by one CTA each 44.1; two rounds of clusters would take longer).  The bits of a row do not
+// depend on it: both forms keep the halves apart and merge them by the same operations.
+template <int N>
+static int launch_few(const void* q, const FewArgs& a, cudaStream_t stream) {
+  return a.K > kFewWhole * kFewBlk && a.T <= sm_count() / 2 ? launch_few<N, true>(q, a, stream) : launch_few<N, false>(q, a, stream);
 }
 
 int sparse_mla_few_launch(const void* q, const void* kv, const int32_t* idx, void* out, int T, int H, int S_kv, int K,

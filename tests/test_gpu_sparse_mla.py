@@ -443,3 +443,35 @@ def test_decode_scores_that_outgrow_the_reference_many_times(form, H):
     out = ops.sparse_mla_decode_paged(q.cuda(), cache.cuda(), table.cuda(), idx.cuda(), scale, workspace=ws)
     ops.check_status("cuda")
     check(out, O.sparse_mla_decode_paged(q.float(), cache, table, idx, scale, round_bf16=True))
+
+
+@pytest.mark.parametrize("H", [1, 16, 17, 32])
+@pytest.mark.parametrize("K", [129, 256, 257, 320, 700, 2048])
+def test_rows_of_few_heads_have_the_same_bits_in_calls_of_any_size(H, K):
+    """Up to one row for every two SMs a row's list is dealt to two CTAs, beyond that one CTA walks both halves: the same bits
+    (a row may be computed by another rank, or in another chunk), over lists that end anywhere, holes and empty rows."""
+    T, P = 160, 40
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    g = torch.Generator(device="cuda").manual_seed(H + K)
+    kv = torch.randn(P * 64, 576, device="cuda", generator=g).to(torch.bfloat16)
+    q = torch.randn(T, H, 576, device="cuda", generator=g).to(torch.bfloat16)
+    idx = _holes(torch.rand(T, P * 64, device="cuda", generator=g).topk(K, dim=-1).indices.int(), g)
+    for t, n in enumerate((0, 1, 64, 65, 128, 129, 192, 193, 256, 257, 321, 1024, 1025)):
+        idx[2 * t, min(n, K):] = -1
+    run = lambda a, b: ops.sparse_mla_prefill(q[a:b], kv, idx[a:b], 0.06)
+    out = run(0, T)
+    for a, n in ((0, 1), (0, pairs), (T - pairs, pairs), (5, pairs - 1), (3, pairs + 1)):
+        for _ in range(3):
+            assert torch.equal(run(a, a + n), out[a:a + n]), (a, n)
+    ops.check_status("cuda")
+    check(out, O.sparse_mla(q.float().cpu(), kv.float().cpu(), idx.cpu(), 0.06))
+
+
+@pytest.mark.parametrize("H", [16, 32])
+def test_halves_of_a_list_are_weighted_by_their_own_references(H):
+    """Scores that climb by hundreds of log2 units along the list, fall, or stay: one CTA to a row and two, the same bits."""
+    q, kv, idx, scale = (x.cuda() if torch.is_tensor(x) else x for x in _climbing(100, H, 1100, seed=H))
+    out = ops.sparse_mla_prefill(q, kv, idx, scale)
+    assert torch.equal(ops.sparse_mla_prefill(q[:40], kv, idx[:40], scale), out[:40])
+    ops.check_status("cuda")
+    check(out, O.sparse_mla(q.float().cpu(), kv.float().cpu(), idx.cpu(), scale))

@@ -7,8 +7,10 @@
 //     what lies above it leaves in column order, the bin's own few elements are ranked against one another.
 //   * sampled (longer rows): a sample of the row (one 128-float block in every 16, more of a row below 32768 columns) is ranked by the
 //     same kind of histogram, a threshold a few standard deviations below the sample's estimate of the k-th value is taken
-//     from it, and one ordered pass stages every element at or above it (at most 4096) and counts it by bins as it does; the
-//     select then reads the candidates once.
+//     from it, one ordered pass stages the columns of every element at or above it (at most 4096), a flat one counts those by
+//     bins, and the select reads the candidates once.  Values far from the others, which would leave a histogram of equal bins
+//     blind, cost a second look at the sample and no more: the rank's bin is cut into bins in turn, and the candidates are binned
+//     by their keys.
 //   * two passes, for what the others give up (a staged count that misses [k, 4096], infinities or NaN in the range, more than 256
 //     elements in the threshold bin, long unaligned rows): the k-th key digit by digit (12 + 12 + 8 bits):
 //       1. histogram the top 12 key bits of the row (shared-memory atomics), suffix-
@@ -24,8 +26,11 @@
 // Compaction uses block prefix sums, never atomics, and no order depends on the number of threads, so a row's output is
 // the same from run to run and whatever the number of rows of the call.
 // What bounds it: latency, of the barriers between a row's steps.  us, against the form before (digit passes behind the sample, two
-// passes below 16384 columns), k = 2048: 7 rows of up to 33000 columns 13.5 -> 8.7, 64 x 131072 21.2 -> 13.3, 160 x 9000 15.0 -> 10.4, 2048 x 16384
+// passes below 16384 columns), k = 2048: 7 rows of up to 33000 columns 13.5 -> 8.7, 64 x 131072 21.2 -> 12.3, 160 x 9000 15.0 -> 10.4, 2048 x 16384
 // causal 104 -> 71, 4096 x 32768 213 -> 172, 4096 x 131072 453 -> 400, 3000 x 3000 30 -> 19; 2048 x 2048, k = 256 42 -> 21.
+// With 64 values of a row at 300 sigma (before; equal bins alone, which give up and pay for two passes as well; now): 64 x 131072 23.2, 56.2,
+// 16.5, 7 x 33000 15.8, 22.7, 10.4, 1024 x 32768 68, 126, 53, 160 x 9000 15.7, 21.8, 13.9; rows in registers, 1024 x 3000 27.8, 49.9, 32.3, 1024 x
+// 8000 35.5, 44.4, 45.6.
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -43,6 +48,7 @@ constexpr int kCandS = 4096;                           // candidates that the sa
 constexpr int kDirectChunk = 4096;
 constexpr int kDirectRow = 2 * kDirectChunk - 4;       // longest row without sample and staging (it may start three columns into a float4)
 constexpr int kTieCap = 256;                           // elements of the threshold bin that are ranked by counting
+constexpr int kMaxLevels = 3;                          // a crowded bin of the sample is cut into bins at most that often
 constexpr int kSampleBlock = 128;                      // floats per sampled block (one float4 per lane)
 constexpr int kSampleMaxBlocks = 64;                   // at most 8192 sampled values
 constexpr int kSampleWant = 16;                        // blocks wanted where a block in 16 gives fewer
@@ -64,6 +70,8 @@ __device__ __forceinline__ float key_value(uint32_t key) {
 // must not come here.
 struct LinBins {
   float hi, scale;
+  uint32_t base = 0;                                    // not 0: the elements' coordinate is how far their key lies above this one
+  __device__ __forceinline__ int of_key(uint32_t key) const { return of(base ? __uint2float_rz(key - base) : key_value(key)); }
   __device__ __forceinline__ bool set(float top, float bottom) {       // false: no usable range (all equal, infinite, NaN)
     hi = top;
     scale = static_cast<float>(kLinBins) / (top - bottom);
@@ -250,18 +258,13 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* x, int wbase, int l
   return fc;
 }
 
-__device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* x, int wbase, int lane, uint32_t fc,
-                                           uint32_t pc, const LinBins& bins) {
-  while (fc) {                               // few bits set: reload the hits (L1) rather than keep 32 values
+__device__ __forceinline__ void stage_hits(TopkSmem& sm, int wbase, int lane, uint32_t fc, uint32_t pc) {
+  while (fc) {                               // few bits set
     const int j = __ffs(fc) - 1;
     fc &= fc - 1;
-    const int col = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
-    const float v = x[col];
-    sm.cand_key[pc] = order_key(v);
-    sm.cand_idx[pc] = col;
-    atomicAdd(&sm.lin[bins.of(v)], 1u);
-    ++pc;
+    sm.cand_idx[pc++] = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
   }
+  __syncwarp();
 }
 
 // The ordered pass of the sampled path: stages every element with key >= thr, two chunks per block scan, and counts them by
@@ -284,12 +287,39 @@ __device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* x, int 
     const uint32_t excl = block_exclusive_scan<TH>(sm, __popc(f0) | (__popc(f1) << 16), c & 1, total);
     const uint32_t t0 = total & 0xffffu, t1 = total >> 16;
     if (staged + t0 + t1 > (uint32_t)kCandS) return 0xffffffffu;   // every thread sees the same totals
-    stage_hits(sm, x, wb0, lane, f0, staged + (excl & 0xffffu), bins);
-    stage_hits(sm, x, wb1, lane, f1, staged + t0 + (excl >> 16), bins);
+    stage_hits(sm, wb0, lane, f0, staged + (excl & 0xffffu));
+    stage_hits(sm, wb1, lane, f1, staged + t0 + (excl >> 16));
     staged += t0 + t1;
   }
   __syncthreads();
+  // their values are read again (from the L1 or L2) by all threads alike
+#pragma unroll
+  for (int a = tid; a < kCandS; a += TH) {
+    if (a < (int)staged) {
+      const uint32_t key = order_key(x[sm.cand_idx[a]]);
+      sm.cand_key[a] = key;
+      atomicAdd(&sm.lin[bins.of_key(key)], 1u);
+    }
+  }
+  __syncthreads();
   return staged;
+}
+
+// Block-wide largest and smallest key (threads without one give 0 and 0xffffffff); clears sm.lin on the way, which is clear and may
+// be counted into when this returns.
+template <int TH>
+__device__ __forceinline__ void key_range(TopkSmem& sm, uint32_t& kmax, uint32_t& kmin) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  if (lane == 0) {
+    sm.warp_tot[0][warp] = kmax;
+    sm.warp_tot[1][warp] = kmin;
+  }
+  zero_bins<TH, kLinBins>(sm.lin);
+  __syncthreads();
+  kmax = __reduce_max_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[0][lane] : 0u);
+  kmin = __reduce_min_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[1][lane] : 0xffffffffu);
 }
 
 // The k largest of a set of elements that sm.lin counts by `bins` (complete, a barrier behind it), in CHUNKS chunks: each(c, ck,
@@ -313,7 +343,7 @@ __device__ __forceinline__ bool select_by_bins(TopkSmem& sm, const LinBins& bins
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
       if ((valid >> j) & 1u) {
-        const int bj = bins.of(key_value(ck[j]));
+        const int bj = bins.of_key(ck[j]);
         fgt |= (uint32_t)(bj < b) << j;
         feq |= (uint32_t)(bj == b) << j;
       }
@@ -337,9 +367,15 @@ __device__ __forceinline__ bool select_by_bins(TopkSmem& sm, const LinBins& bins
     const uint32_t key = sm.tie.key[threadIdx.x];
     const int32_t c = sm.tie.col[threadIdx.x];
     uint32_t rank = 0;
-    for (uint32_t i = 0; i < cnt; ++i) {
-      const uint32_t ki = sm.tie.key[i];
-      rank += ki > key || (ki == key && sm.tie.col[i] < c);
+    // Four at a time: one by one, a bin of 200 elements took 14 us, longer than all the rest of a row of 3000 columns.
+#pragma unroll 2
+    for (uint32_t i = 0; i < cnt; i += 4) {
+      const uint4 ki = *reinterpret_cast<const uint4*>(&sm.tie.key[i]);
+      const int4 ci = *reinterpret_cast<const int4*>(&sm.tie.col[i]);
+      rank += ki.x > key || (ki.x == key && ci.x < c);
+      rank += i + 1 < cnt && (ki.y > key || (ki.y == key && ci.y < c));
+      rank += i + 2 < cnt && (ki.z > key || (ki.z == key && ci.z < c));
+      rank += i + 3 < cnt && (ki.w > key || (ki.w == key && ci.w < c));
     }
     if (rank < need) o[n_above + rank] = c;
   }
@@ -387,27 +423,62 @@ __device__ __forceinline__ bool sample_threshold(TopkSmem& sm, const float* x, i
       }
     }
   }
-  kmax = __reduce_max_sync(0xffffffffu, kmax);
-  kmin = __reduce_min_sync(0xffffffffu, kmin);
-  if (lane == 0) {
-    sm.warp_tot[0][warp] = kmax;
-    sm.warp_tot[1][warp] = kmin;
-  }
-  zero_bins<TH, kLinBins>(sm.lin);
-  __syncthreads();
-  kmax = __reduce_max_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[0][lane] : 0u);
-  kmin = __reduce_min_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[1][lane] : 0xffffffffu);
-  const float top = key_value(kmax), bottom = key_value(kmin);
+  key_range<TH>(sm, kmax, kmin);
+  const float top = key_value(kmax);
   LinBins bins;
-  if (!bins.set(top, bottom)) return false;               // a NaN makes it false too, whatever its sign
+  if (!bins.set(top, key_value(kmin))) return false;      // a NaN makes it false too, whatever its sign
 #pragma unroll
   for (int j = 0; j < NPT; ++j)
     if ((svalid >> j) & 1u) atomicAdd(&sm.lin[bins.of(key_value(skey[j]))], 1u);
   __syncthreads();
   find_threshold_bin<TH, kLinBins, true>(sm, sm.lin, (uint32_t)rf);
-  const float thr = top - (float)(sm.bin + 1) * ((top - bottom) * (1.f / kLinBins));     // the bin's lower edge, give or take a rounding
+  // the bin's lower edge, give or take a rounding
+  float thr = top - (float)(sm.bin + 1) * ((top - key_value(kmin)) * (1.f / kLinBins));
+  const uint32_t enough = max(4, (int)rf / 16);
+  if (sm.cnt > enough) {
+    // Too many in the bin to tell the rank by: a few values far from the others have stretched the range.  The bin's own range
+    // is cut into bins in turn (the sample is read again, so that other rows do not keep it in registers).
+#pragma unroll 1
+    for (int level = 0; level < kMaxLevels && sm.cnt > enough; ++level) {
+      const int b = sm.bin;
+      const uint32_t need = sm.need, hi_key = kmax, lo_key = kmin;
+      kmax = 0;
+      kmin = 0xffffffffu;
+#pragma unroll 1
+      for (int i = tid; i < m; i += TH) {
+        const uint32_t key = order_key(x[first + (i / kSampleBlock * sb + sb / 2) * kSampleBlock + i % kSampleBlock]);
+        if (key >= lo_key && key <= hi_key && bins.of(key_value(key)) == b) {
+          kmax = max(kmax, key);
+          kmin = min(kmin, key);
+        }
+      }
+      __syncwarp();
+      key_range<TH>(sm, kmax, kmin);
+      if (!bins.set(key_value(kmax), key_value(kmin))) {  // all equal, or as good as
+        thr = key_value(kmin);
+        __syncthreads();
+        break;
+      }
+#pragma unroll 1
+      for (int i = tid; i < m; i += TH) {
+        const uint32_t key = order_key(x[first + (i / kSampleBlock * sb + sb / 2) * kSampleBlock + i % kSampleBlock]);
+        if (key >= kmin && key <= kmax) atomicAdd(&sm.lin[bins.of(key_value(key))], 1u);
+      }
+      __syncthreads();
+      find_threshold_bin<TH, kLinBins, true>(sm, sm.lin, need);
+      thr = key_value(kmax) - (float)(sm.bin + 1) * ((key_value(kmax) - key_value(kmin)) * (1.f / kLinBins));
+    }
+    // as many equal values as that cannot be staged
+    if ((float)((int)rf - (int)sm.need + (int)sm.cnt) > (float)kCandS * frac) return false;
+  }
   zero_bins<TH, kLinBins>(sm.lin);                        // for the candidates (all have read the counts)
   thr_out = thr;
+  // candidates of one sign are binned by their keys, near enough by their logarithms: no value stretches that range
+  const uint32_t base = order_key(thr);
+  if (thr > 0.f || top < 0.f) {
+    bins_out.base = base;
+    return bins_out.set(__uint2float_rz(order_key(top) - base), 0.f);
+  }
   return bins_out.set(top, thr);
 }
 
@@ -456,7 +527,7 @@ template <int TH, int CHUNKS>
 __device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* x, bool vec, int lo, int hi, int k,
                                            int32_t* __restrict__ o) {
   constexpr int NPT = kDirectChunk / TH;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   const int i0 = (lo & ~(kVec - 1)) + tid * NPT;
   auto used = [&](int c, int j) { return i0 + c * kDirectChunk + j >= lo && i0 + c * kDirectChunk + j < hi; };
   uint32_t key[CHUNKS][NPT], kmax = 0, kmin = 0xffffffffu;
@@ -488,16 +559,7 @@ __device__ __forceinline__ bool direct_row(TopkSmem& sm, const float* x, bool ve
         kmax = max(kmax, key[c][j]);
         kmin = min(kmin, key[c][j]);
       }
-  kmax = __reduce_max_sync(0xffffffffu, kmax);
-  kmin = __reduce_min_sync(0xffffffffu, kmin);
-  if (lane == 0) {
-    sm.warp_tot[0][warp] = kmax;
-    sm.warp_tot[1][warp] = kmin;
-  }
-  zero_bins<TH, kLinBins>(sm.lin);
-  __syncthreads();
-  kmax = __reduce_max_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[0][lane] : 0u);
-  kmin = __reduce_min_sync(0xffffffffu, lane < TH / 32 ? sm.warp_tot[1][lane] : 0xffffffffu);
+  key_range<TH>(sm, kmax, kmin);
   LinBins bins;
   if (!bins.set(key_value(kmax), key_value(kmin))) return false;       // a NaN makes it false too, whatever its sign
 #pragma unroll

@@ -223,3 +223,49 @@ def test_nan_and_infinities_keep_the_order_of_the_bits(n):
         for t in range(6):
             want = sorted(range(n), key=lambda c, kt=key[t].tolist(): (-kt[c], c))[:k]
             assert sorted(got[t].tolist()) == sorted(want), (t, k)
+
+
+def _stretched_rows(n, g):
+    """Rows of which a few values lie so far from the others that equal bins over the whole range say nothing about them."""
+    rows = []
+    for count, sigma in ((4, 100.0), (64, 100.0), (64, 300.0), (64, 1e4), (300, 1e6)):
+        r = torch.randn(n, device=DEV, generator=g)
+        r[torch.randperm(n, device=DEV, generator=g)[:count]] = sigma * (1 + 0.1 * torch.randn(count, device=DEV, generator=g))
+        rows.append(r)
+    rows += [(2.0 * torch.randn(n, device=DEV, generator=g)).exp(), (3.0 * torch.randn(n, device=DEV, generator=g)).exp(),
+             torch.tan(3.14 * (torch.rand(n, device=DEV, generator=g) - 0.5))]
+    return torch.stack(rows)
+
+
+@pytest.mark.parametrize("n,k", [(9000, 2048), (33000, 2048), (131072, 2048), (131072, 256)])
+def test_values_far_from_the_others_keep_long_rows_on_the_sampled_form(n, k):
+    """The bin of the sample's rank is cut into bins in turn, and the candidates are binned by their keys.  Which form a row took
+    shows in the order of its output: the sampled one ends with the threshold bin's elements by value, the two-pass form lists
+    them by column."""
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    x = torch.zeros(8, (n + 3) // 4 * 4, device=DEV)
+    x[:, :n] = _stretched_rows(n, g)
+    x = x[:, :n]
+    a, b = ops.topk_select(x, k), _two_pass(x, k)
+    _sets_equal_with_ties(x, a, k)
+    assert not (a == b).all(dim=1).any(), (a == b).all(dim=1).tolist()
+    many = ops.topk_select(x.repeat(20, 1) if n % 4 == 0 else torch.cat([x] * 20), k)
+    assert torch.equal(many[:8], a) and torch.equal(many[-8:], a)
+
+
+@pytest.mark.parametrize("n", [2048, 3000, 8188, 8192, 33000])
+@pytest.mark.parametrize("share", [0.05, 0.3, 0.6])
+def test_rows_of_zeros_and_a_few_others(n, share):
+    """What a ReLU leaves: the k-th value may be the zero that most columns hold (lower columns first), of either sign."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    k = min(2048, n // 2)
+    x = torch.randn(6, n, device=DEV, generator=g)
+    x = torch.where(torch.rand(6, n, device=DEV, generator=g) < share, x, torch.zeros_like(x))
+    x[1] = x[1].relu()
+    x[2] = torch.where(x[2] == 0, -x[2], x[2])                  # -0.0
+    x[3] *= 1e-38
+    x[4] = x[4].abs() * 1e30
+    a = ops.topk_select(x, k)
+    _sets_equal_with_ties(x, a, k)
+    assert torch.equal(a.sort(1).values, _two_pass(x, k).sort(1).values)
+    assert torch.equal(ops.topk_select(x.repeat(30, 1), k)[-6:], a)

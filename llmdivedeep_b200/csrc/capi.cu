@@ -247,9 +247,11 @@ int dsa_decode_step(const void* q_fp8, const void* w, int w_dtype, const void* k
   int rc = dsa_indexer_logits_paged(q_fp8, w, w_dtype, kcache, kscale, block_table, table_stride, ctx_len, logits, ld_logits, B,
                                     idx_heads, idx_dim, k_pages, max_ctx, status, stream);
   // Small batches leave SMs to the next kernel while one still runs: each is launched so that it may set itself up under the end
-  // of the one before.  us a step in a plain loop: 1 x 2000 37.0 -> 29.5, 2 x 9000 43.1 -> 36.9, 7 x 33000 50.3 -> 45.1, 12 x 30000 57.5 -> 52.3,
-  // 20 x 20000 65.7 -> 61.6; 30 x 9000 70.2 both (in a CUDA graph, whose launches are closer, the same up to 8 and 1 to 3 % more at 16
-  // and 20, 8 % at 30); from 64 up the top-k's blocks take the first SMs that come free, and the rest waits.
+  // of the one before.  us a step in a plain loop over one set of inputs: 1 x 2000 37.0 -> 29.5, 2 x 9000 43.1 -> 36.9, 7 x 33000 50.3 -> 45.1,
+  // 12 x 30000 57.5 -> 52.3, 20 x 20000 65.7 -> 61.6; 30 x 9000 70.2 both.  In a CUDA graph, whose launches are closer, 40 batches of 4 to 24
+  // with contexts of 3000 to 60000 take 1.4 % less on average: 6 % less at 3000 tokens, up to 6 % more at 20000 and from 18 sequences on
+  // (23 x 20000 62.3 -> 66.5), 2 % more with 8 of 9000 and over, the others less.  From 64 up the top-k's blocks take the first SMs that come
+  // free, and the rest waits.
   const int overlapped = B <= 24;
   if (!rc) rc = topk_select_checked(logits, ld_logits, nullptr, ctx_len, B, max_ctx, k, idx, /*sample=*/1, overlapped, stream);
   if (!rc) rc = sparse_mla_decode_checked(q_bf16, latent, block_table, table_stride, idx, out_bf16, B, H, k, latent_pages, max_ctx,

@@ -100,8 +100,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 
 // The same for a whole warp whose lanes all come here: one answer for all of them.  The first look stands before the loop, so
 // that a wait which finds its phase complete costs a poll, a vote and a branch and leaves nothing to test behind it; with the
-// loop alone (which the compiler unrolls by four at every place) the indexer takes 2379 us for 4096 x 65536 instead of 2204, the
-// sparse MLA of 16 heads 1239 instead of 1183 (4096 x 2048 keys), block-sparse attention 247 instead of 244.
+// loop alone (which the compiler unrolls by four at every place) the indexer took 2379 us for 4096 x 65536 instead of 2204,
+// block-sparse attention 247 instead of 244.
 template <int UNROLL = 1>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;

@@ -7,8 +7,8 @@
 //     what lies above it leaves in column order, the bin's own few elements are ranked against one another.
 //   * sampled (longer rows): a sample of the row (one 128-float block in every 16, more of a row below 32768 columns) is ranked by the
 //     same kind of histogram, a threshold a few standard deviations below the sample's estimate of the k-th value is taken
-//     from it, one ordered pass stages the columns of every element at or above it (at most 4096), a flat one counts those by
-//     bins, and the select reads the candidates once.  Values far from the others, which would leave a histogram of equal bins
+//     from it, one ordered pass stages every element at or above it (at most 4096) and counts it by bins as it does, and the
+//     select reads the candidates once.  Values far from the others, which would leave a histogram of equal bins
 //     blind, cost a second look at the sample and no more: the rank's bin is cut into bins in turn, and the candidates are binned
 //     by their keys.
 //   * two passes, for what the others give up (a staged count that misses [k, 4096], infinities or NaN in the range, more than 256
@@ -27,10 +27,10 @@
 // the same from run to run and whatever the number of rows of the call.
 // What bounds it: latency, of the barriers between a row's steps.  us, against the form before (digit passes behind the sample, two
 // passes below 16384 columns), k = 2048: 7 rows of up to 33000 columns 13.5 -> 8.7, 64 x 131072 21.2 -> 12.3, 160 x 9000 15.0 -> 10.4, 2048 x 16384
-// causal 104 -> 71, 4096 x 32768 213 -> 172, 4096 x 131072 453 -> 400, 3000 x 3000 30 -> 19; 2048 x 2048, k = 256 42 -> 21.
+// causal 104 -> 71, 4096 x 32768 213 -> 166, 4096 x 131072 453 -> 383, 3000 x 3000 30 -> 19; 2048 x 2048, k = 256 42 -> 21.
 // With 64 values of a row at 300 sigma (before; equal bins alone, which give up and pay for two passes as well; now): 64 x 131072 23.2, 56.2,
-// 16.5, 7 x 33000 15.8, 22.7, 10.4, 1024 x 32768 68, 126, 53, 160 x 9000 15.7, 21.8, 13.9; rows in registers, 1024 x 3000 27.8, 49.9, 32.3, 1024 x
-// 8000 35.5, 44.4, 45.6.
+// 16.2, 7 x 33000 15.8, 22.7, 10.3, 1024 x 32768 68, 126, 53, 160 x 9000 15.7, 21.8, 14.0; rows in registers, 1024 x 3000 27.8, 49.9, 32.1, 1024 x
+// 8000 35.5, 44.4, 45.6.  Rows in registers have no second look: bins of the bin, from the registers, made ordinary rows 10 % slower.
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -258,11 +258,24 @@ __device__ __forceinline__ uint32_t chunk_flags(const float* x, int wbase, int l
   return fc;
 }
 
-__device__ __forceinline__ void stage_hits(TopkSmem& sm, int wbase, int lane, uint32_t fc, uint32_t pc) {
+// Stages a lane's hits of a chunk: their columns first, then their values, by the lanes of the warp alike and while the L1 still has
+// them.  (All values at the end of the row, by all threads: 4096 x 131072 478 us instead of 383, the rows in flight do not fit the L2.  A
+// lane's own values in its own loop: 406, and 64 x 131072 13.1 instead of 12.4, or 17.7 where the compiler lets the lanes drift apart.)
+__device__ __forceinline__ void stage_hits(TopkSmem& sm, const float* x, int wbase, int lane, uint32_t fc, uint32_t pc,
+                                           const LinBins& bins) {
+  const uint32_t begin = __shfl_sync(0xffffffffu, pc, 0);
   while (fc) {                               // few bits set
     const int j = __ffs(fc) - 1;
     fc &= fc - 1;
     sm.cand_idx[pc++] = wbase + (j >> 2) * 128 + lane * kVec + (j & 3);
+  }
+  const uint32_t end = __shfl_sync(0xffffffffu, pc, 31);
+  __syncwarp();
+  // the warp's hits, dealt to its lanes: read again (from the L1) rather than kept
+  for (uint32_t a = begin + lane; a < end; a += 32) {
+    const uint32_t key = order_key(x[sm.cand_idx[a]]);
+    sm.cand_key[a] = key;
+    atomicAdd(&sm.lin[bins.of_key(key)], 1u);
   }
   __syncwarp();
 }
@@ -287,19 +300,9 @@ __device__ __forceinline__ uint32_t stage_row(TopkSmem& sm, const float* x, int 
     const uint32_t excl = block_exclusive_scan<TH>(sm, __popc(f0) | (__popc(f1) << 16), c & 1, total);
     const uint32_t t0 = total & 0xffffu, t1 = total >> 16;
     if (staged + t0 + t1 > (uint32_t)kCandS) return 0xffffffffu;   // every thread sees the same totals
-    stage_hits(sm, wb0, lane, f0, staged + (excl & 0xffffu));
-    stage_hits(sm, wb1, lane, f1, staged + t0 + (excl >> 16));
+    stage_hits(sm, x, wb0, lane, f0, staged + (excl & 0xffffu), bins);
+    stage_hits(sm, x, wb1, lane, f1, staged + t0 + (excl >> 16), bins);
     staged += t0 + t1;
-  }
-  __syncthreads();
-  // their values are read again (from the L1 or L2) by all threads alike
-#pragma unroll
-  for (int a = tid; a < kCandS; a += TH) {
-    if (a < (int)staged) {
-      const uint32_t key = order_key(x[sm.cand_idx[a]]);
-      sm.cand_key[a] = key;
-      atomicAdd(&sm.lin[bins.of_key(key)], 1u);
-    }
   }
   __syncthreads();
   return staged;

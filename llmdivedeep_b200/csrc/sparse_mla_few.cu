@@ -18,9 +18,9 @@
 //     number of blocks) and for positions out of range, and sends for Q.
 //   * warps 6-21: gather, four rows of a block each, by cp.async that arrive on the block's barrier by themselves.  The latent
 //     rows lie in a ring of panel pairs (128 dims of 64 keys), freed one by one as P.V has read them, the rope panels in another.
-// What bounds it: the tensor pipe, whose 52 MMAs a block cost 47 cycles each whatever their N (2450 cycles; the gather alone would
-// take 1900); in calls of few tokens the chain of one list.  us, keys of 16384: the kernel for many heads, this one with a list in
-// one piece (and read 16 slots a lane at a time for its end), as it is now.
+// What bounds it: the issue of 52 MMAs a block, 47 cycles each whatever their N (2450 cycles; the tensor pipe itself is 13 % busy
+// with 16 heads, 22 % with 32; the gather alone would take 1900); in calls of few tokens the chain of one list.  us, keys of 16384:
+// the kernel for many heads, this one with a list in one piece (and read 16 slots a lane at a time for its end), as it is now.
 //   16 heads, 2048 keys: 1 token 33.9, 52.2, 25.5; 74 tokens 36.4, 53.1, 27.0; 148 tokens 71.5, 54.0, 44.1; 2048 tokens 1090, 566, 548
 //             256 keys:  1 token 9.9, 10.9, 9.5;   74 tokens 11.0, 11.3, 9.9;  2048 tokens 272, 91, 86
 //   32 heads, 2048 keys: 1 token 34.1, 61.7, 29.8; 74 tokens 36.6, 62.5, 31.6; 148 tokens 71.6, 63.5, 53.2; 2048 tokens 1090, 701, 680
